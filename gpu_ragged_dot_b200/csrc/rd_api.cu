@@ -14,6 +14,7 @@
 #include "rd_dispatch.cuh"
 #include "rd_gemm2.cuh"
 #include "rd_gemm_f32.cuh"
+#include "rd_gemm_f32_pair.cuh"
 #include "rd_gemm_perm.cuh"
 #include "rd_metadata.cuh"
 #include "rd_rows.cuh"
@@ -80,26 +81,34 @@ int encode_map(CUtensorMap* map, const void* base, int dtype, int rank, const ui
   return RD_OK;
 }
 
-// "Column-blocked" view of a dense row-major 16-bit [rows, cols] tensor, cols a multiple of 64:
-// (64 columns, rows, cols / 64 blocks).  A box of (64, box_rows, box_blocks) lands in shared memory
-// as box_blocks slabs of [box_rows][128 B], block after block -- what box_blocks separate 2-D boxes
-// of 64 columns would write -- in ONE TMA instruction.
+// "Column-blocked" view of a dense row-major [rows, cols] tensor, cols a multiple of c = 64 (16-bit) or
+// 32 (float32, in the 32-byte-atom swizzle): (c columns, rows, cols / c blocks).  A box of (c,
+// box_rows, box_blocks) lands in shared memory as box_blocks slabs of [box_rows][128 B], block after
+// block -- what box_blocks separate 2-D boxes of c columns would write -- in ONE TMA instruction.
+// `mats` > 0 adds a fourth dimension: that many such tensors one after the other.
 int encode_blocked_map(CUtensorMap* map, const void* base, int dtype, int cols, int rows, int box_rows,
-                       int box_blocks) {
+                       int box_blocks, int mats = 0) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return RD_ERR_DRIVER;
-  cuuint64_t gdims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
-  cuuint64_t gstrides[2] = {static_cast<cuuint64_t>(cols) * 2, 128};
-  cuuint32_t gbox[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_blocks)};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapDataType dt =
-      dtype == RD_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUresult r = fn(map, dt, 3, const_cast<void*>(base), gdims, gstrides, gbox, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  const bool f32 = dtype == RD_DTYPE_F32;
+  const int c = f32 ? 32 : 64;
+  const cuuint64_t row_bytes = static_cast<cuuint64_t>(cols) * (f32 ? 4 : 2);
+  cuuint64_t gdims[4] = {static_cast<cuuint64_t>(c), static_cast<cuuint64_t>(rows),
+                         static_cast<cuuint64_t>(cols / c), static_cast<cuuint64_t>(mats)};
+  cuuint64_t gstrides[3] = {row_bytes, 128, row_bytes * static_cast<cuuint64_t>(rows)};
+  cuuint32_t gbox[4] = {static_cast<cuuint32_t>(c), static_cast<cuuint32_t>(box_rows),
+                        static_cast<cuuint32_t>(box_blocks), 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUtensorMapDataType dt = dtype == RD_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                 : f32                  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                                        : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUresult r = fn(map, dt, mats > 0 ? 4 : 3, const_cast<void*>(base), gdims, gstrides, gbox, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  f32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "ragged_dot_b200: cuTensorMapEncodeTiled failed (CUresult %d): blocked map base=%p "
-            "rows=%d cols=%d box=(64,%d,%d)\n", static_cast<int>(r), base, rows, cols, box_rows, box_blocks);
+            "rows=%d cols=%d box=(%d,%d,%d)\n", static_cast<int>(r), base, rows, cols, c, box_rows, box_blocks);
     return RD_ERR_TENSOR_MAP;
   }
   return RD_OK;
@@ -275,16 +284,15 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
   return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
 }
 
-// tgmm with 512 x 256 tiles on CTA pairs (rd_gemm2.cuh, kPair).
-int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
-                      const GemmArgs& args, int ctas, cudaStream_t stream) {
-  auto kernel = rd::ragged_gemm2_kernel<false, true, false, true>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kG2PairSmemBytes) !=
-      cudaSuccess)
+// Launch of a persistent kernel on clusters of two CTAs.
+template <typename Kernel>
+int launch_pairs(Kernel kernel, int threads, int smem_bytes, const CUtensorMap& ta, const CUtensorMap& tb,
+                 const CUtensorMap& tout, const GemmArgs& args, int ctas, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
     return RD_ERR_LAUNCH;
   cudaLaunchConfig_t lc = {};
-  lc.blockDim = dim3(rd::kG2Threads, 1, 1);
-  lc.dynamicSmemBytes = rd::kG2PairSmemBytes;
+  lc.blockDim = dim3(threads, 1, 1);
+  lc.dynamicSmemBytes = smem_bytes;
   lc.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -309,6 +317,24 @@ int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtens
   return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
 }
 
+// tgmm with 512 x 256 tiles on CTA pairs (rd_gemm2.cuh, kPair).
+int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
+                      const GemmArgs& args, int ctas, cudaStream_t stream) {
+  return launch_pairs(rd::ragged_gemm2_kernel<false, true, false, true>, rd::kG2Threads, rd::kG2PairSmemBytes, ta,
+                      tb, tout, args, ctas, stream);
+}
+
+// float32 on CTA pairs (rd_gemm_f32_pair.cuh).
+template <bool kBKMajor, bool kTgmm>
+int launch_gemm_f32_pair(bool split, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
+                         const GemmArgs& args, int ctas, cudaStream_t stream) {
+  if (split)
+    return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, true>, rd::f32_pair_threads<true>(),
+                        rd::f32_pair_smem_bytes<true>(), ta, tb, tout, args, ctas, stream);
+  return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, false>, rd::f32_pair_threads<false>(),
+                      rd::f32_pair_smem_bytes<false>(), ta, tb, tout, args, ctas, stream);
+}
+
 // 256-row tiles on one CTA (rd_gemm2.cuh) move a third less data per flop than 128-row tiles.
 // They pay off when a tile's second half usually exists: tgmm with k >= 256, and gmm when the
 // groups are long (mean rows per group >= 512; a half without rows is skipped, so the cost of a
@@ -326,6 +352,19 @@ bool choose_two_half(bool tgmm, long long m, int k, int g, int bn) {
 // (m/g 512 to 2048; k 4096 and 7168; n 1536 to 14336).  Short groups make tgmm output-bound and
 // were not measured: they stay on one CTA.
 bool choose_pair_512(long long m, int k, int g) { return k >= 512 && g > 0 && m / g >= 512; }
+
+// float32 tiles on CTA pairs (rd_gemm_f32_pair.cuh).  A caller who asks for three TF32 passes always
+// gets them: only that kernel splits its operands.  One pass, one CTA against a pair, microseconds:
+//   tgmm   m/g 1024 (k 4096, n 1536, g 8) 212 -> 175;  512 (same, g 64) 985 -> 779;  256 (k 1024, n 2048,
+//          g 32) 126 -> 104;  128 (k 2048, n 4096, g 64) 452 -> 491
+//   gmm    m/g 1024 181 -> 165;  512 759 -> 675;  256 97 -> 91, but 185 -> 222 for unequal groups of
+//          mean 375 with trans_rhs (256-row tiles waste twice the rows of 128-row ones at a group's
+//          end);  128 386 -> 452
+bool choose_f32_pair(bool tgmm, long long m, int k, int g, int bn, const rd_tile_cfg* cfg) {
+  if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return true;
+  if (bn != 256 || g <= 0 || (cfg && (cfg->cta_group == 1 || cfg->tile_m == 128))) return false;
+  return tgmm ? (k >= 256 && m / g >= 256) : m / g >= 512;
+}
 
 // CTA pairs (256 x 256 tiles, B operand split between the two CTAs) pay off where the
 // 256-row granularity wastes nothing: tgmm, whose tile rows are the dense k axis.  For gmm the
@@ -454,9 +493,13 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   int tile_m = cfg ? cfg->tile_m : 0;
   if (tile_m != 0 && tile_m != 128 && tile_m != 256) return RD_ERR_BAD_CONFIG;
   if (tile_m == 256 && (bn != 256 || cta_group != 1)) return RD_ERR_BAD_CONFIG;
-  if (f32) {  // the float32 (TF32) kernels exist as single-CTA 128-row tiles only
-    if (cta_group == 2 || tile_m == 256) return RD_ERR_BAD_CONFIG;
-    cta_group = 1;
+  const bool three_pass = cfg && (cfg->flags & RD_CFG_F32_THREE_PASS);
+  if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
+  if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
+    if ((cfg && cfg->cta_group == 2) || tile_m == 256) return RD_ERR_BAD_CONFIG;
+    const bool pair = choose_f32_pair(false, m, k, g, bn, cfg);
+    if (pair) bn = rd::kF32PairBN;
+    cta_group = pair ? 2 : 1;
     tile_m = 128;
   }
   if (tile_m == 0) tile_m = (cta_group == 1 && choose_two_half(false, m, k, g, bn)) ? 256 : 128;
@@ -471,6 +514,7 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
                            cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0);
   if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
 
+  const bool blocked = f32 && cta_group == 2 && !trans_rhs && n % 32 == 0;
   CUtensorMap ta, tb;
   {
     const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
@@ -483,6 +527,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
                               static_cast<uint64_t>(num_weights)};
     const uint32_t box[3] = {static_cast<uint32_t>(row_elems), static_cast<uint32_t>(bn / cta_group), 1};
     rc = encode_map(&tb, A, dtype, 3, dims, box);
+  } else if (blocked) {  // the float32 pair kernel fetches its four boxes of a stage with one load
+    rc = encode_blocked_map(&tb, A, dtype, n, k, row_elems, rd::kF32PairBN / 2 / 32, num_weights);
   } else {  // A[g, k, n]: rows of n, MN-major operand, [stage-depth k][128 B of n] boxes
     const uint64_t dims[3] = {static_cast<uint64_t>(n), static_cast<uint64_t>(k),
                               static_cast<uint64_t>(num_weights)};
@@ -502,6 +548,7 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   args.m = m; args.k = k; args.n = n; args.g = g;
   args.n_tiles = (n + bn - 1) / bn;
   args.k_tiles = 0;
+  args.blocked_maps = blocked ? 1 : 0;
   args.max_m_tiles = w.layout.max_tiles;
   args.ab_format = dtype;
   args.wait_limit_us = wait_limit_us(cfg);
@@ -524,6 +571,9 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (send != nullptr && send->sender_ctas >= ctas) return RD_ERR_BAD_CONFIG;
   if (f32) {
     if (ready.flags != nullptr) return RD_ERR_BAD_DTYPE;  // the float32 kernels do not wait on flags
+    if (cta_group == 2)
+      return trans_rhs ? launch_gemm_f32_pair<true, false>(three_pass, ta, tb, tout, args, ctas, stream)
+                       : launch_gemm_f32_pair<false, false>(three_pass, ta, tb, tout, args, ctas, stream);
     if (trans_rhs) {
       if (bn == 256) return launch_gemm_f32<256, true, false>(ta, tb, tout, args, ctas, stream);
       if (bn == 128) return launch_gemm_f32<128, true, false>(ta, tb, tout, args, ctas, stream);
@@ -790,9 +840,13 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   if (cta_group < 0 || cta_group > 2 || (cta_group == 2 && bn != 256)) return RD_ERR_BAD_CONFIG;
   if (tile_m != 0 && tile_m != 128 && tile_m != 256) return RD_ERR_BAD_CONFIG;
   if (tile_m == 256 && bn != 256) return RD_ERR_BAD_CONFIG;
-  if (f32) {  // the float32 (TF32) kernels exist as single-CTA 128-row tiles only
+  const bool three_pass = cfg && (cfg->flags & RD_CFG_F32_THREE_PASS);
+  if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
+  if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
     if (cta_group == 2 || tile_m == 256 || seg_count > 1) return RD_ERR_BAD_CONFIG;
-    cta_group = 1;
+    const bool pair = choose_f32_pair(true, m, k, g, bn, cfg);
+    if (pair) bn = rd::kF32PairBN;
+    cta_group = pair ? 2 : 1;
     tile_m = 128;
   }
   if (seg_count > 1) {  // strided segments: one CTA per tile
@@ -825,9 +879,16 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
 
   // 256-row tiles fetch each operand of a stage with one box when the 64-column blocks tile the
   // rows exactly (see rd_gemm2.cuh); otherwise one 2-D box per 64 columns.
-  const bool blocked = two_half && !f32 && k % 64 == 0 && n % 64 == 0;
+  // The float32 pair kernel likewise, with blocks of 32 columns.
+  const bool f32_pair = f32 && cta_group == 2;
+  const bool blocked = f32_pair ? (k % 32 == 0 && n % 32 == 0) : (two_half && !f32 && k % 64 == 0 && n % 64 == 0);
   CUtensorMap ta, tb;
-  if (blocked) {
+  if (blocked && f32_pair) {
+    rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kF32TileK, rd::kTileM / 32);
+    if (rc != RD_OK) return rc;
+    rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kF32TileK, rd::kF32PairBN / 2 / 32);
+    if (rc != RD_OK) return rc;
+  } else if (blocked) {
     rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kTileK, rd::kG2TileRows / 64);
     if (rc != RD_OK) return rc;
     rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kTileK, rd::kG2TileN / 64 / cta_group);
@@ -875,6 +936,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   args.out = out;
 
   const int ctas = pick_ctas(cfg);
+  if (f32_pair) return launch_gemm_f32_pair<false, true>(three_pass, ta, tb, tout, args, ctas, stream);
   if (f32) {
     if (bn == 256) return launch_gemm_f32<256, false, true>(ta, tb, tout, args, ctas, stream);
     if (bn == 128) return launch_gemm_f32<128, false, true>(ta, tb, tout, args, ctas, stream);

@@ -830,7 +830,7 @@ def _gmm_cast(x, A, group_sizes, trans_rhs, compute_dtype, precision):
     back in x's type."""
     cd = compute_dtype or x.dtype
     if cd == torch.float32 and precision == "highest":
-        y = _gmm_3xtf32(x.to(cd), A.to(cd), group_sizes, trans_rhs)
+        y = gmm_forward(x.to(cd), A.to(cd), group_sizes, trans_rhs=trans_rhs, cfg=_THREE_PASS)
     else:
         y = gmm_forward(x.to(cd), A.to(cd), group_sizes, trans_rhs=trans_rhs)
     return y.to(x.dtype)
@@ -839,42 +839,16 @@ def _gmm_cast(x, A, group_sizes, trans_rhs, compute_dtype, precision):
 def _tgmm_cast(x, y, group_sizes, compute_dtype, precision):
     cd = compute_dtype or x.dtype
     if cd == torch.float32 and precision == "highest":
-        out = _tgmm_3xtf32(x.to(cd), y.to(cd), group_sizes)
+        out = tgmm_forward(x.to(cd), y.to(cd), group_sizes, cfg=_THREE_PASS)
     else:
         out = tgmm_forward(x.to(cd), y.to(cd), group_sizes)
     return out.to(x.dtype)
 
 
-def _split_tf32(t: torch.Tensor):
-    """t = hi + lo exactly, hi holding the top 10 explicit mantissa bits rounded to nearest (a
-    value the tensor cores read without loss) and lo the remainder."""
-    bits = t.contiguous().view(torch.int32)
-    hi = ((bits + 0x1000) & ~0x1FFF).view(torch.float32)
-    hi = torch.where(torch.isfinite(hi), hi, t)  # rounding up the largest finite values would overflow
-    return hi, t - hi
-
-
-def _gmm_3xtf32(x, A, group_sizes, trans_rhs):
-    """float32 product to nearly fp32 accuracy on the TF32 tensor cores: with x = xh + xl and
-    A = Ah + Al (TF32 head + remainder), x.A ~ xh.Ah + xh.Al + xl.Ah; the dropped xl.Al term is
-    2^-22 relative.  Three passes of the TF32 kernel, summed in fp32, small terms first."""
-    xh, xl = _split_tf32(x)
-    Ah, Al = _split_tf32(A)
-    ws = _workspace(x.shape[0], _as_i32(group_sizes).numel(), x.device)
-    y = gmm_forward(xl, Ah, group_sizes, trans_rhs=trans_rhs, workspace=ws)
-    y += gmm_forward(xh, Al, group_sizes, trans_rhs=trans_rhs, workspace=ws)
-    y += gmm_forward(xh, Ah, group_sizes, trans_rhs=trans_rhs, workspace=ws)
-    return y
-
-
-def _tgmm_3xtf32(x, y, group_sizes):
-    xh, xl = _split_tf32(x)
-    yh, yl = _split_tf32(y)
-    ws = _workspace(x.shape[0], _as_i32(group_sizes).numel(), x.device)
-    out = tgmm_forward(xl, yh, group_sizes, workspace=ws)
-    out += tgmm_forward(xh, yl, group_sizes, workspace=ws)
-    out += tgmm_forward(xh, yh, group_sizes, workspace=ws)
-    return out
+# float32 product to nearly fp32 accuracy on the TF32 tensor cores: with x = xh + xl and A = Ah + Al
+# (TF32 head, rounded to nearest, + remainder), x.A ~ xl.Ah + xh.Al + xh.Ah; the dropped xl.Al term is
+# 2^-22 relative.  The kernel splits the operands itself (rd_gemm_f32_pair.cuh).
+_THREE_PASS = _lib.TileCfg(0, 0, 0, 0, _lib.RD_CFG_F32_THREE_PASS)
 
 
 class _GmmFn(torch.autograd.Function):

@@ -1205,3 +1205,63 @@ def test_ep_count_share_emulated_ranks(world):
     late = torch.zeros(max(world, 4), dtype=torch.int32, device=DEV)
     ops.ep_plan_ring_when_counted(tables[0][0], late, 1, 0, ops.ep_plan_ring(want, 0), status, wait_limit_ms=5)
     assert ops.device_status(status) == _lib.RD_ERR_DEVICE_WAIT
+
+
+# ------------------------------------------------------------------ float32 on CTA pairs
+@pytest.mark.parametrize("precision", [None, "highest"])
+@pytest.mark.parametrize("m,k,n,sizes", [
+    (1, 4, 4, [1]),                                   # one element of every tile axis
+    (300, 36, 260, [300]),                            # k, n just past a 32-block and a tile
+    (1025, 256, 256, [513, 511]),                     # tiles that end one row off, one unowned row
+    (3100, 320, 292, [257, 0, 1, 255, 256, 2300]),    # tails of 1, 31 and 0 rows; 292 = 32 * 9 + 4
+    (3000, 516, 644, [129, 127, 7, 1000, 1700]),
+])
+def test_float32_pair_kernels(precision, m, k, n, sizes):
+    """256 x 256 tiles on CTA pairs, plain and operand-splitting, at the edges of tiles, stages and
+    groups.  "highest" against float64: 22-bit operands and fp32 sums over `depth` terms that may be
+    truncated: about depth / 8 * 2^-24 relative (one addition per 8-deep MMA), 3e-5 bounds depth 2300;
+    one pass: 10-bit operands, 2e-3 as in test_reference_grid_float32."""
+    g = len(sizes)
+    gs = torch.tensor(sizes, dtype=torch.int32)
+    x, A, dout = _inputs(77, m, k, n, g, dtype=torch.float32)
+    total = int(gs.sum())
+    x[total:] = float("nan")  # rows of no group reach nothing
+    dout[total:] = float("nan")
+    want = torch.zeros((m, n), dtype=torch.float64)
+    want_dx = torch.zeros((m, k), dtype=torch.float64)
+    want_dA = torch.zeros((g, k, n), dtype=torch.float64)
+    off = 0
+    for gi, s_ in enumerate(sizes):
+        xs, ds, w = x[off:off + s_].double(), dout[off:off + s_].double(), A[gi].double()
+        want[off:off + s_], want_dx[off:off + s_], want_dA[gi] = xs @ w, ds @ w.T, xs.T @ ds
+        off += s_
+    xd, Ad, gd, dd = _to_dev(x, A, gs, dout)
+    flags = _lib.RD_CFG_F32_THREE_PASS if precision else 0
+    limit = 3e-5 if precision else 2e-3
+    At = A.transpose(1, 2).contiguous().to(DEV)
+    got = {
+        "gmm": (ops.gmm_forward(xd, Ad, gd, cfg=_lib.TileCfg(256, 0, 0, 0, flags)), want),
+        "gmm_t": (ops.gmm_forward(xd, At, gd, trans_rhs=True, cfg=_lib.TileCfg(256, 0, 0, 0, flags)), want),
+        "dlhs": (ops.gmm_forward(dd, Ad, gd, trans_rhs=True, cfg=_lib.TileCfg(256, 0, 0, 0, flags)), want_dx),
+        "tgmm": (ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, 0, 0, flags)), want_dA),
+    }
+    for name, (y, ref) in got.items():
+        y = y.cpu().double()
+        assert torch.isfinite(y).all(), name
+        err = float((y - ref).norm() / ref.norm())
+        assert err < limit, (name, err)
+    assert float(got["gmm"][0][total:].abs().sum()) == 0.0
+
+
+def test_float32_highest_splits_extreme_values():
+    """The split of the operands at the ends of the float32 range: values that round up to infinity
+    as TF32, infinities and NaN give what the same products give on a split done outside."""
+    big, k, n = 3.4028234e38, 256, 256
+    x = torch.ones((4, k), dtype=torch.float32)
+    x[0, 0], x[1, 3], x[2, 5] = big, float("inf"), float("nan")
+    A = torch.full((1, k, n), 2.0 ** -10, dtype=torch.float32)
+    y = ops.gmm_forward(x.to(DEV), A.to(DEV), torch.tensor([4], dtype=torch.int32, device=DEV),
+                        cfg=_lib.TileCfg(0, 0, 0, 0, _lib.RD_CFG_F32_THREE_PASS)).cpu()
+    assert torch.isfinite(y[0]).all() and float((y[0] / (big * 2.0 ** -10) - 1).abs().max()) < 2.0 ** -9
+    assert not torch.isfinite(y[1:3]).any()
+    assert torch.equal(y[3], torch.full((n,), k * 2.0 ** -10))
