@@ -139,6 +139,16 @@ SIGNATURES = {
         + [_c_int] * 5
         + [ctypes.POINTER(TileCfg), _c_void_p],
     ),
+    "rd_gather_rows_clamped": (_c_int, [_c_void_p, _c_void_p, _c_void_p] + [_c_int] * 3 + [_c_void_p]),
+    "rd_sum_rows_scratch_bytes": (_c_size_t, [_c_int, _c_int]),
+    "rd_sum_rows": (
+        _c_int,
+        [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p] + [_c_int] * 4 + [_c_void_p, _c_size_t, _c_void_p],
+    ),
+    "rd_zero_unwritten_rows": (
+        _c_int,
+        [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p],
+    ),
     "rd_gather_rows": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p]),
     "rd_ep_count": (_c_int, [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p]),
     "rd_ep_plan": (_c_int, [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p,

@@ -615,8 +615,8 @@ int rd_gmm_indexed(const void* x, const void* A, int num_weights, const int32_t*
                   n, g, trans_rhs, dtype, cfg, stream);
 }
 
-int rd_gather_rows(const void* src, const int32_t* row_index, void* dst, int rows_out, int rows_in,
-                   int row_bytes, void* stream) {
+static int gather_rows_impl(const void* src, const int32_t* row_index, void* dst, int rows_out, int rows_in,
+                            int row_bytes, bool clamp, void* stream) {
   if (rows_out < 0 || rows_in < 0 || row_bytes < 0 || (row_bytes & 15)) return RD_ERR_BAD_SHAPE;
   if (rows_out == 0 || row_bytes == 0) return RD_OK;
   if (!aligned16(src) || !aligned16(dst) || row_index == nullptr) return RD_ERR_BAD_POINTER;
@@ -626,7 +626,88 @@ int rd_gather_rows(const void* src, const int32_t* row_index, void* dst, int row
   if (blocks > cap) blocks = cap;
   rd::gather_rows_kernel<<<blocks, rd::kGatherThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(src), row_index, static_cast<uint4*>(dst), rows_out, rows_in,
-      row_bytes / 16);
+      row_bytes / 16, clamp);
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
+int rd_gather_rows(const void* src, const int32_t* row_index, void* dst, int rows_out, int rows_in,
+                   int row_bytes, void* stream) {
+  return gather_rows_impl(src, row_index, dst, rows_out, rows_in, row_bytes, false, stream);
+}
+
+int rd_gather_rows_clamped(const void* src, const int32_t* row_index, void* dst, int rows_out, int rows_in,
+                           int row_bytes, void* stream) {
+  return gather_rows_impl(src, row_index, dst, rows_out, rows_in, row_bytes, true, stream);
+}
+
+size_t rd_sum_rows_scratch_bytes(int rows_in, int rows_out) {
+  if (rows_in < 0 || rows_out < 0) return 0;
+  return (2 * static_cast<size_t>(rows_out) + 1 + 2 * static_cast<size_t>(rows_in)) * sizeof(int32_t);
+}
+
+int rd_sum_rows(const void* src, const int32_t* row_index, const int32_t* group_sizes, int g, void* dst,
+                int rows_in, int rows_out, int cols, int dtype, void* scratch, size_t scratch_bytes,
+                void* stream_v) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (dtype != RD_DTYPE_F16 && dtype != RD_DTYPE_BF16 && dtype != RD_DTYPE_F32) return RD_ERR_BAD_DTYPE;
+  if (rows_in < 0 || rows_out < 0 || cols < 0 || g < 0) return RD_ERR_BAD_SHAPE;
+  if (rows_out == 0 || cols == 0) return RD_OK;
+  if (dst == nullptr) return RD_ERR_BAD_POINTER;
+  const size_t row_bytes = static_cast<size_t>(cols) * (dtype == RD_DTYPE_F32 ? 4 : 2);
+  if (rows_in == 0 || g == 0) {
+    cudaMemsetAsync(dst, 0, row_bytes * rows_out, stream);
+    return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+  }
+  if (src == nullptr || row_index == nullptr || group_sizes == nullptr) return RD_ERR_BAD_POINTER;
+  if (scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 3u)) return RD_ERR_BAD_POINTER;
+  if (scratch_bytes < rd_sum_rows_scratch_bytes(rows_in, rows_out)) return RD_ERR_WORKSPACE;
+  int32_t* count = static_cast<int32_t*>(scratch);
+  int32_t* cursor = count + rows_out;
+  int32_t* start = cursor + 1;
+  int32_t* rank = start + rows_out;
+  int32_t* list = rank + rows_in;
+  if (cudaMemsetAsync(count, 0, sizeof(int32_t) * (static_cast<size_t>(rows_out) + 1), stream) != cudaSuccess)
+    return RD_ERR_LAUNCH;
+  constexpr int kT = rd::kGatherThreads;
+  rd::sum_rows_count_kernel<<<(rows_in + kT - 1) / kT, kT, 0, stream>>>(row_index, rows_in, rows_out, group_sizes,
+                                                                      g, count, rank);
+  rd::sum_rows_start_kernel<<<(rows_out + kT - 1) / kT, kT, 0, stream>>>(count, rows_out, start, cursor);
+  rd::sum_rows_fill_kernel<<<(rows_in + kT - 1) / kT, kT, 0, stream>>>(row_index, rows_in, rows_out, start, rank,
+                                                                     list);
+  const bool wide = row_bytes % 16 == 0 && aligned16(src) && aligned16(dst);
+  const int vec = wide ? (dtype == RD_DTYPE_F32 ? 4 : 8) : 1;
+  const int vecs = cols / vec;
+  const int chunks = (vecs + 127) / 128;
+  const long long warps = static_cast<long long>(rows_out) * chunks;
+  long long blocks = (warps + kT / 32 - 1) / (kT / 32);
+  const long long cap = static_cast<long long>(sm_count()) * 64;
+  if (blocks > cap) blocks = cap;
+#define RD_SUM_ROWS(TY, V)                                                                              \
+  rd::sum_rows_kernel<TY, V><<<static_cast<int>(blocks), kT, 0, stream>>>(                                \
+      static_cast<const uint8_t*>(src), list, start, count, static_cast<uint8_t*>(dst), rows_out, vecs, chunks)
+  if (dtype == RD_DTYPE_F32) { if (wide) RD_SUM_ROWS(2, 4); else RD_SUM_ROWS(2, 1); }
+  else if (dtype == RD_DTYPE_BF16) { if (wide) RD_SUM_ROWS(1, 8); else RD_SUM_ROWS(1, 1); }
+  else { if (wide) RD_SUM_ROWS(0, 8); else RD_SUM_ROWS(0, 1); }
+#undef RD_SUM_ROWS
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
+int rd_zero_unwritten_rows(void* y, int y_rows, int row_bytes, const int32_t* out_rows, int m,
+                           const int32_t* group_sizes, int g, int32_t* scratch, void* stream_v) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (y_rows < 0 || m < 0 || g < 0 || row_bytes < 0 || (row_bytes & 15)) return RD_ERR_BAD_SHAPE;
+  if (y_rows == 0 || row_bytes == 0) return RD_OK;
+  if (!aligned16(y) || scratch == nullptr) return RD_ERR_BAD_POINTER;
+  if (m > 0 && g > 0 && (out_rows == nullptr || group_sizes == nullptr)) return RD_ERR_BAD_POINTER;
+  if (cudaMemsetAsync(scratch, 0, sizeof(int32_t) * y_rows, stream) != cudaSuccess) return RD_ERR_LAUNCH;
+  constexpr int kT = rd::kGatherThreads;
+  if (m > 0 && g > 0)
+    rd::mark_rows_kernel<<<(m + kT - 1) / kT, kT, 0, stream>>>(out_rows, m, y_rows, group_sizes, g, scratch);
+  int blocks = (y_rows + kT / 32 - 1) / (kT / 32);
+  const int cap = sm_count() * 8;
+  if (blocks > cap) blocks = cap;
+  rd::zero_unwritten_rows_kernel<<<blocks, kT, 0, stream>>>(scratch, static_cast<uint4*>(y), y_rows,
+                                                            row_bytes / 16);
   return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
 }
 

@@ -286,8 +286,10 @@ def gmm_fp8_forward(x: torch.Tensor, A: torch.Tensor, group_sizes: torch.Tensor,
     return out
 
 
-def gather_rows(src: torch.Tensor, row_index: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """dst[i] = src[row_index[i]] through ``rd_gather_rows`` (rows must be a multiple of 16 bytes)."""
+def gather_rows(src: torch.Tensor, row_index: torch.Tensor, out: Optional[torch.Tensor] = None,
+                clamp: bool = False) -> torch.Tensor:
+    """dst[i] = src[row_index[i]] through ``rd_gather_rows`` (rows must be a multiple of 16 bytes); an
+    index outside src gives a zero row, or with ``clamp`` the nearest row."""
     lib = _lib.load()
     _require_cuda(src, "src")
     idx = _as_i32(row_index)
@@ -297,9 +299,29 @@ def gather_rows(src: torch.Tensor, row_index: torch.Tensor, out: Optional[torch.
     dst = out if out is not None else torch.empty((rows_out, src.shape[1]), dtype=src.dtype, device=src.device)
     assert dst.is_contiguous() and dst.shape == (rows_out, src.shape[1]) and dst.dtype == src.dtype
     with torch.cuda.device(src.device):
-        rc = lib.rd_gather_rows(src.data_ptr(), idx.data_ptr(), dst.data_ptr(), rows_out, src.shape[0],
-                                row_bytes, _stream_ptr(src.device))
+        fn = lib.rd_gather_rows_clamped if clamp else lib.rd_gather_rows
+        rc = fn(src.data_ptr(), idx.data_ptr(), dst.data_ptr(), rows_out, src.shape[0], row_bytes,
+                _stream_ptr(src.device))
     _lib.check(rc, "rd_gather_rows")
+    return dst
+
+
+def sum_rows(src: torch.Tensor, row_index: torch.Tensor, group_sizes: torch.Tensor, rows_out: int) -> torch.Tensor:
+    """dst[t] = sum of src[i] over the rows i < sum(group_sizes) with row_index[i] == t (clamped), added
+    in float32 (``rd_sum_rows``): the gradient of ``gather_rows(x, row_index, clamp=True)``."""
+    lib = _lib.load()
+    _require_cuda(src, "src")
+    idx, gs = _as_i32(row_index), _as_i32(group_sizes)
+    src = src.contiguous()
+    assert src.dim() == 2 and idx.numel() >= src.shape[0]
+    dst = torch.empty((rows_out, src.shape[1]), dtype=src.dtype, device=src.device)
+    nbytes = lib.rd_sum_rows_scratch_bytes(src.shape[0], rows_out)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=src.device)
+    with torch.cuda.device(src.device):
+        rc = lib.rd_sum_rows(src.data_ptr(), idx.data_ptr(), gs.data_ptr(), gs.numel(), dst.data_ptr(), src.shape[0],
+                             rows_out, src.shape[1], _DTYPE_CODE[src.dtype], scratch.data_ptr(), nbytes,
+                             _stream_ptr(src.device))
+    _lib.check(rc, "rd_sum_rows")
     return dst
 
 
@@ -614,10 +636,9 @@ def gmm_permuted_forward(
     if out is not None and not padded_n:
         assert out.shape == (y_rows, n) and out.dtype == x.dtype and out.is_contiguous()
         y = out
-    elif out_rows is not None:
+    elif out_rows is not None and out is not None:
         y = torch.zeros((y_rows, np_), dtype=x.dtype, device=x.device)
-        if out is not None:
-            y[:, :n] = out
+        y[:, :n] = out
     else:
         y = torch.empty((y_rows, np_), dtype=x.dtype, device=x.device)
     ws = workspace if workspace is not None else _workspace(m, g, x.device)
@@ -630,7 +651,14 @@ def gmm_permuted_forward(
             ws.data_ptr(), ws.numel(), m, kp, np_, g, int(bool(trans_rhs)), _DTYPE_CODE[x.dtype],
             _cfg_ptr(cfg), _stream_ptr(x.device),
         )
-    _lib.check(rc, "rd_gmm_permuted")
+        _lib.check(rc, "rd_gmm_permuted")
+        if out_rows is not None and out is None:
+            # Rows that no sorted row names are zero: clearing only those instead of all of y first
+            # saves a pass over it.
+            marks = torch.empty(y_rows, dtype=torch.int32, device=x.device)
+            rc = lib.rd_zero_unwritten_rows(y.data_ptr(), y_rows, np_ * y.element_size(), out_rows.data_ptr(), m,
+                                            gs.data_ptr(), g, marks.data_ptr(), _stream_ptr(x.device))
+            _lib.check(rc, "rd_zero_unwritten_rows")
     if padded_n:
         y = y[:, :n].contiguous()
         if out is not None:
@@ -703,7 +731,7 @@ def _fused_permute_pays(m: int, g: int, scatter: bool) -> bool:
 
 
 def _gmm_permuted_two_pass(x, A, gs, in_rows, out_rows, y_rows, m, trans_rhs):
-    xs = x if in_rows is None else gather_rows(x, in_rows[:m].clamp(0, x.shape[0] - 1))
+    xs = x if in_rows is None else gather_rows(x, in_rows[:m], clamp=True)
     if xs.shape[0] != m:
         xs = xs[:m] if xs.shape[0] > m else torch.nn.functional.pad(xs, (0, 0, 0, m - xs.shape[0]))
     ys = gmm_forward(xs.contiguous(), A, gs, trans_rhs=trans_rhs)
@@ -746,7 +774,7 @@ class _GmmPermutedFn(torch.autograd.Function):
         use_fused = bool(fused)
         dys = None
         if not use_fused:
-            dys = dy if out_rows is None else gather_rows(dy, out_rows[:m].clamp(0, dy.shape[0] - 1))
+            dys = dy if out_rows is None else gather_rows(dy, out_rows[:m], clamp=True)
         if ctx.needs_input_grad[0]:
             if use_fused:
                 dxs = gmm_permuted_forward(dy, A, gs, in_rows=out_rows, m=m, trans_rhs=not trans_rhs)
@@ -756,9 +784,7 @@ class _GmmPermutedFn(torch.autograd.Function):
                 dx = dxs[: x.shape[0]] if dxs.shape[0] >= x.shape[0] else torch.nn.functional.pad(
                     dxs, (0, 0, 0, x.shape[0] - dxs.shape[0]))
             else:  # a token row may feed several sorted rows (top-k routing): sum them in fp32
-                idx = in_rows[:m].long().clamp_(0, x.shape[0] - 1)
-                dx = torch.zeros(x.shape, dtype=torch.float32, device=x.device).index_add_(0, idx, dxs.float())
-                dx = dx.to(x.dtype)
+                dx = sum_rows(dxs, in_rows, gs, x.shape[0])
         if ctx.needs_input_grad[1]:
             if use_fused:
                 if not trans_rhs:
@@ -766,7 +792,7 @@ class _GmmPermutedFn(torch.autograd.Function):
                 else:
                     dA = tgmm_permuted_forward(dy, x, gs, x_rows_index=out_rows, y_rows_index=in_rows, m=m)
             else:
-                xs = x if in_rows is None else gather_rows(x, in_rows[:m].clamp(0, x.shape[0] - 1))
+                xs = x if in_rows is None else gather_rows(x, in_rows[:m], clamp=True)
                 dA = tgmm_forward(xs, dys, gs) if not trans_rhs else tgmm_forward(dys, xs, gs)
         return dx, dA, None, None, None, None, None, None, None
 

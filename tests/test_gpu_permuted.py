@@ -173,3 +173,54 @@ def test_permuted_argument_checks():
     pair = _lib.TileCfg(256, 0, 2, 0, 0)
     assert call(cfg=ctypes.byref(pair)) == _lib.RD_ERR_BAD_CONFIG
     torch.cuda.synchronize()
+
+
+# ------------------------------------------------------------------ sum of rows by index, unwritten rows
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows_in,rows_out,cols,live", [
+    (1, 1, 8, 1),
+    (300, 7, 1032, 300),     # lists longer than a warp; 1032 = one 128-vector chunk and one vector
+    (257, 400, 4096, 200),   # rows without a source; rows past the groups do not count
+    (64, 64, 37, 64),        # rows that are not multiples of 16 bytes
+    (500, 3, 64, 0),         # no live row
+])
+def test_sum_rows(dtype, rows_in, rows_out, cols, live):
+    """Against a float64 sum: at most one rounding to the result's type (2^-9 bf16, 2^-12 fp16) plus
+    float32 additions of up to 100 terms."""
+    rng = np.random.default_rng(rows_in + cols)
+    index = torch.from_numpy(rng.integers(-2, rows_out + 2, size=rows_in).astype(np.int32))
+    src = oracle.reference_normal(3, (rows_in, cols), torch.float32).to(dtype)
+    src[live:] = float("nan")
+    gs = torch.tensor([live // 3, 0, live - live // 3], dtype=torch.int32)
+    want = torch.zeros((rows_out, cols), dtype=torch.float64)
+    mag = torch.zeros((rows_out, cols), dtype=torch.float64)
+    idx = index[:live].long().clamp(0, rows_out - 1)
+    want.index_add_(0, idx, src[:live].double())
+    mag.index_add_(0, idx, src[:live].double().abs())
+    got = ops.sum_rows(src.to(DEV), index.to(DEV), gs.to(DEV), rows_out)
+    assert got.dtype == dtype
+    again = ops.sum_rows(src.to(DEV), index.to(DEV), gs.to(DEV), rows_out)
+    if rows_in <= 257 and rows_out >= 32:
+        assert torch.equal(got, again)  # short lists are added in a fixed order
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 0.0}[dtype]
+    bound = eps * want.abs() + (128 * 2.0 ** -24) * mag + 2.0 ** -24
+    assert bool(((got.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("tokens,extra,y_rows", [(96, 0, 192), (96, 33, 200), (5, 0, 300)])
+def test_gmm_permuted_clears_unnamed_rows(tokens, extra, y_rows):
+    """Rows of y that no sorted row names are zero, also where memory held something else."""
+    g, k, n = 4, 64, 136
+    gs, in_rows, out_rows = _routing(11, tokens, 2, g, extra)
+    out_rows = torch.where(out_rows % 7 == 0, out_rows + 1000, out_rows)  # some destinations do not exist
+    x = oracle.reference_normal(1, (tokens, k), torch.bfloat16)
+    A = oracle.reference_normal(2, (g, k, n), torch.bfloat16)
+    junk = torch.full((y_rows, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    del junk  # the allocator hands this block out again
+    y = ops.gmm_permuted_forward(x.to(DEV), A.to(DEV), gs.to(DEV), in_rows=in_rows.to(DEV), out_rows=out_rows.to(DEV),
+                                 y_rows=y_rows).cpu()
+    named = torch.zeros(y_rows, dtype=torch.bool)
+    live = out_rows[: int(gs.sum())].long()
+    named[live[(live >= 0) & (live < y_rows)]] = True
+    assert torch.equal(y[~named], torch.zeros_like(y[~named]))
+    assert torch.isfinite(y.float()).all() and bool((y[named].abs().sum(1) > 0).all())
