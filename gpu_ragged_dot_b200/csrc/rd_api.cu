@@ -317,6 +317,17 @@ int launch_pairs(Kernel kernel, int threads, int smem_bytes, const CUtensorMap& 
   return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
 }
 
+// e4m3 on 256-row tiles (rd_gemm2.cuh, kFp8).
+int launch_gemm2_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout, const GemmArgs& args,
+                     int ctas, cudaStream_t stream) {
+  auto kernel = rd::ragged_gemm2_kernel<true, false, false, false, true>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kG2SmemBytes) !=
+      cudaSuccess)
+    return RD_ERR_LAUNCH;
+  kernel<<<ctas, rd::kG2Threads, rd::kG2SmemBytes, stream>>>(ta, tb, tout, args);
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
 // tgmm with 512 x 256 tiles on CTA pairs (rd_gemm2.cuh, kPair).
 int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
                       const GemmArgs& args, int ctas, cudaStream_t stream) {
@@ -341,6 +352,7 @@ int launch_gemm_f32_pair(bool split, const CUtensorMap& ta, const CUtensorMap& t
 // wrong guess is only a shallower smem ring).  At exactly 512 rows per group the picture is mixed:
 // 16 ragged groups over m 8192, k 4096, n 14336 are 5-13 % faster on 128-row tiles, the
 // expert-parallel step (64 segments of about 512 rows over 32 weight matrices) 4 % slower.
+// e4m3 follows the same rule: m 8192, k 4096, n 14336, 8 groups 390 -> 378 us, 475 -> 466 us in a row.
 bool choose_two_half(bool tgmm, long long m, int k, int g, int bn) {
   if (bn != 256) return false;
   if (tgmm) return k >= 256;
@@ -1293,9 +1305,10 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   if (rc != RD_OK) return rc;
   int bn = cfg && cfg->tile_n ? cfg->tile_n : choose_tile_n(0, n, 0);
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
-  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // 128-row tiles only
+  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // the library chooses
+  const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, g, bn);
 
-  launch_internal_metadata(group_sizes, group_to_weight, g, m, rd::kTileM, w, stream,
+  launch_internal_metadata(group_sizes, group_to_weight, g, m, two_half ? rd::kG2TileRows : rd::kTileM, w, stream,
                            cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0);
   if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
 
@@ -1338,6 +1351,7 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   args.out = y;
   args.groups_per_flag = 1;
   const int ctas = pick_ctas(cfg);
+  if (two_half) return launch_gemm2_fp8(ta, tb, tout, args, ctas, stream);
   if (bn == 256) return launch_gemm<256, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);
   if (bn == 128) return launch_gemm<128, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);
   return launch_gemm<64, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);

@@ -101,12 +101,15 @@ __device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, int 
 // `cta_index` / `gemm_ctas` variables cost the plain kernel 3-5 %):
 //   gmm:  the expert-parallel variant (ready flags in the loader, sender CTAs in the grid);
 //   tgmm: strided segments (a block contracts over several row ranges, rd_tgmm_strided).
-template <bool kBKMajor, bool kTgmm, bool kVariant = false, bool kPair = false>
+// kFp8: e4m3 operands, gmm with K-major weights; tiles are byte for byte those of a 16-bit problem with
+// k / 2 elements per row (see rd_gemm.cuh).
+template <bool kBKMajor, bool kTgmm, bool kVariant = false, bool kPair = false, bool kFp8 = false>
 __global__ void __launch_bounds__(kG2Threads, 1)
 ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
   static_assert(!(kTgmm && kBKMajor), "tgmm reads both operands MN-major");
+  static_assert(!kFp8 || (kBKMajor && !kTgmm && !kVariant && !kPair), "8-bit inputs: plain gmm, K-major weights");
   static_assert(!kPair || (kTgmm && !kVariant), "CTA pairs: plain tgmm only");
   constexpr bool kEp = !kTgmm && kVariant;
   constexpr bool kSeg = kTgmm && kVariant;
@@ -323,7 +326,8 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // __syncwarp costs about 160 clocks on B200, a stage's MMAs take 1024).  The one warp-wide
     // job, clearing the rows past a group's end in a tgmm stage, belongs to the fixer warp.
     if (lane == 0 && leader) {
-      const uint32_t idesc = make_idesc_f16(p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM * kCtas, BN);
+      const uint32_t idesc =
+          make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM * kCtas, BN);
       constexpr uint32_t kAStep = (kTgmm ? 2048u : 32u) >> 4;
       constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
       const uint64_t adesc0 = kTgmm ? make_smem_desc(stage_base, kBoxBytes, 1024)
@@ -402,16 +406,16 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
               const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * (kHalfABytes >> 4);
               if (kTgmm && n_mma < kTileK / kUmmaK) {
                 for (int kk = 0; kk < n_mma; ++kk) {
-                  umma_f16<kCtas>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
+                  umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
                                   make_desc64(b_lo + kk * kBStep, desc_hi), idesc,
                                   (kb > 0 || kk > 0) ? 1u : 0u);
                 }
               } else {
-                umma_f16<kCtas>(tmem_d, make_desc64(a_lo, desc_hi), make_desc64(b_lo, desc_hi), idesc,
+                umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo, desc_hi), make_desc64(b_lo, desc_hi), idesc,
                                 kb > 0 ? 1u : 0u);
 #pragma unroll
                 for (int kk = 1; kk < kTileK / kUmmaK; ++kk) {
-                  umma_f16<kCtas>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
+                  umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
                                   make_desc64(b_lo + kk * kBStep, desc_hi), idesc, 1u);
                 }
               }
@@ -545,6 +549,11 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         } else {
 #pragma unroll
           for (int j = 0; j < 64; ++j) v[j] = 0u;
+        }
+        if constexpr (kFp8) {  // dequantise: one scale per weight matrix (1 when none is given)
+          const float sc = p.weight_scale != nullptr ? p.weight_scale[t.weight] : 1.0f;
+#pragma unroll
+          for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * sc);
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {

@@ -1265,3 +1265,17 @@ def test_float32_highest_splits_extreme_values():
     assert torch.isfinite(y[0]).all() and float((y[0] / (big * 2.0 ** -10) - 1).abs().max()) < 2.0 ** -9
     assert not torch.isfinite(y[1:3]).any()
     assert torch.equal(y[3], torch.full((n,), k * 2.0 ** -10))
+
+
+def test_gmm_fp8_on_256_row_tiles():
+    """Long groups (512 rows on average) run on 256-row tiles: bit-equal to the 128-row kernel, which
+    adds the same products in the same order, at tile edges and with and without a scale."""
+    m, k, n = 1601, 272, 264
+    gs = torch.tensor([257, 0, 1279 + 64], dtype=torch.int32)
+    rng = np.random.default_rng(5)
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
+    A = torch.from_numpy(rng.standard_normal((3, n, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
+    for scale in (None, torch.tensor([0.5, 2.0, 0.03125], device=DEV)):
+        want = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale, cfg=_lib.TileCfg(256, 0, 0, 128, 0))
+        got = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale)
+        assert torch.equal(got, want) and float(got[-1].abs().max()) == 0.0
