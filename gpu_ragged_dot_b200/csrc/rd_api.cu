@@ -45,6 +45,29 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// The tensor-map encoder needs a context on the calling thread.  A runtime launch binds the device's
+// primary context, but threads such as torch's autograd workers arrive here without one.
+int ensure_context() {
+  typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
+  static CtxGetCurrentFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
+        qres == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<CtxGetCurrentFn>(sym);
+  });
+  CUcontext ctx = nullptr;
+  if (fn != nullptr && fn(&ctx) == CUDA_SUCCESS && ctx != nullptr) return RD_OK;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return RD_ERR_LAUNCH;
+  }
+  return RD_OK;
+}
+
 // rank-2 or rank-3 tiled map over a dense row-major 16-bit or 32-bit float tensor, 128-byte swizzle,
 // zero fill outside the bounds.  dims / box are innermost first.
 int encode_map(CUtensorMap* map, const void* base, int dtype, int rank, const uint64_t* dims,
@@ -172,6 +195,12 @@ void launch_internal_metadata(const int32_t* group_sizes, const int32_t* group_t
       group_sizes, g, m, tile_m, w.layout.max_tiles, w.group_offsets(), w.tile2group(),
       w.tile2idx(), w.totals(), w.tile_prefix(), w.totals() + 1, w.status(), w.tile_rec(),
       group_to_weight);
+}
+
+// Do the CTAs make their own group table (rd_gemm.cuh), so that no metadata launch is needed?  Not for
+// more groups or row tiles than the table holds.
+bool inline_groups(int m, int g) {
+  return g <= rd::kMaxInlineGroups && max_row_tiles(m, g) <= rd::kMaxInlineRowTiles;
 }
 
 // ------------------------------------------------------------------ tile selection
@@ -517,14 +546,18 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (tile_m == 0) tile_m = (cta_group == 1 && choose_two_half(false, m, k, g, bn)) ? 256 : 128;
   const bool two_half = tile_m == 256;
 
-  // Launch the metadata kernel before encoding the tensor maps: besides being the first step
-  // of the call, a runtime launch binds the device's primary context to the calling thread,
-  // which the driver's tensor-map encoder needs (threads such as torch's autograd workers
-  // arrive here without one).
-  launch_internal_metadata(group_sizes, group_to_weight, g, m,
-                           two_half ? rd::kG2TileRows : rd::kTileM * cta_group, w, stream,
-                           cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0);
-  if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  // The expert-parallel forms (flags, senders, groups visited by weight) keep the metadata launch.
+  const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
+  const bool in_kernel = inline_groups(m, g) && ready.flags == nullptr && send == nullptr &&
+                         !(by_weight && group_to_weight != nullptr);
+  if (in_kernel) {
+    rc = ensure_context();
+    if (rc != RD_OK) return rc;
+  } else {
+    launch_internal_metadata(group_sizes, group_to_weight, g, m,
+                             two_half ? rd::kG2TileRows : rd::kTileM * cta_group, w, stream, by_weight);
+    if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  }
 
   const bool blocked = f32 && cta_group == 2 && !trans_rhs && n % 32 == 0;
   CUtensorMap ta, tb;
@@ -571,6 +604,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   args.totals = w.totals();
   args.status = w.status();
   args.out = y;
+  args.inline_groups = in_kernel ? 1 : 0;
+  args.group_to_weight = group_to_weight;
   args.ready_flags = ready.flags;
   args.groups_per_flag = ready.groups_per_flag > 0 ? ready.groups_per_flag : 1;
   args.ready_epoch = ready.epoch;
@@ -963,12 +998,14 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   const int tile_rows = two_half ? rd::kG2TileRows * cta_group : rd::kTileM * cta_group;
   const long long k_tiles = (k + tile_rows - 1) / tile_rows;
 
-  // Launch the metadata kernel before encoding the tensor maps: besides being the first step
-  // of the call, a runtime launch binds the device's primary context to the calling thread,
-  // which the driver's tensor-map encoder needs (threads such as torch's autograd workers
-  // arrive here without one).
-  launch_internal_metadata(group_sizes, nullptr, g_fine, m, rd::kTileM, w, stream);
-  if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  const bool in_kernel = seg_count == 1 && inline_groups(m, g);
+  if (in_kernel) {
+    rc = ensure_context();
+    if (rc != RD_OK) return rc;
+  } else {
+    launch_internal_metadata(group_sizes, nullptr, g_fine, m, rd::kTileM, w, stream);
+    if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  }
 
   // 256-row tiles fetch each operand of a stage with one box when the 64-column blocks tile the
   // rows exactly (see rd_gemm2.cuh); otherwise one 2-D box per 64 columns.
@@ -1021,6 +1058,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   args.ab_format = dtype;
   args.wait_limit_us = wait_limit_us(cfg);
   args.zero_tail = 0;
+  args.inline_groups = in_kernel ? 1 : 0;
   args.group_sizes = group_sizes;
   args.group_offsets = w.group_offsets();
   args.tile_rec = w.tile_rec();
@@ -1308,9 +1346,16 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // the library chooses
   const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, g, bn);
 
-  launch_internal_metadata(group_sizes, group_to_weight, g, m, two_half ? rd::kG2TileRows : rd::kTileM, w, stream,
-                           cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0);
-  if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
+  const bool in_kernel = inline_groups(m, g) && !(by_weight && group_to_weight != nullptr);
+  if (in_kernel) {
+    rc = ensure_context();
+    if (rc != RD_OK) return rc;
+  } else {
+    launch_internal_metadata(group_sizes, group_to_weight, g, m, two_half ? rd::kG2TileRows : rd::kTileM, w, stream,
+                             by_weight);
+    if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  }
 
   // Both operands are K-major, so a row of k one-byte elements is described to TMA as k/2
   // two-byte elements: the bytes that land in shared memory are the same.
@@ -1350,6 +1395,8 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   args.status = w.status();
   args.out = y;
   args.groups_per_flag = 1;
+  args.inline_groups = in_kernel ? 1 : 0;
+  args.group_to_weight = group_to_weight;
   const int ctas = pick_ctas(cfg);
   if (two_half) return launch_gemm2_fp8(ta, tb, tout, args, ctas, stream);
   if (bn == 256) return launch_gemm<256, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);

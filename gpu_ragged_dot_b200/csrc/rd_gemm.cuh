@@ -76,6 +76,10 @@ struct GemmArgs {
   int blocked_maps;
   uint32_t wait_limit_us;  // how long a bounded wait inside the kernel may last (microseconds)
   const float* weight_scale;  // 8-bit inputs: scale of weight matrix w, applied to the accumulator (null: 1)
+  // Set: every CTA makes its own group table in shared memory (build_group_table); group_offsets,
+  // tile_rec and totals are not read then, and there is no metadata launch.
+  int inline_groups;
+  const int32_t* group_to_weight;  // inline_groups, gmm: weight matrix of each group (null: the group's own index)
   const int32_t* group_sizes;
   const int32_t* group_offsets;
   const TileRecord* tile_rec;  // gmm: one record per live row tile (of 128 * kCtas rows)
@@ -106,24 +110,131 @@ struct TileCoord {
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 __device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
 
+// ------------------------------------------------------------------ group table in shared memory
+// Up to 256 groups, one warp of every CTA scans group_sizes itself (one load per lane and group,
+// two warp scans, about a microsecond beside the barrier and TMEM set-up), instead of one CTA in a
+// launch of its own in front of every GEMM: that launch costs 6 us of stream time (3.5 us and the
+// gaps around it) and 3 us of the host's.  A tile then finds its group with at most eight
+// shared-memory reads.  256 groups are what fits beside 192 KB of stages and the staging boxes.
+constexpr int kMaxInlineGroups = 256;
+constexpr int kMaxInlineRowTiles = 65535;  // tiles are counted in 16 bits
+
+struct GroupTable {
+  int32_t offset[kMaxInlineGroups + 1];  // first row of each group; [g]: sum of the sizes
+  uint16_t tiles[kMaxInlineGroups + 1];  // row tiles of all earlier groups; [g]: of all groups
+};
+
+// One warp.  Rows at or past m count for no tile.
+__device__ __forceinline__ void build_group_table(const GemmArgs& p, int tile_rows, GroupTable* tab, int lane) {
+  constexpr int kPer = kMaxInlineGroups / 32;
+  int rows[kPer], sum = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = lane * kPer + j;
+    rows[j] = i < p.g ? imax(p.group_sizes[i], 0) : 0;
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) sum += rows[j];
+  int off = warp_inclusive_scan(sum, lane) - sum;
+  int tiles[kPer], tsum = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = lane * kPer + j;
+    if (i <= p.g) tab->offset[i] = off;
+    const int live = imin(rows[j], imax(p.m - off, 0));
+    tiles[j] = (live + tile_rows - 1) / tile_rows;
+    tsum += tiles[j];
+    off += rows[j];
+  }
+  int t = warp_inclusive_scan(tsum, lane) - tsum;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = lane * kPer + j;
+    if (i <= p.g) tab->tiles[i] = static_cast<uint16_t>(t);
+    t += tiles[j];
+  }
+  if (lane == 31 && p.g == kMaxInlineGroups) {
+    tab->offset[p.g] = off;
+    tab->tiles[p.g] = static_cast<uint16_t>(t);
+  }
+}
+
+// What one row tile needs to know (from the table, or from the metadata kernel's records).
+struct RowTile {
+  int group, weight, group_offset, group_size, tile_base, tiles;
+};
+
+__device__ __forceinline__ RowTile find_row_tile(const GemmArgs& p, const GroupTable* tab, int mt) {
+  RowTile r;
+  if (p.inline_groups) {
+    int lo = 0, hi = p.g;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (tab->tiles[mid + 1] > mt) hi = mid; else lo = mid + 1;
+    }
+    r.group = lo;
+    r.weight = p.group_to_weight != nullptr ? p.group_to_weight[lo] : lo;
+    r.group_offset = tab->offset[lo];
+    r.group_size = imin(tab->offset[lo + 1] - r.group_offset, p.m - r.group_offset);
+    r.tile_base = tab->tiles[lo];
+    r.tiles = tab->tiles[lo + 1] - r.tile_base;
+  } else {
+    const int4* rp = reinterpret_cast<const int4*>(p.tile_rec + mt);
+    const int4 a = rp[0];  // group, weight, group_offset, group_size
+    const int4 b = rp[1];  // tile_base, tiles, idx, pad
+    r.group = a.x;
+    r.weight = a.y;
+    r.group_offset = a.z;
+    r.group_size = a.w;
+    r.tile_base = b.x;
+    r.tiles = b.y;
+  }
+  return r;
+}
+
+// First row and rows (below m) of a group.
+__device__ __forceinline__ void group_rows(const GemmArgs& p, const GroupTable* tab, int group, int& row0, int& rows) {
+  if (p.inline_groups) {
+    row0 = tab->offset[group];
+    rows = tab->offset[group + 1] - row0;
+  } else {
+    row0 = p.group_offsets[group];
+    rows = imax(p.group_sizes[group], 0);
+  }
+  rows = imax(imin(rows, p.m - row0), 0);
+}
+
+__device__ __forceinline__ int live_row_tiles(const GemmArgs& p, const GroupTable* tab) {
+  return p.inline_groups ? tab->tiles[p.g] : imin(p.totals[0], p.max_m_tiles);
+}
+
+// First row that belongs to no group.
+__device__ __forceinline__ int first_dead_row(const GemmArgs& p, const GroupTable* tab) {
+  return imin(imax(p.inline_groups ? tab->offset[p.g] : p.totals[1], 0), p.m);
+}
+
+// Start of a call: the metadata kernel resets the status words, or the first CTA does.  (A CTA that
+// records an expired wait does so a whole wait limit, at least a millisecond, after it started.)
+__device__ __forceinline__ void reset_status(const GemmArgs& p) {
+  if (p.inline_groups && blockIdx.x == 0) *reinterpret_cast<int4*>(p.status) = make_int4(0, 0, 0, 0);
+}
+
 // gmm tile order: group-major; inside a group the n-tiles are outer and the group's row
 // tiles inner, so CTAs running concurrently share one [k, BN] weight panel through L2 and an
-// expert's weights stream from HBM once.  One 32-byte record load per tile, no dependent loads.
+// expert's weights stream from HBM once.
 template <int BN, int kCtas>
-__device__ __forceinline__ TileCoord decode_gmm_tile(const GemmArgs& p, int tile, int cta_rank) {
+__device__ __forceinline__ TileCoord decode_gmm_tile(const GemmArgs& p, const GroupTable* tab, int tile,
+                                                     int cta_rank) {
   constexpr int kRows = kTileM * kCtas;
-  const int mt = tile / p.n_tiles;
-  const int4* rp = reinterpret_cast<const int4*>(p.tile_rec + mt);
-  const int4 a = rp[0];  // group, weight, group_offset, group_size
-  const int4 b = rp[1];  // tile_base, tiles, idx, pad
-  const int local = tile - b.x * p.n_tiles;
-  const int nt = local / b.y;
-  const int mi = local - nt * b.y;
+  const RowTile r = find_row_tile(p, tab, tile / p.n_tiles);
+  const int local = tile - r.tile_base * p.n_tiles;
+  const int nt = local / r.tiles;
+  const int mi = local - nt * r.tiles;
   TileCoord t;
-  t.group = a.x;
-  t.weight = a.y;
-  t.row0 = a.z + mi * kRows + cta_rank * kTileM;
-  t.rows = imin(kTileM, a.w - mi * kRows - cta_rank * kTileM);
+  t.group = r.group;
+  t.weight = r.weight;
+  t.row0 = r.group_offset + mi * kRows + cta_rank * kTileM;
+  t.rows = imin(kTileM, r.group_size - mi * kRows - cta_rank * kTileM);
   t.rows = imin(t.rows, p.m - t.row0);  // never touch rows past m
   t.n0 = nt * BN;
   t.k0 = 0;
@@ -131,7 +242,8 @@ __device__ __forceinline__ TileCoord decode_gmm_tile(const GemmArgs& p, int tile
 }
 
 template <int BN, int kCtas>
-__device__ __forceinline__ TileCoord decode_tgmm_tile(const GemmArgs& p, int tile, int cta_rank) {
+__device__ __forceinline__ TileCoord decode_tgmm_tile(const GemmArgs& p, const GroupTable* tab, int tile,
+                                                      int cta_rank) {
   const int per_group = p.k_tiles * p.n_tiles;
   const int gi = tile / per_group;
   const int rem = tile - gi * per_group;
@@ -140,8 +252,7 @@ __device__ __forceinline__ TileCoord decode_tgmm_tile(const GemmArgs& p, int til
   TileCoord t;
   t.group = gi;
   t.weight = gi;
-  t.row0 = p.group_offsets[gi];
-  t.rows = imax(imin(imax(p.group_sizes[gi], 0), p.m - t.row0), 0);
+  group_rows(p, tab, gi, t.row0, t.rows);
   t.n0 = nt * BN;
   t.k0 = (kt * kCtas + cta_rank) * kTileM;
   return t;
@@ -311,6 +422,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ __align__(8) uint64_t bar_acc_empty[2];  // leader only when paired
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
+  __shared__ GroupTable group_table;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -333,6 +445,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
+    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -352,6 +465,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<kCtas>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<kCtas>();
   }
+  if (warp == 2 && p.inline_groups) build_group_table(p, kTileM * kCtas, &group_table, lane);
   tc_fence_before_sync();
   __syncthreads();
   if (kPair) cluster_sync();  // the peer's barriers exist before anything arrives on them
@@ -363,7 +477,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (kTgmm) {
     num_tiles = p.g * p.k_tiles * p.n_tiles;
   } else {
-    num_tiles = imin(p.totals[0], p.max_m_tiles) * p.n_tiles;
+    num_tiles = live_row_tiles(p, &group_table) * p.n_tiles;
   }
   const int tile_start = cta_index / kCtas;
   const int tile_step = gemm_ctas / kCtas;
@@ -376,8 +490,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       int ready_slot = -1;  // last ready flag this producer has seen set
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, tile, cta_rank)
-                                  : decode_gmm_tile<BN, kCtas>(p, tile, cta_rank);
+        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank)
+                                  : decode_gmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
         const int nb = t.n0 + cta_rank * kBCols;  // first B column this CTA loads
         const int kb_count = kTgmm ? tgmm_block_count<kSeg>(p, t) : k_blocks_gmm;
         RowBlocks blocks = first_block(t);
@@ -463,8 +577,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t tail_events = 0;  // stages handed to the fixer warp so far
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, tile, cta_rank)
-                                  : decode_gmm_tile<BN, kCtas>(p, tile, cta_rank);
+        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank)
+                                  : decode_gmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
         const int kb_count = kTgmm ? tgmm_block_count<kSeg>(p, t) : k_blocks_gmm;
         const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
         RowBlocks blocks = first_block(t);
@@ -559,7 +673,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t own_parity = 0;  // peer of a pair, bit s: parity of the next landing on its own barrier of slot s
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = decode_tgmm_tile<BN, kCtas>(p, tile, cta_rank);
+        const TileCoord t = decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
         const int kb_count = tgmm_block_count<kSeg>(p, t);
         RowBlocks blocks = first_block(t);
         const bool tail_stage = kb_count > 0 && tail_needs_clearing(t.rows);
@@ -608,8 +722,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
     for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, tile, cta_rank)
-                                : decode_gmm_tile<BN, kCtas>(p, tile, cta_rank);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank)
+                                : decode_gmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
       const int n0 = t.n0;
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;
@@ -743,7 +857,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (!kTgmm && p.zero_tail) {
       // Rows past sum(group_sizes) belong to no group: jax.lax.ragged_dot defines them as 0
       // (the reference writes them from its last live program, gpu_ragged_dot.py:155-165).
-      const int first = imin(imax(p.totals[1], 0), p.m);
+      const int first = first_dead_row(p, &group_table);
       const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
       const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(cta_index) * 128 + (threadIdx.x - 64);

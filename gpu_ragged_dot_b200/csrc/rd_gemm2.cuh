@@ -53,19 +53,16 @@ constexpr uint32_t kG2PairStageBytes = kG2ABytes + kG2BBytes / 2;  // 48 KB
 constexpr int kG2PairSmemBytes = kG2PairStages * kG2PairStageBytes + kG2EpilogueWarps * kOutBoxBytes + 1024;
 
 // rows: valid rows of the whole 256-row tile (gmm) / rows of the group (tgmm).
-__device__ __forceinline__ TileCoord decode_gmm_tile256(const GemmArgs& p, int tile) {
-  const int mt = tile / p.n_tiles;
-  const int4* rp = reinterpret_cast<const int4*>(p.tile_rec + mt);
-  const int4 a = rp[0];  // group, weight, group_offset, group_size
-  const int4 b = rp[1];  // tile_base, tiles, idx, pad
-  const int local = tile - b.x * p.n_tiles;
-  const int nt = local / b.y;
-  const int mi = local - nt * b.y;
+__device__ __forceinline__ TileCoord decode_gmm_tile256(const GemmArgs& p, const GroupTable* tab, int tile) {
+  const RowTile r = find_row_tile(p, tab, tile / p.n_tiles);
+  const int local = tile - r.tile_base * p.n_tiles;
+  const int nt = local / r.tiles;
+  const int mi = local - nt * r.tiles;
   TileCoord t;
-  t.group = a.x;
-  t.weight = a.y;
-  t.row0 = a.z + mi * kG2TileRows;
-  t.rows = imin(kG2TileRows, a.w - mi * kG2TileRows);
+  t.group = r.group;
+  t.weight = r.weight;
+  t.row0 = r.group_offset + mi * kG2TileRows;
+  t.rows = imin(kG2TileRows, r.group_size - mi * kG2TileRows);
   t.rows = imin(t.rows, p.m - t.row0);
   t.n0 = nt * kG2TileN;
   t.k0 = 0;
@@ -73,7 +70,7 @@ __device__ __forceinline__ TileCoord decode_gmm_tile256(const GemmArgs& p, int t
 }
 
 template <int kRows = kG2TileRows>
-__device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, int tile) {
+__device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, const GroupTable* tab, int tile) {
   const int per_group = p.k_tiles * p.n_tiles;
   const int gi = tile / per_group;
   const int rem = tile - gi * per_group;
@@ -89,8 +86,7 @@ __device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, int 
   TileCoord t;
   t.group = gi;
   t.weight = gi;
-  t.row0 = p.group_offsets[gi];
-  t.rows = imax(imin(imax(p.group_sizes[gi], 0), p.m - t.row0), 0);
+  group_rows(p, tab, gi, t.row0, t.rows);
   t.n0 = nt * kG2TileN;
   t.k0 = kt * kRows;
   return t;
@@ -132,6 +128,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp(s) -> MMA thread: its tail rows are cleared
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
+  __shared__ GroupTable group_table;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -155,6 +152,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
+    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -174,6 +172,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<kCtas>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<kCtas>();
   }
+  if (warp == 2 && p.inline_groups) build_group_table(p, kTgmm ? kTileM : kG2TileRows, &group_table, lane);
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (kPair) cluster_sync();  // the peer's barriers exist before anything arrives on them
@@ -182,7 +181,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile WaitCtl* abort_ptr = &wait_ctl;
 
   const int num_tiles =
-      kTgmm ? p.g * p.k_tiles * p.n_tiles : imin(p.totals[0], p.max_m_tiles) * p.n_tiles;
+      kTgmm ? p.g * p.k_tiles * p.n_tiles : live_row_tiles(p, &group_table) * p.n_tiles;
   const int k_blocks_gmm = (p.k + kTileK - 1) / kTileK;
   const int tile_step = kPair ? static_cast<int>(gridDim.x >> 1)
                         : kEp ? static_cast<int>(gridDim.x) - sender_ctas : static_cast<int>(gridDim.x);
@@ -192,9 +191,9 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     return static_cast<int>(blockIdx.x);
   };
   auto decode = [&](int tile) -> TileCoord {
-    if constexpr (kPair) return decode_tgmm_tile256<2 * kG2TileRows>(p, tile);
-    if constexpr (kTgmm) return decode_tgmm_tile256(p, tile);
-    return decode_gmm_tile256(p, tile);
+    if constexpr (kPair) return decode_tgmm_tile256<2 * kG2TileRows>(p, &group_table, tile);
+    if constexpr (kTgmm) return decode_tgmm_tile256(p, &group_table, tile);
+    return decode_gmm_tile256(p, &group_table, tile);
   };
 
   // Number of halves of a tile that exist.
@@ -634,7 +633,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (!kTgmm && p.zero_tail) {
       // Rows past sum(group_sizes) belong to no group and are defined as zero.
       constexpr int kEpiThreads = 32 * kG2EpilogueWarps;
-      const int first = imin(imax(p.totals[1], 0), p.m);
+      const int first = first_dead_row(p, &group_table);
       const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
       const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(kEp ? blockIdx.x - sender_ctas : blockIdx.x) * kEpiThreads +

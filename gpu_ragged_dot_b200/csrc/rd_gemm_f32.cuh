@@ -85,6 +85,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ __align__(8) uint64_t bar_acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
+  __shared__ GroupTable group_table;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -93,6 +94,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
+    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -110,6 +112,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<1>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<1>();
   }
+  if (warp == 2 && p.inline_groups) build_group_table(p, kTileM, &group_table, lane);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -117,7 +120,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile WaitCtl* abort_ptr = &wait_ctl;
 
   const int num_tiles =
-      kTgmm ? p.g * p.k_tiles * p.n_tiles : imin(p.totals[0], p.max_m_tiles) * p.n_tiles;
+      kTgmm ? p.g * p.k_tiles * p.n_tiles : live_row_tiles(p, &group_table) * p.n_tiles;
   const int tile_step = static_cast<int>(gridDim.x);
   const int k_blocks_gmm = (p.k + kF32TileK - 1) / kF32TileK;
 
@@ -127,7 +130,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
         const int kb_count = kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
         for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % kStages;
@@ -180,7 +183,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t local_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
       const int kb_count = kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
       const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing_f32(t.rows);
       const uint32_t acc = local_tile & 1u;
@@ -248,7 +251,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     float* out32 = reinterpret_cast<float*>(p.out);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
       const int n0 = t.n0;
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;
@@ -342,7 +345,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     __syncwarp();
 
     if (!kTgmm && p.zero_tail) {
-      const int first = imin(imax(p.totals[1], 0), p.m);
+      const int first = first_dead_row(p, &group_table);
       const size_t chunks_per_row = static_cast<size_t>(p.n) / 4;
       const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(blockIdx.x) * 128 + (threadIdx.x - 64);

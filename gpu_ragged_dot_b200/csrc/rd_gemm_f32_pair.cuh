@@ -100,6 +100,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ __align__(8) uint64_t bar_acc_empty[2];  // leader's is used
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
+  __shared__ GroupTable group_table;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -110,6 +111,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
+    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -130,6 +132,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<2>(smem_u32(&tmem_slot), 2 * BN);
     tmem_relinquish<2>();
   }
+  if (warp == 2 && p.inline_groups) build_group_table(p, 2 * kTileM, &group_table, lane);
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync();  // the peer's barriers exist before anything arrives on them
@@ -138,12 +141,12 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile WaitCtl* abort_ptr = &wait_ctl;
 
   const int num_tiles =
-      kTgmm ? p.g * p.k_tiles * p.n_tiles : imin(p.totals[0], p.max_m_tiles) * p.n_tiles;
+      kTgmm ? p.g * p.k_tiles * p.n_tiles : live_row_tiles(p, &group_table) * p.n_tiles;
   const int tile_start = static_cast<int>(blockIdx.x >> 1);
   const int tile_step = static_cast<int>(gridDim.x >> 1);
   const int k_blocks_gmm = (p.k + kF32TileK - 1) / kF32TileK;
   auto decode = [&](int tile) -> TileCoord {
-    return kTgmm ? decode_tgmm_tile<BN, 2>(p, tile, cta_rank) : decode_gmm_tile<BN, 2>(p, tile, cta_rank);
+    return kTgmm ? decode_tgmm_tile<BN, 2>(p, &group_table, tile, cta_rank) : decode_gmm_tile<BN, 2>(p, &group_table, tile, cta_rank);
   };
   auto blocks_of = [&](const TileCoord& t) -> int {
     return kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
@@ -502,7 +505,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     __syncwarp();
 
     if (!kTgmm && p.zero_tail) {
-      const int first = imin(imax(p.totals[1], 0), p.m);
+      const int first = first_dead_row(p, &group_table);
       const size_t chunks_per_row = static_cast<size_t>(p.n) / 4;
       const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(blockIdx.x) * 128 + (threadIdx.x - 64);

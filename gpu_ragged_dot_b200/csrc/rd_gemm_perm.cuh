@@ -131,7 +131,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
         const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
         for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % kStages;
@@ -187,7 +187,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t it = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
       const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
       long long arow[kGmmRows];  // gmm: byte offsets of this thread's rows of the tile (-1: no row)
       if (!kTgmm && gather_a) {
@@ -300,7 +300,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t local_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
       const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
       const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
       const uint32_t acc = local_tile & 1u;
@@ -372,7 +372,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, tile, 0) : decode_gmm_tile<BN, 1>(p, tile, 0);
+      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
       const int n0 = t.n0;
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;

@@ -1279,3 +1279,27 @@ def test_gmm_fp8_on_256_row_tiles():
         want = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale, cfg=_lib.TileCfg(256, 0, 0, 128, 0))
         got = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale)
         assert torch.equal(got, want) and float(got[-1].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("g", [1, 31, 255, 256, 257])
+@pytest.mark.parametrize("excess", [0, 40])
+def test_groups_in_shared_memory_or_by_metadata_kernel(g, excess):
+    """Up to 256 groups the GEMM kernels make their own group table; the same groups padded with empty
+    ones to 300 go through the metadata kernel: bit-equal, with groups that share a tile, groups
+    past m (sum of the sizes above m) and repeated weights, for every tile height."""
+    k, n, weights = 72, 136, 5
+    rng = np.random.default_rng(g)
+    sizes = rng.multinomial(4 * g + 700, rng.dirichlet(np.full(g, 0.3))).astype(np.int32)
+    m = int(sizes.sum()) - excess + (9 if excess == 0 else 0)
+    padded = np.concatenate([sizes, np.zeros(300 - g, dtype=np.int32)])
+    to_w = rng.integers(0, weights, size=300).astype(np.int32)
+    x, A, dout = _inputs(3, m, k, n, weights)
+    xd, Ad, dd = _to_dev(x, A, dout)
+    gs, gs_p, tw = (torch.from_numpy(a).to(DEV) for a in (sizes, padded, to_w))
+    for cfg in (None, _lib.TileCfg(256, 0, 1, 256, 0), _lib.TileCfg(256, 0, 2, 128, 0)):
+        y = ops.gmm_forward(xd, Ad, gs, cfg=cfg, group_to_weight=tw[:g])
+        assert torch.equal(y, ops.gmm_forward(xd, Ad, gs_p, cfg=cfg, group_to_weight=tw))
+        out = ops.tgmm_forward(xd, dd, gs, cfg=cfg)
+        assert torch.equal(out, ops.tgmm_forward(xd, dd, gs_p, cfg=cfg)[:g])
+    y32 = ops.gmm_forward(xd.float(), Ad.float(), gs, group_to_weight=tw[:g])
+    assert torch.equal(y32, ops.gmm_forward(xd.float(), Ad.float(), gs_p, group_to_weight=tw))
