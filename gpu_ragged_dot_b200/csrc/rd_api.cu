@@ -16,6 +16,7 @@
 #include "rd_gemm_f32.cuh"
 #include "rd_gemm_f32_pair.cuh"
 #include "rd_gemm_perm.cuh"
+#include "rd_gemm_splitk.cuh"
 #include "rd_metadata.cuh"
 #include "rd_rows.cuh"
 
@@ -375,6 +376,85 @@ int launch_gemm_f32_pair(bool split, const CUtensorMap& ta, const CUtensorMap& t
                       rd::f32_pair_smem_bytes<false>(), ta, tb, tout, args, ctas, stream);
 }
 
+// Cluster size for a gmm whose tiles are too few for the SMs (rd_gemm_splitk.cuh), 1 = no split.
+// `tiles` bounds the live tiles.  All clusters must be resident at once and every CTA gets at least
+// four 64-deep blocks.
+template <bool kBKMajor, bool kFp8>
+int choose_split(long long tiles, int k_blocks) {
+  const int sms = sm_count();
+  if (tiles <= 0 || tiles * 2 > sms || k_blocks < 8) return 1;
+  static std::mutex mu;
+  static int fit[64][rd::kMaxSplit + 1];  // clusters of each size that fit, + 1; 0 = not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  auto kernel = rd::ragged_gemm_splitk_kernel<kBKMajor, kFp8>;
+  std::lock_guard<std::mutex> lock(mu);
+  for (int s = rd::kMaxSplit; s >= 2; --s) {
+    if (tiles * s > sms || k_blocks < 4 * s) continue;
+    if (fit[dev][s] == 0) {
+      cudaLaunchConfig_t lc = {};
+      lc.blockDim = dim3(rd::kGemmThreads, 1, 1);
+      lc.gridDim = dim3(s, 1, 1);
+      lc.dynamicSmemBytes = rd::kSplitSmemBytes;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = s;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      lc.attrs = attr;
+      lc.numAttrs = 1;
+      int clusters = 0;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kSplitSmemBytes) !=
+              cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, kernel, &lc) != cudaSuccess) {
+        (void)cudaGetLastError();
+        clusters = 0;
+      }
+      fit[dev][s] = clusters + 1;
+    }
+    if (tiles <= fit[dev][s] - 1) return s;
+  }
+  return 1;
+}
+
+template <bool kBKMajor, bool kFp8>
+int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args, int split, int tiles,
+                       cudaStream_t stream) {
+  auto kernel = rd::ragged_gemm_splitk_kernel<kBKMajor, kFp8>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kSplitSmemBytes) !=
+      cudaSuccess)
+    return RD_ERR_LAUNCH;
+  cudaLaunchConfig_t lc = {};
+  lc.blockDim = dim3(rd::kGemmThreads, 1, 1);
+  lc.gridDim = dim3(split * tiles, 1, 1);
+  lc.dynamicSmemBytes = rd::kSplitSmemBytes;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  if (cudaLaunchKernelEx(&lc, kernel, ta, tb, args, split) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return RD_ERR_LAUNCH;
+  }
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
+// Upper bound on the live 128 x 256 tiles of a gmm: a group has at least one row, and only whole
+// 128-row steps of m add tiles to that.
+long long split_tiles_bound(int m, int g, int n) {
+  const long long row_tiles = (m < g ? m : g) + m / rd::kTileM;
+  return row_tiles * ((n + rd::kSplitBN - 1) / rd::kSplitBN);
+}
+
+// Only calls that leave the tile and the grid to the library are split.
+bool split_allowed(const rd_tile_cfg* cfg) {
+  return cfg == nullptr || (cfg->tile_n == 0 && cfg->max_ctas == 0 && cfg->cta_group == 0 && cfg->tile_m == 0);
+}
+
 // 256-row tiles on one CTA (rd_gemm2.cuh) move a third less data per flop than 128-row tiles.
 // They pay off when a tile's second half usually exists: tgmm with k >= 256, and gmm when the
 // groups are long (mean rows per group >= 512; a half without rows is skipped, so the cost of a
@@ -550,6 +630,14 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
   const bool in_kernel = inline_groups(m, g) && ready.flags == nullptr && send == nullptr &&
                          !(by_weight && group_to_weight != nullptr);
+  const long long split_tiles = split_tiles_bound(m, g, n);
+  int split = 1;
+  if (in_kernel && !f32 && !two_half && cta_group == 1 && split_allowed(cfg)) {
+    const int k_blocks = (k + rd::kTileK - 1) / rd::kTileK;
+    split = trans_rhs ? choose_split<true, false>(split_tiles, k_blocks)
+                      : choose_split<false, false>(split_tiles, k_blocks);
+    if (split > 1) bn = rd::kSplitBN;
+  }
   if (in_kernel) {
     rc = ensure_context();
     if (rc != RD_OK) return rc;
@@ -630,6 +718,9 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
     if (bn == 128) return launch_gemm_f32<128, false, false>(ta, tb, tout, args, ctas, stream);
     return launch_gemm_f32<64, false, false>(ta, tb, tout, args, ctas, stream);
   }
+  if (split > 1)
+    return trans_rhs ? launch_gemm_splitk<true, false>(ta, tb, args, split, static_cast<int>(split_tiles), stream)
+                     : launch_gemm_splitk<false, false>(ta, tb, args, split, static_cast<int>(split_tiles), stream);
   if (two_half) {
     return trans_rhs ? launch_gemm2<true, false>(ta, tb, tout, args, ctas, stream)
                      : launch_gemm2<false, false>(ta, tb, tout, args, ctas, stream);
@@ -1348,6 +1439,11 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
 
   const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
   const bool in_kernel = inline_groups(m, g) && !(by_weight && group_to_weight != nullptr);
+  const long long split_tiles = split_tiles_bound(m, g, n);
+  const int split = in_kernel && !two_half && split_allowed(cfg)
+                        ? choose_split<true, true>(split_tiles, (k / 2 + rd::kTileK - 1) / rd::kTileK)
+                        : 1;
+  if (split > 1) bn = rd::kSplitBN;
   if (in_kernel) {
     rc = ensure_context();
     if (rc != RD_OK) return rc;
@@ -1398,6 +1494,7 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   args.inline_groups = in_kernel ? 1 : 0;
   args.group_to_weight = group_to_weight;
   const int ctas = pick_ctas(cfg);
+  if (split > 1) return launch_gemm_splitk<true, true>(ta, tb, args, split, static_cast<int>(split_tiles), stream);
   if (two_half) return launch_gemm2_fp8(ta, tb, tout, args, ctas, stream);
   if (bn == 256) return launch_gemm<256, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);
   if (bn == 128) return launch_gemm<128, true, false, 1, false, true>(ta, tb, tout, args, ctas, stream);

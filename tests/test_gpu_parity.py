@@ -1303,3 +1303,36 @@ def test_groups_in_shared_memory_or_by_metadata_kernel(g, excess):
         assert torch.equal(out, ops.tgmm_forward(xd, dd, gs_p, cfg=cfg)[:g])
     y32 = ops.gmm_forward(xd.float(), Ad.float(), gs, group_to_weight=tw[:g])
     assert torch.equal(y32, ops.gmm_forward(xd.float(), Ad.float(), gs_p, group_to_weight=tw))
+
+
+# ------------------------------------------------------------------ few tiles: contraction shared by a cluster
+@pytest.mark.parametrize("m,k,n,sizes", [
+    (1, 512, 8, [1]),                                    # one row, one chunk of columns, two CTAs
+    (4, 4096, 1544, [0, 1, 0, 2, 1, 0]),                 # last tile of 8 columns; empty groups
+    (3, 1096, 260 * 2, [1, 1]),                          # k not a multiple of a stage, an unowned row
+    (200, 2056, 256, [65, 129]),                         # M = 64 and M = 128 tiles, unowned rows
+    (130, 8192, 96, [64, 0, 66]),                        # n below a tile
+])
+def test_split_contraction(m, k, n, sizes):
+    """Split and whole contraction agree within the oracle's tolerance and to fp32 summation order (one
+    16-bit rounding apart), twice the same bits, for both weight layouts and e4m3."""
+    g = len(sizes)
+    x, A, _ = _inputs(21, m, k, n, g)
+    gs = torch.tensor(sizes, dtype=torch.int32)
+    xd, Ad, gd = _to_dev(x, A, gs)
+    At = Ad.transpose(1, 2).contiguous()
+    whole = _lib.TileCfg(0, 0, 1, 0, 0)
+    auto = _lib.TileCfg(0, 0, 0, 0, 0)
+    for w, trans in ((Ad, False), (At, True)):
+        y = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto)
+        assert torch.equal(y, ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto))
+        _assert_close(y.cpu(), oracle.ragged_dot(x, A, gs), "split")
+        ref = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=whole).float()
+        scale = float(ref.abs().max())
+        assert float((y.float() - ref).abs().max()) <= 2.0 ** -7 * scale
+    if k % 16 == 0:
+        x8, A8 = xd.to(torch.float8_e4m3fn), At.to(torch.float8_e4m3fn)
+        sc = torch.rand(g, device=DEV) + 0.5
+        y = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc)
+        ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=whole).float()
+        assert float((y.float() - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
