@@ -139,6 +139,15 @@ SIGNATURES = {
         + [_c_int] * 5
         + [ctypes.POINTER(TileCfg), _c_void_p],
     ),
+    "rd_unaligned_scratch_bytes": (_c_size_t, [ctypes.c_longlong, _c_int, ctypes.c_longlong, _c_int]),
+    "rd_gmm_unaligned": (
+        _c_int,
+        [_c_void_p] * 5 + [_c_size_t, _c_void_p, _c_size_t] + [_c_int] * 6 + [_c_void_p],
+    ),
+    "rd_tgmm_unaligned": (
+        _c_int,
+        [_c_void_p] * 5 + [_c_size_t, _c_void_p, _c_size_t] + [_c_int] * 5 + [_c_void_p],
+    ),
     "rd_gather_rows_clamped": (_c_int, [_c_void_p, _c_void_p, _c_void_p] + [_c_int] * 3 + [_c_void_p]),
     "rd_sum_rows_scratch_bytes": (_c_size_t, [_c_int, _c_int]),
     "rd_sum_rows": (

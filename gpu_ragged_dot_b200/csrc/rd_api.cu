@@ -258,6 +258,20 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
 }
 
+// Rows that are not multiples of 16 bytes (see kUnaligned in rd_gemm.cuh).
+template <int BN, bool kBKMajor, bool kTgmm>
+int launch_gemm_unaligned(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args, int ctas,
+                          cudaStream_t stream) {
+  constexpr int kStageBytes = rd::stage_bytes<BN, 1>();
+  constexpr int kStages = (196608 / kStageBytes) > 8 ? 8 : (196608 / kStageBytes);
+  constexpr int kSmem = kStages * kStageBytes + rd::kOutStagingBytes + 1024;
+  auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, 1, false, false, true>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
+    return RD_ERR_LAUNCH;
+  kernel<<<ctas, rd::kGemmFixerThreads, kSmem, stream>>>(ta, tb, ta, args);
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
 template <int BN, bool kBKMajor, bool kTgmm>
 int launch_gemm_f32(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
                     const GemmArgs& args, int ctas, cudaStream_t stream) {
@@ -1188,6 +1202,162 @@ int rd_tgmm_strided(const void* x, const void* dout, const int32_t* group_sizes,
                     int dtype, const rd_tile_cfg* cfg, void* stream) {
   return tgmm_impl(x, dout, group_sizes, out, workspace, workspace_bytes, m, k, n, g, seg_count, dtype, cfg,
                    stream);
+}
+
+// ------------------------------------------------------------------ rows that are not multiples of 16 bytes
+namespace {
+
+// Tiled map, 128-byte swizzle, over `mats` row-major 16-bit matrices [rows, cols] whose rows are
+// `pitch` elements apart (a multiple of 8); zero fill outside.
+int encode_pitched_map(CUtensorMap* map, const void* base, int dtype, int cols, int rows, int mats, int pitch,
+                       uint32_t box_cols, uint32_t box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return RD_ERR_DRIVER;
+  const cuuint64_t row_bytes = static_cast<cuuint64_t>(pitch) * 2;
+  cuuint64_t gdims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(mats)};
+  cuuint64_t gstrides[2] = {row_bytes, row_bytes * static_cast<cuuint64_t>(rows)};
+  cuuint32_t gbox[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r =
+      fn(map, dtype == RD_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+         mats > 0 ? 3 : 2, const_cast<void*>(base), gdims, gstrides, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? RD_OK : RD_ERR_TENSOR_MAP;
+}
+
+bool tma_rows(const void* p, int cols) { return (cols & 7) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+int padded_cols(int cols) { return (cols + 7) & ~7; }
+
+// Copies whichever of the two matrices TMA cannot read into scratch, in one launch; the pointers
+// returned are what the tensor maps start at.
+int repitch_operands(const void** a, long long a_rows, int a_cols, const void** b, long long b_rows, int b_cols,
+                     void* scratch, size_t scratch_bytes, cudaStream_t stream) {
+  rd::Repitch ra = {}, rb = {};
+  uint8_t* next = static_cast<uint8_t*>(scratch);
+  size_t used = 0;
+  auto plan = [&](rd::Repitch& r, const void** p, long long rows, int cols) {
+    if (tma_rows(*p, cols)) return;
+    r.src = static_cast<const uint16_t*>(*p);
+    r.dst = reinterpret_cast<uint4*>(next + used);
+    r.cols = cols;
+    r.vecs_per_row = padded_cols(cols) / 8;
+    r.vecs = rows * r.vecs_per_row;
+    *p = r.dst;
+    used += static_cast<size_t>(r.vecs) * 16;
+  };
+  plan(ra, a, a_rows, a_cols);
+  plan(rb, b, b_rows, b_cols);
+  if (used == 0) return RD_OK;
+  if (!aligned16(scratch)) return RD_ERR_BAD_POINTER;
+  if (used > scratch_bytes) return RD_ERR_WORKSPACE;
+  const long long vecs = ra.vecs + rb.vecs;
+  long long blocks = (vecs + rd::kGatherThreads - 1) / rd::kGatherThreads;
+  const long long cap = static_cast<long long>(sm_count()) * 8;
+  if (blocks > cap) blocks = cap;
+  rd::repitch_rows_kernel<<<static_cast<int>(blocks), rd::kGatherThreads, 0, stream>>>(ra, rb);
+  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+}
+
+bool aligned2(const void* p) { return p != nullptr && (reinterpret_cast<uintptr_t>(p) & 1u) == 0; }
+
+}  // namespace
+
+size_t rd_unaligned_scratch_bytes(long long a_rows, int a_cols, long long b_rows, int b_cols) {
+  if (a_rows < 0 || a_cols < 0 || b_rows < 0 || b_cols < 0) return 0;
+  return 2 * (static_cast<size_t>(a_rows) * padded_cols(a_cols) + static_cast<size_t>(b_rows) * padded_cols(b_cols));
+}
+
+int rd_gmm_unaligned(const void* x, const void* A, const int32_t* group_sizes, void* y, void* workspace,
+                     size_t workspace_bytes, void* scratch, size_t scratch_bytes, int m, int k, int n, int g,
+                     int trans_rhs, int dtype, void* stream_v) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (dtype != RD_DTYPE_F16 && dtype != RD_DTYPE_BF16) return RD_ERR_BAD_DTYPE;
+  if (m < 0 || k < 0 || n < 0 || g < 0) return RD_ERR_BAD_SHAPE;
+  if (m == 0 || n == 0) return RD_OK;
+  if (!aligned2(y)) return RD_ERR_BAD_POINTER;
+  if (g == 0 || k == 0) {
+    cudaMemsetAsync(y, 0, static_cast<size_t>(m) * n * 2, stream);
+    return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+  }
+  if (!inline_groups(m, g)) return RD_ERR_BAD_SHAPE;
+  if (!aligned2(x) || !aligned2(A) || group_sizes == nullptr) return RD_ERR_BAD_POINTER;
+  Workspace w;
+  int rc = bind_workspace(workspace, workspace_bytes, m, g, &w);
+  if (rc != RD_OK) return rc;
+  rc = ensure_context();
+  if (rc != RD_OK) return rc;
+  const int a_cols = trans_rhs ? k : n, a_rows = trans_rhs ? n : k;
+  rc = repitch_operands(&x, m, k, &A, static_cast<long long>(g) * a_rows, a_cols, scratch, scratch_bytes, stream);
+  if (rc != RD_OK) return rc;
+  const int bn = n <= 64 ? 64 : 128;
+  CUtensorMap ta, tb;
+  rc = encode_pitched_map(&ta, x, dtype, k, m, 0, padded_cols(k), 64, rd::kTileM);
+  if (rc != RD_OK) return rc;
+  rc = encode_pitched_map(&tb, A, dtype, a_cols, a_rows, g, padded_cols(a_cols), 64, trans_rhs ? bn : 64);
+  if (rc != RD_OK) return rc;
+  GemmArgs args = {};
+  args.m = m; args.k = k; args.n = n; args.g = g;
+  args.n_tiles = (n + bn - 1) / bn;
+  args.max_m_tiles = w.layout.max_tiles;
+  args.ab_format = dtype;
+  args.wait_limit_us = wait_limit_us(nullptr);
+  args.zero_tail = 1;
+  args.inline_groups = 1;
+  args.group_sizes = group_sizes;
+  args.status = w.status();
+  args.out = y;
+  args.groups_per_flag = 1;
+  const int ctas = sm_count();
+  if (trans_rhs)
+    return bn == 64 ? launch_gemm_unaligned<64, true, false>(ta, tb, args, ctas, stream)
+                    : launch_gemm_unaligned<128, true, false>(ta, tb, args, ctas, stream);
+  return bn == 64 ? launch_gemm_unaligned<64, false, false>(ta, tb, args, ctas, stream)
+                  : launch_gemm_unaligned<128, false, false>(ta, tb, args, ctas, stream);
+}
+
+int rd_tgmm_unaligned(const void* x, const void* dout, const int32_t* group_sizes, void* out, void* workspace,
+                      size_t workspace_bytes, void* scratch, size_t scratch_bytes, int m, int k, int n, int g,
+                      int dtype, void* stream_v) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (dtype != RD_DTYPE_F16 && dtype != RD_DTYPE_BF16) return RD_ERR_BAD_DTYPE;
+  if (m < 0 || k < 0 || n < 0 || g < 0) return RD_ERR_BAD_SHAPE;
+  if (g == 0 || k == 0 || n == 0) return RD_OK;
+  if (!aligned2(out)) return RD_ERR_BAD_POINTER;
+  if (m == 0) {
+    cudaMemsetAsync(out, 0, static_cast<size_t>(g) * k * n * 2, stream);
+    return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_LAUNCH;
+  }
+  if (!inline_groups(m, g)) return RD_ERR_BAD_SHAPE;
+  if (!aligned2(x) || !aligned2(dout) || group_sizes == nullptr) return RD_ERR_BAD_POINTER;
+  Workspace w;
+  int rc = bind_workspace(workspace, workspace_bytes, m, g, &w);
+  if (rc != RD_OK) return rc;
+  rc = ensure_context();
+  if (rc != RD_OK) return rc;
+  rc = repitch_operands(&x, m, k, &dout, m, n, scratch, scratch_bytes, stream);
+  if (rc != RD_OK) return rc;
+  const int bn = n <= 64 ? 64 : 128;
+  CUtensorMap ta, tb;
+  rc = encode_pitched_map(&ta, x, dtype, k, m, 0, padded_cols(k), 64, rd::kTileK);
+  if (rc != RD_OK) return rc;
+  rc = encode_pitched_map(&tb, dout, dtype, n, m, 0, padded_cols(n), 64, rd::kTileK);
+  if (rc != RD_OK) return rc;
+  GemmArgs args = {};
+  args.m = m; args.k = k; args.n = n; args.g = g;
+  args.n_tiles = (n + bn - 1) / bn;
+  args.k_tiles = (k + rd::kTileM - 1) / rd::kTileM;
+  args.seg_count = 1;
+  args.seg_stride = g;
+  args.max_m_tiles = w.layout.max_tiles;
+  args.ab_format = dtype;
+  args.wait_limit_us = wait_limit_us(nullptr);
+  args.inline_groups = 1;
+  args.group_sizes = group_sizes;
+  args.status = w.status();
+  args.out = out;
+  const int ctas = sm_count();
+  return bn == 64 ? launch_gemm_unaligned<64, false, true>(ta, tb, args, ctas, stream)
+                  : launch_gemm_unaligned<128, false, true>(ta, tb, args, ctas, stream);
 }
 
 int rd_gmm_permuted(const void* x, int x_rows, const int32_t* in_rows, const void* A, int num_weights,

@@ -392,7 +392,11 @@ constexpr int stage_bytes() {
 //                  kBKMajor (trans_rhs: W[g] is [n,k]) else MN-major (W[g] is [k,n]).
 // kTgmm == true  : tgmm.  A operand = x^T tile (MN-major), B operand = dout tile (MN-major);
 //                  kBKMajor must be false.
-template <int BN, bool kBKMajor, int kStages, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false>
+// kUnaligned: rows of the output are not multiples of 16 bytes (n odd, say).  Operands come through
+// maps whose rows have a pitch of their own; the output is staged as usual and stored element
+// by element, a warp covering 32 consecutive columns of a row at a time.
+template <int BN, bool kBKMajor, int kStages, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false,
+          bool kUnaligned = false>
 __global__ void __launch_bounds__(kGemmFixerThreads, 1)
 ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                    const __grid_constant__ CUtensorMap tmap_b,
@@ -406,6 +410,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   // GemmArgs::k describe); only the MMA kind differs, 32 elements = 32 bytes per instruction, and
   // the epilogue multiplies by the weight matrix's scale.  Output is bf16.
   static_assert(!kFp8 || (kBKMajor && !kTgmm && kCtas == 1), "8-bit inputs: gmm with K-major weights, one CTA");
+  static_assert(!kUnaligned || (kCtas == 1 && !kSeg && !kFp8), "unaligned rows: plain 16-bit products, one CTA");
   constexpr bool kPair = kCtas == 2;
   constexpr int kBCols = BN / kCtas;  // B-operand columns this CTA loads
   constexpr uint32_t kABytes = kTileM * kTileK * 2;
@@ -804,7 +809,35 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           o[q].z = pack2(__uint_as_float(v[q * 8 + 4]), __uint_as_float(v[q * 8 + 5]), p.ab_format);
           o[q].w = pack2(__uint_as_float(v[q * 8 + 6]), __uint_as_float(v[q * 8 + 7]), p.ab_format);
         }
-        if (slab_by_tma) {
+        if constexpr (kUnaligned) {
+          const uint32_t row_addr = staging + lane * 128;
+          __syncwarp();  // the previous chunk has been read out
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t a = row_addr + (((q ^ (lane & 7)) & 7) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(o[q].x),
+                         "r"(o[q].y), "r"(o[q].z), "r"(o[q].w)
+                         : "memory");
+          }
+          __syncwarp();
+          const uint32_t rows_ok = __ballot_sync(0xffffffffu, row_ok);
+          const size_t row_of = static_cast<size_t>(kTgmm ? t.group : 0) * p.k + out_row0;
+#pragma unroll 4
+          for (int rr = 0; rr < 32; ++rr) {
+            if (!((rows_ok >> rr) & 1u)) continue;
+            uint16_t* dst = out16 + (row_of + rr) * static_cast<size_t>(p.n) + col;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int cc = h * 32 + lane;
+              uint16_t val;
+              asm volatile("ld.shared.u16 %0, [%1];"
+                           : "=h"(val)
+                           : "r"(staging + rr * 128 + ((((cc >> 3) ^ (rr & 7)) & 7) << 4) + (cc & 7) * 2)
+                           : "memory");
+              if (col + cc < p.n) dst[cc] = val;
+            }
+          }
+        } else if (slab_by_tma) {
           const uint32_t buf = staging + (boxes_stored & 1u) * kOutBoxBytes;
           // The box stored two boxes ago used this buffer: wait until TMA has read it out.
           if (lane == 0) bulk_wait_group_read<1>();
@@ -858,10 +891,14 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       // Rows past sum(group_sizes) belong to no group: jax.lax.ragged_dot defines them as 0
       // (the reference writes them from its last live program, gpu_ragged_dot.py:155-165).
       const int first = first_dead_row(p, &group_table);
-      const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
-      const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(cta_index) * 128 + (threadIdx.x - 64);
       const size_t stride = static_cast<size_t>(gemm_ctas) * 128;
+      if constexpr (kUnaligned) {
+        const size_t end = static_cast<size_t>(p.m) * p.n;
+        for (size_t i = static_cast<size_t>(first) * p.n + tid; i < end; i += stride) out16[i] = 0;
+      }
+      const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
+      const size_t total = kUnaligned ? 0 : static_cast<size_t>(p.m - first) * chunks_per_row;
       uint4* dst = reinterpret_cast<uint4*>(out16 + static_cast<size_t>(first) * p.n);
       const uint4 z = make_uint4(0u, 0u, 0u, 0u);
       for (size_t i = tid; i < total; i += stride) dst[i] = z;

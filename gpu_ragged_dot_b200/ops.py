@@ -45,6 +45,12 @@ __all__ = [
     "BlockSizes",
 ]
 
+# Elements of the three tensors up to which rows that are not multiples of 16 bytes take the route of
+# _use_unaligned.  Microseconds of a gmm, padded against this: 0.1 M 89 -> 29 (host time), 10 M 58 -> 38,
+# 55 M 186 -> 88, 155 M 501 -> 197; its 128 x 128 tiles lose on long groups beyond that.
+_UNALIGNED_MAX_ELEMENTS = 1 << 26
+_UNALIGNED_MAX_ROWS = 1 << 20
+
 DEFAULT_BLOCK_M = 64
 DEFAULT_BLOCK_N = 64
 DEFAULT_BLOCK_K = 64
@@ -162,6 +168,20 @@ def make_group_metadata(group_sizes: torch.Tensor, m: int, chunk_m: int) -> GMMG
     return GMMGroupLookupMetadata(gs, offsets, it2group, it2it, total)
 
 
+def _use_unaligned(elements: int, m: int, g: int, dtype: torch.dtype, *row_lengths: int) -> bool:
+    """Small 16-bit products with rows that are not multiples of 16 bytes: ``rd_gmm_unaligned`` /
+    ``rd_tgmm_unaligned`` (two launches) instead of padding with torch, the plain kernel and a copy
+    of the result."""
+    return (dtype != torch.float32 and g <= 256 and m <= _UNALIGNED_MAX_ROWS and elements <= _UNALIGNED_MAX_ELEMENTS
+            and any(r % 8 for r in row_lengths))
+
+
+def _unaligned_scratch(lib, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
+    nbytes = lib.rd_unaligned_scratch_bytes(a.numel() // max(a.shape[-1], 1), a.shape[-1],
+                                            b.numel() // max(b.shape[-1], 1), b.shape[-1])
+    return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=a.device)
+
+
 def gmm_forward(
     x: torch.Tensor,
     A: torch.Tensor,
@@ -197,6 +217,24 @@ def gmm_forward(
     n = A.shape[-1] if not trans_rhs else A.shape[-2]
     k_rhs = A.shape[-2] if not trans_rhs else A.shape[-1]
     assert k_rhs == k, f"contraction mismatch: x has k={k}, A has {k_rhs}"
+
+    if (cfg is None and group_to_weight is None
+            and _use_unaligned(m * k + A.numel() + m * n, m, g, x.dtype, k, n)):
+        x, A = x.contiguous(), A.contiguous()
+        y = out if out is not None else torch.empty((m, n), dtype=x.dtype, device=x.device)
+        assert y.shape == (m, n) and y.dtype == x.dtype
+        res = y if y.is_contiguous() else torch.empty_like(y, memory_format=torch.contiguous_format)
+        ws = workspace if workspace is not None else _workspace(m, g, x.device)
+        scratch = _unaligned_scratch(lib, x, A)
+        with torch.cuda.device(x.device):
+            rc = lib.rd_gmm_unaligned(
+                x.data_ptr(), A.data_ptr(), gs.data_ptr(), res.data_ptr(), ws.data_ptr(), ws.numel(),
+                scratch.data_ptr(), scratch.numel(), m, k, n, g, int(bool(trans_rhs)), _DTYPE_CODE[x.dtype],
+                _stream_ptr(x.device),
+            )
+        _lib.check(rc, "rd_gmm_unaligned")
+        _maybe_check_status(ws, "rd_gmm_unaligned")
+        return res if res is y else y.copy_(res)
 
     # TMA needs 16-byte row strides: pad k and n up to multiples of 16 bytes with zeros (exact).
     mult = 16 // x.element_size()
@@ -521,6 +559,21 @@ def tgmm_forward(
     (m, k), n = x.shape, y.shape[-1]
     assert seg_count >= 1 and gs.numel() % seg_count == 0
     g = gs.numel() // seg_count
+    if cfg is None and seg_count == 1 and _use_unaligned(m * k + m * n + g * k * n, m, g, x.dtype, k, n):
+        x, y = x.contiguous(), y.contiguous()
+        res = out if out is not None else torch.empty((g, k, n), dtype=x.dtype, device=x.device)
+        assert res.shape == (g, k, n) and res.dtype == x.dtype
+        dst = res if res.is_contiguous() else torch.empty_like(res, memory_format=torch.contiguous_format)
+        ws = workspace if workspace is not None else _workspace(m, g, x.device)
+        scratch = _unaligned_scratch(lib, x, y)
+        with torch.cuda.device(x.device):
+            rc = lib.rd_tgmm_unaligned(
+                x.data_ptr(), y.data_ptr(), gs.data_ptr(), dst.data_ptr(), ws.data_ptr(), ws.numel(),
+                scratch.data_ptr(), scratch.numel(), m, k, n, g, _DTYPE_CODE[x.dtype], _stream_ptr(x.device),
+            )
+        _lib.check(rc, "rd_tgmm_unaligned")
+        _maybe_check_status(ws, "rd_tgmm_unaligned")
+        return dst if dst is res else res.copy_(dst)
     mult = 16 // x.element_size()
     xp = _dense16(_pad_last(x, mult))
     yp = _dense16(_pad_last(y, mult))

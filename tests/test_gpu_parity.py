@@ -1336,3 +1336,43 @@ def test_split_contraction(m, k, n, sizes):
         y = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc)
         ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=whole).float()
         assert float((y.float() - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
+
+
+# ------------------------------------------------------------------ rows that are not multiples of 16 bytes
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k,n,sizes", [
+    (1, 1, 1, [1]),
+    (171, 58, 77, [30, 0, 40, 1, 49]),     # unowned rows
+    (300, 63, 65, [129, 64, 107]),         # one off a box in either direction
+    (257, 129, 64, [255, 1]),              # only k unaligned; both tile heights
+    (130, 64, 131, [0, 0, 130]),           # only n unaligned; empty groups
+    (400, 513, 259, [17, 383]),
+])
+def test_unaligned_rows(dtype, m, k, n, sizes):
+    """Small products whose rows TMA cannot read, against the oracle and bit for bit against the padded
+    route, also from tensors that start at an odd element."""
+    g = len(sizes)
+    x, A, dout = _inputs(33, m, k, n, g, dtype=dtype)
+    gs = torch.tensor(sizes, dtype=torch.int32)
+    total = int(gs.sum())
+    xd, Ad, dd, gd = _to_dev(x, A, dout, gs)
+    At = Ad.transpose(1, 2).contiguous()
+    off = torch.empty(x.numel() + 1, dtype=dtype, device=DEV)
+    xo = off[1:].view(m, k)
+    xo.copy_(xd)
+    padded = _lib.TileCfg(0, 0, 0, 128, 0)  # a caller's tile choice takes the padded route
+    for xi in (xd, xo):
+        y = ops.gmm_forward(xi, Ad, gd)
+        assert torch.equal(y, ops.gmm_forward(xi, Ad, gd, cfg=padded))
+        out = ops.tgmm_forward(xi, dd, gd)
+        assert torch.equal(out, ops.tgmm_forward(xi, dd, gd, cfg=padded))
+    yt = ops.gmm_forward(xd, At, gd, trans_rhs=True)
+    assert torch.equal(yt, y)
+    dx = ops.gmm_forward(dd, Ad, gd, trans_rhs=True)
+    assert torch.equal(dx, ops.gmm_forward(dd, Ad, gd, trans_rhs=True, cfg=padded))
+    _assert_close(y.cpu(), oracle.ragged_dot(x, A, gs), "y")
+    _assert_close(out.cpu(), oracle.trans_ragged_dot(x, dout, gs), "out")
+    if total < m:
+        assert float(y[total:].abs().max()) == 0.0 and float(dx[total:].abs().max()) == 0.0
+    buf = torch.empty((m, n + 3), dtype=dtype, device=DEV)
+    assert torch.equal(ops.gmm_forward(xd, Ad, gd, out=buf[:, :n]), y) and torch.equal(buf[:, :n], y)
