@@ -212,6 +212,24 @@ def load() -> ctypes.CDLL:
         return lib
 
 
+_host = None
+
+
+def host():
+    """The native host path of the torch layer (csrc/rd_torch.cpp), loaded once; raises if it is not built."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _rd_host
+        except ImportError as e:
+            raise RuntimeError(
+                f"{PKG_DIR}/_rd_host.so cannot be loaded ({e}). Run `python -m gpu_ragged_dot_b200.build`."
+            ) from e
+        _host = _rd_host
+    return _host
+
+
 def status_string(code: int) -> str:
     return load().rd_status_string(code).decode()
 

@@ -3,7 +3,8 @@
     python -m gpu_ragged_dot_b200.build [--force]
 
 The shared object lands next to this file as ``librd_b200.so``; nvcc cross-compiles, so no
-GPU is needed to build.
+GPU is needed to build.  ``_rd_host.so`` beside it is the native host path of the torch layer
+(csrc/rd_torch.cpp), linked against it and against torch.
 """
 
 from __future__ import annotations
@@ -16,6 +17,9 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC_DIR = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "librd_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_rd_host.so")
+HOST_SOURCE = os.path.join(CSRC_DIR, "rd_torch.cpp")
+HEADER = os.path.join(PKG_DIR, "..", "include", "ragged_dot_b200.h")
 SOURCES = ["rd_api.cu"]
 
 NVCC_FLAGS = [
@@ -62,5 +66,32 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def build_host(force: bool = False) -> str:
+    """Compile _rd_host.so if it is missing or older than its sources; return its path."""
+    deps = [HOST_SOURCE, HEADER]
+    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           "-DTORCH_EXTENSION_NAME=_rd_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for path in [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", path]
+    cmd += ["-o", HOST_PATH, HOST_SOURCE, f"-L{PKG_DIR}", "-lrd_b200", "-Wl,-rpath,$ORIGIN"]
+    for path in cpp_extension.library_paths():
+        cmd += [f"-L{path}", f"-Wl,-rpath,{path}"]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"g++ failed ({proc.returncode}):\n{proc.stdout}\n{proc.stderr}")
+    return HOST_PATH
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

@@ -168,6 +168,30 @@ def make_group_metadata(group_sizes: torch.Tensor, m: int, chunk_m: int) -> GMMG
     return GMMGroupLookupMetadata(gs, offsets, it2group, it2it, total)
 
 
+def _tensors(x, x_dim: int, w, w_dim: int, group_sizes) -> bool:
+    return (isinstance(x, torch.Tensor) and x.dim() == x_dim and isinstance(w, torch.Tensor) and w.dim() == w_dim
+            and isinstance(group_sizes, torch.Tensor) and group_sizes.dim() == 1)
+
+
+def _native(where: str, fn, op: str, x, w, group_sizes, m_k_n, cfg, *args):
+    """A call of the plain form (nothing given by the caller but operands and perhaps a tile) through the
+    native host path (csrc/rd_torch.cpp), or None when it is not of that form."""
+    if _check_status_enabled():
+        return None
+    if cfg is None and x.dtype != torch.float32:
+        cfg = tile_table.lookup(op, *m_k_n, group_sizes.shape[0])
+    if cfg is None:
+        res = fn(x, w, group_sizes, *args, 0, 0, 0, 0, 0, _UNALIGNED_MAX_ELEMENTS)
+    elif cfg.wait_limit_ms == 0:
+        res = fn(x, w, group_sizes, *args, cfg.tile_n, cfg.cta_group, cfg.tile_m, cfg.max_ctas, cfg.flags,
+                 _UNALIGNED_MAX_ELEMENTS)
+    else:
+        return None
+    if isinstance(res, int):
+        _lib.check(res, where)
+    return res
+
+
 def _use_unaligned(elements: int, m: int, g: int, dtype: torch.dtype, *row_lengths: int) -> bool:
     """Small 16-bit products with rows that are not multiples of 16 bytes: ``rd_gmm_unaligned`` /
     ``rd_tgmm_unaligned`` (two launches) instead of padding with torch, the plain kernel and a copy
@@ -199,6 +223,13 @@ def gmm_forward(
     group i multiplies by A[group_to_weight[i]] and g may differ from A.shape[0].
     With ``ready = (flags int32 tensor, groups_per_flag, epoch)`` it is
     ``rd_gmm_indexed_when_ready``: group i's rows are read once flags[i // groups_per_flag] >= epoch."""
+    if (out is None and workspace is None and group_to_weight is None and ready is None
+            and _tensors(x, 2, A, 3, group_sizes)):
+        m_k_n = (x.shape[0], x.shape[1], A.shape[1 if trans_rhs else 2])
+        y = _native("rd_gmm", _lib.host().gmm, "gmm_t" if trans_rhs else "gmm", x, A, group_sizes, m_k_n, cfg,
+                    bool(trans_rhs))
+        if y is not None:
+            return y
     lib = _lib.load()
     _require_cuda(x, "x")
     _require_cuda(A, "A")
@@ -290,6 +321,14 @@ def gmm_fp8_forward(x: torch.Tensor, A: torch.Tensor, group_sizes: torch.Tensor,
     """``rd_gmm_fp8``: ragged x[m,k] . A[w]^T for e4m3 operands (``torch.float8_e4m3fn``), A stored
     ``[num_weights, n, k]``; fp32 accumulation, times ``weight_scale[w]`` (float32, optional), bf16
     result.  Forward only (an inference path): there is no 8-bit tgmm."""
+    if (out is None and workspace is None and group_to_weight is None and cfg is None
+            and _tensors(x, 2, A, 3, group_sizes) and isinstance(weight_scale, (torch.Tensor, type(None)))
+            and not _check_status_enabled()):
+        y = _lib.host().gmm_fp8(x, A, group_sizes, weight_scale)
+        if isinstance(y, int):
+            _lib.check(y, "rd_gmm_fp8")
+        if y is not None:
+            return y
     lib = _lib.load()
     _require_cuda(x, "x")
     _require_cuda(A, "A")
@@ -549,6 +588,10 @@ def tgmm_forward(
 
     With ``seg_count > 1`` it is ``rd_tgmm_strided``: ``group_sizes`` has ``g * seg_count`` entries
     and block i sums the groups i, i + g, i + 2g, ... (the expert-parallel receive layout)."""
+    if out is None and workspace is None and seg_count == 1 and _tensors(x, 2, y, 2, group_sizes):
+        res = _native("rd_tgmm", _lib.host().tgmm, "tgmm", x, y, group_sizes, (x.shape[0], x.shape[1], y.shape[1]), cfg)
+        if res is not None:
+            return res
     lib = _lib.load()
     _require_cuda(x, "x")
     _require_cuda(y, "y")
@@ -908,6 +951,8 @@ def _gmm_cast(x, A, group_sizes, trans_rhs, compute_dtype, precision):
     ``compute_dtype`` (default: x's type), the product is accumulated in fp32, the result comes
     back in x's type."""
     cd = compute_dtype or x.dtype
+    if x.dtype == cd == A.dtype:
+        return gmm_forward(x, A, group_sizes, trans_rhs, _THREE_PASS if precision == "highest" and cd == torch.float32 else None)
     if cd == torch.float32 and precision == "highest":
         y = gmm_forward(x.to(cd), A.to(cd), group_sizes, trans_rhs=trans_rhs, cfg=_THREE_PASS)
     else:
@@ -917,6 +962,8 @@ def _gmm_cast(x, A, group_sizes, trans_rhs, compute_dtype, precision):
 
 def _tgmm_cast(x, y, group_sizes, compute_dtype, precision):
     cd = compute_dtype or x.dtype
+    if x.dtype == cd == y.dtype:
+        return tgmm_forward(x, y, group_sizes, _THREE_PASS if precision == "highest" and cd == torch.float32 else None)
     if cd == torch.float32 and precision == "highest":
         out = tgmm_forward(x.to(cd), y.to(cd), group_sizes, cfg=_THREE_PASS)
     else:
