@@ -213,10 +213,20 @@ __device__ __forceinline__ int first_dead_row(const GemmArgs& p, const GroupTabl
   return imin(imax(p.inline_groups ? tab->offset[p.g] : p.totals[1], 0), p.m);
 }
 
-// Start of a call: the metadata kernel resets the status words, or the first CTA does.  (A CTA that
-// records an expired wait does so a whole wait limit, at least a millisecond, after it started.)
-__device__ __forceinline__ void reset_status(const GemmArgs& p) {
-  if (p.inline_groups && blockIdx.x == 0) *reinterpret_cast<int4*>(p.status) = make_int4(0, 0, 0, 0);
+// Part of every kernel's set-up, after the barriers and tensor memory and before the block's first
+// barrier.  With inline_groups this launch may have begun while the kernel before it was still
+// running (launch_early in rd_api.cu; what came before this touches nothing another kernel writes):
+// every thread waits for that kernel here.  The next launch may begin once every CTA of this grid
+// has got this far.
+// The first CTA resets the status words, as the metadata kernel does for the other calls.  (A CTA
+// that records an expired wait does so a whole wait limit, at least a millisecond, after it started.)
+__device__ __forceinline__ void start_inline_groups(const GemmArgs& p, int tile_rows, GroupTable* tab, int warp,
+                                                    int lane) {
+  if (!p.inline_groups) return;
+  pdl_wait();
+  pdl_release();
+  if (warp == 2) build_group_table(p, tile_rows, tab, lane);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int4*>(p.status) = make_int4(0, 0, 0, 0);
 }
 
 // gmm tile order: group-major; inside a group the n-tiles are outer and the group's row
@@ -450,7 +460,6 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
-    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -470,7 +479,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<kCtas>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<kCtas>();
   }
-  if (warp == 2 && p.inline_groups) build_group_table(p, kTileM * kCtas, &group_table, lane);
+  start_inline_groups(p, kTileM * kCtas, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
   if (kPair) cluster_sync();  // the peer's barriers exist before anything arrives on them

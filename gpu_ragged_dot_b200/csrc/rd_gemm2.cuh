@@ -152,7 +152,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
-    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -172,7 +171,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<kCtas>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<kCtas>();
   }
-  if (warp == 2 && p.inline_groups) build_group_table(p, kTgmm ? kTileM : kG2TileRows, &group_table, lane);
+  start_inline_groups(p, kTgmm ? kTileM : kG2TileRows, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (kPair) cluster_sync();  // the peer's barriers exist before anything arrives on them

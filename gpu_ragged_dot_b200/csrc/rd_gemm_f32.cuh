@@ -94,7 +94,6 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
-    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -112,7 +111,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<1>(smem_u32(&tmem_slot), kTmemCols);
     tmem_relinquish<1>();
   }
-  if (warp == 2 && p.inline_groups) build_group_table(p, kTileM, &group_table, lane);
+  start_inline_groups(p, kTileM, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

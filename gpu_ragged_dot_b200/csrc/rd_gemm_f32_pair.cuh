@@ -111,7 +111,6 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
-    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     tma_prefetch_desc(&tmap_out);
@@ -132,7 +131,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     tmem_alloc<2>(smem_u32(&tmem_slot), 2 * BN);
     tmem_relinquish<2>();
   }
-  if (warp == 2 && p.inline_groups) build_group_table(p, 2 * kTileM, &group_table, lane);
+  start_inline_groups(p, 2 * kTileM, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync();  // the peer's barriers exist before anything arrives on them

@@ -71,7 +71,6 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   if (threadIdx.x == 0) {
     wait_ctl.abort = 0;
     wait_ctl.limit_us = p.wait_limit_us;
-    reset_status(p);
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     for (int s = 0; s < kStages; ++s) {
@@ -85,7 +84,7 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     tmem_alloc<1>(smem_u32(&tmem_slot), BN);
     tmem_relinquish<1>();
   }
-  if (warp == 2) build_group_table(p, kTileM, &group_table, lane);
+  start_inline_groups(p, kTileM, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rd_ptx.cuh"
+
 namespace rd {
 
 constexpr int kGatherThreads = 256;
@@ -61,6 +63,8 @@ struct Repitch {
 
 __global__ void __launch_bounds__(kGatherThreads)
 repitch_rows_kernel(const Repitch a, const Repitch b) {
+  pdl_wait();  // launched early, as the product that follows it
+  pdl_release();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < a.vecs + b.vecs; i += stride) {
     const bool second = i >= a.vecs;

@@ -1376,3 +1376,58 @@ def test_unaligned_rows(dtype, m, k, n, sizes):
         assert float(y[total:].abs().max()) == 0.0 and float(dx[total:].abs().max()) == 0.0
     buf = torch.empty((m, n + 3), dtype=dtype, device=DEV)
     assert torch.equal(ops.gmm_forward(xd, Ad, gd, out=buf[:, :n]), y) and torch.equal(buf[:, :n], y)
+
+
+def test_launched_before_the_predecessor_ends():
+    """Products that feed one another back to back, each allowed to start before the one before it has
+    finished, in a stream and as a captured graph replayed on new inputs: the bits of the same calls
+    with a synchronisation between them."""
+    g, sizes = 4, torch.tensor([100, 0, 300, 112], dtype=torch.int32)
+    m, k, n = 512, 256, 384
+    x, A, _ = _inputs(41, m, k, n, g)
+    xd, Ad, gd = _to_dev(x, A, sizes)
+    xo = xd[:, :251].contiguous()  # rows that are not multiples of 16 bytes
+    Ao = Ad[:, :251, :].contiguous()
+    xf, Af = xd.float(), Ad.float()
+    x1, w1, g1 = xd[:3].clone(), torch.randn(g, k, 8 * k, device=DEV).to(x.dtype) / k ** 0.5, torch.tensor(
+        [1, 1, 0, 1], dtype=torch.int32, device=DEV)
+
+    def chain(sync):
+        res = []
+
+        def step(fn, *args, **kw):
+            res.append(fn(*args, **kw))
+            if sync:
+                torch.cuda.synchronize()
+            return res[-1]
+
+        for _ in range(3):
+            y = step(ops.gmm_forward, xd, Ad, gd)
+            dx = step(ops.gmm_forward, y, Ad, gd, trans_rhs=True)
+            dA = step(ops.tgmm_forward, dx, y, gd)
+            step(ops.gmm_forward, dx, dA, gd)
+            yo = step(ops.gmm_forward, xo, Ao, gd)
+            step(ops.tgmm_forward, xo, yo, gd)
+            yf = step(ops.gmm_forward, xf, Af, gd)
+            step(ops.tgmm_forward, xf, yf, gd, cfg=ops._THREE_PASS)
+            h = step(ops.gmm_forward, x1, w1, g1)
+            step(ops.gmm_forward, h, w1, g1, trans_rhs=True)
+        return res
+
+    want = chain(True)
+    for a, b in zip(chain(False), want):
+        assert torch.equal(a, b)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain(False)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(False)
+    xd.mul_(2.0)  # exact: everything computed from xd alone doubles
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0] * 2) and torch.equal(got[1], want[1] * 2)
+    assert torch.equal(got[4], want[4]) and torch.equal(got[7], want[7]) and torch.equal(got[9], want[9])
+    graph.reset()
