@@ -17,6 +17,7 @@
 #include "rd_gemm_f32_pair.cuh"
 #include "rd_gemm_perm.cuh"
 #include "rd_gemm_splitk.cuh"
+#include "rd_gemm_swap.cuh"
 #include "rd_metadata.cuh"
 #include "rd_rows.cuh"
 
@@ -69,10 +70,10 @@ int ensure_context() {
   return RD_OK;
 }
 
-// rank-2 or rank-3 tiled map over a dense row-major 16-bit or 32-bit float tensor, 128-byte swizzle,
+// rank-2 or rank-3 tiled map over a dense row-major 16-bit or 32-bit float tensor, 128-byte swizzle (or none),
 // zero fill outside the bounds.  dims / box are innermost first.
 int encode_map(CUtensorMap* map, const void* base, int dtype, int rank, const uint64_t* dims,
-               const uint32_t* box, bool atom32 = false) {
+               const uint32_t* box, bool atom32 = false, bool swizzled = true) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return RD_ERR_DRIVER;
   cuuint64_t gdims[3];
@@ -91,7 +92,9 @@ int encode_map(CUtensorMap* map, const void* base, int dtype, int rank, const ui
                                                          : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUresult r = fn(map, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, gstrides,
                   gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  !swizzled ? CU_TENSOR_MAP_SWIZZLE_NONE
+                  : atom32  ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
+                            : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr,
@@ -409,12 +412,15 @@ int launch_gemm_f32_pair(bool split, const CUtensorMap& ta, const CUtensorMap& t
 }
 
 // Cluster size for a gmm whose tiles are too few for the SMs (rd_gemm_splitk.cuh), 1 = no split.
-// `tiles` bounds the live tiles.  All clusters must be resident at once and every CTA gets at least
-// four 64-deep blocks.
+// `tiles` bounds the live tiles, `rows` is what a large tile may hold.  All clusters must be resident at
+// once and every CTA gets at least four 64-deep blocks.  A block takes a lone CTA 0.3 to 0.4 us;
+// adding the partial sums up costs about 1 us and 10 us more for 128 rows (1024 rows in 2 groups, k
+// 1024, n 1024: 17 us whole, 25 us split; 300 rows in 4 groups, k 8192, n 256: 55 and 27).
 template <bool kBKMajor, bool kFp8>
-int choose_split(long long tiles, int k_blocks) {
+int choose_split(long long tiles, int rows, int k_blocks) {
   const int sms = sm_count();
   if (tiles <= 0 || tiles * 2 > sms || k_blocks < 8) return 1;
+  if (0.3 * k_blocks < 3.0 + 15.0 * rows / rd::kTileM) return 1;
   static std::mutex mu;
   static int fit[64][rd::kMaxSplit + 1];  // clusters of each size that fit, + 1; 0 = not asked yet
   int dev = 0;
@@ -460,11 +466,65 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
                        split);
 }
 
+// Should a gmm put its rows on the N side of the MMAs (rd_gemm_swap.cuh)?  When groups are long, there
+// are at least three rounds of tiles for the pairs and the last 512-column tile is nearly full.
+// Microseconds, one-CTA tiles (better of the two heights) against swapped: m 8192, k 4096, n 14336, 8
+// groups 694 -> 687, trans_rhs with k 14336, n 4096 687 -> 669 (alone; in a row with the backward pass
+// 2.58 -> 2.48 ms a step); 16 unequal groups 816 -> 751; 64 groups of 512, k 4096, n 1536 402 -> 384.
+// Below: 4096, 4096, 4096, 8 (1.7 rounds) 177 -> 212; n 2304 (last tile half full) 160 -> 171; 256 rows
+// per group 288 -> 273 at best, 1058 -> 1160 at worst; 128 rows 222 -> 233.
+bool choose_swap(long long m, int n, int g, bool trans_rhs) {
+  if (g <= 0 || m / g < 512 || (!trans_rhs && n % 64 != 0)) return false;
+  const long long col_tiles = (static_cast<long long>(n) + rd::kSwapCols - 1) / rd::kSwapCols;
+  if ((col_tiles * rd::kSwapCols - n) * 16 > n) return false;
+  return m / rd::kSwapRows * col_tiles >= 3LL * (sm_count() / 2);
+}
+
+// Tensor maps and launch of the swapped kernel; k in 2-byte units (kFp8: half of the elements).
+template <bool kBKMajor, bool kFp8, bool kScatter = false>
+int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_weights, GemmArgs args,
+                     cudaStream_t stream) {
+  CUtensorMap tw, tx, tout;
+  int rc;
+  {
+    const uint64_t dims[2] = {static_cast<uint64_t>(args.k), static_cast<uint64_t>(args.m)};
+    const uint32_t box[2] = {64, rd::kSwapRows / 2};
+    rc = encode_map(&tx, x, dtype, 2, dims, box);
+    if (rc != RD_OK) return rc;
+  }
+  if (kBKMajor) {
+    const uint64_t dims[3] = {static_cast<uint64_t>(args.k), static_cast<uint64_t>(args.n),
+                              static_cast<uint64_t>(num_weights)};
+    const uint32_t box[3] = {64, rd::kSwapCtaCols, 1};
+    rc = encode_map(&tw, A, dtype, 3, dims, box);
+  } else {
+    rc = encode_blocked_map(&tw, A, dtype, args.n, args.k, rd::kTileK, rd::kSwapCtaCols / 64, num_weights);
+  }
+  if (rc != RD_OK) return rc;
+  if (kScatter) {
+    tout = tx;  // rows are stored one by one
+  } else {
+    const uint64_t dims[2] = {static_cast<uint64_t>(args.n), static_cast<uint64_t>(args.m)};
+    const uint32_t box[2] = {32, 32};
+    rc = encode_map(&tout, y, dtype, 2, dims, box, false, /*swizzled=*/false);
+    if (rc != RD_OK) return rc;
+  }
+  args.n_tiles = (args.n + rd::kSwapCols - 1) / rd::kSwapCols;
+  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8, kScatter>, rd::kSwapThreads, rd::kSwapSmemBytes, tw, tx, tout,
+                      args, sm_count(), stream);
+}
+
 // Upper bound on the live 128 x 256 tiles of a gmm: a group has at least one row, and only whole
 // 128-row steps of m add tiles to that.
 long long split_tiles_bound(int m, int g, int n) {
   const long long row_tiles = (m < g ? m : g) + m / rd::kTileM;
   return row_tiles * ((n + rd::kSplitBN - 1) / rd::kSplitBN);
+}
+
+// Rows of a large tile: twice the mean of the groups that can have rows.
+int split_tile_rows(int m, int g) {
+  const long long mean2 = 2LL * m / (m < g ? m : g);
+  return mean2 < rd::kTileM ? static_cast<int>(mean2) : rd::kTileM;
 }
 
 // Only calls that leave the tile and the grid to the library are split.
@@ -474,15 +534,24 @@ bool split_allowed(const rd_tile_cfg* cfg) {
 
 // 256-row tiles on one CTA (rd_gemm2.cuh) move a third less data per flop than 128-row tiles.
 // They pay off when a tile's second half usually exists: tgmm with k >= 256, and gmm when the
-// groups are long (mean rows per group >= 512; a half without rows is skipped, so the cost of a
-// wrong guess is only a shallower smem ring).  At exactly 512 rows per group the picture is mixed:
-// 16 ragged groups over m 8192, k 4096, n 14336 are 5-13 % faster on 128-row tiles, the
-// expert-parallel step (64 segments of about 512 rows over 32 weight matrices) 4 % slower.
+// groups are long (a half without rows is skipped, so the cost of a wrong guess is only a
+// shallower smem ring) -- unless the larger tiles fill the SMs badly.  A 256-row tile takes as long
+// as 1.84 128-row tiles; with fewer than six rounds of tiles the rounds are compared (128 rows against
+// 256, microseconds): m 4096, k 4096, n 4096, g 8 (4 rounds against 3) 177 -> 210; 512, 4096, 4096, 1 (1
+// against 1) 36 -> 52; 8192, 4096, 2304, 8 (5 against 3) 160 -> 169; but 6000, 4096, 1024, 8 (2 against
+// 1) 77 -> 70; 2048, 7168, 2048, 8 (2 against 1) 116 -> 101.  With many rounds 512 rows per group on
+// average is the line: 32768, 1536, 4096, 64 364 -> 335, 8192, 4096, 14336, 32 (256 rows) 1060 -> 1131.
 // e4m3 follows the same rule: m 8192, k 4096, n 14336, 8 groups 390 -> 378 us, 475 -> 466 us in a row.
-bool choose_two_half(bool tgmm, long long m, int k, int g, int bn) {
-  if (bn != 256) return false;
+bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn) {
+  if (bn != 256 || g <= 0) return false;
   if (tgmm) return k >= 256;
-  return g > 0 && m / g >= 512;
+  if (m / g < 256) return false;
+  const int sms = sm_count();
+  const long long n_tiles = (static_cast<long long>(n) + 255) / 256;
+  // a group's last tile is half full on average
+  const long long tiles128 = ((m + 127) / 128 + g / 2) * n_tiles, tiles256 = ((m + 255) / 256 + g / 2) * n_tiles;
+  if (tiles256 >= 6LL * sms) return m / g >= 512;
+  return 1.84 * static_cast<double>((tiles256 + sms - 1) / sms) < static_cast<double>((tiles128 + sms - 1) / sms);
 }
 
 // tgmm with 256-row tiles: 512 x 256 tiles on CTA pairs (a quarter less L2 -> SM traffic, a
@@ -640,7 +709,7 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
     cta_group = pair ? 2 : 1;
     tile_m = 128;
   }
-  if (tile_m == 0) tile_m = (cta_group == 1 && choose_two_half(false, m, k, g, bn)) ? 256 : 128;
+  if (tile_m == 0) tile_m = (cta_group == 1 && choose_two_half(false, m, k, n, g, bn)) ? 256 : 128;
   const bool two_half = tile_m == 256;
 
   // The expert-parallel forms (flags, senders, groups visited by weight) keep the metadata launch.
@@ -651,8 +720,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   int split = 1;
   if (in_kernel && !f32 && !two_half && cta_group == 1 && split_allowed(cfg)) {
     const int k_blocks = (k + rd::kTileK - 1) / rd::kTileK;
-    split = trans_rhs ? choose_split<true, false>(split_tiles, k_blocks)
-                      : choose_split<false, false>(split_tiles, k_blocks);
+    split = trans_rhs ? choose_split<true, false>(split_tiles, split_tile_rows(m, g), k_blocks)
+                      : choose_split<false, false>(split_tiles, split_tile_rows(m, g), k_blocks);
     if (split > 1) bn = rd::kSplitBN;
   }
   if (in_kernel) {
@@ -662,6 +731,21 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
     launch_internal_metadata(group_sizes, group_to_weight, g, m,
                              two_half ? rd::kG2TileRows : rd::kTileM * cta_group, w, stream, by_weight);
     if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  }
+  if (in_kernel && !f32 && split == 1 && split_allowed(cfg) && choose_swap(m, n, g, trans_rhs != 0)) {
+    GemmArgs args = {};
+    args.m = m; args.k = k; args.n = n; args.g = g;
+    args.max_m_tiles = w.layout.max_tiles;
+    args.ab_format = dtype;
+    args.wait_limit_us = wait_limit_us(cfg);
+    args.zero_tail = (cfg && (cfg->flags & RD_CFG_NO_ZERO_TAIL)) ? 0 : 1;
+    args.inline_groups = 1;
+    args.group_to_weight = group_to_weight;
+    args.group_sizes = group_sizes;
+    args.status = w.status();
+    args.out = y;
+    return trans_rhs ? launch_gemm_swap<true, false>(x, A, y, dtype, num_weights, args, stream)
+                     : launch_gemm_swap<false, false>(x, A, y, dtype, num_weights, args, stream);
   }
 
   const bool blocked = f32 && cta_group == 2 && !trans_rhs && n % 32 == 0;
@@ -1091,7 +1175,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   }
   // Preference order when nothing is forced: 256-row tiles on one CTA, then a CTA pair, then
   // plain 128-row tiles.
-  if (tile_m == 0 && cta_group != 2) tile_m = choose_two_half(true, m, k, g, bn) ? 256 : 128;
+  if (tile_m == 0 && cta_group != 2) tile_m = choose_two_half(true, m, k, n, g, bn) ? 256 : 128;
   if (tile_m == 0) tile_m = 128;
   if (cta_group == 0) {
     if (tile_m == 256) {
@@ -1395,6 +1479,27 @@ int rd_gmm_permuted(const void* x, int x_rows, const int32_t* in_rows, const voi
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;
 
+  // Rows in order, results scattered: the swapped kernel, where the plain gmm would use it.
+  if (in_rows == nullptr && out_rows != nullptr && inline_groups(m, g) && split_allowed(cfg) &&
+      choose_swap(m, n, g, trans_rhs != 0)) {
+    rc = ensure_context();
+    if (rc != RD_OK) return rc;
+    GemmArgs args = {};
+    args.m = m; args.k = k; args.n = n; args.g = g;
+    args.max_m_tiles = w.layout.max_tiles;
+    args.ab_format = dtype;
+    args.wait_limit_us = wait_limit_us(cfg);
+    args.inline_groups = 1;
+    args.group_to_weight = group_to_weight;
+    args.group_sizes = group_sizes;
+    args.status = w.status();
+    args.out = y;
+    args.scatter_rows = out_rows;
+    args.scatter_rows_n = y_rows;
+    return trans_rhs ? launch_gemm_swap<true, false, true>(x, A, y, dtype, num_weights, args, stream)
+                     : launch_gemm_swap<false, false, true>(x, A, y, dtype, num_weights, args, stream);
+  }
+
   launch_internal_metadata(group_sizes, group_to_weight, g, m, rd::kTileM, w, stream);
   if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
 
@@ -1608,13 +1713,13 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   int bn = cfg && cfg->tile_n ? cfg->tile_n : choose_tile_n(0, n, 0);
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // the library chooses
-  const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, g, bn);
+  const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, n, g, bn);
 
   const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
   const bool in_kernel = inline_groups(m, g) && !(by_weight && group_to_weight != nullptr);
   const long long split_tiles = split_tiles_bound(m, g, n);
   const int split = in_kernel && !two_half && split_allowed(cfg)
-                        ? choose_split<true, true>(split_tiles, (k / 2 + rd::kTileK - 1) / rd::kTileK)
+                        ? choose_split<true, true>(split_tiles, split_tile_rows(m, g), (k / 2 + rd::kTileK - 1) / rd::kTileK)
                         : 1;
   if (split > 1) bn = rd::kSplitBN;
   if (in_kernel) {
@@ -1624,6 +1729,22 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
     launch_internal_metadata(group_sizes, group_to_weight, g, m, two_half ? rd::kG2TileRows : rd::kTileM, w, stream,
                              by_weight);
     if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
+  }
+
+  if (in_kernel && split == 1 && split_allowed(cfg) && choose_swap(m, n, g, true)) {
+    GemmArgs args = {};
+    args.m = m; args.k = k / 2; args.n = n; args.g = g;
+    args.max_m_tiles = w.layout.max_tiles;
+    args.ab_format = RD_DTYPE_BF16;
+    args.wait_limit_us = wait_limit_us(cfg);
+    args.weight_scale = weight_scale;
+    args.zero_tail = (cfg && (cfg->flags & RD_CFG_NO_ZERO_TAIL)) ? 0 : 1;
+    args.inline_groups = 1;
+    args.group_to_weight = group_to_weight;
+    args.group_sizes = group_sizes;
+    args.status = w.status();
+    args.out = y;
+    return launch_gemm_swap<true, true>(x, A, y, RD_DTYPE_BF16, num_weights, args, stream);
   }
 
   // Both operands are K-major, so a row of k one-byte elements is described to TMA as k/2

@@ -1,0 +1,337 @@
+// gmm with the roles of the operands swapped: the weights' columns are the M side of the MMAs and the
+// ragged rows the N side, on CTA pairs.
+//
+// Two things bound the 256 x 256 tiles of rd_gemm2.cuh on long groups.  Shared memory: a 64-deep
+// stage takes 64 KB of TMA writes and 96 KB of operand reads per 1024 clocks of MMAs, 156 bytes per
+// clock where a shared memory gives 128, so the tensor cores cannot pass 82 % (and every byte
+// costs power, of which a long run of these GEMMs uses all there is).  And rows: M comes in steps of
+// 128, so a group pays for 64 rows on average that are not there.
+// Here a pair of CTAs owns 512 columns x up to 256 rows.  CTA c holds the accumulators of columns [256 c,
+// 256 c + 256) as two 128-lane halves; each half is ONE tcgen05.mma.cta_group::2 with M = 256 (128
+// columns of either CTA) and N = the tile's rows in steps of 32.  Each CTA loads its own columns of
+// the weights (32 KB a stage) and half of the rows (16 KB); shared memory moves 48 KB in and 64 KB
+// out per 1024 clocks.  A group's rows are dealt evenly to ceil(rows / 256) tiles.
+//
+// Measured against the 256 x 256 one-CTA tiles: m 8192, k 4096, n 14336, 8 unequal groups 694 -> 687 us
+// and trans_rhs 687 -> 669 us alone; as part of a training step at the power limit, where less
+// traffic and fewer empty rows mean a higher clock, 2.58 -> 2.48 ms for the step.  64 groups of about 512
+// rows, k 4096, n 1536, fp16: 402 -> 384 us, in a loop 487 -> 449 us.  e4m3 (m 8192, k 4096, n 14336) 466 -> 447 us
+// in a row.  What bounds it now: power; alone, the exposed drain of the accumulators, which fill
+// tensor memory, and the last round of tiles.
+//
+// Accumulator lanes are output columns, so a warp's 32 x 32 block is transposed on its way through
+// shared memory (two-byte stores, 64 contiguous bytes per row) and leaves by TMA; blocks that cross
+// the end of the tile's rows are stored from registers, 64 bytes per row.
+//
+// kScatter: every row goes to a destination of its own, from registers, 64 bytes per row and warp (the MoE
+// layer's un-sort; forward of 4096 tokens, top-2, k 4096, n 14336: gather 19 + product 690 us against 755
+// us for the kernel that gathers row by row).
+//
+// Roles, barriers and waits as in rd_gemm2.cuh (kPair); loads are plain, nothing is broadcast.
+// kFp8: e4m3 operands, K-major weights, tiles byte for byte those of a 16-bit problem.
+#pragma once
+
+#include "rd_gemm2.cuh"
+
+namespace rd {
+
+constexpr int kSwapStages = 4;
+constexpr int kSwapCols = 512;      // output columns of a pair's tile
+constexpr int kSwapCtaCols = 256;   // of one CTA
+constexpr int kSwapRows = 256;      // most rows of a tile
+constexpr uint32_t kSwapABytes = kSwapCtaCols * kTileK * 2;      // 32 KB: weights
+constexpr uint32_t kSwapBBytes = (kSwapRows / 2) * kTileK * 2;   // 16 KB: rows
+constexpr uint32_t kSwapStageBytes = kSwapABytes + kSwapBBytes;  // 48 KB
+constexpr int kSwapEpilogueWarps = 8;
+constexpr int kSwapThreads = 64 + 32 * kSwapEpilogueWarps;
+constexpr uint32_t kSwapBoxBytes = 32 * 64;  // [32 rows][32 columns] of the output
+constexpr int kSwapSmemBytes = kSwapStages * kSwapStageBytes + kSwapEpilogueWarps * 2 * kSwapBoxBytes + 1024;
+
+// The tile's rows [row0, row0 + rows) of its group and the pair's first column.
+struct SwapTile {
+  int weight, row0, rows, n0;
+  int mma_n;  // rows in steps of 32: the N of the MMAs
+};
+
+__device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const GroupTable* tab, int tile) {
+  const RowTile r = find_row_tile(p, tab, tile / p.n_tiles);
+  const int local = tile - r.tile_base * p.n_tiles;
+  const int nt = local / r.tiles;
+  const int mi = local - nt * r.tiles;
+  // equal shares in steps of 32 rows; the last tiles may be shorter, never empty or above 256
+  const int per = ((r.group_size + r.tiles - 1) / r.tiles + 31) & ~31;
+  SwapTile t;
+  t.weight = r.weight;
+  t.row0 = r.group_offset + mi * per;
+  t.rows = imax(imin(per, r.group_size - mi * per), 0);
+  t.mma_n = imax((t.rows + 31) & ~31, 32);
+  t.n0 = nt * kSwapCols;
+  return t;
+}
+
+template <bool kBKMajor, bool kFp8, bool kScatter>
+__global__ void __launch_bounds__(kSwapThreads, 1)
+ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                        const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
+  static_assert(!kFp8 || kBKMajor, "8-bit inputs: K-major weights");
+  constexpr int kStages = kSwapStages;
+  constexpr uint32_t kStageBytes = kSwapStageBytes;
+
+  extern __shared__ uint8_t smem_dyn[];
+  __shared__ __align__(8) uint64_t bar_full[kStages];   // leader's is used
+  __shared__ __align__(8) uint64_t bar_empty[kStages];
+  __shared__ __align__(8) uint64_t bar_acc_full[2];     // per half
+  __shared__ __align__(8) uint64_t bar_acc_empty[2];    // per half, leader's is used
+  __shared__ uint32_t tmem_slot;
+  __shared__ WaitCtl wait_ctl;
+  __shared__ GroupTable group_table;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int cta_rank = static_cast<int>(cluster_cta_rank());
+  const bool leader = cta_rank == 0;
+  const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+
+  if (threadIdx.x == 0) {
+    wait_ctl.abort = 0;
+    wait_ctl.limit_us = p.wait_limit_us;
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+    tma_prefetch_desc(&tmap_out);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(smem_u32(&bar_full[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), 1);
+    }
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(smem_u32(&bar_acc_full[h]), 1);
+      mbar_init(smem_u32(&bar_acc_empty[h]), 8);  // four epilogue warps of either CTA
+    }
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc<2>(smem_u32(&tmem_slot), 512);
+    tmem_relinquish<2>();
+  }
+  start_inline_groups(p, kSwapRows, &group_table, warp, lane);
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync();  // the peer's barriers exist before anything arrives on them
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_slot;
+  volatile WaitCtl* abort_ptr = &wait_ctl;
+
+  const int num_tiles = live_row_tiles(p, &group_table) * p.n_tiles;
+  const int tile_start = static_cast<int>(blockIdx.x >> 1);
+  const int tile_step = static_cast<int>(gridDim.x >> 1);
+  const int k_blocks = (p.k + kTileK - 1) / kTileK;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
+        const SwapTile t = decode_swap_tile(p, &group_table, tile);
+        const int col = t.n0 + cta_rank * kSwapCtaCols;
+        const int row = t.row0 + cta_rank * (t.mma_n >> 1);
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const uint32_t s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1u;
+          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+            ok = false;
+            break;
+          }
+          uint32_t full = smem_u32(&bar_full[s]);
+          const uint32_t sa = stage_base + s * kStageBytes;
+          const uint32_t sb = sa + kSwapABytes;
+          if (leader) {
+            mbar_arrive_expect_tx(full, 2 * kStageBytes);
+            tma_load_2d(sb, &tmap_x, full, kb * kTileK, row);
+            if constexpr (kBKMajor) {
+              tma_load_3d(sa, &tmap_w, full, kb * kTileK, col, t.weight);
+            } else {
+              tma_load_4d(sa, &tmap_w, full, 0, kb * kTileK, col >> 6, t.weight);
+            }
+          } else {
+            full = map_to_cta(full, 0);
+            tma_load_2d_pair(sb, &tmap_x, full, kb * kTileK, row);
+            if constexpr (kBKMajor) {
+              tma_load_3d_pair(sa, &tmap_w, full, kb * kTileK, col, t.weight);
+            } else {
+              tma_load_4d_pair(sa, &tmap_w, full, 0, kb * kTileK, col >> 6, t.weight);
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (one thread)
+    if (lane == 0 && leader) {
+      constexpr uint32_t kAStep = (kBKMajor ? 32u : 2048u) >> 4;
+      constexpr uint32_t kBStep = 32u >> 4;
+      constexpr uint32_t kHalfA = (kBKMajor ? 128u * 128u : 2u * kBoxBytes) >> 4;  // the next 128 columns
+      const uint64_t adesc0 = kBKMajor ? make_smem_desc(stage_base, 16, 1024)
+                                       : make_smem_desc(stage_base, kBoxBytes, 1024);
+      const uint64_t bdesc0 = make_smem_desc(stage_base + kSwapABytes, 16, 1024);
+      const uint32_t adesc0_lo = static_cast<uint32_t>(adesc0);
+      const uint32_t bdesc0_lo = static_cast<uint32_t>(bdesc0);
+      const uint32_t a_hi = static_cast<uint32_t>(adesc0 >> 32);
+      const uint32_t b_hi = static_cast<uint32_t>(bdesc0 >> 32);
+      uint32_t it = 0;
+      uint32_t local_tile = 0;
+      bool ok = true;
+      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
+        const SwapTile t = decode_swap_tile(p, &group_table, tile);
+        const uint32_t idesc =
+            make_idesc_f16(kFp8 ? 0 : p.ab_format, kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n);
+        uint32_t s = it % kStages;
+        uint32_t ph = (it / kStages) & 1u;
+        for (int kb = 0; kb < k_blocks; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
+          if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (kb == 0) {  // the half's accumulator must have been drained by both CTAs
+              if (!mbar_wait<true>(smem_u32(&bar_acc_empty[h]), (local_tile & 1u) ^ 1u, abort_ptr)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after_sync();
+            }
+            const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * kHalfA;
+            const uint32_t tmem_d = tmem_base + h * kSwapRows;
+#pragma unroll
+            for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
+              umma_ab<2, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, a_hi),
+                               make_desc64(b_lo + kk * kBStep, b_hi), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
+          }
+          if (!ok) break;
+          umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue (warps 2..9)
+    const int half = (warp - 2) >> 2;
+    const int quarter = warp & 3;
+    const uint32_t staging = stage_base + kStages * kStageBytes + (warp - 2) * 2 * kSwapBoxBytes;
+    const int col_in_tile = cta_rank * kSwapCtaCols + half * kTileM + quarter * 32;
+    uint32_t local_tile = 0;
+    uint32_t boxes_stored = 0;
+    bool ok = true;
+    uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
+    for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
+      const SwapTile t = decode_swap_tile(p, &group_table, tile);
+      const int col0 = t.n0 + col_in_tile;  // this warp's first output column; lane = column
+      if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), local_tile & 1u, abort_ptr)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      const int chunks = col0 < p.n ? (t.rows + 31) >> 5 : 0;
+      const float sc = kFp8 && p.weight_scale != nullptr ? p.weight_scale[t.weight] : 1.0f;
+      // All rows leave tensor memory first (packed to 16 bits, 16 registers per 32 rows), so that the
+      // next tile's MMAs wait for nothing but the loads below.
+      uint32_t o[kSwapRows / 32][16];
+#pragma unroll
+      for (int c = 0; c < kSwapRows / 32; ++c) {
+        if (c < chunks) {
+          uint32_t v[32];
+          tmem_ld_32x32(tmem_base + half * kSwapRows + c * 32 + (static_cast<uint32_t>(quarter * 32) << 16), v);
+          tmem_ld_wait();
+          if constexpr (kFp8) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * sc);
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            o[c][j] = pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), p.ab_format);
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(smem_u32(&bar_acc_empty[half]), 0);
+#pragma unroll
+      for (int c = 0; c < kSwapRows / 32; ++c) {
+        if (c >= chunks) continue;
+        const int row0 = t.row0 + c * 32;
+        const int rows = t.rows - c * 32;
+        if constexpr (kScatter) {  // 64 contiguous bytes per row, straight from registers
+          int dst_row = lane < rows ? p.scatter_rows[row0 + lane] : -1;
+          if (dst_row >= p.scatter_rows_n) dst_row = -1;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int r = __shfl_sync(0xffffffffu, dst_row, j);
+            if (r >= 0 && col0 + lane < p.n)
+              out16[static_cast<size_t>(r) * p.n + col0 + lane] = static_cast<uint16_t>(o[c][j >> 1] >> (16 * (j & 1)));
+          }
+        } else if (rows >= 32) {
+          const uint32_t buf = staging + (boxes_stored & 1u) * kSwapBoxBytes;
+          if (lane == 0) bulk_wait_group_read<1>();  // the box stored two boxes ago has been read out
+          __syncwarp();
+          const uint32_t a = buf + lane * 2;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            asm volatile(
+                "{\n\t"
+                ".reg .b16 lo, hi;\n\t"
+                "mov.b32 {lo, hi}, %1;\n\t"
+                "st.shared.b16 [%0], lo;\n\t"
+                "st.shared.b16 [%0 + 64], hi;\n\t"
+                "}\n" ::"r"(a + j * 128),
+                "r"(o[c][j])
+                : "memory");
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmap_out, buf, col0, row0);
+            bulk_commit_group();
+          }
+          ++boxes_stored;
+        } else if (col0 + lane < p.n) {  // crosses the end of the tile's rows
+          uint16_t* dst = out16 + static_cast<size_t>(row0) * p.n + col0 + lane;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (j < rows) dst[static_cast<size_t>(j) * p.n] = static_cast<uint16_t>(o[c][j >> 1] >> (16 * (j & 1)));
+          }
+        }
+      }
+    }
+    if (lane == 0) bulk_wait_group<0>();
+    __syncwarp();
+
+    if (p.zero_tail) {
+      constexpr int kEpiThreads = 32 * kSwapEpilogueWarps;
+      const int first = first_dead_row(p, &group_table);
+      const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
+      const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
+      const size_t tid = static_cast<size_t>(blockIdx.x) * kEpiThreads + (threadIdx.x - 64);
+      const size_t stride = static_cast<size_t>(gridDim.x) * kEpiThreads;
+      uint4* dst = reinterpret_cast<uint4*>(out16 + static_cast<size_t>(first) * p.n);
+      const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+      for (size_t i = tid; i < total; i += stride) dst[i] = z;
+    }
+  }
+
+  // ------------------------------------------------------------ tear-down
+  __syncthreads();
+  if (wait_ctl.abort) {
+    if (threadIdx.x == 0) atomicMax(p.status, static_cast<int32_t>(kStatusWaitExpired));
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  cluster_sync();  // neither CTA may leave while the other can still reach its barriers or smem
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc<2>(tmem_base, 512);
+  }
+}
+
+}  // namespace rd

@@ -401,9 +401,21 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
         : "memory");
 }
 
-// Same for 8-bit floating-point inputs (kind::f8f6f4; K = 32 per instruction), one CTA.
+// Same for 8-bit floating-point inputs (kind::f8f6f4; K = 32 per instruction).
+template <int kCtaGroup>
 __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
+  if (kCtaGroup == 2) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+    return;
+  }
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
@@ -419,7 +431,7 @@ template <int kCtaGroup, bool kFp8>
 __device__ __forceinline__ void umma_ab(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
   if constexpr (kFp8) {
-    umma_f8(tmem_d, adesc, bdesc, idesc, accumulate);
+    umma_f8<kCtaGroup>(tmem_d, adesc, bdesc, idesc, accumulate);
   } else {
     umma_f16<kCtaGroup>(tmem_d, adesc, bdesc, idesc, accumulate);
   }

@@ -1310,7 +1310,7 @@ def test_groups_in_shared_memory_or_by_metadata_kernel(g, excess):
     (1, 512, 8, [1]),                                    # one row, one chunk of columns, two CTAs
     (4, 4096, 1544, [0, 1, 0, 2, 1, 0]),                 # last tile of 8 columns; empty groups
     (3, 1096, 260 * 2, [1, 1]),                          # k not a multiple of a stage, an unowned row
-    (200, 2056, 256, [65, 129]),                         # M = 64 and M = 128 tiles, unowned rows
+    (200, 8200, 256, [65, 129]),                         # M = 64 and M = 128 tiles, unowned rows
     (130, 8192, 96, [64, 0, 66]),                        # n below a tile
 ])
 def test_split_contraction(m, k, n, sizes):
@@ -1431,3 +1431,41 @@ def test_launched_before_the_predecessor_ends():
     assert torch.equal(got[0], want[0] * 2) and torch.equal(got[1], want[1] * 2)
     assert torch.equal(got[4], want[4]) and torch.equal(got[7], want[7]) and torch.equal(got[9], want[9])
     graph.reset()
+
+
+# ------------------------------------------------------------------ gmm with rows on the N side
+@pytest.mark.parametrize("m,k,n,sizes", [
+    (1030, 72, 512, [1, 1025]),                          # a single row; five tiles of 224 rows and less
+    (1600, 136, 576 * 2, [513, 0, 1000]),                # 3 x 192 rows; n ends 128 columns into a tile
+    (1540, 64, 1024, [256, 257, 1027]),                  # exactly one tile; one row more
+    (2600, 4096, 960, [31, 33, 2500]),                   # around one 32-row step; unowned rows
+])
+def test_rows_on_the_n_side(m, k, n, sizes):
+    """The swapped kernel at the edges of its row shares, against the oracle and the 128-row kernel (the
+    same products summed in fp32; one 16-bit rounding apart), with NaN in unowned rows, both
+    weight layouts, e4m3 and repeated weights."""
+    g = len(sizes)
+    x, A, _ = _inputs(61, m, k, n, g)
+    gs = torch.tensor(sizes, dtype=torch.int32)
+    total = int(gs.sum())
+    x[total:] = float("nan")
+    xd, Ad, gd = _to_dev(x, A, gs)
+    At = Ad.transpose(1, 2).contiguous()
+    auto, rows128 = _lib.TileCfg(0, 0, 0, 0, 0), _lib.TileCfg(256, 0, 1, 128, 0)
+    want = oracle.ragged_dot(x, A, gs)
+    for w, trans in ((Ad, False), (At, True)):
+        y = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto)
+        _assert_close(y.cpu(), want, f"trans={trans}")
+        ref = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=rows128)
+        assert float((y.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
+        if total < m:
+            assert float(y[total:].abs().max()) == 0.0
+    to_w = torch.tensor([g - 1] * g, dtype=torch.int32, device=DEV)
+    y = ops.gmm_forward(xd, Ad, gd, cfg=auto, group_to_weight=to_w)
+    _assert_close(y.cpu(), oracle.ragged_dot(x, A[[g - 1] * g], gs), "indexed")
+    if k % 16 == 0:
+        x8, A8 = xd.nan_to_num().to(torch.float8_e4m3fn), At.to(torch.float8_e4m3fn)
+        sc = torch.rand(g, device=DEV) + 0.5
+        got = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc).float()
+        ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=rows128).float()
+        assert float((got - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
