@@ -224,3 +224,20 @@ def test_gmm_permuted_clears_unnamed_rows(tokens, extra, y_rows):
     named[live[(live >= 0) & (live < y_rows)]] = True
     assert torch.equal(y[~named], torch.zeros_like(y[~named]))
     assert torch.isfinite(y.float()).all() and bool((y[named].abs().sum(1) > 0).all())
+
+
+@pytest.mark.parametrize("trans_rhs", [False, True])
+def test_long_groups_gather_then_scatter(trans_rhs):
+    """The route a call with long groups takes: rows gathered, results scattered by the kernel that has the
+    rows on its N side; bit-equal to the kernel that gathers and scatters itself, junk indices past
+    the groups and destinations that do not exist included."""
+    tokens, g, k, n = 4400, 2, 136, 2048 * 8
+    gs, in_rows, out_rows = _routing(5, tokens, 1, g, 77)
+    out_rows = torch.where(out_rows % 11 == 0, out_rows - 100000, out_rows)
+    in_rows[3] = tokens + 9  # a zero row
+    x = oracle.reference_normal(1, (tokens, k), torch.bfloat16).to(DEV)
+    A = oracle.reference_normal(2, (g, n, k) if trans_rhs else (g, k, n), torch.bfloat16).to(DEV)
+    gd, ird, ord_ = gs.to(DEV), in_rows.to(DEV), out_rows.to(DEV)
+    want = rd.ragged_dot_permuted(x, A, gd, in_rows=ird, out_rows=ord_, y_rows=tokens, trans_rhs=trans_rhs, fused=True)
+    got = rd.ragged_dot_permuted(x, A, gd, in_rows=ird, out_rows=ord_, y_rows=tokens, trans_rhs=trans_rhs)
+    assert torch.equal(got, want)
