@@ -197,14 +197,24 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     for (int i = threadIdx.x; i < my_pairs * t.rows; i += kGemmThreads) {
       const int row = i / my_pairs;
       const int pr = (i - row * my_pairs) * split + rank;
+      // all parts are fetched before the first is added: one trip through the cluster, not `split`
+      float4 a[kMaxSplit], b[kMaxSplit];
+#pragma unroll
+      for (int r = 0; r < kMaxSplit; ++r) {
+        if (r < split) {
+          a[r] = ld_cluster_f4(stage_base + split_chunk_offset(row, 2 * pr), r);
+          b[r] = ld_cluster_f4(stage_base + split_chunk_offset(row, 2 * pr + 1), r);
+        }
+      }
       float f[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = 0.0f;
-      for (int r = 0; r < split; ++r) {
-        const float4 a = ld_cluster_f4(stage_base + split_chunk_offset(row, 2 * pr), r);
-        const float4 b = ld_cluster_f4(stage_base + split_chunk_offset(row, 2 * pr + 1), r);
-        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-        f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+#pragma unroll
+      for (int r = 0; r < kMaxSplit; ++r) {
+        if (r < split) {
+          f[0] += a[r].x; f[1] += a[r].y; f[2] += a[r].z; f[3] += a[r].w;
+          f[4] += b[r].x; f[5] += b[r].y; f[6] += b[r].z; f[7] += b[r].w;
+        }
       }
       if constexpr (kFp8) {
 #pragma unroll
