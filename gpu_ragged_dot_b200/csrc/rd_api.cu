@@ -573,6 +573,15 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int g, int bn, const rd_tile
   return tgmm ? (k >= 256 && m / g >= 256) : m / g >= 512;
 }
 
+// Is a tgmm bound by an output whose rows are not multiples of 32 bytes?  Boxes then begin and end inside
+// sectors, which costs L2 reads of what it has not got; the 128-row kernel, whose boxes of a row
+// follow one another more closely, suffers least.  128-row against 256-row tiles, microseconds: n 3240 (k
+// 11600, 45 groups of 97 rows) 1047 and 1394, n 11672 (k 2216, 51 groups of 99) 884 and 990, where n 3232
+// and 11680 take 702 and 652; long groups are bound by the MMAs: n 4104 (8 groups of 1024 rows) 294 and 228.
+// (Cache hints on loads or stores change nothing; storing whole rows of a tile, or eight rows of four
+// boxes together, was slower.)
+bool split_sector_output(long long m, int n, int g) { return n % 16 != 0 && g > 0 && m / g < 256; }
+
 // CTA pairs (256 x 256 tiles, B operand split between the two CTAs) pay off where the
 // 256-row granularity wastes nothing: tgmm, whose tile rows are the dense k axis.  For gmm the
 // tile rows are a group's ragged token rows and the wider tile wastes more than the pair
@@ -1171,6 +1180,10 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   }
   if (seg_count > 1) {  // strided segments: one CTA per tile
     if (cta_group == 2) return RD_ERR_BAD_CONFIG;
+    cta_group = 1;
+  }
+  if (tile_m == 0 && cta_group == 0 && bn == 256 && split_sector_output(m, n, g)) {
+    tile_m = 128;
     cta_group = 1;
   }
   // Preference order when nothing is forced: 256-row tiles on one CTA, then a CTA pair, then

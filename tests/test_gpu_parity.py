@@ -1469,3 +1469,21 @@ def test_rows_on_the_n_side(m, k, n, sizes):
         got = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc).float()
         ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=rows128).float()
         assert float((got - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("n", [8, 248, 264, 520, 1432])
+@pytest.mark.parametrize("tile", [(256, 1, 256), (256, 2, 256), None])
+def test_tgmm_rows_that_split_sectors(n, tile):
+    """n % 16 == 8: output rows begin inside a 32-byte sector.  Every tile and the library's choice, bit-equal
+    to the 128-row kernel, k around the tile heights, an empty group's zeros included."""
+    g = 3
+    for k in (256, 520, 776):
+        gs = torch.tensor([70, 0, 133], dtype=torch.int32)
+        x, _, dout = _inputs(13, 210, k, n, g)
+        xd, dd, gd = _to_dev(x, dout, gs)
+        cfg = _lib.TileCfg(tile[0], 0, tile[1], tile[2], 0) if tile else None
+        out = torch.full((g, k, n), float("nan"), dtype=x.dtype, device=DEV)
+        ops.tgmm_forward(xd, dd, gd, cfg=cfg, out=out)
+        ref = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
+        assert torch.equal(out, ref), (k, n)
+        assert float(out[1].abs().max()) == 0.0
