@@ -582,6 +582,22 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int g, int bn, const rd_tile
 // boxes together, was slower.)
 bool split_sector_output(long long m, int n, int g) { return n % 16 != 0 && g > 0 && m / g < 256; }
 
+// Tile height of a tgmm with few rounds of tiles: 128 or 256 on one CTA, or 0 when there are six rounds of
+// 256-row tiles and more, or pairs need fewer rounds (then the rules above decide).  A 128-row tile
+// takes 0.58 times as long as a 256-row one.  Microseconds for 128 rows, 256 rows, pair: m 4096, k 1024, n
+// 1024, 4 groups (1, 1, 1 rounds) 17.3, 23.4, 23.5; 32768, 512, 512, 8 (1, 1, 1) 38, 54, 54; 8192, 4096, 1536, 2
+// (3, 2, 2) 87, 99, 99; 8106, 2552, 384, 9 (3, 2, 2) 34, 36, 38; 4096, 768, 3072, 8 (4, 2, 3) 27.6, 27.7, 33.8;
+// 8192, 1024, 768, 8 (2, 1, 1) 25.5, 23.5, 25.6; 3000, 4096, 4096, 1 (4, 2, 2) 87, 77, 79.
+int tgmm_tile_by_rounds(int k, int n, int g) {
+  if (k < 256) return 0;
+  const long long sms = sm_count(), cols = (static_cast<long long>(n) + 255) / 256 * g;
+  auto rounds = [&](int rows, long long units) { return ((k + rows - 1) / rows * cols + units - 1) / units; };
+  const long long r128 = rounds(128, sms), r256 = rounds(256, sms), r512 = rounds(512, sms / 2);
+  if (r256 >= 6) return 0;
+  if (0.58 * static_cast<double>(r128) < static_cast<double>(r256)) return 128;
+  return r256 <= r512 ? 256 : 0;
+}
+
 // CTA pairs (256 x 256 tiles, B operand split between the two CTAs) pay off where the
 // 256-row granularity wastes nothing: tgmm, whose tile rows are the dense k axis.  For gmm the
 // tile rows are a group's ragged token rows and the wider tile wastes more than the pair
@@ -1182,9 +1198,13 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (cta_group == 2) return RD_ERR_BAD_CONFIG;
     cta_group = 1;
   }
-  if (tile_m == 0 && cta_group == 0 && bn == 256 && split_sector_output(m, n, g)) {
-    tile_m = 128;
-    cta_group = 1;
+  if (tile_m == 0 && cta_group == 0 && bn == 256 && !f32 && seg_count == 1) {
+    if (split_sector_output(m, n, g)) {
+      tile_m = 128;
+    } else {
+      tile_m = tgmm_tile_by_rounds(k, n, g);
+    }
+    if (tile_m != 0) cta_group = 1;
   }
   // Preference order when nothing is forced: 256-row tiles on one CTA, then a CTA pair, then
   // plain 128-row tiles.

@@ -1487,3 +1487,15 @@ def test_tgmm_rows_that_split_sectors(n, tile):
         ref = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
         assert torch.equal(out, ref), (k, n)
         assert float(out[1].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("m,k,n,g", [(300, 256, 264, 2), (900, 1032, 1024, 4), (2000, 776, 3072, 8), (700, 4104, 4096, 1)])
+def test_tgmm_tile_by_rounds(m, k, n, g):
+    """Sizes on either side of the rule that picks the tile height from rounds of tiles: the library's choice
+    has the bits of every tile height."""
+    x, _, dout = _inputs(17, m, k, n, g)
+    gs = torch.from_numpy(oracle.reference_group_sizes(5, g, m - 3))
+    xd, dd, gd = _to_dev(x, dout, gs)
+    out = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(0, 0, 0, 0, 0))
+    for cfg in (_lib.TileCfg(256, 0, 1, 128, 0), _lib.TileCfg(256, 0, 1, 256, 0), _lib.TileCfg(256, 0, 2, 256, 0)):
+        assert torch.equal(out, ops.tgmm_forward(xd, dd, gd, cfg=cfg))
