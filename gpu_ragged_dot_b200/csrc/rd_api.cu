@@ -567,10 +567,13 @@ bool choose_pair_512(long long m, int k, int g) { return k >= 512 && g > 0 && m 
 //   gmm    m/g 1024 181 -> 165;  512 759 -> 675;  256 97 -> 91, but 185 -> 222 for unequal groups of
 //          mean 375 with trans_rhs (256-row tiles waste twice the rows of 128-row ones at a group's
 //          end);  128 386 -> 452
-bool choose_f32_pair(bool tgmm, long long m, int k, int g, int bn, const rd_tile_cfg* cfg) {
+// MN-major operands (tgmm, weights [k, n]) need rows that are multiples of 32: without the column-blocked
+// box the pair is slower (tgmm k 1056, n 12976, 17 groups of 400 457 -> 650, n 13056 410 -> 343).
+bool choose_f32_pair(bool tgmm, bool trans_rhs, long long m, int k, int n, int g, int bn, const rd_tile_cfg* cfg) {
   if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return true;
   if (bn != 256 || g <= 0 || (cfg && (cfg->cta_group == 1 || cfg->tile_m == 128))) return false;
-  return tgmm ? (k >= 256 && m / g >= 256) : m / g >= 512;
+  if (tgmm) return k >= 256 && m / g >= 256 && k % 32 == 0 && n % 32 == 0;
+  return m / g >= 512 && (trans_rhs || n % 32 == 0);
 }
 
 // Is a tgmm bound by an output whose rows are not multiples of 32 bytes?  Boxes then begin and end inside
@@ -729,7 +732,7 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
   if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
     if ((cfg && cfg->cta_group == 2) || tile_m == 256) return RD_ERR_BAD_CONFIG;
-    const bool pair = choose_f32_pair(false, m, k, g, bn, cfg);
+    const bool pair = choose_f32_pair(false, trans_rhs != 0, m, k, n, g, bn, cfg);
     if (pair) bn = rd::kF32PairBN;
     cta_group = pair ? 2 : 1;
     tile_m = 128;
@@ -1189,7 +1192,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
   if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
     if (cta_group == 2 || tile_m == 256 || seg_count > 1) return RD_ERR_BAD_CONFIG;
-    const bool pair = choose_f32_pair(true, m, k, g, bn, cfg);
+    const bool pair = choose_f32_pair(true, false, m, k, n, g, bn, cfg);
     if (pair) bn = rd::kF32PairBN;
     cta_group = pair ? 2 : 1;
     tile_m = 128;

@@ -1215,6 +1215,7 @@ def test_ep_count_share_emulated_ranks(world):
     (1025, 256, 256, [513, 511]),                     # tiles that end one row off, one unowned row
     (3100, 320, 292, [257, 0, 1, 255, 256, 2300]),    # tails of 1, 31 and 0 rows; 292 = 32 * 9 + 4
     (3000, 516, 644, [129, 127, 7, 1000, 1700]),
+    (2600, 288, 544, [33, 1500, 1000]),               # rows that are multiples of 32: column-blocked boxes
 ])
 def test_float32_pair_kernels(precision, m, k, n, sizes):
     """256 x 256 tiles on CTA pairs, plain and operand-splitting, at the edges of tiles, stages and
