@@ -508,7 +508,8 @@ def run_single(args):
         }),
         "method": "CUDA events on the launch stream; per-kernel events inside the timed region",
         "clocks": clocks,
-        "gpu_launches": 2 * len(kernels) * args.steps,
+        # one launch per GEMM; above 256 groups the group metadata is a launch of its own
+        "gpu_launches": (1 if shape.g <= 256 else 2) * len(kernels) * args.steps,
         "roofline": roofline,
     }
 
@@ -799,8 +800,8 @@ EP_COLLECTIVE = {
              "back with peer loads after a symmetric-memory barrier",
 }
 # our kernels per step (forward + backward), collectives and torch's own kernels not counted
-EP_LAUNCHES = {"nccl": 1 + 2 + 2 + 2, "p2p": 4 + 2 + 2 + 2 + 1, "fused": 6 + 2 + 2 + 1}  # fused: count+share,
-# plan, assign, own rows, metadata, send+GEMM; metadata + dlhs; metadata + drhs; pull
+EP_LAUNCHES = {"nccl": 1 + 1 + 1 + 2, "p2p": 4 + 1 + 1 + 2 + 1, "fused": 6 + 1 + 2 + 1}  # fused: count+share,
+# plan, assign, own rows, metadata, send+GEMM; dlhs; metadata + drhs; pull
 
 
 def ep_parity_check(layer, mode, out, dy, dx, dW, routing, world, dev, sample_tokens=48):
