@@ -169,7 +169,7 @@ def make_group_metadata(group_sizes: torch.Tensor, m: int, chunk_m: int) -> GMMG
 
 
 def _tensors(x, x_dim: int, w, w_dim: int, group_sizes) -> bool:
-    return (isinstance(x, torch.Tensor) and x.dim() == x_dim and isinstance(w, torch.Tensor) and w.dim() == w_dim
+    return (isinstance(x, torch.Tensor) and x.is_cuda and x.dim() == x_dim and isinstance(w, torch.Tensor) and w.dim() == w_dim
             and isinstance(group_sizes, torch.Tensor) and group_sizes.dim() == 1)
 
 
