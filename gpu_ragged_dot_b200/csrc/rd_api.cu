@@ -401,14 +401,11 @@ int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtens
 }
 
 // float32 on CTA pairs (rd_gemm_f32_pair.cuh).
-template <bool kBKMajor, bool kTgmm>
-int launch_gemm_f32_pair(bool split, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
-                         const GemmArgs& args, int ctas, cudaStream_t stream) {
-  if (split)
-    return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, true>, rd::f32_pair_threads<true>(),
-                        rd::f32_pair_smem_bytes<true>(), ta, tb, tout, args, ctas, stream);
-  return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, false>, rd::f32_pair_threads<false>(),
-                      rd::f32_pair_smem_bytes<false>(), ta, tb, tout, args, ctas, stream);
+template <bool kBKMajor, bool kTgmm, bool kSplit>
+int launch_gemm_f32_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout, const GemmArgs& args,
+                         int ctas, cudaStream_t stream) {
+  return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, kSplit>, rd::f32_pair_threads<kSplit>(),
+                      rd::f32_pair_smem_bytes<kSplit>(), ta, tb, tout, args, ctas, stream);
 }
 
 // Cluster size for a gmm whose tiles are too few for the SMs (rd_gemm_splitk.cuh), 1 = no split.
@@ -561,19 +558,16 @@ bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn) {
 bool choose_pair_512(long long m, int k, int g) { return k >= 512 && g > 0 && m / g >= 512; }
 
 // float32 tiles on CTA pairs (rd_gemm_f32_pair.cuh).  A caller who asks for three TF32 passes always
-// gets them: only that kernel splits its operands.  One pass, one CTA against a pair, microseconds:
-//   tgmm   m/g 1024 (k 4096, n 1536, g 8) 212 -> 175;  512 (same, g 64) 985 -> 779;  256 (k 1024, n 2048,
-//          g 32) 126 -> 104;  128 (k 2048, n 4096, g 64) 452 -> 491
-//   gmm    m/g 1024 181 -> 165;  512 759 -> 675;  256 97 -> 91, but 185 -> 222 for unequal groups of
-//          mean 375 with trans_rhs (256-row tiles waste twice the rows of 128-row ones at a group's
-//          end);  128 386 -> 452
-// MN-major operands (tgmm, weights [k, n]) need rows that are multiples of 32: without the column-blocked
-// box the pair is slower (tgmm k 1056, n 12976, 17 groups of 400 457 -> 650, n 13056 410 -> 343).
-bool choose_f32_pair(bool tgmm, bool trans_rhs, long long m, int k, int n, int g, int bn, const rd_tile_cfg* cfg) {
+// gets them: only that kernel splits its operands.  One pass: tgmm on groups of 256 rows and more with
+// rows that are multiples of 32.  One CTA against a pair, microseconds: k 1024, n 4096, 32 groups of 256
+// 181 -> 167; n 13056, 17 groups of 399 450 -> 421; k 4096, n 1536, 64 groups of 512 973 -> 939; m/g 1024 equal
+// within 3 %; k 2048, n 4096, 64 groups of 128 413 -> 491; without the column-blocked boxes (n 12976) 457 ->
+// 650.  gmm stays on one CTA: 8192, 4096, 14336, 8 1588 -> 1832, 16384, 1024, 4096, 32 267 -> 302, with
+// trans_rhs 3 % either way.
+bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const rd_tile_cfg* cfg) {
   if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return true;
-  if (bn != 256 || g <= 0 || (cfg && (cfg->cta_group == 1 || cfg->tile_m == 128))) return false;
-  if (tgmm) return k >= 256 && m / g >= 256 && k % 32 == 0 && n % 32 == 0;
-  return m / g >= 512 && (trans_rhs || n % 32 == 0);
+  if (!tgmm || bn != 256 || g <= 0 || (cfg && (cfg->cta_group == 1 || cfg->tile_m == 128))) return false;
+  return k >= 256 && m / g >= 256 && k % 32 == 0 && n % 32 == 0;
 }
 
 // Is a tgmm bound by an output whose rows are not multiples of 32 bytes?  Boxes then begin and end inside
@@ -732,7 +726,7 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
   if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
     if ((cfg && cfg->cta_group == 2) || tile_m == 256) return RD_ERR_BAD_CONFIG;
-    const bool pair = choose_f32_pair(false, trans_rhs != 0, m, k, n, g, bn, cfg);
+    const bool pair = choose_f32_pair(false, m, k, n, g, bn, cfg);
     if (pair) bn = rd::kF32PairBN;
     cta_group = pair ? 2 : 1;
     tile_m = 128;
@@ -776,7 +770,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
                      : launch_gemm_swap<false, false>(x, A, y, dtype, num_weights, args, stream);
   }
 
-  const bool blocked = f32 && cta_group == 2 && !trans_rhs && n % 32 == 0;
+  // float32 weights [k, n] with rows that are multiples of 32: one box per stage instead of one per 32 columns.
+  const bool blocked = f32 && !trans_rhs && n % 32 == 0;
   CUtensorMap ta, tb;
   {
     const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
@@ -789,8 +784,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
                               static_cast<uint64_t>(num_weights)};
     const uint32_t box[3] = {static_cast<uint32_t>(row_elems), static_cast<uint32_t>(bn / cta_group), 1};
     rc = encode_map(&tb, A, dtype, 3, dims, box);
-  } else if (blocked) {  // the float32 pair kernel fetches its four boxes of a stage with one load
-    rc = encode_blocked_map(&tb, A, dtype, n, k, row_elems, rd::kF32PairBN / 2 / 32, num_weights);
+  } else if (blocked) {
+    rc = encode_blocked_map(&tb, A, dtype, n, k, row_elems, bn / cta_group / 32, num_weights);
   } else {  // A[g, k, n]: rows of n, MN-major operand, [stage-depth k][128 B of n] boxes
     const uint64_t dims[3] = {static_cast<uint64_t>(n), static_cast<uint64_t>(k),
                               static_cast<uint64_t>(num_weights)};
@@ -835,9 +830,9 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (send != nullptr && send->sender_ctas >= ctas) return RD_ERR_BAD_CONFIG;
   if (f32) {
     if (ready.flags != nullptr) return RD_ERR_BAD_DTYPE;  // the float32 kernels do not wait on flags
-    if (cta_group == 2)
-      return trans_rhs ? launch_gemm_f32_pair<true, false>(three_pass, ta, tb, tout, args, ctas, stream)
-                       : launch_gemm_f32_pair<false, false>(three_pass, ta, tb, tout, args, ctas, stream);
+    if (cta_group == 2)  // three passes
+      return trans_rhs ? launch_gemm_f32_pair<true, false, true>(ta, tb, tout, args, ctas, stream)
+                       : launch_gemm_f32_pair<false, false, true>(ta, tb, tout, args, ctas, stream);
     if (trans_rhs) {
       if (bn == 256) return launch_gemm_f32<256, true, false>(ta, tb, tout, args, ctas, stream);
       if (bn == 128) return launch_gemm_f32<128, true, false>(ta, tb, tout, args, ctas, stream);
@@ -1192,7 +1187,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   if (three_pass && !f32) return RD_ERR_BAD_CONFIG;
   if (f32) {  // the float32 kernels choose between one CTA and a pair themselves
     if (cta_group == 2 || tile_m == 256 || seg_count > 1) return RD_ERR_BAD_CONFIG;
-    const bool pair = choose_f32_pair(true, false, m, k, n, g, bn, cfg);
+    const bool pair = choose_f32_pair(true, m, k, n, g, bn, cfg);
     if (pair) bn = rd::kF32PairBN;
     cta_group = pair ? 2 : 1;
     tile_m = 128;
@@ -1237,14 +1232,14 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
 
   // 256-row tiles fetch each operand of a stage with one box when the 64-column blocks tile the
   // rows exactly (see rd_gemm2.cuh); otherwise one 2-D box per 64 columns.
-  // The float32 pair kernel likewise, with blocks of 32 columns.
+  // The float32 kernels likewise, with blocks of 32 columns.
   const bool f32_pair = f32 && cta_group == 2;
-  const bool blocked = f32_pair ? (k % 32 == 0 && n % 32 == 0) : (two_half && !f32 && k % 64 == 0 && n % 64 == 0);
+  const bool blocked = f32 ? (k % 32 == 0 && n % 32 == 0) : (two_half && k % 64 == 0 && n % 64 == 0);
   CUtensorMap ta, tb;
-  if (blocked && f32_pair) {
+  if (blocked && f32) {
     rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kF32TileK, rd::kTileM / 32);
     if (rc != RD_OK) return rc;
-    rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kF32TileK, rd::kF32PairBN / 2 / 32);
+    rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kF32TileK, bn / cta_group / 32);
     if (rc != RD_OK) return rc;
   } else if (blocked) {
     rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kTileK, rd::kG2TileRows / 64);
@@ -1295,7 +1290,9 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   args.out = out;
 
   const int ctas = pick_ctas(cfg);
-  if (f32_pair) return launch_gemm_f32_pair<false, true>(three_pass, ta, tb, tout, args, ctas, stream);
+  if (f32_pair)
+    return three_pass ? launch_gemm_f32_pair<false, true, true>(ta, tb, tout, args, ctas, stream)
+                      : launch_gemm_f32_pair<false, true, false>(ta, tb, tout, args, ctas, stream);
   if (f32) {
     if (bn == 256) return launch_gemm_f32<256, false, true>(ta, tb, tout, args, ctas, stream);
     if (bn == 128) return launch_gemm_f32<128, false, true>(ta, tb, tout, args, ctas, stream);

@@ -11,6 +11,10 @@
 // moves 32 fp32 columns (one 128-byte row) per staging box.  MN-major 32-bit operands must use
 // the 128-byte swizzle with 32-byte atoms (TMA: SWIZZLE_128B_ATOM_32B; descriptor layout type
 // 1); with the ordinary 16-byte-atom swizzle the tensor core returns zeros.
+//
+// Where its rows are multiples of 32 elements an MN-major operand is described to TMA as (32 columns,
+// rows, blocks of 32 columns, matrices), so that one box per stage fetches what four to eight 4 KB boxes
+// would: m 8192, k 4096, n 1536, 8 groups gmm 181 -> 160 us, tgmm 204 -> 160 us.
 #pragma once
 
 #include "rd_gemm.cuh"
@@ -144,16 +148,23 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
           mbar_arrive_expect_tx(full, kStageBytes);
           if (kTgmm) {
             const int r = t.row0 + kb * kF32TileK;
+            if (p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, blocks of 32 columns)
+              tma_load_3d(sa, &tmap_a, full, 0, r, t.k0 >> 5);
+              tma_load_3d(sb, &tmap_b, full, 0, r, t.n0 >> 5);
+            } else {
 #pragma unroll
-            for (int j = 0; j < kTileM / 32; ++j)
-              tma_load_2d(sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
+              for (int j = 0; j < kTileM / 32; ++j)
+                tma_load_2d(sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
 #pragma unroll
-            for (int j = 0; j < BN / 32; ++j)
-              tma_load_2d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, r);
+              for (int j = 0; j < BN / 32; ++j)
+                tma_load_2d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, r);
+            }
           } else {
             tma_load_2d(sa, &tmap_a, full, kb * kF32TileK, t.row0);
             if (kBKMajor) {
               tma_load_3d(sb, &tmap_b, full, kb * kF32TileK, t.n0, t.weight);
+            } else if (p.blocked_maps) {
+              tma_load_4d(sb, &tmap_b, full, 0, kb * kF32TileK, t.n0 >> 5, t.weight);
             } else {
 #pragma unroll
               for (int j = 0; j < BN / 32; ++j)

@@ -1,6 +1,6 @@
-// float32 grouped GEMM kernels on CTA pairs: gmm / gmm trans_rhs / tgmm, float32 output.
+// float32 grouped GEMM kernels on CTA pairs, float32 output: three-pass gmm / gmm trans_rhs / tgmm, one-pass tgmm.
 //
-//   kSplit == false  one TF32 pass (the same arithmetic as ragged_gemm_f32_kernel)
+//   kSplit == false  one TF32 pass (the same arithmetic as ragged_gemm_f32_kernel), tgmm only
 //   kSplit == true   nearly float32 accuracy: every operand is split into a TF32 head and a
 //                    remainder, t = hi + lo, and a.b ~ lo.hi + hi.lo + hi.hi (the dropped lo.lo
 //                    term is 2^-22 relative).  The two small products have an accumulator of
@@ -23,10 +23,9 @@
 //
 // Measured (m 4096, k 4096, n 1536, 8 groups, three products): 0.25 / 0.25 / 0.24 ms for gmm / trans_rhs
 // / tgmm = 610 to 640 TFLOP/s of TF32 MMAs, where splitting in torch and three launches took 0.99 /
-// 0.92 / 0.85 ms; forward + backward 2.78 -> 0.87 ms.  One product (m 8192): 0.165 / 0.146 / 0.175 ms
-// against 0.181 / 0.159 / 0.212 on one CTA per tile.  The four [32][32] boxes of an MN-major operand
-// come as ONE box of a column-blocked view where its rows are multiples of 32: with four 4 KB boxes the
-// one-product gmm took 0.220 ms.
+// 0.92 / 0.85 ms; forward + backward 2.78 -> 0.87 ms.  The [32][32] boxes of an MN-major operand come as ONE
+// box of a column-blocked view where its rows are multiples of 32: with four 4 KB boxes a
+// one-product gmm took 0.220 instead of 0.161 ms.  One product: see choose_f32_pair in rd_api.cu.
 //
 // Roles: warp 0 = TMA producer, warp 1 = MMA issuer (one thread, of the leader CTA), warps 2..5 =
 // epilogue, warps 6.. = converters (kSplit, eight) or the tail fixer (one, tgmm).  tgmm rows past
@@ -84,6 +83,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             const __grid_constant__ CUtensorMap tmap_b,
                             const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
   static_assert(!(kTgmm && kBKMajor), "tgmm reads both operands MN-major");
+  static_assert(kSplit || kTgmm, "one-pass gmm runs on one CTA per tile");
   constexpr int BN = kF32PairBN;
   constexpr int kBCols = BN / 2;
   constexpr int kStages = f32_pair_stages<kSplit>();

@@ -1500,3 +1500,23 @@ def test_tgmm_tile_by_rounds(m, k, n, g):
     out = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(0, 0, 0, 0, 0))
     for cfg in (_lib.TileCfg(256, 0, 1, 128, 0), _lib.TileCfg(256, 0, 1, 256, 0), _lib.TileCfg(256, 0, 2, 256, 0)):
         assert torch.equal(out, ops.tgmm_forward(xd, dd, gd, cfg=cfg))
+
+
+@pytest.mark.parametrize("tile_n", [64, 128, 256])
+@pytest.mark.parametrize("k,n", [(32, 32), (96, 288), (288, 544)])
+def test_float32_blocked_boxes_one_cta(tile_n, k, n):
+    """float32 rows that are multiples of 32, where an MN-major operand comes as one box per stage: every
+    tile width, box blocks past the last column, against the same sizes padded by one row of 4
+    elements (one box per 32 columns), bit for bit on the common part."""
+    m, g = 300, 3
+    x, A, dout = _inputs(23, m, k, n, g, dtype=torch.float32)
+    gs = torch.tensor([129, 0, 170], dtype=torch.int32)
+    xd, Ad, dd, gd = _to_dev(x, A, dout, gs)
+    cfg = _lib.TileCfg(tile_n, 0, 1, 128, 0)
+    pad = lambda t: torch.nn.functional.pad(t, (0, 4))  # noqa: E731
+    y = ops.gmm_forward(xd, Ad, gd, cfg=cfg)
+    assert torch.equal(y, ops.gmm_forward(xd, pad(Ad), gd, cfg=cfg)[:, :n])
+    out = ops.tgmm_forward(xd, dd, gd, cfg=cfg)
+    assert torch.equal(out, ops.tgmm_forward(pad(xd), pad(dd), gd, cfg=cfg)[:, :k, :n])
+    rows = torch.arange(m) < int(gs.sum())
+    assert float(oracle.rel_l2_err(y.cpu(), oracle.ragged_dot(x, A, gs), axis=-1, mask=rows).max()) < 2e-3
