@@ -1510,7 +1510,8 @@ int rd_gmm_permuted(const void* x, int x_rows, const int32_t* in_rows, const voi
   if (rc != RD_OK) return rc;
   int bn = cfg && cfg->tile_n ? cfg->tile_n : choose_tile_n(0, n, 0);
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
-  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;
+  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256 || (cfg->flags & RD_CFG_F32_THREE_PASS)))
+    return RD_ERR_BAD_CONFIG;
 
   // Rows in order, results scattered: the swapped kernel, where the plain gmm would use it.
   if (in_rows == nullptr && out_rows != nullptr && inline_groups(m, g) && split_allowed(cfg) &&
@@ -1615,7 +1616,8 @@ int rd_tgmm_permuted(const void* x, int x_rows, const int32_t* x_row_index, cons
   if (rc != RD_OK) return rc;
   int bn = cfg && cfg->tile_n ? cfg->tile_n : choose_tile_n(0, n, 0);
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
-  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;
+  if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256 || (cfg->flags & RD_CFG_F32_THREE_PASS)))
+    return RD_ERR_BAD_CONFIG;
 
   launch_internal_metadata(group_sizes, nullptr, g, m, rd::kTileM, w, stream);
   if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
@@ -1746,6 +1748,7 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   int bn = cfg && cfg->tile_n ? cfg->tile_n : choose_tile_n(0, n, 0);
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // the library chooses
+  if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return RD_ERR_BAD_CONFIG;
   const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, n, g, bn);
 
   const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;

@@ -107,6 +107,22 @@ def test_argument_validation_happens_on_the_host(lib):
     assert lib.rd_device_status(None, None) == 3
 
 
+@pytest.mark.parametrize("entry", ["rd_gmm", "rd_tgmm", "rd_gmm_fp8", "rd_gmm_permuted", "rd_tgmm_permuted"])
+def test_three_pass_flag_is_refused_for_other_types(lib, entry):
+    """RD_CFG_F32_THREE_PASS belongs to float32: every entry point of other types refuses it on the host."""
+    a16, ws = 0x1000, 1 << 20
+    cfg = ctypes.byref(_lib.TileCfg(0, 0, 0, 0, _lib.RD_CFG_F32_THREE_PASS))
+    m, k, n, g, bf16 = 128, 64, 64, 2, _lib.RD_DTYPE_BF16
+    args = {
+        "rd_gmm": (a16, a16, a16, a16, a16, ws, m, k, n, g, 0, bf16),
+        "rd_tgmm": (a16, a16, a16, a16, a16, ws, m, k, n, g, bf16),
+        "rd_gmm_fp8": (a16, a16, g, a16, None, None, a16, a16, ws, m, k, n, g),
+        "rd_gmm_permuted": (a16, m, a16, a16, g, a16, None, a16, m, a16, a16, ws, m, k, n, g, 0, bf16),
+        "rd_tgmm_permuted": (a16, m, a16, a16, m, a16, a16, a16, a16, ws, m, k, n, g, bf16),
+    }[entry]
+    assert getattr(lib, entry)(*args, cfg, None) == 5
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
