@@ -5,6 +5,8 @@
 // (two allocations, a device guard, a stream object, a 16-argument ctypes call) 21 us a call.
 // Every function returns the result; None when the call is not of the plain form (the Python layer
 // then takes its general path, which pads, converts or raises); or the C ABI's error code.
+// From the first allocation on the GIL is released: cudaMalloc may wait for the device and a launch for
+// room in the queue, and other Python threads run meanwhile.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -79,17 +81,21 @@ py::object gmm(const Tensor& x, const Tensor& A, const Tensor& gs, bool trans_rh
     return py::none();
   const c10::cuda::OptionalCUDAGuard guard(x.device());
   void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  Tensor y = at::empty({m, n}, x.options());
-  Tensor ws = workspace(m, g, x);
+  Tensor y;
   int rc;
-  if (odd) {
-    const int64_t a_cols = trans_rhs ? k : n, a_rows = g * (trans_rhs ? n : k);
-    Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, a_rows, a_cols), x);
-    rc = rd_gmm_unaligned(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(),
-                          scratch.data_ptr(), scratch.numel(), m, k, n, g, trans_rhs, dtype, stream);
-  } else {
-    rc = rd_gmm(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
-                trans_rhs, dtype, cfg.ptr(), stream);
+  {
+    const py::gil_scoped_release no_gil;
+    y = at::empty({m, n}, x.options());
+    Tensor ws = workspace(m, g, x);
+    if (odd) {
+      const int64_t a_cols = trans_rhs ? k : n, a_rows = g * (trans_rhs ? n : k);
+      Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, a_rows, a_cols), x);
+      rc = rd_gmm_unaligned(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(),
+                            scratch.data_ptr(), scratch.numel(), m, k, n, g, trans_rhs, dtype, stream);
+    } else {
+      rc = rd_gmm(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
+                  trans_rhs, dtype, cfg.ptr(), stream);
+    }
   }
   return result(rc, y);
 }
@@ -113,16 +119,20 @@ py::object tgmm(const Tensor& x, const Tensor& y, const Tensor& gs, int tile_n, 
     return py::none();
   const c10::cuda::OptionalCUDAGuard guard(x.device());
   void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  Tensor out = at::empty({g, k, n}, x.options());
-  Tensor ws = workspace(m, g, x);
+  Tensor out;
   int rc;
-  if (odd) {
-    Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, m, n), x);
-    rc = rd_tgmm_unaligned(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(),
-                           scratch.data_ptr(), scratch.numel(), m, k, n, g, dtype, stream);
-  } else {
-    rc = rd_tgmm(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
-                 dtype, cfg.ptr(), stream);
+  {
+    const py::gil_scoped_release no_gil;
+    out = at::empty({g, k, n}, x.options());
+    Tensor ws = workspace(m, g, x);
+    if (odd) {
+      Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, m, n), x);
+      rc = rd_tgmm_unaligned(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(),
+                             scratch.data_ptr(), scratch.numel(), m, k, n, g, dtype, stream);
+    } else {
+      rc = rd_tgmm(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
+                   dtype, cfg.ptr(), stream);
+    }
   }
   return result(rc, out);
 }
@@ -145,10 +155,15 @@ py::object gmm_fp8(const Tensor& x, const Tensor& A, const Tensor& gs, const c10
   }
   const c10::cuda::OptionalCUDAGuard guard(x.device());
   void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  Tensor y = at::empty({m, n}, x.options().dtype(at::kBFloat16));
-  Tensor ws = workspace(m, g, x);
-  const int rc = rd_gmm_fp8(x.data_ptr(), A.data_ptr(), g, gs.data_ptr<int>(), nullptr, sc, y.data_ptr(),
-                            ws.data_ptr(), ws.numel(), m, k, n, g, nullptr, stream);
+  Tensor y;
+  int rc;
+  {
+    const py::gil_scoped_release no_gil;
+    y = at::empty({m, n}, x.options().dtype(at::kBFloat16));
+    Tensor ws = workspace(m, g, x);
+    rc = rd_gmm_fp8(x.data_ptr(), A.data_ptr(), g, gs.data_ptr<int>(), nullptr, sc, y.data_ptr(), ws.data_ptr(),
+                    ws.numel(), m, k, n, g, nullptr, stream);
+  }
   return result(rc, y);
 }
 

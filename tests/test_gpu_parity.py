@@ -1520,3 +1520,45 @@ def test_float32_blocked_boxes_one_cta(tile_n, k, n):
     assert torch.equal(out, ops.tgmm_forward(pad(xd), pad(dd), gd, cfg=cfg)[:, :k, :n])
     rows = torch.arange(m) < int(gs.sum())
     assert float(oracle.rel_l2_err(y.cpu(), oracle.ragged_dot(x, A, gs), axis=-1, mask=rows).max()) < 2e-3
+
+
+# ------------------------------------------------------------------ native host path
+@pytest.mark.parametrize("op", ["gmm", "tgmm", "gmm_fp8"])
+def test_other_threads_run_while_a_launch_waits(op):
+    """Calls behind a kernel of 0.3 s fill the launch queue, so that one of them waits for it: another Python
+    thread must keep running meanwhile."""
+    import threading
+    import time
+
+    gs = torch.tensor([16], dtype=torch.int32, device=DEV)
+    x, A = torch.ones((16, 64), dtype=torch.bfloat16, device=DEV), torch.ones((1, 64, 64), dtype=torch.bfloat16, device=DEV)
+    x8, A8 = x.to(torch.float8_e4m3fn), A.to(torch.float8_e4m3fn)
+    call = {"gmm": lambda: ops.gmm_forward(x, A, gs), "tgmm": lambda: ops.tgmm_forward(x, x, gs),
+            "gmm_fp8": lambda: ops.gmm_fp8_forward(x8, A8, gs)}[op]
+    call()
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), []
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(600_000_000)  # clocks
+        longest, t0 = 0.0, time.perf_counter()
+        while longest < 0.1 and time.perf_counter() - t0 < 2.0:
+            t1 = time.perf_counter()
+            call()
+            longest = max(longest, time.perf_counter() - t1)
+    finally:
+        stop.set()
+        thread.join()
+        torch.cuda.synchronize()
+    assert longest >= 0.1, "no call waited: the launch queue never filled"
+    assert max(gaps) < 0.5 * longest, (max(gaps), longest)
