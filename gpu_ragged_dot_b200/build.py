@@ -67,14 +67,15 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_host(force: bool = False) -> str:
-    """Compile _rd_host.so if it is missing or older than its sources; return its path."""
-    deps = [HOST_SOURCE, HEADER]
-    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
-        return HOST_PATH
+    """Compile _rd_host.so if it is missing or older than its sources or the installed torch; return its path."""
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension
+
+    deps = [HOST_SOURCE, HEADER, torch.version.__file__]  # built for one torch's headers and libraries
+    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
+        return HOST_PATH
 
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",

@@ -123,6 +123,29 @@ def test_three_pass_flag_is_refused_for_other_types(lib, entry):
     assert getattr(lib, entry)(*args, cfg, None) == 5
 
 
+def test_host_path_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    """_rd_host.so holds for the torch it was compiled against: a torch installed later makes it stale."""
+    import subprocess
+
+    import torch
+
+    commands = []
+    monkeypatch.setattr(subprocess, "run", lambda cmd, **kw: commands.append(cmd) or subprocess.CompletedProcess(cmd, 0, "", ""))
+    built, version = tmp_path / "_rd_host.so", tmp_path / "version.py"
+    for path in (built, version):
+        path.write_text("")
+    monkeypatch.setattr(build, "HOST_PATH", str(built))
+    monkeypatch.setattr(torch.version, "__file__", str(version))
+    newest = max(os.path.getmtime(p) for p in (build.HOST_SOURCE, build.HEADER))
+    os.utime(built, (newest + 10, newest + 10))
+    os.utime(version, (newest + 5, newest + 5))
+    build.build_host()
+    assert not commands
+    os.utime(version, (newest + 20, newest + 20))
+    build.build_host()
+    assert len(commands) == 1 and str(built) in commands[0]
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
