@@ -200,11 +200,31 @@ def test_sum_rows(dtype, rows_in, rows_out, cols, live):
     got = ops.sum_rows(src.to(DEV), index.to(DEV), gs.to(DEV), rows_out)
     assert got.dtype == dtype
     again = ops.sum_rows(src.to(DEV), index.to(DEV), gs.to(DEV), rows_out)
-    if rows_in <= 257 and rows_out >= 32:
-        assert torch.equal(got, again)  # short lists are added in a fixed order
+    assert torch.equal(got, again)
     eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 0.0}[dtype]
     bound = eps * want.abs() + (128 * 2.0 ** -24) * mag + 2.0 ** -24
     assert bool(((got.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows_in,rows_out,live", [
+    (32, 1, 32), (33, 1, 33),      # either side of what is ranked in registers
+    (4096, 2, 4096),               # one window of indices
+    (9001, 2, 9000),               # windows, the last one part full
+    (9001, 150, 9001),             # lists of about 60 rows that span all windows
+])
+def test_sum_rows_adds_in_ascending_order(rows_in, rows_out, live):
+    """Bit for bit the float32 sum in ascending order of the source rows, whatever the length of the lists:
+    magnitudes over eight decades make any other order differ."""
+    rng = np.random.default_rng(rows_in + rows_out)
+    src = (rng.standard_normal((rows_in, 12)) * 10.0 ** rng.uniform(-4, 4, (rows_in, 1))).astype(np.float32)
+    index = rng.integers(0, rows_out, size=rows_in).astype(np.int32)
+    want = np.zeros((rows_out, 12), dtype=np.float32)
+    for i in range(live):
+        want[index[i]] += src[i]
+    gs = torch.tensor([live], dtype=torch.int32, device=DEV)
+    for _ in range(3):
+        got = ops.sum_rows(torch.from_numpy(src).to(DEV), torch.from_numpy(index).to(DEV), gs, rows_out)
+        assert np.array_equal(got.cpu().numpy(), want)
 
 
 @pytest.mark.parametrize("tokens,extra,y_rows", [(96, 0, 192), (96, 33, 200), (5, 0, 300)])
