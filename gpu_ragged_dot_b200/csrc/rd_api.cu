@@ -478,7 +478,7 @@ bool choose_swap(long long m, int n, int g, bool trans_rhs) {
 }
 
 // Tensor maps and launch of the swapped kernel; k in 2-byte units (kFp8: half of the elements).
-template <bool kBKMajor, bool kFp8, bool kScatter = false>
+template <bool kBKMajor, bool kFp8>
 int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_weights, GemmArgs args,
                      cudaStream_t stream) {
   CUtensorMap tw, tx, tout;
@@ -498,16 +498,14 @@ int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_w
     rc = encode_blocked_map(&tw, A, dtype, args.n, args.k, rd::kTileK, rd::kSwapCtaCols / 64, num_weights);
   }
   if (rc != RD_OK) return rc;
-  if (kScatter) {
-    tout = tx;  // rows are stored one by one
-  } else {
+  {
     const uint64_t dims[2] = {static_cast<uint64_t>(args.n), static_cast<uint64_t>(args.m)};
     const uint32_t box[2] = {32, 32};
     rc = encode_map(&tout, y, dtype, 2, dims, box, false, /*swizzled=*/false);
     if (rc != RD_OK) return rc;
   }
   args.n_tiles = (args.n + rd::kSwapCols - 1) / rd::kSwapCols;
-  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8, kScatter>, rd::kSwapThreads, rd::kSwapSmemBytes, tw, tx, tout,
+  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8>, rd::kSwapThreads, rd::kSwapSmemBytes, tw, tx, tout,
                       args, sm_count(), stream);
 }
 
@@ -1512,27 +1510,6 @@ int rd_gmm_permuted(const void* x, int x_rows, const int32_t* in_rows, const voi
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256 || (cfg->flags & RD_CFG_F32_THREE_PASS)))
     return RD_ERR_BAD_CONFIG;
-
-  // Rows in order, results scattered: the swapped kernel, where the plain gmm would use it.
-  if (in_rows == nullptr && out_rows != nullptr && inline_groups(m, g) && split_allowed(cfg) &&
-      choose_swap(m, n, g, trans_rhs != 0)) {
-    rc = ensure_context();
-    if (rc != RD_OK) return rc;
-    GemmArgs args = {};
-    args.m = m; args.k = k; args.n = n; args.g = g;
-    args.max_m_tiles = w.layout.max_tiles;
-    args.ab_format = dtype;
-    args.wait_limit_us = wait_limit_us(cfg);
-    args.inline_groups = 1;
-    args.group_to_weight = group_to_weight;
-    args.group_sizes = group_sizes;
-    args.status = w.status();
-    args.out = y;
-    args.scatter_rows = out_rows;
-    args.scatter_rows_n = y_rows;
-    return trans_rhs ? launch_gemm_swap<true, false, true>(x, A, y, dtype, num_weights, args, stream)
-                     : launch_gemm_swap<false, false, true>(x, A, y, dtype, num_weights, args, stream);
-  }
 
   launch_internal_metadata(group_sizes, group_to_weight, g, m, rd::kTileM, w, stream);
   if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;

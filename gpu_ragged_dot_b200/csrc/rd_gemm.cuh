@@ -79,10 +79,6 @@ struct GemmArgs {
   // Set: every CTA makes its own group table in shared memory (build_group_table); group_offsets,
   // tile_rec and totals are not read then, and there is no metadata launch.
   int inline_groups;
-  // ragged_gemm_swap_kernel, kScatter: row r of the product goes to row scatter_rows[r] of out, which has
-  // scatter_rows_n rows (others are dropped).
-  const int32_t* scatter_rows;
-  int scatter_rows_n;
   const int32_t* group_to_weight;  // inline_groups, gmm: weight matrix of each group (null: the group's own index)
   const int32_t* group_sizes;
   const int32_t* group_offsets;

@@ -23,10 +23,6 @@
 // shared memory (two-byte stores, 64 contiguous bytes per row) and leaves by TMA; blocks that cross
 // the end of the tile's rows are stored from registers, 64 bytes per row.
 //
-// kScatter: every row goes to a destination of its own, from registers, 64 bytes per row and warp (the MoE
-// layer's un-sort; forward of 4096 tokens, top-2, k 4096, n 14336: gather 19 + product 690 us against 755
-// us for the kernel that gathers row by row).
-//
 // Roles, barriers and waits as in rd_gemm2.cuh (kPair); loads are plain, nothing is broadcast.
 // kFp8: e4m3 operands, K-major weights, tiles byte for byte those of a 16-bit problem.
 #pragma once
@@ -69,7 +65,7 @@ __device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const Gr
   return t;
 }
 
-template <bool kBKMajor, bool kFp8, bool kScatter>
+template <bool kBKMajor, bool kFp8>
 __global__ void __launch_bounds__(kSwapThreads, 1)
 ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
@@ -261,16 +257,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (c >= chunks) continue;
         const int row0 = t.row0 + c * 32;
         const int rows = t.rows - c * 32;
-        if constexpr (kScatter) {  // 64 contiguous bytes per row, straight from registers
-          int dst_row = lane < rows ? p.scatter_rows[row0 + lane] : -1;
-          if (dst_row >= p.scatter_rows_n) dst_row = -1;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int r = __shfl_sync(0xffffffffu, dst_row, j);
-            if (r >= 0 && col0 + lane < p.n)
-              out16[static_cast<size_t>(r) * p.n + col0 + lane] = static_cast<uint16_t>(o[c][j >> 1] >> (16 * (j & 1)));
-          }
-        } else if (rows >= 32) {
+        if (rows >= 32) {
           const uint32_t buf = staging + (boxes_stored & 1u) * kSwapBoxBytes;
           if (lane == 0) bulk_wait_group_read<1>();  // the box stored two boxes ago has been read out
           __syncwarp();

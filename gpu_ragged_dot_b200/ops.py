@@ -855,10 +855,6 @@ class _GmmPermutedFn(torch.autograd.Function):
         g = group_sizes.numel()
         use_fused = fused if fused is not None else _fused_permute_pays(m, g, out_rows is not None)
         if use_fused:
-            if fused is None and in_rows is not None and x.shape[1] % 8 == 0:
-                # Rows gathered once, results scattered by the GEMM's epilogue: the gather (19 us for
-                # 8192 rows of 4096) buys the kernel of the plain product, which takes its rows by TMA.
-                x, in_rows = gather_rows(x, in_rows[:m]), None
             return gmm_permuted_forward(x, A, group_sizes, in_rows=in_rows, out_rows=out_rows, y_rows=y_rows,
                                         m=m, trans_rhs=trans_rhs)
         return _gmm_permuted_two_pass(x, A, _as_i32(group_sizes), in_rows, out_rows, y_rows, m, trans_rhs)

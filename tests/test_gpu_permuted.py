@@ -14,6 +14,7 @@ sys.path.insert(0, os.path.join(os.path.dirname(__file__), ".."))
 import gpu_ragged_dot_b200 as rd  # noqa: E402
 from gpu_ragged_dot_b200 import _lib, ops  # noqa: E402
 from oracle import ragged_dot_oracle as oracle  # noqa: E402
+from tests import launched  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0) if torch.cuda.is_available() else None
@@ -247,10 +248,10 @@ def test_gmm_permuted_clears_unnamed_rows(tokens, extra, y_rows):
 
 
 @pytest.mark.parametrize("trans_rhs", [False, True])
-def test_long_groups_gather_then_scatter(trans_rhs):
-    """The route a call with long groups takes: rows gathered, results scattered by the kernel that has the
-    rows on its N side; bit-equal to the kernel that gathers and scatters itself, junk indices past
-    the groups and destinations that do not exist included."""
+def test_long_groups_gather_and_scatter_in_one_kernel(trans_rhs):
+    """The route a call with long groups takes: one product that gathers and scatters itself, nothing gathered
+    before it; bit-equal to gather_rows, the plain product and a scatter, junk indices past the
+    groups and destinations that do not exist included."""
     tokens, g, k, n = 4400, 2, 136, 2048 * 8
     gs, in_rows, out_rows = _routing(5, tokens, 1, g, 77)
     out_rows = torch.where(out_rows % 11 == 0, out_rows - 100000, out_rows)
@@ -258,6 +259,13 @@ def test_long_groups_gather_then_scatter(trans_rhs):
     x = oracle.reference_normal(1, (tokens, k), torch.bfloat16).to(DEV)
     A = oracle.reference_normal(2, (g, n, k) if trans_rhs else (g, k, n), torch.bfloat16).to(DEV)
     gd, ird, ord_ = gs.to(DEV), in_rows.to(DEV), out_rows.to(DEV)
-    want = rd.ragged_dot_permuted(x, A, gd, in_rows=ird, out_rows=ord_, y_rows=tokens, trans_rhs=trans_rhs, fused=True)
-    got = rd.ragged_dot_permuted(x, A, gd, in_rows=ird, out_rows=ord_, y_rows=tokens, trans_rhs=trans_rhs)
+    ys = ops.gmm_forward(ops.gather_rows(x, ird), A, gd, trans_rhs=trans_rhs)
+    live = torch.arange(ird.numel(), device=DEV) < int(gs.sum())
+    named = live & (ord_ >= 0) & (ord_ < tokens)
+    want = torch.zeros((tokens, n), dtype=torch.bfloat16, device=DEV)
+    want[ord_[named].long()] = ys[named]
+    got, names = launched.kernels(lambda: rd.ragged_dot_permuted(x, A, gd, in_rows=ird, out_rows=ord_, y_rows=tokens,
+                                                         trans_rhs=trans_rhs))
     assert torch.equal(got, want)
+    assert sum("ragged_gemm" in name for name in names) == 1 and any("ragged_gemm_perm" in name for name in names)
+    assert not any("gather_rows" in name for name in names)
