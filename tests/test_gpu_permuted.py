@@ -228,7 +228,7 @@ def test_sum_rows_adds_in_ascending_order(rows_in, rows_out, live):
         assert np.array_equal(got.cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("tokens,extra,y_rows", [(96, 0, 192), (96, 33, 200), (5, 0, 300)])
+@pytest.mark.parametrize("tokens,extra,y_rows", [(96, 0, 192), (96, 33, 200), (5, 0, 300), (96, 33, 190000)])
 def test_gmm_permuted_clears_unnamed_rows(tokens, extra, y_rows):
     """Rows of y that no sorted row names are zero, also where memory held something else."""
     g, k, n = 4, 64, 136
@@ -245,6 +245,22 @@ def test_gmm_permuted_clears_unnamed_rows(tokens, extra, y_rows):
     named[live[(live >= 0) & (live < y_rows)]] = True
     assert torch.equal(y[~named], torch.zeros_like(y[~named]))
     assert torch.isfinite(y.float()).all() and bool((y[named].abs().sum(1) > 0).all())
+
+
+@pytest.mark.parametrize("y_rows,marks", [(1 << 14, False), (3 << 15, True)])
+def test_small_results_are_cleared_whole(y_rows, marks):
+    """Rows of 512 bytes: 8 MB of result are cleared by one memset, 48 MB by marking what is written."""
+    g, k, n = 2, 64, 256
+    gs, in_rows, out_rows = _routing(3, 64, 1, g)
+    x = oracle.reference_normal(1, (64, k), torch.bfloat16).to(DEV)
+    A = oracle.reference_normal(2, (g, k, n), torch.bfloat16).to(DEV)
+    args = [t.to(DEV) for t in (gs, in_rows, out_rows)]
+    y, names = launched.kernels(lambda: ops.gmm_permuted_forward(x, A, args[0], in_rows=args[1], out_rows=args[2],
+                                                                   y_rows=y_rows))
+    assert any("mark_rows" in name for name in names) == marks
+    rows = torch.zeros(y_rows, dtype=torch.bool)
+    rows[out_rows.long()] = True
+    assert bool((y.cpu().float().abs().sum(1) > 0).eq(rows).all())
 
 
 @pytest.mark.parametrize("trans_rhs", [False, True])
