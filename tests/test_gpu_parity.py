@@ -16,6 +16,7 @@ import torch
 import gpu_ragged_dot_b200 as rd
 from gpu_ragged_dot_b200 import _lib, ops, workloads
 from oracle import ragged_dot_oracle as oracle
+from tests import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -1269,17 +1270,18 @@ def test_float32_highest_splits_extreme_values():
 
 
 def test_gmm_fp8_on_256_row_tiles():
-    """Long groups (512 rows on average) run on 256-row tiles: bit-equal to the 128-row kernel, which
+    """Long groups whose 256-row tiles need fewer rounds run on them: bit-equal to the 128-row kernel, which
     adds the same products in the same order, at tile edges and with and without a scale."""
-    m, k, n = 1601, 272, 264
-    gs = torch.tensor([257, 0, 1279 + 64], dtype=torch.int32)
+    m, k, n = 6000, 272, 1024
+    gs = torch.tensor([257, 0, 1279 + 64, 1, 128, 256, 3000, 900], dtype=torch.int32)
     rng = np.random.default_rng(5)
     x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
-    A = torch.from_numpy(rng.standard_normal((3, n, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
-    for scale in (None, torch.tensor([0.5, 2.0, 0.03125], device=DEV)):
+    A = torch.from_numpy(rng.standard_normal((8, n, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
+    for scale in (None, torch.rand(8, device=DEV) + 0.5):
         want = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale, cfg=_lib.TileCfg(256, 0, 0, 128, 0))
-        got = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale)
-        assert torch.equal(got, want) and float(got[-1].abs().max()) == 0.0
+        got, names = launched.kernels(lambda: ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale))
+        assert any("ragged_gemm2_kernel" in name for name in names), names
+        assert torch.equal(got, want) and float(got[int(gs.sum()):].abs().max()) == 0.0
 
 
 @pytest.mark.parametrize("g", [1, 31, 255, 256, 257])
@@ -1308,7 +1310,7 @@ def test_groups_in_shared_memory_or_by_metadata_kernel(g, excess):
 
 # ------------------------------------------------------------------ few tiles: contraction shared by a cluster
 @pytest.mark.parametrize("m,k,n,sizes", [
-    (1, 512, 8, [1]),                                    # one row, one chunk of columns, two CTAs
+    (1, 704, 8, [1]),                                    # one row, one chunk of columns, two CTAs
     (4, 4096, 1544, [0, 1, 0, 2, 1, 0]),                 # last tile of 8 columns; empty groups
     (3, 1096, 260 * 2, [1, 1]),                          # k not a multiple of a stage, an unowned row
     (200, 8200, 256, [65, 129]),                         # M = 64 and M = 128 tiles, unowned rows
@@ -1325,7 +1327,8 @@ def test_split_contraction(m, k, n, sizes):
     whole = _lib.TileCfg(0, 0, 1, 0, 0)
     auto = _lib.TileCfg(0, 0, 0, 0, 0)
     for w, trans in ((Ad, False), (At, True)):
-        y = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto)
+        y, names = launched.kernels(lambda: ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto))
+        assert any("ragged_gemm_splitk_kernel" in name for name in names), names
         assert torch.equal(y, ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto))
         _assert_close(y.cpu(), oracle.ragged_dot(x, A, gs), "split")
         ref = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=whole).float()
@@ -1334,7 +1337,8 @@ def test_split_contraction(m, k, n, sizes):
     if k % 16 == 0:
         x8, A8 = xd.to(torch.float8_e4m3fn), At.to(torch.float8_e4m3fn)
         sc = torch.rand(g, device=DEV) + 0.5
-        y = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc)
+        y, names = launched.kernels(lambda: ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc))
+        assert k < 1024 or any("ragged_gemm_splitk_kernel" in name for name in names), names
         ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=whole).float()
         assert float((y.float() - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
 
@@ -1435,41 +1439,52 @@ def test_launched_before_the_predecessor_ends():
 
 
 # ------------------------------------------------------------------ gmm with rows on the N side
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("m,k,n,sizes", [
-    (1030, 72, 512, [1, 1025]),                          # a single row; five tiles of 224 rows and less
-    (1600, 136, 576 * 2, [513, 0, 1000]),                # 3 x 192 rows; n ends 128 columns into a tile
-    (1540, 64, 1024, [256, 257, 1027]),                  # exactly one tile; one row more
-    (2600, 4096, 960, [31, 33, 2500]),                   # around one 32-row step; unowned rows
+    (1030, 584, 32768, [1, 1025]),                       # a single row; five tiles of 224 rows and less
+    (1600, 520, 19264, [513, 0, 1000]),                  # 3 x 192 rows; n ends 320 columns into a tile
+    (1540, 576, 19456, [256, 257, 1027]),                # exactly one tile; one row more
+    (2600, 1040, 11776, [31, 33, 2500]),                 # around one 32-row step; unowned rows
+    (1030, 576, 32744, [5, 1020]),                       # trans_rhs: n ends inside a 32-column block
 ])
-def test_rows_on_the_n_side(m, k, n, sizes):
+def test_rows_on_the_n_side(dtype, m, k, n, sizes):
     """The swapped kernel at the edges of its row shares, against the oracle and the 128-row kernel (the
     same products summed in fp32; one 16-bit rounding apart), with NaN in unowned rows, both
     weight layouts, e4m3 and repeated weights."""
     g = len(sizes)
-    x, A, _ = _inputs(61, m, k, n, g)
+    x, A, _ = _inputs(61, m, k, n, g, dtype=dtype)
     gs = torch.tensor(sizes, dtype=torch.int32)
     total = int(gs.sum())
     x[total:] = float("nan")
     xd, Ad, gd = _to_dev(x, A, gs)
     At = Ad.transpose(1, 2).contiguous()
     auto, rows128 = _lib.TileCfg(0, 0, 0, 0, 0), _lib.TileCfg(256, 0, 1, 128, 0)
+
+    def swapped(fn):
+        res, names = launched.kernels(fn)
+        assert any("ragged_gemm_swap_kernel" in name for name in names), names
+        return res
+
     want = oracle.ragged_dot(x, A, gs)
     for w, trans in ((Ad, False), (At, True)):
-        y = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto)
+        if not trans and n % 64:
+            continue
+        y = swapped(lambda: ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=auto))
         _assert_close(y.cpu(), want, f"trans={trans}")
         ref = ops.gmm_forward(xd, w, gd, trans_rhs=trans, cfg=rows128)
         assert float((y.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
         if total < m:
             assert float(y[total:].abs().max()) == 0.0
     to_w = torch.tensor([g - 1] * g, dtype=torch.int32, device=DEV)
-    y = ops.gmm_forward(xd, Ad, gd, cfg=auto, group_to_weight=to_w)
+    y = swapped(lambda: ops.gmm_forward(xd, At, gd, trans_rhs=True, cfg=auto, group_to_weight=to_w))
     _assert_close(y.cpu(), oracle.ragged_dot(x, A[[g - 1] * g], gs), "indexed")
-    if k % 16 == 0:
-        x8, A8 = xd.nan_to_num().to(torch.float8_e4m3fn), At.to(torch.float8_e4m3fn)
-        sc = torch.rand(g, device=DEV) + 0.5
-        got = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc).float()
-        ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=rows128).float()
-        assert float((got - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
+    # e4m3: twice the elements, the same bytes per row
+    x8 = torch.cat([xd, xd.flip(1)], dim=1).nan_to_num().to(torch.float8_e4m3fn)
+    A8 = torch.cat([At, At.flip(2)], dim=2).to(torch.float8_e4m3fn)
+    sc = torch.rand(g, device=DEV) + 0.5
+    got = swapped(lambda: ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc)).float()
+    ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=rows128).float()
+    assert float((got - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
 
 
 @pytest.mark.parametrize("n", [8, 248, 264, 520, 1432])
