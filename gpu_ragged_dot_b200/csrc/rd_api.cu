@@ -467,14 +467,25 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
 // are at least three rounds of tiles for the pairs and the last 512-column tile is nearly full.
 // Microseconds, one-CTA tiles (better of the two heights) against swapped: m 8192, k 4096, n 14336, 8
 // groups 694 -> 687, trans_rhs with k 14336, n 4096 687 -> 669 (alone; in a row with the backward pass
-// 2.58 -> 2.48 ms a step); 16 unequal groups 816 -> 751; 64 groups of 512, k 4096, n 1536 402 -> 384.
-// Below: 4096, 4096, 4096, 8 (1.7 rounds) 177 -> 212; n 2304 (last tile half full) 160 -> 171; 256 rows
-// per group 288 -> 273 at best, 1058 -> 1160 at worst; 128 rows 222 -> 233.
-bool choose_swap(long long m, int n, int g, bool trans_rhs) {
+// 2.58 -> 2.48 ms a step); 13304, 2824, 11264, 16 804 -> 683; 28320, 5656, 1536, 32 605 -> 523; 64 groups of 512, k
+// 4096, n 1536 402 -> 384.  Below: 4096, 4096, 4096, 8 (1.7 rounds) 177 -> 212; n 2304 (last tile half full)
+// 160 -> 171; 256 rows per group 288 -> 273 at best, 1058 -> 1160 at worst; 128 rows 222 -> 233.
+// A short contraction (fewer than nine 64-deep blocks) leaves the drain of both accumulators exposed once per
+// tile: 4928, 264, 7232, 4 40 -> 50, 22000, 512, 4032, 12 112 -> 120; 16 bits win again from twenty rounds on (17184, 456,
+// 13568, 32 288 -> 255), e4m3 does not (25960, 448, 4928, 24 112 -> 124).
+// e4m3 (128-row tiles otherwise) with few rounds: they are compared, a swapped tile taking 1.7 times as long
+// as a 128-row one; 8192, 14336, 4096, 16 (5 against 8) 422 -> 433, in a row 425 -> 453.
+bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool fp8) {
   if (g <= 0 || m / g < 512 || (!trans_rhs && n % 64 != 0)) return false;
+  const long long pairs = sm_count() / 2;
   const long long col_tiles = (static_cast<long long>(n) + rd::kSwapCols - 1) / rd::kSwapCols;
-  if ((col_tiles * rd::kSwapCols - n) * 16 > n) return false;
-  return m / rd::kSwapRows * col_tiles >= 3LL * (sm_count() / 2);
+  if ((col_tiles * rd::kSwapCols - n) * 16 > n || m / rd::kSwapRows * col_tiles < 3 * pairs) return false;
+  const long long tiles = (m / rd::kSwapRows + g / 2) * col_tiles;  // half a tile more per group
+  if (k_blocks < 9 && (fp8 || tiles < 20 * pairs)) return false;
+  if (!fp8 || tiles >= 6 * pairs) return true;
+  const long long tiles128 = ((m + 127) / 128 + g / 2) * ((static_cast<long long>(n) + 255) / 256);
+  return 1.7 * static_cast<double>((tiles + pairs - 1) / pairs) <
+         static_cast<double>((tiles128 + 2 * pairs - 1) / (2 * pairs));
 }
 
 // Tensor maps and launch of the swapped kernel; k in 2-byte units (kFp8: half of the elements).
@@ -530,23 +541,34 @@ bool split_allowed(const rd_tile_cfg* cfg) {
 // 256-row tiles on one CTA (rd_gemm2.cuh) move a third less data per flop than 128-row tiles.
 // They pay off when a tile's second half usually exists: tgmm with k >= 256, and gmm when the
 // groups are long (a half without rows is skipped, so the cost of a wrong guess is only a
-// shallower smem ring) -- unless the larger tiles fill the SMs badly.  A 256-row tile takes as long
-// as 1.84 128-row tiles; with fewer than six rounds of tiles the rounds are compared (128 rows against
-// 256, microseconds): m 4096, k 4096, n 4096, g 8 (4 rounds against 3) 177 -> 210; 512, 4096, 4096, 1 (1
-// against 1) 36 -> 52; 8192, 4096, 2304, 8 (5 against 3) 160 -> 169; but 6000, 4096, 1024, 8 (2 against
-// 1) 77 -> 70; 2048, 7168, 2048, 8 (2 against 1) 116 -> 101.  With many rounds 512 rows per group on
-// average is the line: 32768, 1536, 4096, 64 364 -> 335, 8192, 4096, 14336, 32 (256 rows) 1060 -> 1131.
-// e4m3 follows the same rule: m 8192, k 4096, n 14336, 8 groups 390 -> 378 us, 475 -> 466 us in a row.
-bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn) {
+// shallower smem ring) -- unless the larger tiles fill the SMs badly.
+// 512 rows per group and more: always from three rounds of 256-row tiles on (128 rows against 256, microseconds, m,
+// k, n, groups: 6120, 6528, 3304, 8 390 -> 319; 8304, 1768, 5112, 16 198 -> 173; 28448, 952, 576, 16 75 -> 69; 24104, 304, 2560, 6
+// 75 -> 68).  Below, the rounds are compared, a 256-row tile taking 1.5 times as long as a 128-row one: 4096, 4096,
+// 4096, 8 (4 rounds against 3) 177 -> 210; 512, 4096, 4096, 1 (1 against 1) 36 -> 52; but 6000, 4096, 1024, 8 (2 against 1)
+// 77 -> 70; 4352, 2928, 2232, 2 (3 against 2) 103 -> 93; 7184, 448, 2296, 8 (4 against 2) 38 -> 32.
+// 256 to 511 rows: only where 256-row tiles need fewer rounds even with a tile more per group than m asks for and
+// no tile more for 128 rows; 2048, 7168, 2048, 8 would take 2 rounds against 1 with unequal groups (116 -> 101) but
+// 1 against 1 with equal ones (74 -> 91), and 6352, 968, 896, 24 loses (30 -> 40).
+// e4m3, whose MMAs take half as long: 1.7 times, always from six rounds on, never with fewer than nine blocks of
+// the contraction (m 8192, k 4096, n 14336, 8 groups 390 -> 378; but 8192, 14336, 4096, 16, five rounds against
+// eight, 422 -> 472; 31480, 640, 1088, 32, five blocks, 46 -> 48).
+bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn, bool fp8 = false) {
   if (bn != 256 || g <= 0) return false;
   if (tgmm) return k >= 256;
-  if (m / g < 256) return false;
-  const int sms = sm_count();
+  const long long rows = m / g, sms = sm_count();
   const long long n_tiles = (static_cast<long long>(n) + 255) / 256;
+  auto rounds = [&](long long row_tiles) { return (row_tiles * n_tiles + sms - 1) / sms; };
+  const long long m128 = (m + 127) / 128, m256 = (m + 255) / 256;
+  if (rows < 512) return !fp8 && rows >= 256 && 1.84 * rounds(m256 + g) < static_cast<double>(rounds(m128));
   // a group's last tile is half full on average
-  const long long tiles128 = ((m + 127) / 128 + g / 2) * n_tiles, tiles256 = ((m + 255) / 256 + g / 2) * n_tiles;
-  if (tiles256 >= 6LL * sms) return m / g >= 512;
-  return 1.84 * static_cast<double>((tiles256 + sms - 1) / sms) < static_cast<double>((tiles128 + sms - 1) / sms);
+  const long long tiles256 = (m256 + g / 2) * n_tiles, r128 = rounds(m128 + g / 2);
+  if (fp8)
+    return (k + 127) / 128 >= 9 && (tiles256 >= 6 * sms || 1.7 * rounds(m256 + g / 2) < static_cast<double>(r128));
+  if (tiles256 >= 3 * sms) return true;
+  // a twentieth of a round is no round: the tiles of a group are an estimate
+  const long long r256 = (tiles256 - sms / 20 + sms - 1) / sms;
+  return 1.5 * (r256 > 0 ? r256 : 1) <= static_cast<double>(r128);
 }
 
 // tgmm with 256-row tiles: 512 x 256 tiles on CTA pairs (a quarter less L2 -> SM traffic, a
@@ -752,7 +774,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
                              two_half ? rd::kG2TileRows : rd::kTileM * cta_group, w, stream, by_weight);
     if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
   }
-  if (in_kernel && !f32 && split == 1 && split_allowed(cfg) && choose_swap(m, n, g, trans_rhs != 0)) {
+  if (in_kernel && !f32 && split == 1 && split_allowed(cfg) &&
+      choose_swap(m, (k + rd::kTileK - 1) / rd::kTileK, n, g, trans_rhs != 0, false)) {
     GemmArgs args = {};
     args.m = m; args.k = k; args.n = n; args.g = g;
     args.max_m_tiles = w.layout.max_tiles;
@@ -1726,7 +1749,7 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   if (cfg && (cfg->cta_group == 2 || cfg->tile_m == 256)) return RD_ERR_BAD_CONFIG;  // the library chooses
   if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return RD_ERR_BAD_CONFIG;
-  const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, n, g, bn);
+  const bool two_half = !(cfg && cfg->tile_m == 128) && choose_two_half(false, m, k, n, g, bn, true);
 
   const bool by_weight = cfg != nullptr && (cfg->flags & RD_CFG_GROUP_BY_WEIGHT) != 0;
   const bool in_kernel = inline_groups(m, g) && !(by_weight && group_to_weight != nullptr);
@@ -1744,7 +1767,8 @@ int rd_gmm_fp8(const void* x, const void* A, int num_weights, const int32_t* gro
     if (cudaGetLastError() != cudaSuccess) return RD_ERR_LAUNCH;
   }
 
-  if (in_kernel && split == 1 && split_allowed(cfg) && choose_swap(m, n, g, true)) {
+  if (in_kernel && split == 1 && split_allowed(cfg) &&
+      choose_swap(m, (k / 2 + rd::kTileK - 1) / rd::kTileK, n, g, true, true)) {
     GemmArgs args = {};
     args.m = m; args.k = k / 2; args.n = n; args.g = g;
     args.max_m_tiles = w.layout.max_tiles;

@@ -1272,7 +1272,7 @@ def test_float32_highest_splits_extreme_values():
 def test_gmm_fp8_on_256_row_tiles():
     """Long groups whose 256-row tiles need fewer rounds run on them: bit-equal to the 128-row kernel, which
     adds the same products in the same order, at tile edges and with and without a scale."""
-    m, k, n = 6000, 272, 1024
+    m, k, n = 6000, 1168, 1024
     gs = torch.tensor([257, 0, 1279 + 64, 1, 128, 256, 3000, 900], dtype=torch.int32)
     rng = np.random.default_rng(5)
     x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
@@ -1485,6 +1485,39 @@ def test_rows_on_the_n_side(dtype, m, k, n, sizes):
     got = swapped(lambda: ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc)).float()
     ref = ops.gmm_fp8_forward(x8, A8, gd, weight_scale=sc, cfg=rows128).float()
     assert float((got - ref).abs().max()) <= 2.0 ** -7 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("dtype,m,k,n,g,kernel", [
+    ("bf16", 6120, 72, 3304, 8, "ragged_gemm2_kernel"),       # three rounds of 256-row tiles
+    ("bf16", 7184, 448, 2296, 8, "ragged_gemm2_kernel"),      # two rounds and a hundredth
+    ("bf16", 4096, 72, 4096, 8, "ragged_gemm_kernel"),        # two rounds and a sixth
+    ("bf16", 6352, 72, 896, 24, "ragged_gemm_kernel"),        # 264 rows per group, as many rounds of either height
+    ("bf16", 4928, 264, 7232, 4, "ragged_gemm2_kernel"),      # a contraction of five blocks
+    ("bf16", 4928, 584, 7232, 4, "ragged_gemm_swap_kernel"),  # of ten
+    ("bf16", 26112, 264, 7168, 24, "ragged_gemm_swap_kernel"),  # of five, more than twenty rounds
+    ("e4m3", 8192, 1152, 4096, 16, "ragged_gemm_kernel"),     # five rounds against eight of half the size
+    ("e4m3", 8192, 1152, 4096, 8, "ragged_gemm_swap_kernel"),  # four against eight
+    ("e4m3", 4928, 528, 7232, 4, "ragged_gemm_kernel"),       # a contraction of five blocks
+])
+def test_tiles_of_long_groups(dtype, m, k, n, g, kernel):
+    """The kernel chosen on either side of the rules for long groups, and its result against that of 128-row
+    tiles (one 16-bit rounding apart), the last row in no group."""
+    gen = torch.Generator(device=DEV).manual_seed(m + n)
+    x = torch.randn((m, k), device=DEV, generator=gen).bfloat16()
+    A = torch.randn((g, n, k), device=DEV, generator=gen).bfloat16()
+    gs = torch.full((g,), m // g, dtype=torch.int32, device=DEV)
+    gs[0] -= 1
+    whole = _lib.TileCfg(256, 0, 1, 128, 0)
+    if dtype == "e4m3":
+        x, A = x.to(torch.float8_e4m3fn), A.to(torch.float8_e4m3fn)
+        got, names = launched.kernels(lambda: ops.gmm_fp8_forward(x, A, gs))
+        ref = ops.gmm_fp8_forward(x, A, gs, cfg=whole)
+    else:
+        got, names = launched.kernels(lambda: ops.gmm_forward(x, A, gs, trans_rhs=True))
+        ref = ops.gmm_forward(x, A, gs, trans_rhs=True, cfg=whole)
+    assert any(kernel + "<" in name for name in names), names
+    assert float((got.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
+    assert float(got[int(gs.sum()):].abs().max()) == 0.0
 
 
 @pytest.mark.parametrize("n", [8, 248, 264, 520, 1432])
