@@ -410,9 +410,10 @@ int launch_gemm_f32_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
 
 // Cluster size for a gmm whose tiles are too few for the SMs (rd_gemm_splitk.cuh), 1 = no split.
 // `tiles` bounds the live tiles, `rows` is what a large tile may hold.  All clusters must be resident at
-// once and every CTA gets at least four 64-deep blocks.  A block takes a lone CTA 0.3 to 0.4 us;
-// adding the partial sums up costs about 1 us and 10 us more for 128 rows (1024 rows in 2 groups, k
-// 1024, n 1024: 17 us whole, 25 us split; 300 rows in 4 groups, k 8192, n 256: 55 and 27).
+// once and every CTA gets at least four 64-deep blocks.  Split where the contraction of a tile on one CTA
+// (0.3 us per block) takes longer than 3 us and 15 us more for 128 rows: adding the partial sums up costs
+// about 1 us and 10 us more for 128 rows, the rest is a margin (1024 rows in 2 groups, k 1024, n 1024,
+// 16 blocks: 17 us whole, 25 us split; 300 rows in 4 groups, k 8192, n 256, 128 blocks: 55 and 27).
 template <bool kBKMajor, bool kFp8>
 int choose_split(long long tiles, int rows, int k_blocks) {
   const int sms = sm_count();
@@ -1256,6 +1257,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   // The float32 kernels likewise, with blocks of 32 columns.
   const bool f32_pair = f32 && cta_group == 2;
   const bool blocked = f32 ? (k % 32 == 0 && n % 32 == 0) : (two_half && k % 64 == 0 && n % 64 == 0);
+  if (f32_pair && !three_pass && !blocked) return RD_ERR_BAD_CONFIG;  // choose_f32_pair does not ask for it
   CUtensorMap ta, tb;
   if (blocked && f32) {
     rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kF32TileK, rd::kTileM / 32);

@@ -24,8 +24,8 @@
 // Measured (m 4096, k 4096, n 1536, 8 groups, three products): 0.25 / 0.25 / 0.24 ms for gmm / trans_rhs
 // / tgmm = 610 to 640 TFLOP/s of TF32 MMAs, where splitting in torch and three launches took 0.99 /
 // 0.92 / 0.85 ms; forward + backward 2.78 -> 0.87 ms.  The [32][32] boxes of an MN-major operand come as ONE
-// box of a column-blocked view where its rows are multiples of 32: with four 4 KB boxes a
-// one-product gmm took 0.220 instead of 0.161 ms.  One product: see choose_f32_pair in rd_api.cu.
+// box of a column-blocked view where its rows are multiples of 32; other rows, four 4 KB boxes per operand,
+// only reach the three-product form.  One product, measured on both sides: choose_f32_pair in rd_api.cu.
 //
 // Roles: warp 0 = TMA producer, warp 1 = MMA issuer (one thread, of the leader CTA), warps 2..5 =
 // epilogue, warps 6.. = converters (kSplit, eight) or the tail fixer (one, tgmm).  tgmm rows past
@@ -184,7 +184,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           if (kTgmm) {
             const int r = t.row0 + kb * kF32TileK;
-            if (p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, 4 blocks of 32 columns)
+            if (!kSplit || p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, 4 blocks of 32 columns)
               load_3d(remote_bar, sa, &tmap_a, full, 0, r, t.k0 >> 5);
               load_3d(remote_bar, sb, &tmap_b, full, 0, r, nb >> 5);
             } else {
