@@ -51,6 +51,15 @@ def test_tile_table_lookup(tmp_path, monkeypatch):
     monkeypatch.setattr(tile_table, "_entries", None)
 
 
+def test_tile_table_entries_are_bounded():
+    """An entry is an exception to the library's rules at the sizes it was measured at: a finite range of m."""
+    assert tile_table.lookup("gmm_t", 8192, 14336, 4096, 16) is not None
+    for e in tile_table._load():
+        assert 0 < e["m_min"] <= e["m_max"] <= 4 * e["m_min"], e
+        assert tile_table.lookup(e["op"], e["m_min"] // 8, e["k"], e["n"], e["g"]) is None
+        assert tile_table.lookup(e["op"], e["m_max"] * 8, e["k"], e["n"], e["g"]) is None
+
+
 def test_reference_signature_is_kept():
     import inspect
 
