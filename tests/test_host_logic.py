@@ -60,6 +60,25 @@ def test_tile_table_entries_are_bounded():
         assert tile_table.lookup(e["op"], e["m_max"] * 8, e["k"], e["n"], e["g"]) is None
 
 
+def test_tuner_writes_no_entry_where_the_rules_win(tmp_path, monkeypatch):
+    """A sweep competes with the library's own choice, which may be a kernel that no tile configuration names."""
+    import json
+    import sys
+
+    from gpu_ragged_dot_b200 import tune
+
+    assert tune.RULES in tune.CANDIDATES
+    path = tmp_path / "t.json"
+    path.write_text('{"entries": []}')
+    monkeypatch.setattr(tile_table, "_TABLE_PATH", str(path))
+    monkeypatch.setattr(tune._lib, "load", lambda: None)
+    monkeypatch.setattr(tune, "sweep_shape", lambda *a, **kw: {"gmm": [(1.0, tune.RULES), (1.1, (256, 1, 128))],
+                                                               "tgmm": [(1.0, (256, 1, 128)), (1.1, tune.RULES)]})
+    monkeypatch.setattr(sys, "argv", ["tune", "--shape", "512,256,384,8", "--write"])
+    tune.main()
+    assert [e["op"] for e in json.loads(path.read_text())["entries"]] == ["tgmm"]
+
+
 def test_reference_signature_is_kept():
     import inspect
 
