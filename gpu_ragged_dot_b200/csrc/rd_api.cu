@@ -20,6 +20,7 @@
 #include "rd_gemm_swap.cuh"
 #include "rd_metadata.cuh"
 #include "rd_rows.cuh"
+#include "rd_tgmm.cuh"
 
 namespace {
 
@@ -254,11 +255,11 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 // then land on SMs in the order in which the kernel before leaves them, and neighbours in the tile
 // order, which share operand panels, no longer lie side by side (Mixtral-shaped training step 2.57 ->
 // 2.70 ms, 64 groups 1.41 -> 1.54 ms, 256 groups 5.1 -> 5.5 ms).
-bool launch_early(const GemmArgs& args) {
+bool launch_early(const GemmArgs& args, int ctas_per_tile = 1) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
                                                : static_cast<long long>(args.m < args.g ? args.m : args.g) + args.m / rd::kTileM;
-  return row_tiles * args.n_tiles <= sm_count();
+  return row_tiles * args.n_tiles * ctas_per_tile <= sm_count();
 }
 
 // How many clusters of two CTAs can be resident at once (0: the query failed).
@@ -284,9 +285,9 @@ int resident_pairs(Kernel kernel, int threads, size_t smem_bytes) {
 }
 
 // A persistent grid of pairs must be fully co-resident.
-template <typename Kernel>
-int launch_pairs(Kernel kernel, int threads, int smem_bytes, const CUtensorMap& ta, const CUtensorMap& tb,
-                 const CUtensorMap& tout, const GemmArgs& args, int ctas, cudaStream_t stream) {
+template <typename Kernel, typename... Maps>
+int launch_pairs(Kernel kernel, int threads, int smem_bytes, const GemmArgs& args, int ctas, cudaStream_t stream,
+                 const Maps&... maps) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
     return RD_ERR_LAUNCH;
   const int clusters = resident_pairs(kernel, threads, smem_bytes);
@@ -294,7 +295,7 @@ int launch_pairs(Kernel kernel, int threads, int smem_bytes, const CUtensorMap& 
   int pairs = ctas / 2;
   if (pairs > clusters) pairs = clusters;
   if (pairs < 1) pairs = 1;
-  return launch_kernel(kernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args), stream, ta, tb, tout, args);
+  return launch_kernel(kernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args, 2), stream, maps..., args);
 }
 
 template <int BN, bool kBKMajor, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false>
@@ -304,7 +305,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   constexpr int kStages = (196608 / kStageBytes) > 8 ? 8 : (196608 / kStageBytes);
   constexpr int kSmem = kStages * kStageBytes + rd::kOutStagingBytes + 1024;
   auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, kCtas, kSeg, kFp8>;
-  if (kCtas == 2) return launch_pairs(kernel, rd::kGemmFixerThreads, kSmem, ta, tb, tout, args, ctas, stream);
+  if (kCtas == 2) return launch_pairs(kernel, rd::kGemmFixerThreads, kSmem, args, ctas, stream, ta, tb, tout);
   // The attribute is per device; setting it again is cheap, so do it on every call rather
   // than track which devices have seen it.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -371,9 +372,6 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
     if (args.ready_flags != nullptr || args.send.world > 0)
       return launch_gemm2<kBKMajor, false, true>(ta, tb, tout, args, ctas, stream);
   }
-  if constexpr (kTgmm && !kVariant) {
-    if (args.seg_count > 1) return launch_gemm2<false, true, true>(ta, tb, tout, args, ctas, stream);
-  }
   auto kernel = rd::ragged_gemm2_kernel<kBKMajor, kTgmm, kVariant>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kG2SmemBytes) !=
       cudaSuccess)
@@ -385,7 +383,7 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
 // e4m3 on 256-row tiles (rd_gemm2.cuh, kFp8).
 int launch_gemm2_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout, const GemmArgs& args,
                      int ctas, cudaStream_t stream) {
-  auto kernel = rd::ragged_gemm2_kernel<true, false, false, false, true>;
+  auto kernel = rd::ragged_gemm2_kernel<true, false, false, true>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kG2SmemBytes) !=
       cudaSuccess)
     return RD_ERR_LAUNCH;
@@ -393,19 +391,12 @@ int launch_gemm2_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
                        args);
 }
 
-// tgmm with 512 x 256 tiles on CTA pairs (rd_gemm2.cuh, kPair).
-int launch_gemm2_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
-                      const GemmArgs& args, int ctas, cudaStream_t stream) {
-  return launch_pairs(rd::ragged_gemm2_kernel<false, true, false, true>, rd::kG2Threads, rd::kG2PairSmemBytes, ta,
-                      tb, tout, args, ctas, stream);
-}
-
 // float32 on CTA pairs (rd_gemm_f32_pair.cuh).
 template <bool kBKMajor, bool kTgmm, bool kSplit>
 int launch_gemm_f32_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout, const GemmArgs& args,
                          int ctas, cudaStream_t stream) {
   return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, kSplit>, rd::f32_pair_threads<kSplit>(),
-                      rd::f32_pair_smem_bytes<kSplit>(), ta, tb, tout, args, ctas, stream);
+                      rd::f32_pair_smem_bytes<kSplit>(), args, ctas, stream, ta, tb, tout);
 }
 
 // Cluster size for a gmm whose tiles are too few for the SMs (rd_gemm_splitk.cuh), 1 = no split.
@@ -494,13 +485,8 @@ template <bool kBKMajor, bool kFp8>
 int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_weights, GemmArgs args,
                      cudaStream_t stream) {
   CUtensorMap tw, tx, tout;
-  int rc;
-  {
-    const uint64_t dims[2] = {static_cast<uint64_t>(args.k), static_cast<uint64_t>(args.m)};
-    const uint32_t box[2] = {64, rd::kSwapRows / 2};
-    rc = encode_map(&tx, x, dtype, 2, dims, box);
-    if (rc != RD_OK) return rc;
-  }
+  int rc = encode_rows_map(&tx, x, dtype, args.k, args.m, rd::kSwapRows / 2);
+  if (rc != RD_OK) return rc;
   if (kBKMajor) {
     const uint64_t dims[3] = {static_cast<uint64_t>(args.k), static_cast<uint64_t>(args.n),
                               static_cast<uint64_t>(num_weights)};
@@ -517,8 +503,33 @@ int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_w
     if (rc != RD_OK) return rc;
   }
   args.n_tiles = (args.n + rd::kSwapCols - 1) / rd::kSwapCols;
-  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8>, rd::kSwapThreads, rd::kSwapSmemBytes, tw, tx, tout,
-                      args, sm_count(), stream);
+  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8>, rd::kSwapThreads, rd::kSwapSmemBytes, args,
+                      sm_count(), stream, tw, tx, tout);
+}
+
+// Tensor maps and launch of tgmm with two accumulators per CTA (rd_tgmm.cuh); args.k_tiles and n_tiles are set.
+template <int kCtas>
+int launch_tgmm(const void* x, const void* dout, const CUtensorMap& tout, int dtype, const GemmArgs& args, int ctas,
+                cudaStream_t stream) {
+  CUtensorMap ta, ta2, tb, tb2;
+  int rc = encode_rows_map(&ta2, x, dtype, args.k, args.m, rd::kTileK);
+  if (rc != RD_OK) return rc;
+  rc = encode_rows_map(&tb2, dout, dtype, args.n, args.m, rd::kTileK);
+  if (rc != RD_OK) return rc;
+  // Whole blocks of 64 columns only; the kernel reads what is left through the plain maps.
+  ta = ta2;
+  tb = tb2;
+  if (args.k >= 64) rc = encode_blocked_map(&ta, x, dtype, args.k, args.m, rd::kTileK, rd::kTileM / 64);
+  if (rc == RD_OK && args.n >= 64)
+    rc = encode_blocked_map(&tb, dout, dtype, args.n, args.m, rd::kTileK, rd::kTgTileN / 64 / kCtas);
+  if (rc != RD_OK) return rc;
+  auto kernel = rd::ragged_tgmm_kernel<kCtas>;
+  constexpr int kSmem = rd::tg_smem_bytes<kCtas>();
+  if constexpr (kCtas == 2)
+    return launch_pairs(kernel, rd::kTgThreads, kSmem, args, ctas, stream, ta, ta2, tb, tb2, tout);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
+    return RD_ERR_LAUNCH;
+  return launch_kernel(kernel, ctas, rd::kTgThreads, kSmem, 1, launch_early(args), stream, ta, ta2, tb, tb2, tout, args);
 }
 
 // Upper bound on the live 128 x 256 tiles of a gmm: a group has at least one row, and only whole
@@ -572,12 +583,6 @@ bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn, bool f
   return 1.5 * (r256 > 0 ? r256 : 1) <= static_cast<double>(r128);
 }
 
-// tgmm with 256-row tiles: 512 x 256 tiles on CTA pairs (a quarter less L2 -> SM traffic, a
-// fourth stage) were 0.6-2.4 % faster than one CTA per tile on every compute-bound shape swept
-// (m/g 512 to 2048; k 4096 and 7168; n 1536 to 14336).  Short groups make tgmm output-bound and
-// were not measured: they stay on one CTA.
-bool choose_pair_512(long long m, int k, int g) { return k >= 512 && g > 0 && m / g >= 512; }
-
 // float32 tiles on CTA pairs (rd_gemm_f32_pair.cuh).  A caller who asks for three TF32 passes always
 // gets them: only that kernel splits its operands.  One pass: tgmm on groups of 256 rows and more with
 // rows that are multiples of 32.  One CTA against a pair, microseconds: k 1024, n 4096, 32 groups of 256
@@ -591,38 +596,24 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
   return k >= 256 && m / g >= 256 && k % 32 == 0 && n % 32 == 0;
 }
 
-// Is a tgmm bound by an output whose rows are not multiples of 32 bytes?  Boxes then begin and end inside
-// sectors, which costs L2 reads of what it has not got; the 128-row kernel, whose boxes of a row
-// follow one another more closely, suffers least.  128-row against 256-row tiles, microseconds: n 3240 (k
-// 11600, 45 groups of 97 rows) 1047 and 1394, n 11672 (k 2216, 51 groups of 99) 884 and 990, where n 3232
-// and 11680 take 702 and 652; long groups are bound by the MMAs: n 4104 (8 groups of 1024 rows) 294 and 228.
-// (Cache hints on loads or stores change nothing; storing whole rows of a tile, or eight rows of four
-// boxes together, was slower.)
-bool split_sector_output(long long m, int n, int g) { return n % 16 != 0 && g > 0 && m / g < 256; }
-
-// Tile height of a tgmm with few rounds of tiles: 128 or 256 on one CTA, or 0 when there are six rounds of
-// 256-row tiles and more, or pairs need fewer rounds (then the rules above decide).  A 128-row tile
-// takes 0.58 times as long as a 256-row one.  Microseconds for 128 rows, 256 rows, pair: m 4096, k 1024, n
-// 1024, 4 groups (1, 1, 1 rounds) 17.3, 23.4, 23.5; 32768, 512, 512, 8 (1, 1, 1) 38, 54, 54; 8192, 4096, 1536, 2
-// (3, 2, 2) 87, 99, 99; 8106, 2552, 384, 9 (3, 2, 2) 34, 36, 38; 4096, 768, 3072, 8 (4, 2, 3) 27.6, 27.7, 33.8;
-// 8192, 1024, 768, 8 (2, 1, 1) 25.5, 23.5, 25.6; 3000, 4096, 4096, 1 (4, 2, 2) 87, 77, 79.
-int tgmm_tile_by_rounds(int k, int n, int g) {
-  if (k < 256) return 0;
+// tgmm with 256-column tiles (rd_tgmm.cuh): 256 x 256 on CTA pairs, or 128 x 256 on one CTA each?  A pair moves a third
+// less data into shared memory.  Microseconds in a row, one CTA against a pair:
+// - Groups of 256 rows and more: pairs, up to a quarter more rounds of tiles (m 8192, k 4096, n 14336, 8 groups 908 ->
+//   722; 21272, 600, 5440, 49, 37 rounds against 44, 207 -> 190; 20312, 288, 280, 38, 2 against 3, equal).
+// - Shorter groups: pairs where they take no more rounds and more than two (16384, 7168, 2048, 128 972 -> 851; 3000,
+//   2048, 2048, 30 72 -> 69; 5024, 272, 1352, 124, 16 against 21 rounds, 35 -> 37).  With one or two rounds the start of a
+//   cluster is a good part of the time (512, 256, 384, 8, one round, alone 11 -> 13).
+// - Output rows that are not multiples of 32 bytes, groups of 100 rows and less: boxes begin and end inside sectors,
+//   which costs L2 reads of what it has not got; the one-CTA tiles, whose boxes of a row follow one another more
+//   closely, suffer less (4365, 11600, 3240, 45 1134 -> 1299; 6192, 3480, 840, 74 147 -> 173; 103 rows per group, 3512,
+//   8168, 648, 34 119 -> 112).
+bool choose_tgmm_pair(long long m, int k, int n, int g) {
   const long long sms = sm_count(), cols = (static_cast<long long>(n) + 255) / 256 * g;
-  auto rounds = [&](int rows, long long units) { return ((k + rows - 1) / rows * cols + units - 1) / units; };
-  const long long r128 = rounds(128, sms), r256 = rounds(256, sms), r512 = rounds(512, sms / 2);
-  if (r256 >= 6) return 0;
-  if (0.58 * static_cast<double>(r128) < static_cast<double>(r256)) return 128;
-  return r256 <= r512 ? 256 : 0;
-}
-
-// CTA pairs (256 x 256 tiles, B operand split between the two CTAs) pay off where the
-// 256-row granularity wastes nothing: tgmm, whose tile rows are the dense k axis.  For gmm the
-// tile rows are a group's ragged token rows and the wider tile wastes more than the pair
-// saves at the benchmark group sizes, so gmm pairs only on request (rd_tile_cfg.cta_group).
-bool choose_pair(bool tgmm, long long tiles256, int bn, int sms) {
-  if (!tgmm || bn != 256) return false;
-  return tiles256 >= 2LL * (sms / 2);
+  const long long r1 = ((k + 127) / 128 * cols + sms - 1) / sms;
+  const long long r2 = ((k + 255) / 256 * cols + sms / 2 - 1) / (sms / 2);
+  if (m / g >= 256) return 4 * r2 <= 5 * r1;
+  if (n % 16 != 0 && m / g <= 100) return false;
+  return r2 <= r1 && r1 > 2;
 }
 
 // Limit of every bounded wait inside a kernel, in microseconds: rd_tile_cfg.wait_limit_ms if
@@ -739,7 +730,8 @@ static int gmm_impl(const void* x, const void* A, const int32_t* group_sizes,
   if (bn != 64 && bn != 128 && bn != 256) return RD_ERR_BAD_CONFIG;
   int cta_group = cfg ? cfg->cta_group : 0;
   if (cta_group < 0 || cta_group > 2 || (cta_group == 2 && bn != 256)) return RD_ERR_BAD_CONFIG;
-  if (cta_group == 0) cta_group = choose_pair(false, 0, bn, sms) ? 2 : 1;
+  // 256-row tiles on pairs waste more of a group's last rows than the pair saves: only on request.
+  if (cta_group == 0) cta_group = 1;
   int tile_m = cfg ? cfg->tile_m : 0;
   if (tile_m != 0 && tile_m != 128 && tile_m != 256) return RD_ERR_BAD_CONFIG;
   if (tile_m == 256 && (bn != 256 || cta_group != 1)) return RD_ERR_BAD_CONFIG;
@@ -1218,29 +1210,16 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (cta_group == 2) return RD_ERR_BAD_CONFIG;
     cta_group = 1;
   }
-  if (tile_m == 0 && cta_group == 0 && bn == 256 && !f32 && seg_count == 1) {
-    if (split_sector_output(m, n, g)) {
-      tile_m = 128;
-    } else {
-      tile_m = tgmm_tile_by_rounds(k, n, g);
-    }
-    if (tile_m != 0) cta_group = 1;
+  // 256 columns, plain: the kernel with two accumulators, whatever tile height the caller names.
+  const bool two_acc = !f32 && bn == 256 && seg_count == 1;
+  if (two_acc) {
+    tile_m = 128;
+    if (cta_group == 0) cta_group = choose_tgmm_pair(m, k, n, g) ? 2 : 1;
   }
-  // Preference order when nothing is forced: 256-row tiles on one CTA, then a CTA pair, then
-  // plain 128-row tiles.
-  if (tile_m == 0 && cta_group != 2) tile_m = choose_two_half(true, m, k, n, g, bn) ? 256 : 128;
-  if (tile_m == 0) tile_m = 128;
-  if (cta_group == 0) {
-    if (tile_m == 256) {
-      cta_group = (seg_count == 1 && choose_pair_512(m, k, g)) ? 2 : 1;
-    } else {
-      cta_group = choose_pair(true, static_cast<long long>((k + 255) / 256) * g * ((n + 255) / 256), bn, sms)
-                      ? 2
-                      : 1;
-    }
-  }
+  if (cta_group == 0) cta_group = 1;
+  if (tile_m == 0) tile_m = choose_two_half(true, m, k, n, g, bn) ? 256 : 128;
   const bool two_half = tile_m == 256;
-  const int tile_rows = two_half ? rd::kG2TileRows * cta_group : rd::kTileM * cta_group;
+  const int tile_rows = two_half ? rd::kG2TileRows : rd::kTileM * cta_group;
   const long long k_tiles = (k + tile_rows - 1) / tile_rows;
 
   const bool in_kernel = seg_count == 1 && inline_groups(m, g);
@@ -1256,7 +1235,8 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   // rows exactly (see rd_gemm2.cuh); otherwise one 2-D box per 64 columns.
   // The float32 kernels likewise, with blocks of 32 columns.
   const bool f32_pair = f32 && cta_group == 2;
-  const bool blocked = f32 ? (k % 32 == 0 && n % 32 == 0) : (two_half && k % 64 == 0 && n % 64 == 0);
+  const bool blocked = f32 ? (k % 32 == 0 && n % 32 == 0)
+                           : (two_half && k % 64 == 0 && n % 64 == 0);
   if (f32_pair && !three_pass && !blocked) return RD_ERR_BAD_CONFIG;  // choose_f32_pair does not ask for it
   CUtensorMap ta, tb;
   if (blocked && f32) {
@@ -1267,7 +1247,7 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   } else if (blocked) {
     rc = encode_blocked_map(&ta, x, dtype, k, m, rd::kTileK, rd::kG2TileRows / 64);
     if (rc != RD_OK) return rc;
-    rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kTileK, rd::kG2TileN / 64 / cta_group);
+    rc = encode_blocked_map(&tb, dout, dtype, n, m, rd::kTileK, rd::kG2TileN / 64);
     if (rc != RD_OK) return rc;
   } else {
     {
@@ -1321,15 +1301,15 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (bn == 128) return launch_gemm_f32<128, false, true>(ta, tb, tout, args, ctas, stream);
     return launch_gemm_f32<64, false, true>(ta, tb, tout, args, ctas, stream);
   }
-  if (two_half && cta_group == 2) return launch_gemm2_pair(ta, tb, tout, args, ctas, stream);
-  if (two_half) return launch_gemm2<false, true>(ta, tb, tout, args, ctas, stream);
+  if (two_half) return launch_gemm2<false, true, true>(ta, tb, tout, args, ctas, stream);  // strided segments
   if (seg_count > 1) {
     if (bn == 256) return launch_gemm<256, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
     if (bn == 128) return launch_gemm<128, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
     return launch_gemm<64, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
   }
-  if (cta_group == 2) return launch_gemm<256, false, true, 2>(ta, tb, tout, args, ctas, stream);
-  if (bn == 256) return launch_gemm<256, false, true, 1>(ta, tb, tout, args, ctas, stream);
+  if (two_acc)
+    return cta_group == 2 ? launch_tgmm<2>(x, dout, tout, dtype, args, ctas, stream)
+                          : launch_tgmm<1>(x, dout, tout, dtype, args, ctas, stream);
   if (bn == 128) return launch_gemm<128, false, true, 1>(ta, tb, tout, args, ctas, stream);
   return launch_gemm<64, false, true, 1>(ta, tb, tout, args, ctas, stream);
 }

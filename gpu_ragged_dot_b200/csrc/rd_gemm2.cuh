@@ -18,14 +18,6 @@
 // staging + TMA stores, row-masked stores where a gmm slab crosses its group's end) as
 // rd_gemm.cuh; the helpers of that file are reused.
 //
-// kPair (tgmm only): two CTAs of a cluster own a 512 x 256 tile, CTA c its rows [256 c, 256 c +
-// 256).  Half h is ONE tcgen05.mma.cta_group::2 product of 256 rows, rows [128 h, 128 h + 128) of
-// either CTA; each CTA loads its own rows of the A operand (32 KB) and HALF of the B operand's
-// columns (16 KB), so a stage is 48 KB for the same MMAs per SM, a quarter less L2 -> SM traffic
-// per flop, and four stages fit.  The hand-shakes between the two CTAs are those of the 128-row
-// pair kernel in rd_gemm.cuh.  Measured on the Mixtral-shaped weight gradient it moves 5.8 GB
-// instead of 7.75 GB from L2 and takes 0.71-0.73 ms against 0.72-0.74 ms for one CTA per tile.
-//
 // Blocked operand maps (GemmArgs::blocked_maps, tgmm): x and dout are described to TMA as
 // (64 columns, rows, blocks of 64 columns), so ONE box of (64, 64 rows, 4 blocks) = 32 KB lands as
 // the same four [64 rows][128 B] slabs that four 2-D boxes would write: two TMA instructions per
@@ -41,7 +33,6 @@ constexpr int kG2EpilogueWarps = 8;
 constexpr int kG2FixerWarp = 2 + kG2EpilogueWarps;  // warp 10: clears tail rows of tgmm stages
 constexpr int kG2Threads = 64 + 32 * kG2EpilogueWarps + 32;
 constexpr int kG2Stages = 3;
-constexpr int kG2PairStages = 4;  // 48 KB stages when a CTA pair shares the B operand
 constexpr int kG2TileN = 256;
 constexpr int kG2TileRows = 2 * kTileM;
 constexpr int kG2TgmmBand = 8;  // column tiles per band of the tgmm tile order
@@ -49,8 +40,6 @@ constexpr uint32_t kG2ABytes = 2 * kTileM * kTileK * 2;   // two 128-row halves
 constexpr uint32_t kG2BBytes = kG2TileN * kTileK * 2;
 constexpr uint32_t kG2StageBytes = kG2ABytes + kG2BBytes;  // 64 KB
 constexpr int kG2SmemBytes = kG2Stages * kG2StageBytes + kG2EpilogueWarps * kOutBoxBytes + 1024;
-constexpr uint32_t kG2PairStageBytes = kG2ABytes + kG2BBytes / 2;  // 48 KB
-constexpr int kG2PairSmemBytes = kG2PairStages * kG2PairStageBytes + kG2EpilogueWarps * kOutBoxBytes + 1024;
 
 // rows: valid rows of the whole 256-row tile (gmm) / rows of the group (tgmm).
 __device__ __forceinline__ TileCoord decode_gmm_tile256(const GemmArgs& p, const GroupTable* tab, int tile) {
@@ -99,31 +88,28 @@ __device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, cons
 //   tgmm: strided segments (a block contracts over several row ranges, rd_tgmm_strided).
 // kFp8: e4m3 operands, gmm with K-major weights; tiles are byte for byte those of a 16-bit problem with
 // k / 2 elements per row (see rd_gemm.cuh).
-template <bool kBKMajor, bool kTgmm, bool kVariant = false, bool kPair = false, bool kFp8 = false>
+template <bool kBKMajor, bool kTgmm, bool kVariant = false, bool kFp8 = false>
 __global__ void __launch_bounds__(kG2Threads, 1)
 ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
   static_assert(!(kTgmm && kBKMajor), "tgmm reads both operands MN-major");
-  static_assert(!kFp8 || (kBKMajor && !kTgmm && !kVariant && !kPair), "8-bit inputs: plain gmm, K-major weights");
-  static_assert(!kPair || (kTgmm && !kVariant), "CTA pairs: plain tgmm only");
+  static_assert(!kFp8 || (kBKMajor && !kTgmm && !kVariant), "8-bit inputs: plain gmm, K-major weights");
+  static_assert(!kTgmm || kVariant, "plain tgmm: rd_tgmm.cuh");
   constexpr bool kEp = !kTgmm && kVariant;
   constexpr bool kSeg = kTgmm && kVariant;
-  constexpr int kCtas = kPair ? 2 : 1;
   constexpr int BN = kG2TileN;
-  constexpr int kBCols = BN / kCtas;  // B-operand columns this CTA loads
-  constexpr int kStages = kPair ? kG2PairStages : kG2Stages;
+  constexpr int kStages = kG2Stages;
   constexpr uint32_t kHalfABytes = kTileM * kTileK * 2;  // 16 KB
-  constexpr uint32_t kBBytes = kBCols * kTileK * 2;
-  constexpr uint32_t kStageBytes = kG2ABytes + kBBytes;  // 64 KB, 48 KB in a pair
+  constexpr uint32_t kBBytes = BN * kTileK * 2;
+  constexpr uint32_t kStageBytes = kG2ABytes + kBBytes;  // 64 KB
   constexpr uint32_t kTmemCols = 2 * BN;                 // accumulator of half h at column h * BN
-  constexpr int kCtaRows = 2 * kTileM;                   // output rows of one CTA (both halves)
 
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kStages];
   __shared__ __align__(8) uint64_t bar_empty[kStages];
   __shared__ __align__(8) uint64_t bar_acc_full[2];   // per half
-  __shared__ __align__(8) uint64_t bar_acc_empty[2];  // per half (pair: the leader's is used)
+  __shared__ __align__(8) uint64_t bar_acc_empty[2];  // per half
   __shared__ __align__(8) uint64_t bar_tail_go;    // MMA thread -> fixer warp(s): a stage with tail rows has landed
   __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp(s) -> MMA thread: its tail rows are cleared
   __shared__ uint32_t tmem_slot;
@@ -133,8 +119,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
-  const int cta_rank = kPair ? static_cast<int>(cluster_cta_rank()) : 0;
-  const bool leader = cta_rank == 0;
 
   // Fused expert-parallel exchange: some CTAs of the grid send rows instead of multiplying.
   // The senders are the FIRST CTAs of the grid, so they are resident before any CTA that may wait
@@ -161,20 +145,19 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     for (int h = 0; h < 2; ++h) {
       mbar_init(smem_u32(&bar_acc_full[h]), 1);
-      mbar_init(smem_u32(&bar_acc_empty[h]), 4 * kCtas);  // the four epilogue warps of that half (per CTA)
+      mbar_init(smem_u32(&bar_acc_empty[h]), 4);  // the four epilogue warps of that half
     }
     mbar_init(smem_u32(&bar_tail_go), 1);
-    mbar_init(smem_u32(&bar_tail_done), kCtas);  // one arrival per CTA's fixer warp (pair: the leader's is used)
+    mbar_init(smem_u32(&bar_tail_done), 1);
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc<kCtas>(smem_u32(&tmem_slot), kTmemCols);
-    tmem_relinquish<kCtas>();
+    tmem_alloc<1>(smem_u32(&tmem_slot), kTmemCols);
+    tmem_relinquish<1>();
   }
   start_inline_groups(p, kTgmm ? kTileM : kG2TileRows, &group_table, warp, lane);
   tc_fence_before_sync();
   __syncthreads();
-  if constexpr (kPair) cluster_sync();  // the peer's barriers exist before anything arrives on them
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
   volatile WaitCtl* abort_ptr = &wait_ctl;
@@ -182,15 +165,12 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int num_tiles =
       kTgmm ? p.g * p.k_tiles * p.n_tiles : live_row_tiles(p, &group_table) * p.n_tiles;
   const int k_blocks_gmm = (p.k + kTileK - 1) / kTileK;
-  const int tile_step = kPair ? static_cast<int>(gridDim.x >> 1)
-                        : kEp ? static_cast<int>(gridDim.x) - sender_ctas : static_cast<int>(gridDim.x);
+  const int tile_step = kEp ? static_cast<int>(gridDim.x) - sender_ctas : static_cast<int>(gridDim.x);
   auto first_tile = [&]() -> int {
-    if constexpr (kPair) return static_cast<int>(blockIdx.x >> 1);
     if constexpr (kEp) return static_cast<int>(blockIdx.x) - sender_ctas;
     return static_cast<int>(blockIdx.x);
   };
   auto decode = [&](int tile) -> TileCoord {
-    if constexpr (kPair) return decode_tgmm_tile256<2 * kG2TileRows>(p, &group_table, tile);
     if constexpr (kTgmm) return decode_tgmm_tile256(p, &group_table, tile);
     return decode_gmm_tile256(p, &group_table, tile);
   };
@@ -238,46 +218,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const uint32_t sa = stage_base + s * kStageBytes;
           const uint32_t sb = sa + kG2ABytes;
           const uint32_t own_bytes = halves * kHalfABytes + kBBytes;
-          if constexpr (kPair) {
-            // The peer's bytes are counted on the leader's barrier, except for the stage whose tail
-            // rows the peer has to clear first (it then needs to see its own data land).
-            const bool local_stage = kb == kb_count - 1 && tail_needs_clearing(t.rows);
-            int r, live;
-            tgmm_block<false>(p, t, blocks, kb, r, live);
-            const int ka = t.k0 + cta_rank * kCtaRows;
-            const int nb = t.n0 + cta_rank * kBCols;
-            const uint32_t bytes = p.blocked_maps ? kStageBytes : own_bytes;  // a blocked A box always has both halves
-            if (leader || local_stage) {
-              mbar_arrive_expect_tx(full, (leader && !local_stage) ? 2 * bytes : bytes);
-              if (p.blocked_maps) {
-                tma_load_3d_hint(sa, &tmap_a, full, 0, r, ka >> 6, keep);
-                tma_load_3d_hint(sb, &tmap_b, full, 0, r, nb >> 6, keep);
-              } else {
-                for (int h = 0; h < halves; ++h) {
-                  tma_load_2d_hint(sa + h * kHalfABytes, &tmap_a, full, ka + h * kTileM, r, keep);
-                  tma_load_2d_hint(sa + h * kHalfABytes + kBoxBytes, &tmap_a, full, ka + h * kTileM + 64, r, keep);
-                }
-#pragma unroll
-                for (int j = 0; j < kBCols / 64; ++j)
-                  tma_load_2d_hint(sb + j * kBoxBytes, &tmap_b, full, nb + j * 64, r, keep);
-              }
-            } else {
-              full = map_to_cta(full, 0);
-              if (p.blocked_maps) {
-                tma_load_3d_pair_hint(sa, &tmap_a, full, 0, r, ka >> 6, keep);
-                tma_load_3d_pair_hint(sb, &tmap_b, full, 0, r, nb >> 6, keep);
-              } else {
-                for (int h = 0; h < halves; ++h) {
-                  tma_load_2d_pair_hint(sa + h * kHalfABytes, &tmap_a, full, ka + h * kTileM, r, keep);
-                  tma_load_2d_pair_hint(sa + h * kHalfABytes + kBoxBytes, &tmap_a, full, ka + h * kTileM + 64, r, keep);
-                }
-#pragma unroll
-                for (int j = 0; j < kBCols / 64; ++j)
-                  tma_load_2d_pair_hint(sb + j * kBoxBytes, &tmap_b, full, nb + j * 64, r, keep);
-              }
-            }
-            continue;
-          }
           if (kTgmm) {
             int r, live;
             tgmm_block<kSeg>(p, t, blocks, kb, r, live);
@@ -318,14 +258,14 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // ONE thread runs the whole loop (in a pair: of the leader CTA).  The loop sits on the ring's
+    // ONE thread runs the whole loop.  The loop sits on the ring's
     // critical path -- a stage can be refilled only after its MMAs, and they only start after
     // this thread has seen the stage land -- and warp-wide steps are expensive there (a
     // __syncwarp costs about 160 clocks on B200, a stage's MMAs take 1024).  The one warp-wide
     // job, clearing the rows past a group's end in a tgmm stage, belongs to the fixer warp.
-    if (lane == 0 && leader) {
+    if (lane == 0) {
       const uint32_t idesc =
-          make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM * kCtas, BN);
+          make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM, BN);
       constexpr uint32_t kAStep = (kTgmm ? 2048u : 32u) >> 4;
       constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
       const uint64_t adesc0 = kTgmm ? make_smem_desc(stage_base, kBoxBytes, 1024)
@@ -356,7 +296,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
               }
               ++uses[h];
               mbar_arrive(smem_u32(&bar_acc_full[h]));
-              if constexpr (kPair) mbar_arrive_cluster(smem_u32(&bar_acc_full[h]), 1);
             }
           }
           continue;
@@ -377,10 +316,9 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const int n_mma = live >= kTileK ? kTileK / kUmmaK : (live + kUmmaK - 1) / kUmmaK;
           if (kTgmm && (kSeg ? block_needs_clearing(live) : (tail_stage && kb == kb_count - 1))) {
             // Rows past the end of the group belong to the next group (or to nobody): the fixer
-            // warp (of either CTA in a pair) clears them before the MMAs read the stage.
+            // warp clears them before the MMAs read the stage.
             mbar_arrive(smem_u32(&bar_tail_go));
-            if constexpr (kPair) mbar_arrive_cluster(smem_u32(&bar_tail_go), 1);
-            if (!mbar_wait<kPair>(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
+            if (!mbar_wait(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
               ok = false;
               break;
             }
@@ -404,35 +342,26 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
               const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * (kHalfABytes >> 4);
               if (kTgmm && n_mma < kTileK / kUmmaK) {
                 for (int kk = 0; kk < n_mma; ++kk) {
-                  umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
+                  umma_ab<1, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
                                   make_desc64(b_lo + kk * kBStep, desc_hi), idesc,
                                   (kb > 0 || kk > 0) ? 1u : 0u);
                 }
               } else {
-                umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo, desc_hi), make_desc64(b_lo, desc_hi), idesc,
+                umma_ab<1, kFp8>(tmem_d, make_desc64(a_lo, desc_hi), make_desc64(b_lo, desc_hi), idesc,
                                 kb > 0 ? 1u : 0u);
 #pragma unroll
                 for (int kk = 1; kk < kTileK / kUmmaK; ++kk) {
-                  umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
+                  umma_ab<1, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
                                   make_desc64(b_lo + kk * kBStep, desc_hi), idesc, 1u);
                 }
               }
               if (last) {  // this half is complete
-                if constexpr (kPair) {
-                  umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
-                } else {
-                  umma_commit(smem_u32(&bar_acc_full[h]));
-                }
+                umma_commit(smem_u32(&bar_acc_full[h]));
               }
             }
           }
           if (!ok) break;
-          // both halves have read the stage (in both CTAs of a pair)
-          if constexpr (kPair) {
-            umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
-          } else {
-            umma_commit(smem_u32(&bar_empty[s]));
-          }
+          umma_commit(smem_u32(&bar_empty[s]));  // both halves have read the stage
         }
       }
     }
@@ -444,7 +373,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if constexpr (kTgmm) {
       uint32_t it = 0;
       uint32_t events = 0;
-      uint32_t own_parity = 0;  // peer of a pair, bit s: parity of the next landing on its own barrier of slot s
       bool ok = true;
       for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
         const TileCoord t = decode(tile);
@@ -456,32 +384,14 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (!(kSeg ? block_needs_clearing(live) : tail_stage)) continue;
           const uint32_t s = (it + kb) % kStages;
-          if (!mbar_wait<kPair>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
+          if (!mbar_wait(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
             ok = false;
             break;
-          }
-          if constexpr (kPair) {
-            // The peer's bytes of such a stage are counted on its own barrier of that slot (see
-            // the producer), which is used for nothing else.
-            if (!leader) {
-              const uint32_t par = (own_parity >> s) & 1u;
-              own_parity ^= 1u << s;
-              if (!mbar_wait(smem_u32(&bar_full[s]), par, abort_ptr)) {
-                ok = false;
-                break;
-              }
-            }
           }
           ++events;
           clear_tail_rows<kStageBytes / kBoxBytes>(stage_base + s * kStageBytes, live, lane);
           __syncwarp();
-          if (lane == 0) {
-            if constexpr (kPair) {
-              mbar_arrive_cluster(smem_u32(&bar_tail_done), 0);
-            } else {
-              mbar_arrive(smem_u32(&bar_tail_done));
-            }
-          }
+          if (lane == 0) mbar_arrive(smem_u32(&bar_tail_done));
         }
         it += kb_count;
       }
@@ -492,7 +402,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // of its quarter (warp index mod 4).
     const int half = (warp - 2) >> 2;
     const int quarter = warp & 3;
-    const int r_in_tile = cta_rank * kCtaRows + half * kTileM + quarter * 32 + lane;
+    const int r_in_tile = half * kTileM + quarter * 32 + lane;
     const uint32_t buf = stage_base + kStages * kStageBytes + (warp - 2) * kOutBoxBytes;
     uint32_t uses = 0;
     bool ok = true;
@@ -512,7 +422,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool row_ok, warp_has_rows, slab_by_tma, zero_only = false;
       size_t row_off;
       int out_row0;
-      const int slab0 = cta_rank * kCtaRows + half * kTileM + quarter * 32;  // first tile row of this warp's slab
+      const int slab0 = half * kTileM + quarter * 32;  // first tile row of this warp's slab
       if (kTgmm) {
         const int kr = t.k0 + r_in_tile;
         out_row0 = t.k0 + slab0;
@@ -602,13 +512,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (n_chunks > 0) {  // the accumulator is in registers: hand it back
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          if constexpr (kPair) {
-            mbar_arrive_cluster(acc_empty_bar, 0);
-          } else {
-            mbar_arrive(acc_empty_bar);
-          }
-        }
+        if (lane == 0) mbar_arrive(acc_empty_bar);
       }
 #pragma unroll
       for (int c = 1; c < BN / 64; ++c) {
@@ -617,13 +521,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (n_chunks == 0) {
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          if constexpr (kPair) {
-            mbar_arrive_cluster(acc_empty_bar, 0);
-          } else {
-            mbar_arrive(acc_empty_bar);
-          }
-        }
+        if (lane == 0) mbar_arrive(acc_empty_bar);
       }
     }
     if (lane == 0) bulk_wait_group<0>();
@@ -652,11 +550,9 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
     __syncthreads();
   }
-  // Neither CTA of a pair may leave while the other can still reach its barriers or smem.
-  if constexpr (kPair) cluster_sync();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc<kCtas>(tmem_base, kTmemCols);
+    tmem_dealloc<1>(tmem_base, kTmemCols);
   }
 }
 

@@ -159,6 +159,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same wait by a whole warp, whose result every lane (and the compiler) knows to be the same.
+template <bool kClusterScope = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile WaitCtl* ctl) {
+  return __all_sync(0xffffffffu, mbar_wait<kClusterScope>(bar, parity, ctl));
+}
+
 // Bounded wait until the 32-bit word at `flag` (written by a kernel on this or another GPU, at
 // system scope, after the data it guards) is >= `value`.  The proxy fence orders the TMA loads
 // that follow after the acquire.  Same expiry rule as mbar_wait.

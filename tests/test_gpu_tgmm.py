@@ -1,0 +1,46 @@
+"""tgmm with 256-column tiles (two accumulators per CTA): the tile order, both ways to fetch the operands,
+narrow last tiles and the choice between one CTA and a pair, against the oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_ragged_dot_b200 import _lib, ops
+from oracle import ragged_dot_oracle as oracle
+from tests import launched
+
+pytestmark = pytest.mark.gpu
+ONE, PAIR = "ragged_tgmm_kernel<1>", "ragged_tgmm_kernel<2>"
+
+
+@pytest.mark.parametrize("dtype,rel", [(torch.bfloat16, 2e-3), (torch.float16, 3e-4)])
+@pytest.mark.parametrize("m,k,n,g,kernel", [
+    (40, 136, 264, 3, ONE),        # fewer tiles than CTAs
+    (900, 520, 2384, 9, PAIR),     # two bands of column tiles, the last tile 80 wide, rows not of whole blocks
+    (700, 1032, 2176, 4, PAIR),    # the same with a last tile of 128 and whole blocks in n only
+    (64, 504, 2176, 40, PAIR),     # two rows per group
+    (300, 392, 840, 60, ONE),      # output rows that split sectors, short groups
+    (3000, 320, 2048, 3, PAIR),    # long groups: several stages per tile
+    (500, 264, 136, 300, ONE),     # more groups than the table in shared memory holds; most rounds on one CTA
+])
+def test_tgmm_two_accumulators(m, k, n, g, kernel, dtype, rel):
+    rng = np.random.default_rng(m + k)
+    live = m - m // 10
+    sizes = torch.from_numpy(rng.multinomial(live, rng.dirichlet(np.full(g, 0.7))).astype(np.int32))
+    x = oracle.reference_normal(3 * m, (m, k), dtype)
+    dout = oracle.reference_normal(3 * m + 1, (m, n), dtype)
+    x[live:] = float("nan")  # rows of no group reach nothing
+    dout[live:] = float("inf")
+    want = oracle.trans_ragged_dot(x, dout, sizes).float()
+    xd, dd, gd = x.cuda(), dout.cuda(), sizes.cuda()
+    got, names = launched.kernels(lambda: ops.tgmm_forward(xd, dd, gd))
+    assert any(kernel in name for name in names), names
+    ws = ops._workspace(m, g, xd.device)
+    for ctas in (1, 2):  # the same bits from either: the order of a contraction does not depend on the tile
+        other = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, ctas, 128), workspace=ws)
+        assert ops.device_status(ws) == 0
+        assert torch.equal(other, got)
+    got = got.cpu().float()
+    assert torch.isfinite(got).all()
+    # float32 sums in another order, and one rounding to 16 bits (2^-9 or 2^-12 at most)
+    assert float((got - want).norm() / want.norm()) < rel
