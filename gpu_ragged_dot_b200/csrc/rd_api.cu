@@ -484,7 +484,7 @@ bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool f
 template <bool kBKMajor, bool kFp8>
 int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_weights, GemmArgs args,
                      cudaStream_t stream) {
-  CUtensorMap tw, tx, tout;
+  CUtensorMap tw, tx, tout, tout16;
   int rc = encode_rows_map(&tx, x, dtype, args.k, args.m, rd::kSwapRows / 2);
   if (rc != RD_OK) return rc;
   if (kBKMajor) {
@@ -498,13 +498,15 @@ int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_w
   if (rc != RD_OK) return rc;
   {
     const uint64_t dims[2] = {static_cast<uint64_t>(args.n), static_cast<uint64_t>(args.m)};
-    const uint32_t box[2] = {32, 32};
+    const uint32_t box[2] = {32, 32}, box16[2] = {32, 16};
     rc = encode_map(&tout, y, dtype, 2, dims, box, false, /*swizzled=*/false);
+    if (rc != RD_OK) return rc;
+    rc = encode_map(&tout16, y, dtype, 2, dims, box16, false, /*swizzled=*/false);
     if (rc != RD_OK) return rc;
   }
   args.n_tiles = (args.n + rd::kSwapCols - 1) / rd::kSwapCols;
   return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8>, rd::kSwapThreads, rd::kSwapSmemBytes, args,
-                      sm_count(), stream, tw, tx, tout);
+                      sm_count(), stream, tw, tx, tout, tout16);
 }
 
 // Tensor maps and launch of tgmm with two accumulators per CTA (rd_tgmm.cuh); args.k_tiles and n_tiles are set.

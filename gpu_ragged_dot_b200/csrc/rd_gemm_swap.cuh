@@ -8,20 +8,26 @@
 // 128, so a group pays for 64 rows on average that are not there.
 // Here a pair of CTAs owns 512 columns x up to 256 rows.  CTA c holds the accumulators of columns [256 c,
 // 256 c + 256) as two 128-lane halves; each half is ONE tcgen05.mma.cta_group::2 with M = 256 (128
-// columns of either CTA) and N = the tile's rows in steps of 32.  Each CTA loads its own columns of
+// columns of either CTA) and N = the tile's rows in steps of 16 (e4m3 32).  Each CTA loads its own columns of
 // the weights (32 KB a stage) and half of the rows (16 KB); shared memory moves 48 KB in and 64 KB
-// out per 1024 clocks.  A group's rows are dealt evenly to ceil(rows / 256) tiles.
+// out per 1024 clocks.  A group's rows are dealt evenly to ceil(rows / 256) tiles, in steps of 16.
 //
 // Measured against the 256 x 256 one-CTA tiles: m 8192, k 4096, n 14336, 8 unequal groups 694 -> 687 us
 // and trans_rhs 687 -> 669 us alone; as part of a training step at the power limit, where less
 // traffic and fewer empty rows mean a higher clock, 2.58 -> 2.48 ms for the step.  64 groups of about 512
 // rows, k 4096, n 1536, fp16: 402 -> 384 us, in a loop 487 -> 449 us.  e4m3 (m 8192, k 4096, n 14336) 466 -> 447 us
-// in a row.  What bounds it now: power; alone, the exposed drain of the accumulators, which fill
+// in a row.
+// Rows in steps of 16, heights in order and loops run by whole warps (see SwapGroupTable and rd_tgmm.cuh) against
+// steps of 32, groups as they come and loops of one thread, microseconds in a row: m 8192, k 14336, n 4096, 8
+// groups, trans_rhs 739 -> 732, 986 -> 925 thousand clocks; k 4096, n 14336 759 -> 732, trans_rhs 757 -> 744, e4m3 413 ->
+// 396; 64 groups of 512, k 1536, n 4096, fp16, trans_rhs 393 -> 353.  The faster loops alone lost 8 % at k 14336:
+// one thread's MMAs had held short tiles to the pace of full ones.
+// What bounds it now: power; alone, the exposed drain of the accumulators, which fill
 // tensor memory, and the last round of tiles.
 //
 // Accumulator lanes are output columns, so a warp's 32 x 32 block is transposed on its way through
-// shared memory (two-byte stores, 64 contiguous bytes per row) and leaves by TMA; blocks that cross
-// the end of the tile's rows are stored from registers, 64 bytes per row.
+// shared memory (two-byte stores, 64 contiguous bytes per row) and leaves by TMA, as 32 rows or 16; the last
+// rows of a group, fewer than 16, are stored from registers, 64 bytes per row.
 //
 // Roles, barriers and waits as in rd_gemm2.cuh (kPair); loads are plain, nothing is broadcast.
 // kFp8: e4m3 operands, K-major weights, tiles byte for byte those of a 16-bit problem.
@@ -46,21 +52,95 @@ constexpr int kSwapSmemBytes = kSwapStages * kSwapStageBytes + kSwapEpilogueWarp
 // The tile's rows [row0, row0 + rows) of its group and the pair's first column.
 struct SwapTile {
   int weight, row0, rows, n0;
-  int mma_n;  // rows in steps of 32: the N of the MMAs
+  int mma_n;  // rows in steps of kStep (16; e4m3 32): the N of the MMAs
 };
 
-__device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const GroupTable* tab, int tile) {
+// Groups in the order of their tiles' height, tallest first: `tiles` counts by position in that order.
+// A tile's time is its rows, and pairs that share panels of x or of the weights should run side by side: with
+// groups as they come, pairs go into a group after tiles of different heights, far apart, and fetch its x once
+// more (m 8192, k 14336, n 4096, 8 groups: 2.4 GB from HBM instead of 1.3, at the power limit 8 % of the time).
+// The launch always has the table (GemmArgs::inline_groups).
+struct SwapGroupTable : GroupTable {
+  uint8_t order[kMaxInlineGroups];
+};
+
+// One warp.  Counting sort on the possible heights in steps of 16 (0: no rows); equal ones keep their order.
+__device__ __forceinline__ void build_group_table(const GemmArgs& p, int tile_rows, SwapGroupTable* tab, int lane) {
+  constexpr int kPer = kMaxInlineGroups / 32;
+  int rows[kPer], sum = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = lane * kPer + j;
+    rows[j] = i < p.g ? imax(p.group_sizes[i], 0) : 0;
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) sum += rows[j];
+  int off = warp_inclusive_scan(sum, lane) - sum;
+  int tiles[kPer], height[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = lane * kPer + j;
+    if (i <= p.g) tab->offset[i] = off;
+    const int live = imin(rows[j], imax(p.m - off, 0));
+    tiles[j] = (live + tile_rows - 1) / tile_rows;
+    height[j] = i >= p.g ? -1 : live > 0 ? ((live + 15) / 16 + tiles[j] - 1) / tiles[j] : 0;
+    off += rows[j];
+  }
+  if (lane == 31 && p.g == kMaxInlineGroups) tab->offset[p.g] = off;
+  int pos = 0, before = 0;
+  for (int h = kSwapRows / 16; h >= 0; --h) {
+    int count = 0;  // groups of this height << 20 | their tiles
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) count += height[j] == h ? (1 << 20) + tiles[j] : 0;
+    if (!__any_sync(0xffffffffu, count != 0)) continue;
+    const int incl = warp_inclusive_scan(count, lane);
+    int at = pos + ((incl - count) >> 20), tile = before + ((incl - count) & 0xfffff);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (height[j] != h) continue;
+      tab->order[at] = static_cast<uint8_t>(lane * kPer + j);
+      tab->tiles[at++] = static_cast<uint16_t>(tile);
+      tile += tiles[j];
+    }
+    const int all = __shfl_sync(0xffffffffu, incl, 31);
+    pos += all >> 20;
+    before += all & 0xfffff;
+  }
+  if (lane == 0) tab->tiles[p.g] = static_cast<uint16_t>(before);
+}
+
+__device__ __forceinline__ RowTile find_row_tile(const GemmArgs& p, const SwapGroupTable* tab, int mt) {
+  int lo = 0, hi = p.g;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (tab->tiles[mid + 1] > mt) hi = mid; else lo = mid + 1;
+  }
+  RowTile r;
+  r.group = tab->order[lo];
+  r.weight = p.group_to_weight != nullptr ? p.group_to_weight[r.group] : r.group;
+  r.group_offset = tab->offset[r.group];
+  r.group_size = imin(tab->offset[r.group + 1] - r.group_offset, p.m - r.group_offset);
+  r.tile_base = tab->tiles[lo];
+  r.tiles = tab->tiles[lo + 1] - r.tile_base;
+  return r;
+}
+
+template <int kStep>
+__device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const SwapGroupTable* tab, int tile) {
   const RowTile r = find_row_tile(p, tab, tile / p.n_tiles);
   const int local = tile - r.tile_base * p.n_tiles;
   const int nt = local / r.tiles;
   const int mi = local - nt * r.tiles;
-  // equal shares in steps of 32 rows; the last tiles may be shorter, never empty or above 256
-  const int per = ((r.group_size + r.tiles - 1) / r.tiles + 31) & ~31;
+  // The group's rows in blocks of kStep, dealt evenly: a tile's time is its rows, and tiles side by side that
+  // take equally long keep sharing panels.  No tile is empty or above 256 rows.
+  const int blocks = (r.group_size + kStep - 1) / kStep;
+  const int per = blocks / r.tiles, more = blocks - per * r.tiles;  // the first `more` tiles have one more
+  const int first = (mi * per + imin(mi, more)) * kStep;
   SwapTile t;
   t.weight = r.weight;
-  t.row0 = r.group_offset + mi * per;
-  t.rows = imax(imin(per, r.group_size - mi * per), 0);
-  t.mma_n = imax((t.rows + 31) & ~31, 32);
+  t.row0 = r.group_offset + first;
+  t.mma_n = imax((per + (mi < more ? 1 : 0)) * kStep, kStep);
+  t.rows = imax(imin(t.mma_n, r.group_size - first), 0);
   t.n0 = nt * kSwapCols;
   return t;
 }
@@ -68,10 +148,12 @@ __device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const Gr
 template <bool kBKMajor, bool kFp8>
 __global__ void __launch_bounds__(kSwapThreads, 1)
 ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                        const __grid_constant__ CUtensorMap tmap_out, const GemmArgs p) {
+                        const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_out16,
+                        const GemmArgs p) {
   static_assert(!kFp8 || kBKMajor, "8-bit inputs: K-major weights");
   constexpr int kStages = kSwapStages;
   constexpr uint32_t kStageBytes = kSwapStageBytes;
+  constexpr int kStep = kFp8 ? 32 : 16;  // what N comes in, M = 256 on a pair
 
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kStages];   // leader's is used
@@ -80,9 +162,9 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   __shared__ __align__(8) uint64_t bar_acc_empty[2];    // per half, leader's is used
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
-  __shared__ GroupTable group_table;
+  __shared__ SwapGroupTable group_table;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int cta_rank = static_cast<int>(cluster_cta_rank());
   const bool leader = cta_rank == 0;
@@ -94,6 +176,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
     tma_prefetch_desc(&tmap_out);
+    tma_prefetch_desc(&tmap_out16);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -121,25 +204,36 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int tile_step = static_cast<int>(gridDim.x >> 1);
   const int k_blocks = (p.k + kTileK - 1) / kTileK;
 
+  // The producer and the MMA warp run their loops as whole warps on values that the compiler knows to be uniform
+  // and elect a lane for the TMA and tcgen05 instructions alone, which take uniform registers (rd_tgmm.cuh).
+  auto uniform_tile = [&](int tile) {
+    SwapTile t = decode_swap_tile<kStep>(p, &group_table, tile);
+    t.weight = __shfl_sync(0xffffffffu, t.weight, 0);
+    t.row0 = __shfl_sync(0xffffffffu, t.row0, 0);
+    t.n0 = __shfl_sync(0xffffffffu, t.n0, 0);
+    t.mma_n = __shfl_sync(0xffffffffu, t.mma_n, 0);
+    return t;
+  };
+
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
-        const SwapTile t = decode_swap_tile(p, &group_table, tile);
-        const int col = t.n0 + cta_rank * kSwapCtaCols;
-        const int row = t.row0 + cta_rank * (t.mma_n >> 1);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
-            ok = false;
-            break;
-          }
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
+      const SwapTile t = uniform_tile(tile);
+      const int col = t.n0 + cta_rank * kSwapCtaCols;
+      const int row = t.row0 + cta_rank * (t.mma_n >> 1);
+      for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kSwapABytes;
+        if (elect_one()) {
           uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kSwapABytes;
           if (leader) {
             mbar_arrive_expect_tx(full, 2 * kStageBytes);
             tma_load_2d(sb, &tmap_x, full, kb * kTileK, row);
@@ -161,8 +255,8 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0 && leader) {
+    // ------------------------------------------------------------ MMA issuer (of the leader)
+    if (leader) {
       constexpr uint32_t kAStep = (kBKMajor ? 32u : 2048u) >> 4;
       constexpr uint32_t kBStep = 32u >> 4;
       constexpr uint32_t kHalfA = (kBKMajor ? 128u * 128u : 2u * kBoxBytes) >> 4;  // the next 128 columns
@@ -177,22 +271,23 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       uint32_t local_tile = 0;
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-        const SwapTile t = decode_swap_tile(p, &group_table, tile);
+        const SwapTile t = uniform_tile(tile);
         const uint32_t idesc =
             make_idesc_f16(kFp8 ? 0 : p.ab_format, kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n);
         uint32_t s = it % kStages;
         uint32_t ph = (it / kStages) & 1u;
         for (int kb = 0; kb < k_blocks; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
-          if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+          if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
+          const uint32_t more = kb > 0 ? 1u : 0u;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (kb == 0) {  // the half's accumulator must have been drained by both CTAs
-              if (!mbar_wait<true>(smem_u32(&bar_acc_empty[h]), (local_tile & 1u) ^ 1u, abort_ptr)) {
+              if (!mbar_wait_warp<true>(smem_u32(&bar_acc_empty[h]), (local_tile & 1u) ^ 1u, abort_ptr)) {
                 ok = false;
                 break;
               }
@@ -200,14 +295,16 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             }
             const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * kHalfA;
             const uint32_t tmem_d = tmem_base + h * kSwapRows;
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
-              umma_ab<2, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, a_hi),
-                               make_desc64(b_lo + kk * kBStep, b_hi), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
+              for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
+                umma_ab<2, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, a_hi),
+                                 make_desc64(b_lo + kk * kBStep, b_hi), idesc, kk > 0 ? 1u : more);
+              if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
+              if (h == 1) umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
+            }
           }
           if (!ok) break;
-          umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
         }
       }
     }
@@ -222,7 +319,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     bool ok = true;
     uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
     for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const SwapTile t = decode_swap_tile(p, &group_table, tile);
+      const SwapTile t = decode_swap_tile<kStep>(p, &group_table, tile);
       const int col0 = t.n0 + col_in_tile;  // this warp's first output column; lane = column
       if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), local_tile & 1u, abort_ptr)) {
         ok = false;
@@ -257,7 +354,8 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (c >= chunks) continue;
         const int row0 = t.row0 + c * 32;
         const int rows = t.rows - c * 32;
-        if (rows >= 32) {
+        const int by_tma = rows >= 32 ? 32 : rows & 16;  // rows stored as one box of 32 or 16
+        if (by_tma > 0) {
           const uint32_t buf = staging + (boxes_stored & 1u) * kSwapBoxBytes;
           if (lane == 0) bulk_wait_group_read<1>();  // the box stored two boxes ago has been read out
           __syncwarp();
@@ -277,15 +375,16 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(&tmap_out, buf, col0, row0);
+            tma_store_2d(by_tma == 32 ? &tmap_out : &tmap_out16, buf, col0, row0);
             bulk_commit_group();
           }
           ++boxes_stored;
-        } else if (col0 + lane < p.n) {  // crosses the end of the tile's rows
+        }
+        if (by_tma < imin(rows, 32) && col0 + lane < p.n) {  // the group's last rows
           uint16_t* dst = out16 + static_cast<size_t>(row0) * p.n + col0 + lane;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (j < rows) dst[static_cast<size_t>(j) * p.n] = static_cast<uint16_t>(o[c][j >> 1] >> (16 * (j & 1)));
+            if (j >= by_tma && j < rows) dst[static_cast<size_t>(j) * p.n] = static_cast<uint16_t>(o[c][j >> 1] >> (16 * (j & 1)));
           }
         }
       }

@@ -1,0 +1,46 @@
+"""gmm with rows on the N side: rows dealt to tiles in steps of 16, and groups visited by the height of their
+tiles, against 128-row tiles that multiply the same operands in the order of the groups."""
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_ragged_dot_b200 import _lib, ops
+from tests import launched
+
+pytestmark = pytest.mark.gpu
+# around whole steps, tiles and both: 1 row, 16 and 32 more or less one, one tile and a row, 17 blocks for two tiles
+EDGES = [1, 15, 16, 17, 31, 32, 33, 47, 0, 255, 256, 257, 272, 273, 511, 512, 513, 528, 0, 1500, 3000]
+
+
+@pytest.mark.parametrize("m,k,n,g,over", [
+    (11000, 576, 8192, 21, 0),     # every edge, heights in no order
+    (11000, 600, 8184, 21, 700),   # sizes that add up to more rows than there are: the last group is cut
+    (131072, 576, 512, 256, 0),    # as many groups as the table in shared memory holds
+])
+def test_rows_in_steps_of_16(m, k, n, g, over):
+    rng = np.random.default_rng(m + g)
+    sizes = np.array((EDGES * (g // len(EDGES) + 1))[:g])
+    rng.shuffle(sizes)
+    sizes[int(rng.integers(g))] += m + over - 5 - sizes.sum()  # the last five rows in no group
+    gs = torch.from_numpy(sizes.astype(np.int32)).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), device="cuda", generator=gen).bfloat16()
+    w = torch.randn((g, n, k), device="cuda", generator=gen).bfloat16()
+    if not over:
+        x[m - 5:] = float("nan")
+    whole = _lib.TileCfg(256, 0, 1, 128, 0)
+    ws = ops._workspace(m, g, x.device)
+    for weights, trans in ((w, True), (w.transpose(1, 2).contiguous(), False)):
+        if not trans and n % 64:
+            continue
+        got, names = launched.kernels(lambda: ops.gmm_forward(x, weights, gs, trans_rhs=trans, workspace=ws,
+                                                              cfg=_lib.TileCfg(0, 0, 0, 0, 0)))
+        assert any("ragged_gemm_swap_kernel" in name for name in names), names
+        assert ops.device_status(ws) == 0
+        ref = ops.gmm_forward(x, weights, gs, trans_rhs=trans, cfg=whole).float()
+        # the same products summed in fp32: a result differs by one rounding to 16 bits at most
+        assert torch.isfinite(got).all()
+        assert float(((got.float() - ref).abs() - 2.0 ** -7 * ref.abs()).max()) <= 1e-4 * float(ref.abs().max())
+        if not over:
+            assert float(got[m - 5:].abs().max()) == 0.0
