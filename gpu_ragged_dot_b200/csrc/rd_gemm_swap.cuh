@@ -31,9 +31,14 @@
 //
 // Roles, barriers and waits as in rd_gemm2.cuh (kPair); loads are plain, nothing is broadcast.
 // kFp8: e4m3 operands, K-major weights, tiles byte for byte those of a 16-bit problem.
+// kF32: one TF32 pass, stages 32 deep, [k, n] weights in the 32-byte-atom swizzle (rd_gemm_f32.cuh), the same sums in
+// the same order as there.  One CTA per 128 x 256 tile moves 187 bytes of shared memory per clock of MMAs and stops at 70 %
+// of the tensor pipe; microseconds in a row, m 8192, k 4096, n 14336, 8 groups 1500 -> 1390, trans_rhs with k 14336, n
+// 4096 1529 -> 1420; 16384, 1024, 4096, 32 268 -> 249.
 #pragma once
 
 #include "rd_gemm2.cuh"
+#include "rd_gemm_f32_pair.cuh"
 
 namespace rd {
 
@@ -145,15 +150,16 @@ __device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const Sw
   return t;
 }
 
-template <bool kBKMajor, bool kFp8>
+template <bool kBKMajor, bool kFp8, bool kF32 = false>
 __global__ void __launch_bounds__(kSwapThreads, 1)
 ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_out16,
                         const GemmArgs p) {
-  static_assert(!kFp8 || kBKMajor, "8-bit inputs: K-major weights");
+  static_assert(!kFp8 || (kBKMajor && !kF32), "8-bit inputs: K-major weights");
   constexpr int kStages = kSwapStages;
   constexpr uint32_t kStageBytes = kSwapStageBytes;
   constexpr int kStep = kFp8 ? 32 : 16;  // what N comes in, M = 256 on a pair
+  constexpr int kDeep = kF32 ? kF32TileK : kTileK;  // elements in a stage's 128 bytes of the contraction
 
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kStages];   // leader's is used
@@ -202,7 +208,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int num_tiles = live_row_tiles(p, &group_table) * p.n_tiles;
   const int tile_start = static_cast<int>(blockIdx.x >> 1);
   const int tile_step = static_cast<int>(gridDim.x >> 1);
-  const int k_blocks = (p.k + kTileK - 1) / kTileK;
+  const int k_blocks = (p.k + kDeep - 1) / kDeep;
 
   // The producer and the MMA warp run their loops as whole warps on values that the compiler knows to be uniform
   // and elect a lane for the TMA and tcgen05 instructions alone, which take uniform registers (rd_tgmm.cuh).
@@ -236,19 +242,19 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           uint32_t full = smem_u32(&bar_full[s]);
           if (leader) {
             mbar_arrive_expect_tx(full, 2 * kStageBytes);
-            tma_load_2d(sb, &tmap_x, full, kb * kTileK, row);
+            tma_load_2d(sb, &tmap_x, full, kb * kDeep, row);
             if constexpr (kBKMajor) {
-              tma_load_3d(sa, &tmap_w, full, kb * kTileK, col, t.weight);
+              tma_load_3d(sa, &tmap_w, full, kb * kDeep, col, t.weight);
             } else {
-              tma_load_4d(sa, &tmap_w, full, 0, kb * kTileK, col >> 6, t.weight);
+              tma_load_4d(sa, &tmap_w, full, 0, kb * kDeep, col / kDeep, t.weight);
             }
           } else {
             full = map_to_cta(full, 0);
-            tma_load_2d_pair(sb, &tmap_x, full, kb * kTileK, row);
+            tma_load_2d_pair(sb, &tmap_x, full, kb * kDeep, row);
             if constexpr (kBKMajor) {
-              tma_load_3d_pair(sa, &tmap_w, full, kb * kTileK, col, t.weight);
+              tma_load_3d_pair(sa, &tmap_w, full, kb * kDeep, col, t.weight);
             } else {
-              tma_load_4d_pair(sa, &tmap_w, full, 0, kb * kTileK, col >> 6, t.weight);
+              tma_load_4d_pair(sa, &tmap_w, full, 0, kb * kDeep, col / kDeep, t.weight);
             }
           }
         }
@@ -257,10 +263,11 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (of the leader)
     if (leader) {
-      constexpr uint32_t kAStep = (kBKMajor ? 32u : 2048u) >> 4;
+      constexpr uint32_t kAStep = (kBKMajor ? 32u : kF32 ? 1024u : 2048u) >> 4;
       constexpr uint32_t kBStep = 32u >> 4;
       constexpr uint32_t kHalfA = (kBKMajor ? 128u * 128u : 2u * kBoxBytes) >> 4;  // the next 128 columns
       const uint64_t adesc0 = kBKMajor ? make_smem_desc(stage_base, 16, 1024)
+                              : kF32   ? make_smem_desc(stage_base, kF32BoxBytes, 512, 1)
                                        : make_smem_desc(stage_base, kBoxBytes, 1024);
       const uint64_t bdesc0 = make_smem_desc(stage_base + kSwapABytes, 16, 1024);
       const uint32_t adesc0_lo = static_cast<uint32_t>(adesc0);
@@ -273,7 +280,8 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
         const SwapTile t = uniform_tile(tile);
         const uint32_t idesc =
-            make_idesc_f16(kFp8 ? 0 : p.ab_format, kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n);
+            kF32 ? make_idesc_tf32(kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n)
+                 : make_idesc_f16(kFp8 ? 0 : p.ab_format, kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n);
         uint32_t s = it % kStages;
         uint32_t ph = (it / kStages) & 1u;
         for (int kb = 0; kb < k_blocks; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
@@ -297,9 +305,14 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             const uint32_t tmem_d = tmem_base + h * kSwapRows;
             if (elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
-                umma_ab<2, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, a_hi),
-                                 make_desc64(b_lo + kk * kBStep, b_hi), idesc, kk > 0 ? 1u : more);
+              for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of the contraction each
+                const uint64_t a = make_desc64(a_lo + kk * kAStep, a_hi), b = make_desc64(b_lo + kk * kBStep, b_hi);
+                if constexpr (kF32) {
+                  umma_tf32_pair(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
+                } else {
+                  umma_ab<2, kFp8>(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
+                }
+              }
               if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
               if (h == 1) umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
             }
@@ -328,6 +341,62 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       tc_fence_after_sync();
       const int chunks = col0 < p.n ? (t.rows + 31) >> 5 : 0;
       const float sc = kFp8 && p.weight_scale != nullptr ? p.weight_scale[t.weight] : 1.0f;
+      if constexpr (kF32) {
+        // 32 rows at a time as they are; the last four of these leave tensor memory together, then the accumulator
+        // is handed back.  A row of 32 columns is 128 bytes: stores of a warp meet no bank twice.
+        float* out32 = reinterpret_cast<float*>(p.out);
+        auto store = [&](int c, const uint32_t (&v)[32]) {
+          const int row0 = t.row0 + c * 32;
+          const int rows = t.rows - c * 32;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {  // boxes of 16 rows
+            if (rows < 16 * h + 16) break;
+            const uint32_t buf = staging + (boxes_stored & 1u) * kSwapBoxBytes;
+            if (lane == 0) bulk_wait_group_read<1>();
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              asm volatile("st.shared.b32 [%0], %1;" ::"r"(buf + j * 128 + lane * 4), "r"(v[16 * h + j]) : "memory");
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(&tmap_out16, buf, col0, row0 + 16 * h);
+              bulk_commit_group();
+            }
+            ++boxes_stored;
+          }
+          if (rows < 32 && (rows & 15) != 0 && col0 + lane < p.n) {  // the group's last rows
+            float* dst = out32 + static_cast<size_t>(row0) * p.n + col0 + lane;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (j >= (rows & 16) && j < rows) dst[static_cast<size_t>(j) * p.n] = __uint_as_float(v[j]);
+            }
+          }
+        };
+        const uint32_t tmem = tmem_base + half * kSwapRows + (static_cast<uint32_t>(quarter * 32) << 16);
+        const int early = imax(chunks - 4, 0);
+#pragma unroll 1
+        for (int c = 0; c < early; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32(tmem + c * 32, v);
+          tmem_ld_wait();
+          store(c, v);
+        }
+        uint32_t v[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (early + c < chunks) tmem_ld_32x32(tmem + (early + c) * 32, v[c]);
+        }
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(smem_u32(&bar_acc_empty[half]), 0);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (early + c < chunks) store(early + c, v[c]);
+        }
+        continue;
+      }
       // All rows leave tensor memory first (packed to 16 bits, 16 registers per 32 rows), so that the
       // next tile's MMAs wait for nothing but the loads below.
       uint32_t o[kSwapRows / 32][16];
@@ -395,11 +464,11 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     if (p.zero_tail) {
       constexpr int kEpiThreads = 32 * kSwapEpilogueWarps;
       const int first = first_dead_row(p, &group_table);
-      const size_t chunks_per_row = static_cast<size_t>(p.n) / 8;
+      const size_t chunks_per_row = static_cast<size_t>(p.n) / (kF32 ? 4 : 8);
       const size_t total = static_cast<size_t>(p.m - first) * chunks_per_row;
       const size_t tid = static_cast<size_t>(blockIdx.x) * kEpiThreads + (threadIdx.x - 64);
       const size_t stride = static_cast<size_t>(gridDim.x) * kEpiThreads;
-      uint4* dst = reinterpret_cast<uint4*>(out16 + static_cast<size_t>(first) * p.n);
+      uint4* dst = reinterpret_cast<uint4*>(p.out) + static_cast<size_t>(first) * chunks_per_row;
       const uint4 z = make_uint4(0u, 0u, 0u, 0u);
       for (size_t i = tid; i < total; i += stride) dst[i] = z;
     }

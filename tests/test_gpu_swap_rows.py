@@ -44,3 +44,28 @@ def test_rows_in_steps_of_16(m, k, n, g, over):
         assert float(((got.float() - ref).abs() - 2.0 ** -7 * ref.abs()).max()) <= 1e-4 * float(ref.abs().max())
         if not over:
             assert float(got[m - 5:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("m,k,n,g,trans", [
+    (11000, 388, 4096, 21, False),   # the fewest rounds it takes, every edge of a tile's rows; k ends inside a stage
+    (11000, 388, 4092, 21, True),    # n ends inside a block of 32 columns
+    (5001, 1032, 6176, 3, False),    # n ends a block of 32 into a tile
+])
+def test_float32_rows_in_steps_of_16(m, k, n, g, trans):
+    rng = np.random.default_rng(m + n)
+    sizes = np.array(EDGES if g == len(EDGES) else [1000, 0, 1500])
+    rng.shuffle(sizes)
+    sizes[int(rng.integers(g))] += m - 5 - sizes.sum()
+    gs = torch.from_numpy(sizes.astype(np.int32)).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), device="cuda", generator=gen)
+    w = torch.randn((g, n, k) if trans else (g, k, n), device="cuda", generator=gen)
+    x[m - 5:] = float("nan")
+    ws = ops._workspace(m, g, x.device)
+    got, names = launched.kernels(lambda: ops.gmm_forward(x, w, gs, trans_rhs=trans, workspace=ws,
+                                                          cfg=_lib.TileCfg(0, 0, 0, 0, 0)))
+    assert any("ragged_gemm_swap_kernel" in name for name in names), names
+    assert ops.device_status(ws) == 0
+    ref = ops.gmm_forward(x, w, gs, trans_rhs=trans, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
+    assert torch.equal(got[:m - 5], ref[:m - 5])  # the same TF32 products, added in the same order
+    assert float(got[m - 5:].abs().max()) == 0.0
