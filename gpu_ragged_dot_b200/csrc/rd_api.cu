@@ -455,6 +455,28 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
                        split);
 }
 
+// Fewer rounds than choose_swap asks for: the clocks of both kernels, from their rounds of tiles.  A pair takes 4 clocks per
+// row and block of the contraction and 5000 to drain a tile, a last half round costs 0.55 of one (SwapWork), one CTA 560
+// per block of a 128 x 256 tile; a group's last tile is half full on average.  Timed on both sides on 300 float32, 500
+// 16-bit and 300 e4m3 sizes (1 to 64 groups, equal and unequal, 128 to 14336 deep and wide), this and the rules
+// below against the rules below alone: float32 1.024 times as fast on average over all sizes instead of 1.010, 16 bits
+// 1.012 instead of 1.006, e4m3 1.009 instead of 1.003; slower by more than 2 % in 2, 2 and 0 of them, 7 % at most.  Under
+// half a round, and for groups shorter than `least`, it is wrong too often.
+bool swap_takes_less(long long m, int k_blocks, int n, int g, int least, double margin) {
+  if (m / g < least) return false;
+  const double sms = sm_count(), rows = static_cast<double>(m) / g;
+  const double per = rows > 128.0 ? rows / rd::kSwapRows + 0.5 : 1.0;
+  const double exact = g * per * ((n + rd::kSwapCols - 1) / rd::kSwapCols) / (sms / 2);
+  if (exact < 0.5) return false;
+  const double whole = static_cast<double>(static_cast<long long>(exact)), left = exact - whole;
+  const double rounds = whole + (left < 0.03 ? 0.0 : left <= 0.5 ? 0.55 : 1.0);
+  double height = rows / per + 8.0;
+  if (height > rd::kSwapRows) height = rd::kSwapRows;
+  const double per128 = rows > 64.0 ? rows / rd::kTileM + 0.5 : 1.0;
+  const double rounds128 = static_cast<double>(static_cast<long long>(g * per128 * ((n + 255) / 256) / sms + 0.97));
+  return rounds * (4.0 * height * k_blocks + 5000.0) * margin < (rounds128 > 1.0 ? rounds128 : 1.0) * 560.0 * k_blocks;
+}
+
 // Should a gmm put its rows on the N side of the MMAs (rd_gemm_swap.cuh)?  When groups are long, there
 // are at least three rounds of tiles for the pairs and the last 512-column tile is nearly full.
 // Microseconds, one-CTA tiles (better of the two heights) against swapped: m 8192, k 4096, n 14336, 8
@@ -468,7 +490,9 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
 // e4m3 (128-row tiles otherwise) with few rounds: they are compared, a swapped tile taking 1.7 times as long
 // as a 128-row one; 8192, 14336, 4096, 16 (5 against 8) 422 -> 433, in a row 425 -> 453.
 bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool fp8) {
-  if (g <= 0 || m / g < 512 || (!trans_rhs && n % 64 != 0)) return false;
+  if (g <= 0 || (!trans_rhs && n % 64 != 0)) return false;
+  if (swap_takes_less(m, k_blocks, n, g, fp8 ? 128 : 384, fp8 ? 1.2 : 1.0)) return true;
+  if (m / g < 512) return false;
   const long long pairs = sm_count() / 2;
   const long long col_tiles = (static_cast<long long>(n) + rd::kSwapCols - 1) / rd::kSwapCols;
   if ((col_tiles * rd::kSwapCols - n) * 16 > n || m / rd::kSwapRows * col_tiles < 3 * pairs) return false;
@@ -484,7 +508,9 @@ bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool f
 // sides it takes 15, 1.11 times as fast on average and 6 % slower in one: m 32768, k 2624, n 928, 26 groups 282 -> 237
 // us, 32768, 368, 7584, 28 384 -> 349.  Below three rounds either side wins by up to 1.6, by how rounds fall.
 bool choose_swap_f32(long long m, int k_blocks, int n, int g, bool trans_rhs) {
-  if (g <= 0 || m / g < 256 || k_blocks < 12 || (!trans_rhs && n % 32 != 0)) return false;
+  if (g <= 0 || (!trans_rhs && n % 32 != 0)) return false;
+  if (swap_takes_less(m, k_blocks, n, g, 384, 1.0)) return true;
+  if (m / g < 256 || k_blocks < 12) return false;
   const long long col_tiles = (static_cast<long long>(n) + rd::kSwapCols - 1) / rd::kSwapCols;
   return (col_tiles * rd::kSwapCols - n) * 10 <= n && (m / rd::kSwapRows + g / 2) * col_tiles >= 3 * (sm_count() / 2);
 }
@@ -505,10 +531,10 @@ int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_w
   if (kBKMajor) {
     const uint64_t dims[3] = {static_cast<uint64_t>(args.k), static_cast<uint64_t>(args.n),
                               static_cast<uint64_t>(num_weights)};
-    const uint32_t box[3] = {kDeep, rd::kSwapCtaCols, 1};
+    const uint32_t box[3] = {kDeep, rd::kTileM, 1};  // one half of a CTA's columns
     rc = encode_map(&tw, A, dtype, 3, dims, box);
   } else {
-    rc = encode_blocked_map(&tw, A, dtype, args.n, args.k, kDeep, rd::kSwapCtaCols / kDeep, num_weights);
+    rc = encode_blocked_map(&tw, A, dtype, args.n, args.k, kDeep, rd::kTileM / kDeep, num_weights);
   }
   if (rc != RD_OK) return rc;
   {

@@ -57,6 +57,7 @@ constexpr int kSwapSmemBytes = kSwapStages * kSwapStageBytes + kSwapEpilogueWarp
 // The tile's rows [row0, row0 + rows) of its group and the pair's first column.
 struct SwapTile {
   int weight, row0, rows, n0;
+  int halves;  // 128-lane halves of each CTA: 2, or 1 for a half tile of 256 columns
   int mma_n;  // rows in steps of kStep (16; e4m3 32): the N of the MMAs
 };
 
@@ -130,8 +131,25 @@ __device__ __forceinline__ RowTile find_row_tile(const GemmArgs& p, const SwapGr
   return r;
 }
 
+// What the pairs walk: whole tiles for whole rounds, and what is left too; where that is half a round or less it is
+// cut into half tiles of 256 columns, one for a pair at most.  Microseconds, alone: m 8192, k 4096, n 5120, 8 groups,
+// trans_rhs 271 -> 233; 8192, 2048, 4096, 8 139 -> 106 (in a row, at the power limit, equal: 264 and 266, 114 and 114);
+// in a row float32 8192, 4096, 14336, 8 1285 -> 1254, bf16 727 -> 707.
+struct SwapWork {
+  int whole, items;
+  __device__ __forceinline__ SwapWork(int tiles, int pairs) {
+    const int left = tiles % pairs;
+    const bool cut = 2 * left <= pairs;
+    whole = cut ? tiles - left : tiles;
+    items = cut ? tiles + left : tiles;
+  }
+};
+
 template <int kStep>
-__device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const SwapGroupTable* tab, int tile) {
+__device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const SwapGroupTable* tab, const SwapWork& work,
+                                                     int item) {
+  const int past = item - work.whole;
+  const int tile = past < 0 ? item : work.whole + (past >> 1);
   const RowTile r = find_row_tile(p, tab, tile / p.n_tiles);
   const int local = tile - r.tile_base * p.n_tiles;
   const int nt = local / r.tiles;
@@ -146,7 +164,8 @@ __device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const Sw
   t.row0 = r.group_offset + first;
   t.mma_n = imax((per + (mi < more ? 1 : 0)) * kStep, kStep);
   t.rows = imax(imin(t.mma_n, r.group_size - first), 0);
-  t.n0 = nt * kSwapCols;
+  t.halves = past < 0 ? 2 : 1;
+  t.n0 = nt * kSwapCols + (past < 0 ? 0 : (past & 1) * kSwapCtaCols);
   return t;
 }
 
@@ -205,7 +224,8 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const uint32_t tmem_base = tmem_slot;
   volatile WaitCtl* abort_ptr = &wait_ctl;
 
-  const int num_tiles = live_row_tiles(p, &group_table) * p.n_tiles;
+  const SwapWork work(live_row_tiles(p, &group_table) * p.n_tiles, static_cast<int>(gridDim.x >> 1));
+  const int num_tiles = work.items;
   const int tile_start = static_cast<int>(blockIdx.x >> 1);
   const int tile_step = static_cast<int>(gridDim.x >> 1);
   const int k_blocks = (p.k + kDeep - 1) / kDeep;
@@ -213,10 +233,11 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   // The producer and the MMA warp run their loops as whole warps on values that the compiler knows to be uniform
   // and elect a lane for the TMA and tcgen05 instructions alone, which take uniform registers (rd_tgmm.cuh).
   auto uniform_tile = [&](int tile) {
-    SwapTile t = decode_swap_tile<kStep>(p, &group_table, tile);
+    SwapTile t = decode_swap_tile<kStep>(p, &group_table, work, tile);
     t.weight = __shfl_sync(0xffffffffu, t.weight, 0);
     t.row0 = __shfl_sync(0xffffffffu, t.row0, 0);
     t.n0 = __shfl_sync(0xffffffffu, t.n0, 0);
+    t.halves = __shfl_sync(0xffffffffu, t.halves, 0);
     t.mma_n = __shfl_sync(0xffffffffu, t.mma_n, 0);
     return t;
   };
@@ -227,7 +248,8 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     bool ok = true;
     for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
       const SwapTile t = uniform_tile(tile);
-      const int col = t.n0 + cta_rank * kSwapCtaCols;
+      const int col = t.n0 + cta_rank * t.halves * kTileM;
+      const uint32_t bytes = t.halves * (kSwapABytes / 2) + kSwapBBytes;  // of one CTA
       const int row = t.row0 + cta_rank * (t.mma_n >> 1);
       for (int kb = 0; kb < k_blocks; ++kb, ++it) {
         const uint32_t s = it % kStages;
@@ -241,20 +263,26 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (elect_one()) {
           uint32_t full = smem_u32(&bar_full[s]);
           if (leader) {
-            mbar_arrive_expect_tx(full, 2 * kStageBytes);
+            mbar_arrive_expect_tx(full, 2 * bytes);
             tma_load_2d(sb, &tmap_x, full, kb * kDeep, row);
             if constexpr (kBKMajor) {
               tma_load_3d(sa, &tmap_w, full, kb * kDeep, col, t.weight);
+              if (t.halves == 2) tma_load_3d(sa + kSwapABytes / 2, &tmap_w, full, kb * kDeep, col + kTileM, t.weight);
             } else {
               tma_load_4d(sa, &tmap_w, full, 0, kb * kDeep, col / kDeep, t.weight);
+              if (t.halves == 2)
+                tma_load_4d(sa + kSwapABytes / 2, &tmap_w, full, 0, kb * kDeep, (col + kTileM) / kDeep, t.weight);
             }
           } else {
             full = map_to_cta(full, 0);
             tma_load_2d_pair(sb, &tmap_x, full, kb * kDeep, row);
             if constexpr (kBKMajor) {
               tma_load_3d_pair(sa, &tmap_w, full, kb * kDeep, col, t.weight);
+              if (t.halves == 2) tma_load_3d_pair(sa + kSwapABytes / 2, &tmap_w, full, kb * kDeep, col + kTileM, t.weight);
             } else {
               tma_load_4d_pair(sa, &tmap_w, full, 0, kb * kDeep, col / kDeep, t.weight);
+              if (t.halves == 2)
+                tma_load_4d_pair(sa + kSwapABytes / 2, &tmap_w, full, 0, kb * kDeep, (col + kTileM) / kDeep, t.weight);
             }
           }
         }
@@ -291,33 +319,36 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           }
           tc_fence_after_sync();
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
-          const uint32_t more = kb > 0 ? 1u : 0u;
+          auto issue = [&](int h, uint32_t more) {
+            const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * kHalfA;
+            const uint32_t tmem_d = tmem_base + h * kSwapRows;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (kb == 0) {  // the half's accumulator must have been drained by both CTAs
+            for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of the contraction each
+              const uint64_t a = make_desc64(a_lo + kk * kAStep, a_hi), b = make_desc64(b_lo + kk * kBStep, b_hi);
+              if constexpr (kF32) {
+                umma_tf32_pair(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
+              } else {
+                umma_ab<2, kFp8>(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
+              }
+            }
+            if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
+          };
+          if (kb == 0) {  // a half's accumulator must have been drained by both CTAs
+            for (int h = 0; h < t.halves; ++h) {
               if (!mbar_wait_warp<true>(smem_u32(&bar_acc_empty[h]), (local_tile & 1u) ^ 1u, abort_ptr)) {
                 ok = false;
                 break;
               }
               tc_fence_after_sync();
+              if (elect_one()) issue(h, 0u);
             }
-            const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * kHalfA;
-            const uint32_t tmem_d = tmem_base + h * kSwapRows;
-            if (elect_one()) {
-#pragma unroll
-              for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of the contraction each
-                const uint64_t a = make_desc64(a_lo + kk * kAStep, a_hi), b = make_desc64(b_lo + kk * kBStep, b_hi);
-                if constexpr (kF32) {
-                  umma_tf32_pair(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
-                } else {
-                  umma_ab<2, kFp8>(tmem_d, a, b, idesc, kk > 0 ? 1u : more);
-                }
-              }
-              if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
-              if (h == 1) umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
-            }
+            if (!ok) break;
+            if (elect_one()) umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
+          } else if (elect_one()) {
+            issue(0, 1u);
+            if (t.halves == 2) issue(1, 1u);
+            umma_commit_pair(smem_u32(&bar_empty[s]), 0x3);
           }
-          if (!ok) break;
         }
       }
     }
@@ -326,14 +357,14 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int half = (warp - 2) >> 2;
     const int quarter = warp & 3;
     const uint32_t staging = stage_base + kStages * kStageBytes + (warp - 2) * 2 * kSwapBoxBytes;
-    const int col_in_tile = cta_rank * kSwapCtaCols + half * kTileM + quarter * 32;
     uint32_t local_tile = 0;
     uint32_t boxes_stored = 0;
     bool ok = true;
     uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
     for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const SwapTile t = decode_swap_tile<kStep>(p, &group_table, tile);
-      const int col0 = t.n0 + col_in_tile;  // this warp's first output column; lane = column
+      const SwapTile t = decode_swap_tile<kStep>(p, &group_table, work, tile);
+      if (half >= t.halves) break;  // a half tile is a pair's last
+      const int col0 = t.n0 + (cta_rank * t.halves + half) * kTileM + quarter * 32;  // this warp's first output column; lane = column
       if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), local_tile & 1u, abort_ptr)) {
         ok = false;
         break;
