@@ -643,20 +643,46 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 // less data into shared memory.  Microseconds in a row, one CTA against a pair:
 // - Groups of 256 rows and more: pairs, up to a quarter more rounds of tiles (m 8192, k 4096, n 14336, 8 groups 908 ->
 //   722; 21272, 600, 5440, 49, 37 rounds against 44, 207 -> 190; 20312, 288, 280, 38, 2 against 3, equal).
-// - Shorter groups: pairs where they take no more rounds and more than two (16384, 7168, 2048, 128 972 -> 851; 3000,
+// - Groups of less than 64 rows: one CTA (5331, 4096, 1536, 128 299 against 325; 2816 548 against 586; at 64 rows equal).
+// - Groups between: pairs where they take no more rounds and more than two (16384, 7168, 2048, 128 972 -> 851; 3000,
 //   2048, 2048, 30 72 -> 69; 5024, 272, 1352, 124, 16 against 21 rounds, 35 -> 37).  With one or two rounds the start of a
 //   cluster is a good part of the time (512, 256, 384, 8, one round, alone 11 -> 13).
 // - Output rows that are not multiples of 32 bytes, groups of 100 rows and less: boxes begin and end inside sectors,
 //   which costs L2 reads of what it has not got; the one-CTA tiles, whose boxes of a row follow one another more
 //   closely, suffer less (4365, 11600, 3240, 45 1134 -> 1299; 6192, 3480, 840, 74 147 -> 173; 103 rows per group, 3512,
-//   8168, 648, 34 119 -> 112).
+//   8168, 648, 34 119 -> 112).  Rows that are not whole 256 bytes likewise, below 100 rows (5331, 4096, 1216, 128 242 -> 276;
+//   n 1600 293 -> 358).
 bool choose_tgmm_pair(long long m, int k, int n, int g) {
   const long long sms = sm_count(), cols = (static_cast<long long>(n) + 255) / 256 * g;
   const long long r1 = ((k + 127) / 128 * cols + sms - 1) / sms;
   const long long r2 = ((k + 255) / 256 * cols + sms / 2 - 1) / (sms / 2);
   if (m / g >= 256) return 4 * r2 <= 5 * r1;
   if (n % 16 != 0 && m / g <= 100) return false;
+  if (m / g < (n % 128 != 0 ? 100 : 64)) return false;
   return r2 <= r1 && r1 > 2;
+}
+
+// 128 x 256 tiles on one CTA each, groups that are not long and output rows that are not whole 256 bytes: a column tile's
+// edge falls inside 256 bytes (or a sector) of every other row, and what counts is that the CTAs that write either side
+// of it stay side by side.  A CTA steps over `ctas` tiles; `d` is what that shares with the tiles of a row.
+// - d > 1 and CTAs that would meet more wide columns than others: the order is turned.  128 groups of 42, k 4096, plain kernel
+//   (rd_gemm.cuh), two accumulators, those turned, microseconds: n 776 301, 327, 196; 1288 546, 509, 370; 1800 714, 716, 542.
+// - d > 1, narrow columns spread over all of them: as it is; n 1392 360, 261, 263; 1400 560, 428, 422.
+// - otherwise the plain kernel, whose CTAs write one tile at a time: n 1160 275, 319, 381; 1560 388, 443, 463; 1600 293, 331, 302;
+//   1000 231, 281, 277; 2112 391, 484, 440; groups of 8, k 2048, n 1216 109, 104, 107.
+enum class TgmmOneCta { kAsIs, kTurned, kPlain };
+TgmmOneCta tgmm_one_cta(long long m, int n, int g, int ctas) {
+  const int tiles = (n + 255) / 256;
+  if (n % 128 == 0 || tiles == 1 || m / g >= 256) return TgmmOneCta::kAsIs;
+  int d = tiles;
+  for (int r = ctas; r != 0;) {
+    const int t = d % r;
+    d = r;
+    r = t;
+  }
+  const int wide = (n + 63) / 64 % tiles;  // tiles with a block of 64 columns more than the others
+  if (d > 1 && (wide % d != 0 || (n % 64 != 0 && n % 64 < 40))) return TgmmOneCta::kTurned;
+  return d > 1 && wide != 0 ? TgmmOneCta::kAsIs : TgmmOneCta::kPlain;
 }
 
 // Limit of every bounded wait inside a kernel, in microseconds: rd_tile_cfg.wait_limit_ms if
@@ -1353,6 +1379,11 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (bn == 256) return launch_gemm<256, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
     if (bn == 128) return launch_gemm<128, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
     return launch_gemm<64, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
+  }
+  if (two_acc && cta_group == 1) {
+    const TgmmOneCta way = tgmm_one_cta(m, n, g, ctas);
+    if (way == TgmmOneCta::kPlain) return launch_gemm<256, false, true, 1>(ta, tb, tout, args, ctas, stream);
+    args.turn_columns = way == TgmmOneCta::kTurned ? 1 : 0;
   }
   if (two_acc)
     return cta_group == 2 ? launch_tgmm<2>(x, dout, tout, dtype, args, ctas, stream)

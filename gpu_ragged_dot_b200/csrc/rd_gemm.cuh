@@ -74,6 +74,7 @@ struct GemmArgs {
   // tgmm on 256-row tiles: the operand maps are "column-blocked" views (64 columns, rows, blocks
   // of 64 columns), so that ONE box fetches all the 64-column slabs an operand has in a stage.
   int blocked_maps;
+  int turn_columns;  // tgmm with two accumulators: turn the columns of the tile order (rd_tgmm.cuh)
   uint32_t wait_limit_us;  // how long a bounded wait inside the kernel may last (microseconds)
   const float* weight_scale;  // 8-bit inputs: scale of weight matrix w, applied to the accumulator (null: 1)
   // Set: every CTA makes its own group table in shared memory (build_group_table); group_offsets,
