@@ -457,17 +457,19 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
 
 // Fewer rounds than choose_swap asks for: the clocks of both kernels, from their rounds of tiles.  A pair takes 4 clocks per
 // row and block of the contraction and 5000 to drain a tile, a last half round costs 0.55 of one (SwapWork), one CTA 560
-// per block of a 128 x 256 tile; a group's last tile is half full on average.  Timed on both sides on 300 float32, 500
-// 16-bit and 300 e4m3 sizes (1 to 64 groups, equal and unequal, 128 to 14336 deep and wide), this and the rules
-// below against the rules below alone: float32 1.024 times as fast on average over all sizes instead of 1.010, 16 bits
-// 1.012 instead of 1.006, e4m3 1.009 instead of 1.003; slower by more than 2 % in 2, 2 and 0 of them, 7 % at most.  Under
-// half a round, and for groups shorter than `least`, it is wrong too often.
+// per block of a 128 x 256 tile; a group's last tile is half full on average.  Timed on both sides on 400 float32, 600
+// 16-bit and 350 e4m3 sizes (1 to 64 groups, equal and unequal, 256 to 14336 deep and wide), this and the rules
+// below against the rules below alone: float32 1.019 times as fast on average over all sizes instead of 1.012, 16 bits
+// 1.010 instead of 1.004, e4m3 1.005 instead of 1.001; slower by more than 2 % in 0, 2 and 0 of them, 4 % at most.  A
+// last tile of a row that is a half tile counts whole: pairs do not share such tiles evenly (counted half, 704 columns
+// were up to 29 % slower).  Under half a round, and for groups shorter than `least`, it is wrong too often.
 bool swap_takes_less(long long m, int k_blocks, int n, int g, int least, double margin) {
   if (m / g < least) return false;
   const double sms = sm_count(), rows = static_cast<double>(m) / g;
   const double per = rows > 128.0 ? rows / rd::kSwapRows + 0.5 : 1.0;
   const double exact = g * per * ((n + rd::kSwapCols - 1) / rd::kSwapCols) / (sms / 2);
   if (exact < 0.5) return false;
+  if (exact < 1.0) margin = 1.25;
   const double whole = static_cast<double>(static_cast<long long>(exact)), left = exact - whole;
   const double rounds = whole + (left < 0.03 ? 0.0 : left <= 0.5 ? 0.55 : 1.0);
   double height = rows / per + 8.0;

@@ -57,7 +57,7 @@ constexpr int kSwapSmemBytes = kSwapStages * kSwapStageBytes + kSwapEpilogueWarp
 // The tile's rows [row0, row0 + rows) of its group and the pair's first column.
 struct SwapTile {
   int weight, row0, rows, n0;
-  int halves;  // 128-lane halves of each CTA: 2, or 1 for a half tile of 256 columns
+  int halves;  // 128-lane halves of each CTA: 2, or 1 for a half tile of 256 columns, or where no more are left
   int mma_n;  // rows in steps of kStep (16; e4m3 32): the N of the MMAs
 };
 
@@ -132,7 +132,8 @@ __device__ __forceinline__ RowTile find_row_tile(const GemmArgs& p, const SwapGr
 }
 
 // What the pairs walk: whole tiles for whole rounds, and what is left too; where that is half a round or less it is
-// cut into half tiles of 256 columns, one for a pair at most.  Microseconds, alone: m 8192, k 4096, n 5120, 8 groups,
+// cut into half tiles of 256 columns, one for a pair at most.  (A last tile of a row with 256 columns or less is
+// a half tile anyway.)  Microseconds, alone: m 8192, k 4096, n 5120, 8 groups,
 // trans_rhs 271 -> 233; 8192, 2048, 4096, 8 139 -> 106 (in a row, at the power limit, equal: 264 and 266, 114 and 114);
 // in a row float32 8192, 4096, 14336, 8 1285 -> 1254, bf16 727 -> 707.
 struct SwapWork {
@@ -164,7 +165,7 @@ __device__ __forceinline__ SwapTile decode_swap_tile(const GemmArgs& p, const Sw
   t.row0 = r.group_offset + first;
   t.mma_n = imax((per + (mi < more ? 1 : 0)) * kStep, kStep);
   t.rows = imax(imin(t.mma_n, r.group_size - first), 0);
-  t.halves = past < 0 ? 2 : 1;
+  t.halves = past < 0 && p.n - nt * kSwapCols > kSwapCtaCols ? 2 : 1;
   t.n0 = nt * kSwapCols + (past < 0 ? 0 : (past & 1) * kSwapCtaCols);
   return t;
 }
@@ -303,9 +304,9 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       const uint32_t a_hi = static_cast<uint32_t>(adesc0 >> 32);
       const uint32_t b_hi = static_cast<uint32_t>(bdesc0 >> 32);
       uint32_t it = 0;
-      uint32_t local_tile = 0;
+      uint32_t uses[2] = {0u, 0u};  // of either half's accumulator
       bool ok = true;
-      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
+      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
         const SwapTile t = uniform_tile(tile);
         const uint32_t idesc =
             kF32 ? make_idesc_tf32(kBKMajor ? 0 : 1, 0, 2 * kTileM, t.mma_n)
@@ -334,11 +335,14 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             if (kb == k_blocks - 1) umma_commit_pair(smem_u32(&bar_acc_full[h]), 0x3);
           };
           if (kb == 0) {  // a half's accumulator must have been drained by both CTAs
-            for (int h = 0; h < t.halves; ++h) {
-              if (!mbar_wait_warp<true>(smem_u32(&bar_acc_empty[h]), (local_tile & 1u) ^ 1u, abort_ptr)) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (h >= t.halves) break;
+              if (!mbar_wait_warp<true>(smem_u32(&bar_acc_empty[h]), (uses[h] & 1u) ^ 1u, abort_ptr)) {
                 ok = false;
                 break;
               }
+              ++uses[h];
               tc_fence_after_sync();
               if (elect_one()) issue(h, 0u);
             }
@@ -357,18 +361,19 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int half = (warp - 2) >> 2;
     const int quarter = warp & 3;
     const uint32_t staging = stage_base + kStages * kStageBytes + (warp - 2) * 2 * kSwapBoxBytes;
-    uint32_t local_tile = 0;
+    uint32_t uses = 0;
     uint32_t boxes_stored = 0;
     bool ok = true;
     uint16_t* out16 = reinterpret_cast<uint16_t*>(p.out);
-    for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
+    for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
       const SwapTile t = decode_swap_tile<kStep>(p, &group_table, work, tile);
-      if (half >= t.halves) break;  // a half tile is a pair's last
+      if (half >= t.halves) continue;
       const int col0 = t.n0 + (cta_rank * t.halves + half) * kTileM + quarter * 32;  // this warp's first output column; lane = column
-      if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), local_tile & 1u, abort_ptr)) {
+      if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), uses & 1u, abort_ptr)) {
         ok = false;
         break;
       }
+      ++uses;
       tc_fence_after_sync();
       const int chunks = col0 < p.n ? (t.rows + 31) >> 5 : 0;
       const float sc = kFp8 && p.weight_scale != nullptr ? p.weight_scale[t.weight] : 1.0f;
