@@ -91,7 +91,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
 
@@ -129,47 +129,46 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
-        const int kb_count = kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
-        for (int kb = 0; kb < kb_count; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
-            ok = false;
-            break;
-          }
-          const uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kABytes;
-          mbar_arrive_expect_tx(full, kStageBytes);
-          if (kTgmm) {
-            const int r = t.row0 + kb * kF32TileK;
-            if (p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, blocks of 32 columns)
-              tma_load_3d(sa, &tmap_a, full, 0, r, t.k0 >> 5);
-              tma_load_3d(sb, &tmap_b, full, 0, r, t.n0 >> 5);
-            } else {
-#pragma unroll
-              for (int j = 0; j < kTileM / 32; ++j)
-                tma_load_2d(sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
-#pragma unroll
-              for (int j = 0; j < BN / 32; ++j)
-                tma_load_2d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, r);
-            }
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
+      const TileCoord t = uniform_coord(kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0));
+      const int kb_count = kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
+      for (int kb = 0; kb < kb_count; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        if (!elect_one()) continue;
+        const uint32_t full = smem_u32(&bar_full[s]);
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kABytes;
+        mbar_arrive_expect_tx(full, kStageBytes);
+        if (kTgmm) {
+          const int r = t.row0 + kb * kF32TileK;
+          if (p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, blocks of 32 columns)
+            tma_load_3d(sa, &tmap_a, full, 0, r, t.k0 >> 5);
+            tma_load_3d(sb, &tmap_b, full, 0, r, t.n0 >> 5);
           } else {
-            tma_load_2d(sa, &tmap_a, full, kb * kF32TileK, t.row0);
-            if (kBKMajor) {
-              tma_load_3d(sb, &tmap_b, full, kb * kF32TileK, t.n0, t.weight);
-            } else if (p.blocked_maps) {
-              tma_load_4d(sb, &tmap_b, full, 0, kb * kF32TileK, t.n0 >> 5, t.weight);
-            } else {
 #pragma unroll
-              for (int j = 0; j < BN / 32; ++j)
-                tma_load_3d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, kb * kF32TileK, t.weight);
-            }
+            for (int j = 0; j < kTileM / 32; ++j)
+              tma_load_2d(sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
+#pragma unroll
+            for (int j = 0; j < BN / 32; ++j)
+              tma_load_2d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, r);
+          }
+        } else {
+          tma_load_2d(sa, &tmap_a, full, kb * kF32TileK, t.row0);
+          if (kBKMajor) {
+            tma_load_3d(sb, &tmap_b, full, kb * kF32TileK, t.n0, t.weight);
+          } else if (p.blocked_maps) {
+            tma_load_4d(sb, &tmap_b, full, 0, kb * kF32TileK, t.n0 >> 5, t.weight);
+          } else {
+#pragma unroll
+            for (int j = 0; j < BN / 32; ++j)
+              tma_load_3d(sb + j * kF32BoxBytes, &tmap_b, full, t.n0 + j * 32, kb * kF32TileK, t.weight);
           }
         }
       }
@@ -193,12 +192,12 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t local_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
+      const TileCoord t = uniform_coord(kTgmm ? decode_tgmm_tile<BN, 1>(p, &group_table, tile, 0) : decode_gmm_tile<BN, 1>(p, &group_table, tile, 0));
       const int kb_count = kTgmm ? (t.rows + kF32TileK - 1) / kF32TileK : k_blocks_gmm;
       const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing_f32(t.rows);
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
+      if (!mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
         ok = false;
         break;
       }
@@ -207,7 +206,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t s = it % kStages;
       uint32_t ph = (it / kStages) & 1u;
       for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
-        if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+        if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
           ok = false;
           break;
         }
@@ -219,7 +218,7 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
           __syncwarp();
         }
         tc_fence_after_sync();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4);
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
           if (kTgmm && n_mma < kF32TileK / kF32UmmaK) {
@@ -238,10 +237,9 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           umma_commit(smem_u32(&bar_empty[s]));
         }
-        __syncwarp();
       }
       if (!ok) break;
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t bar = smem_u32(&bar_acc_full[acc]);
         if (kb_count > 0) {
           umma_commit(bar);
@@ -249,7 +247,6 @@ ragged_gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,
           mbar_arrive(bar);  // empty group: nothing to wait for
         }
       }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)

@@ -27,10 +27,12 @@
 // box of a column-blocked view where its rows are multiples of 32; other rows, four 4 KB boxes per operand,
 // only reach the three-product form.  One product, measured on both sides: choose_f32_pair in rd_api.cu.
 //
-// Roles: warp 0 = TMA producer, warp 1 = MMA issuer (one thread, of the leader CTA), warps 2..5 =
+// Roles: warp 0 = TMA producer, warp 1 = MMA issuer (of the leader CTA), warps 2..5 =
 // epilogue, warps 6.. = converters (kSplit, eight) or the tail fixer (one, tgmm).  tgmm rows past
 // a group's end are cleared by the converters as they pass, or by the fixer as in rd_gemm.cuh.
 // Operand layouts are those of rd_gemm_f32.cuh; waits are bounded as everywhere.
+// The producer and the MMA warp run their loops as whole warps and elect a lane per stage (rd_tgmm.cuh): one-product tgmm,
+// m 8192, k 4096, n 1536, 8 groups 201 -> 182 us, three products forward + backward, m 4096, 872 -> 863.
 #pragma once
 
 #include "rd_gemm_f32.cuh"
@@ -102,7 +104,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int cta_rank = static_cast<int>(cluster_cta_rank());
   const bool leader = cta_rank == 0;
@@ -153,70 +155,69 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = decode(tile);
-        const int nb = t.n0 + cta_rank * kBCols;  // first B column this CTA loads
-        const int kb_count = blocks_of(t);
-        for (int kb = 0; kb < kb_count; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
-            ok = false;
-            break;
-          }
-          uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kF32PairABytes;
-          // kSplit: each CTA's converters wait for that CTA's own data.  Otherwise the peer's bytes
-          // are counted on the leader's barrier, except for a stage whose tail rows it clears first.
-          const bool local_stage = kSplit || (kTgmm && kb == kb_count - 1 && tail_needs_clearing_f32(t.rows));
-          bool remote_bar = false;
-          if (leader) {
-            mbar_arrive_expect_tx(full, local_stage ? kF32PairRawBytes : 2 * kF32PairRawBytes);
-          } else if (local_stage) {
-            mbar_arrive_expect_tx(full, kF32PairRawBytes);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
+      const TileCoord t = uniform_coord(decode(tile));
+      const int nb = t.n0 + cta_rank * kBCols;  // first B column this CTA loads
+      const int kb_count = blocks_of(t);
+      for (int kb = 0; kb < kb_count; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        if (!elect_one()) continue;
+        uint32_t full = smem_u32(&bar_full[s]);
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kF32PairABytes;
+        // kSplit: each CTA's converters wait for that CTA's own data.  Otherwise the peer's bytes
+        // are counted on the leader's barrier, except for a stage whose tail rows it clears first.
+        const bool local_stage = kSplit || (kTgmm && kb == kb_count - 1 && tail_needs_clearing_f32(t.rows));
+        bool remote_bar = false;
+        if (leader) {
+          mbar_arrive_expect_tx(full, local_stage ? kF32PairRawBytes : 2 * kF32PairRawBytes);
+        } else if (local_stage) {
+          mbar_arrive_expect_tx(full, kF32PairRawBytes);
+        } else {
+          full = map_to_cta(full, 0);
+          remote_bar = true;
+        }
+        if (kTgmm) {
+          const int r = t.row0 + kb * kF32TileK;
+          if (!kSplit || p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, 4 blocks of 32 columns)
+            load_3d(remote_bar, sa, &tmap_a, full, 0, r, t.k0 >> 5);
+            load_3d(remote_bar, sb, &tmap_b, full, 0, r, nb >> 5);
           } else {
-            full = map_to_cta(full, 0);
-            remote_bar = true;
+#pragma unroll
+            for (int j = 0; j < kTileM / 32; ++j)
+              load_2d(remote_bar, sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
+#pragma unroll
+            for (int j = 0; j < kBCols / 32; ++j)
+              load_2d(remote_bar, sb + j * kF32BoxBytes, &tmap_b, full, nb + j * 32, r);
           }
-          if (kTgmm) {
-            const int r = t.row0 + kb * kF32TileK;
-            if (!kSplit || p.blocked_maps) {  // one box per operand: (32 columns, 32 rows, 4 blocks of 32 columns)
-              load_3d(remote_bar, sa, &tmap_a, full, 0, r, t.k0 >> 5);
-              load_3d(remote_bar, sb, &tmap_b, full, 0, r, nb >> 5);
+        } else {
+          load_2d(remote_bar, sa, &tmap_a, full, kb * kF32TileK, t.row0);
+          if (kBKMajor) {
+            load_3d(remote_bar, sb, &tmap_b, full, kb * kF32TileK, nb, t.weight);
+          } else if (p.blocked_maps) {  // (32 columns, 32 rows of k, 4 blocks of 32 columns, weight)
+            if (remote_bar) {
+              tma_load_4d_pair(sb, &tmap_b, full, 0, kb * kF32TileK, nb >> 5, t.weight);
             } else {
-#pragma unroll
-              for (int j = 0; j < kTileM / 32; ++j)
-                load_2d(remote_bar, sa + j * kF32BoxBytes, &tmap_a, full, t.k0 + j * 32, r);
-#pragma unroll
-              for (int j = 0; j < kBCols / 32; ++j)
-                load_2d(remote_bar, sb + j * kF32BoxBytes, &tmap_b, full, nb + j * 32, r);
+              tma_load_4d(sb, &tmap_b, full, 0, kb * kF32TileK, nb >> 5, t.weight);
             }
           } else {
-            load_2d(remote_bar, sa, &tmap_a, full, kb * kF32TileK, t.row0);
-            if (kBKMajor) {
-              load_3d(remote_bar, sb, &tmap_b, full, kb * kF32TileK, nb, t.weight);
-            } else if (p.blocked_maps) {  // (32 columns, 32 rows of k, 4 blocks of 32 columns, weight)
-              if (remote_bar) {
-                tma_load_4d_pair(sb, &tmap_b, full, 0, kb * kF32TileK, nb >> 5, t.weight);
-              } else {
-                tma_load_4d(sb, &tmap_b, full, 0, kb * kF32TileK, nb >> 5, t.weight);
-              }
-            } else {
 #pragma unroll
-              for (int j = 0; j < kBCols / 32; ++j)
-                load_3d(remote_bar, sb + j * kF32BoxBytes, &tmap_b, full, nb + j * 32, kb * kF32TileK, t.weight);
-            }
+            for (int j = 0; j < kBCols / 32; ++j)
+              load_3d(remote_bar, sb + j * kF32BoxBytes, &tmap_b, full, nb + j * 32, kb * kF32TileK, t.weight);
           }
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0 && leader) {
+    // ------------------------------------------------------------ MMA issuer (of the leader)
+    if (leader) {
       const uint32_t idesc = make_idesc_tf32(kTgmm ? 1 : 0, kBKMajor ? 0 : 1, 2 * kTileM, BN);
       constexpr uint32_t kAStep = (kTgmm ? 1024u : 32u) >> 4;  // 8 k-rows of 128 B, or 8 k-elements
       constexpr uint32_t kBStep = (kBKMajor ? 32u : 1024u) >> 4;
@@ -234,13 +235,13 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t tail_events = 0;
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-        const TileCoord t = decode(tile);
+        const TileCoord t = uniform_coord(decode(tile));
         const int kb_count = blocks_of(t);
         const bool tail_stage = !kSplit && kTgmm && kb_count > 0 && tail_needs_clearing_f32(t.rows);
         // kSplit: one tile at a time, large products in columns [0, BN), small ones in [BN, 2 BN).
         const uint32_t acc = kSplit ? 0u : (local_tile & 1u);
         const uint32_t acc_ph = kSplit ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
-        if (!mbar_wait<true>(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
+        if (!mbar_wait_warp<true>(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
           ok = false;
           break;
         }
@@ -250,14 +251,16 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         uint32_t ph = (it / kStages) & 1u;
         for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
           const uint32_t landed = kSplit ? smem_u32(&bar_conv[s]) : smem_u32(&bar_full[s]);
-          if (!mbar_wait<kSplit>(landed, ph, abort_ptr)) {
+          if (!mbar_wait_warp<kSplit>(landed, ph, abort_ptr)) {
             ok = false;
             break;
           }
           if (!kSplit && kTgmm && tail_stage && kb == kb_count - 1) {
-            mbar_arrive(smem_u32(&bar_tail_go));
-            mbar_arrive_cluster(smem_u32(&bar_tail_go), 1);
-            if (!mbar_wait<true>(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
+            if (elect_one()) {
+              mbar_arrive(smem_u32(&bar_tail_go));
+              mbar_arrive_cluster(smem_u32(&bar_tail_go), 1);
+            }
+            if (!mbar_wait_warp<true>(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
               ok = false;
               break;
             }
@@ -267,6 +270,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4);
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
           const uint32_t more = kb > 0 ? 1u : 0u;
+          if (!elect_one()) continue;
           if constexpr (kSplit) {
 #pragma unroll
             for (int kk = 0; kk < kF32TileK / kF32UmmaK; ++kk)  // lo . hi
@@ -293,11 +297,13 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         if (!ok) break;
         const uint32_t bar = smem_u32(&bar_acc_full[acc]);
-        if (kb_count > 0) {
-          umma_commit_pair(bar, 0x3);
-        } else {  // empty group: nothing to wait for
-          mbar_arrive(bar);
-          mbar_arrive_cluster(bar, 1);
+        if (elect_one()) {
+          if (kb_count > 0) {
+            umma_commit_pair(bar, 0x3);
+          } else {  // empty group: nothing to wait for
+            mbar_arrive(bar);
+            mbar_arrive_cluster(bar, 1);
+          }
         }
       }
     }

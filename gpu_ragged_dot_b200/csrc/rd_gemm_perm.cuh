@@ -82,7 +82,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
 
@@ -126,48 +126,47 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     // Posts each stage's TMA byte count and loads the operands that need no gather.
-    if (lane == 0) {
-      const uint32_t tma_bytes = (gather_a ? 0u : kABytes) + (gather_b ? 0u : kBBytes);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
-        const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
-        for (int kb = 0; kb < kb_count; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
-            ok = false;
-            break;
+    const uint32_t tma_bytes = (gather_a ? 0u : kABytes) + (gather_b ? 0u : kBBytes);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step) {
+      const TileCoord t = uniform_coord(kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0));
+      const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
+      for (int kb = 0; kb < kb_count; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        if (!elect_one()) continue;
+        const uint32_t full = smem_u32(&bar_full[s]);
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kABytes;
+        if (tma_bytes != 0) {
+          mbar_arrive_expect_tx(full, tma_bytes);
+        } else {
+          mbar_arrive(full);
+        }
+        if (kTgmm) {
+          const int r = t.row0 + kb * kTileK;
+          if (!gather_a) {
+            tma_load_2d(sa, &tmap_a, full, t.k0, r);
+            tma_load_2d(sa + kBoxBytes, &tmap_a, full, t.k0 + 64, r);
           }
-          const uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kABytes;
-          if (tma_bytes != 0) {
-            mbar_arrive_expect_tx(full, tma_bytes);
-          } else {
-            mbar_arrive(full);
+          if (!gather_b) {
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j)
+              tma_load_2d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, r);
           }
-          if (kTgmm) {
-            const int r = t.row0 + kb * kTileK;
-            if (!gather_a) {
-              tma_load_2d(sa, &tmap_a, full, t.k0, r);
-              tma_load_2d(sa + kBoxBytes, &tmap_a, full, t.k0 + 64, r);
-            }
-            if (!gather_b) {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, r);
-            }
+        } else {
+          if (!gather_a) tma_load_2d(sa, &tmap_a, full, kb * kTileK, t.row0);
+          if (kBKMajor) {
+            tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
           } else {
-            if (!gather_a) tma_load_2d(sa, &tmap_a, full, kb * kTileK, t.row0);
-            if (kBKMajor) {
-              tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
-            } else {
 #pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
-            }
+            for (int j = 0; j < BN / 64; ++j)
+              tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
           }
         }
       }
@@ -300,12 +299,12 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t local_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-      const TileCoord t = kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0);
+      const TileCoord t = uniform_coord(kTgmm ? decode_tgmm_tile<BN, 1>(p, nullptr, tile, 0) : decode_gmm_tile<BN, 1>(p, nullptr, tile, 0));
       const int kb_count = kTgmm ? (t.rows + kTileK - 1) / kTileK : k_blocks_gmm;
       const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
+      if (!mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
         ok = false;
         break;
       }
@@ -314,7 +313,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t s = it % kStages;
       uint32_t ph = (it / kStages) & 1u;
       for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
-        if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+        if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
           ok = false;
           break;
         }
@@ -329,7 +328,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           __syncwarp();
         }
         tc_fence_after_sync();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4);
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
           if (kTgmm && n_mma < kTileK / kUmmaK) {
@@ -348,10 +347,9 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           umma_commit(smem_u32(&bar_empty[s]));
         }
-        __syncwarp();
       }
       if (!ok) break;
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t bar = smem_u32(&bar_acc_full[acc]);
         if (kb_count > 0) {
           umma_commit(bar);
@@ -359,7 +357,6 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           mbar_arrive(bar);
         }
       }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)

@@ -63,7 +63,7 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_cta_rank());
   const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -104,59 +104,57 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   bool ok = true;           // a wait that expired ends this thread's waiting, not the tile loop:
                             // every CTA of the cluster must reach the same cluster barriers
   for (int tile = static_cast<int>(blockIdx.x) / split; tile < num_tiles; tile += clusters, ++local_tile) {
-    const TileCoord t = decode_gmm_tile<BN, 1>(p, &group_table, tile, 0);
+    const TileCoord t = uniform_coord(decode_gmm_tile<BN, 1>(p, &group_table, tile, 0));
     const bool half = t.rows <= 64;
     if (warp == 0) {
-      if (lane == 0) {
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
-            ok = false;
-            break;
-          }
-          const uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kABytes;
-          mbar_arrive_expect_tx(full, kStageBytes);
-          tma_load_2d(sa, &tmap_a, full, kb * kTileK, t.row0);
-          if (kBKMajor) {
-            tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
-          } else {
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        if (!elect_one()) continue;
+        const uint32_t full = smem_u32(&bar_full[s]);
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kABytes;
+        mbar_arrive_expect_tx(full, kStageBytes);
+        tma_load_2d(sa, &tmap_a, full, kb * kTileK, t.row0);
+        if (kBKMajor) {
+          tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
+        } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
-          }
+          for (int j = 0; j < BN / 64; ++j)
+            tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
         }
       }
       __syncwarp();
     } else if (warp == 1) {
-      if (lane == 0) {
-        const uint32_t idesc =
-            make_idesc_f16(kFp8 ? 0 : p.ab_format, 0, kBKMajor ? 0 : 1, half ? 64 : kTileM, BN);
-        constexpr uint32_t kAStep = 32u >> 4;
-        constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
-        const uint64_t adesc0 = make_smem_desc(stage_base, 16, 1024);
-        const uint64_t bdesc0 = kBKMajor ? make_smem_desc(stage_base + kABytes, 16, 1024)
-                                         : make_smem_desc(stage_base + kABytes, kBoxBytes, 1024);
-        const uint32_t desc_hi = static_cast<uint32_t>(adesc0 >> 32);
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          if (!mbar_wait(smem_u32(&bar_full[s]), (it / kStages) & 1u, abort_ptr)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint32_t a_lo = static_cast<uint32_t>(adesc0) + s * (kStageBytes >> 4);
-          const uint32_t b_lo = static_cast<uint32_t>(bdesc0) + s * (kStageBytes >> 4);
-#pragma unroll
-          for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
-            umma_ab<1, kFp8>(tmem_base, make_desc64(a_lo + kk * kAStep, desc_hi),
-                             make_desc64(b_lo + kk * kBStep, desc_hi), idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-          umma_commit(smem_u32(&bar_empty[s]));
+      const uint32_t idesc =
+          make_idesc_f16(kFp8 ? 0 : p.ab_format, 0, kBKMajor ? 0 : 1, half ? 64 : kTileM, BN);
+      constexpr uint32_t kAStep = 32u >> 4;
+      constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
+      const uint64_t adesc0 = make_smem_desc(stage_base, 16, 1024);
+      const uint64_t bdesc0 = kBKMajor ? make_smem_desc(stage_base + kABytes, 16, 1024)
+                                       : make_smem_desc(stage_base + kABytes, kBoxBytes, 1024);
+      const uint32_t desc_hi = static_cast<uint32_t>(adesc0 >> 32);
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        if (!mbar_wait_warp(smem_u32(&bar_full[s]), (it / kStages) & 1u, abort_ptr)) {
+          ok = false;
+          break;
         }
-        if (ok) umma_commit(smem_u32(&bar_acc_full));
+        tc_fence_after_sync();
+        if (!elect_one()) continue;
+        const uint32_t a_lo = static_cast<uint32_t>(adesc0) + s * (kStageBytes >> 4);
+        const uint32_t b_lo = static_cast<uint32_t>(bdesc0) + s * (kStageBytes >> 4);
+#pragma unroll
+        for (int kk = 0; kk < kTileK / kUmmaK; ++kk)
+          umma_ab<1, kFp8>(tmem_base, make_desc64(a_lo + kk * kAStep, desc_hi),
+                           make_desc64(b_lo + kk * kBStep, desc_hi), idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&bar_empty[s]));
       }
+      if (ok && elect_one()) umma_commit(smem_u32(&bar_acc_full));
       __syncwarp();
     } else {
       // The accumulator is complete when all MMAs have retired, so the ring is idle and its memory
