@@ -250,16 +250,22 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 }
 
 // Start a kernel while the one before it still runs?  Only kernels that wait for it themselves, and
-// only where no CTA has more than one tile: there the launch is a good part of the time (4 rows through
+// where no CTA has more than one tile: there the launch is a good part of the time (4 rows through
 // 4 of 64 experts, k 4096, n 1536: 17.9 -> 15.7 us a call back to back).  With more tiles it costs: CTAs
 // then land on SMs in the order in which the kernel before leaves them, and neighbours in the tile
 // order, which share operand panels, no longer lie side by side (Mixtral-shaped training step 2.57 ->
 // 2.70 ms, 64 groups 1.41 -> 1.54 ms, 256 groups 5.1 -> 5.5 ms).
+// Groups of 64 rows and less read (or write) weights that no neighbour shares, so there it gains its 2 us too, up to some
+// 512 MB of weights, 80 us: 256 rows, k 4096, n 1536, 64 groups of e4m3 67.7 -> 65.4; 4000, 1024, 1024, 64 30.9 -> 29.5, tgmm
+// 37.0 -> 34.9; 300, 1000, 2000, 100 tgmm 72.5 -> 69.1.  Above, nothing or less: the first in bf16 119.0 -> 119.3; 512, 7168,
+// 2048, 256 755 -> 770.
 bool launch_early(const GemmArgs& args, int ctas_per_tile = 1) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
                                                : static_cast<long long>(args.m < args.g ? args.m : args.g) + args.m / rd::kTileM;
-  return row_tiles * args.n_tiles * ctas_per_tile <= sm_count();
+  if (row_tiles * args.n_tiles * ctas_per_tile <= sm_count()) return true;
+  const double weight_bytes = 2.0 * (args.m < args.g ? args.m : args.g) * args.k * args.n;
+  return args.m <= 64LL * args.g && weight_bytes <= 512e6;
 }
 
 // How many clusters of two CTAs can be resident at once (0: the query failed).
