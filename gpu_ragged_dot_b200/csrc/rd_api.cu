@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "../../include/ragged_dot_b200.h"
@@ -290,18 +291,33 @@ int resident_pairs(Kernel kernel, int threads, size_t smem_bytes) {
   return clusters;
 }
 
+// The same, asked once for a kernel and device (the query takes longer than the launch).  A template argument, so that
+// every kernel has its own answers.
+template <auto kKernel>
+int resident_pairs_once(int threads, size_t smem_bytes) {
+  static std::atomic<int> known[64];  // pairs + 1; 0 = not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return resident_pairs(kKernel, threads, smem_bytes);
+  int n = known[dev].load(std::memory_order_relaxed) - 1;
+  if (n <= 0) {
+    n = resident_pairs(kKernel, threads, smem_bytes);
+    known[dev].store(n + 1, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 // A persistent grid of pairs must be fully co-resident.
-template <typename Kernel, typename... Maps>
-int launch_pairs(Kernel kernel, int threads, int smem_bytes, const GemmArgs& args, int ctas, cudaStream_t stream,
+template <auto kKernel, typename... Maps>
+int launch_pairs(int threads, int smem_bytes, const GemmArgs& args, int ctas, cudaStream_t stream,
                  const Maps&... maps) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
     return RD_ERR_LAUNCH;
-  const int clusters = resident_pairs(kernel, threads, smem_bytes);
+  const int clusters = resident_pairs_once<kKernel>(threads, smem_bytes);
   if (clusters <= 0) return RD_ERR_LAUNCH;
   int pairs = ctas / 2;
   if (pairs > clusters) pairs = clusters;
   if (pairs < 1) pairs = 1;
-  return launch_kernel(kernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args, 2), stream, maps..., args);
+  return launch_kernel(kKernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args, 2), stream, maps..., args);
 }
 
 template <int BN, bool kBKMajor, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false>
@@ -310,8 +326,8 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   constexpr int kStageBytes = rd::stage_bytes<BN, kCtas>();
   constexpr int kStages = (196608 / kStageBytes) > 8 ? 8 : (196608 / kStageBytes);
   constexpr int kSmem = kStages * kStageBytes + rd::kOutStagingBytes + 1024;
-  auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, kCtas, kSeg, kFp8>;
-  if (kCtas == 2) return launch_pairs(kernel, rd::kGemmFixerThreads, kSmem, args, ctas, stream, ta, tb, tout);
+  constexpr auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, kCtas, kSeg, kFp8>;
+  if constexpr (kCtas == 2) return launch_pairs<kernel>(rd::kGemmFixerThreads, kSmem, args, ctas, stream, ta, tb, tout);
   // The attribute is per device; setting it again is cheap, so do it on every call rather
   // than track which devices have seen it.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -401,7 +417,7 @@ int launch_gemm2_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
 template <bool kBKMajor, bool kTgmm, bool kSplit>
 int launch_gemm_f32_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout, const GemmArgs& args,
                          int ctas, cudaStream_t stream) {
-  return launch_pairs(rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, kSplit>, rd::f32_pair_threads<kSplit>(),
+  return launch_pairs<rd::ragged_gemm_f32_pair_kernel<kBKMajor, kTgmm, kSplit>>(rd::f32_pair_threads<kSplit>(),
                       rd::f32_pair_smem_bytes<kSplit>(), args, ctas, stream, ta, tb, tout);
 }
 
@@ -554,7 +570,7 @@ int launch_gemm_swap(const void* x, const void* A, void* y, int dtype, int num_w
     if (rc != RD_OK) return rc;
   }
   args.n_tiles = (args.n + rd::kSwapCols - 1) / rd::kSwapCols;
-  return launch_pairs(rd::ragged_gemm_swap_kernel<kBKMajor, kFp8, kF32>, rd::kSwapThreads, rd::kSwapSmemBytes, args,
+  return launch_pairs<rd::ragged_gemm_swap_kernel<kBKMajor, kFp8, kF32>>(rd::kSwapThreads, rd::kSwapSmemBytes, args,
                       sm_count(), stream, tw, tx, tout, tout16);
 }
 
@@ -574,10 +590,10 @@ int launch_tgmm(const void* x, const void* dout, const CUtensorMap& tout, int dt
   if (rc == RD_OK && args.n >= 64)
     rc = encode_blocked_map(&tb, dout, dtype, args.n, args.m, rd::kTileK, rd::kTgTileN / 64 / kCtas);
   if (rc != RD_OK) return rc;
-  auto kernel = rd::ragged_tgmm_kernel<kCtas>;
+  constexpr auto kernel = rd::ragged_tgmm_kernel<kCtas>;
   constexpr int kSmem = rd::tg_smem_bytes<kCtas>();
   if constexpr (kCtas == 2)
-    return launch_pairs(kernel, rd::kTgThreads, kSmem, args, ctas, stream, ta, ta2, tb, tb2, tout);
+    return launch_pairs<kernel>(rd::kTgThreads, kSmem, args, ctas, stream, ta, ta2, tb, tb2, tout);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
     return RD_ERR_LAUNCH;
   return launch_kernel(kernel, ctas, rd::kTgThreads, kSmem, 1, launch_early(args), stream, ta, ta2, tb, tb2, tout, args);

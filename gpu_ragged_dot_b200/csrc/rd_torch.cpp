@@ -59,82 +59,102 @@ struct Cfg {
   const rd_tile_cfg* ptr() const { return set ? &cfg : nullptr; }
 };
 
+// One product in the plain form: what its call needs, and whether the operands are of that form at all.
 // max_unaligned: elements up to which rows that are not multiples of 16 bytes go to rd_*_unaligned.
-py::object gmm(const Tensor& x, const Tensor& A, const Tensor& gs, bool trans_rhs, int tile_n, int cta_group,
-               int tile_m, int max_ctas, int flags, int64_t max_unaligned) {
-  if (!x.is_cuda()) return py::none();
-  const auto device = x.device().index();
-  if (!dense(x, device) || !dense(A, device) || !dense(gs, device)) return py::none();
-  const int dtype = dtype_code(x.scalar_type());
-  if (dtype < 0 || A.scalar_type() != x.scalar_type() || gs.scalar_type() != at::kInt) return py::none();
-  if (x.dim() != 2 || A.dim() != 3 || gs.dim() != 1 || A.size(0) != gs.size(0)) return py::none();
-  const int64_t m = x.size(0), k = x.size(1), g = gs.size(0);
-  const int64_t n = A.size(trans_rhs ? 1 : 2);
-  if (A.size(trans_rhs ? 2 : 1) != k) return py::none();
-  if (!fits_int(m) || !fits_int(k) || !fits_int(n) || !fits_int(g)) return py::none();
-  const int mask = dtype == RD_DTYPE_F32 ? 3 : 7;
-  const bool odd = (k & mask) || (n & mask);
-  if (!odd && (!aligned16(x) || !aligned16(A))) return py::none();
-  const Cfg cfg(tile_n, cta_group, tile_m, max_ctas, flags);
-  if (odd && (dtype == RD_DTYPE_F32 || cfg.set || g > 256 || m > (1 << 20) ||
-              m * k + g * k * n + m * n > max_unaligned))
-    return py::none();
-  const c10::cuda::OptionalCUDAGuard guard(x.device());
-  void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  Tensor y;
+struct Product {
+  Tensor a, b, gs, out;  // gmm: x, A; tgmm: x, y
+  int64_t m = 0, k = 0, n = 0, g = 0;
+  int dtype = -1;
+  bool tgmm, trans_rhs, odd = false;
+  Cfg cfg;
+
+  Product(bool tgmm_, const Tensor& a_, const Tensor& b_, const Tensor& gs_, bool trans_rhs_, const Cfg& cfg_)
+      : a(a_), b(b_), gs(gs_), tgmm(tgmm_), trans_rhs(trans_rhs_), cfg(cfg_) {}
+
+  bool plain(int64_t max_unaligned) {
+    if (!a.is_cuda()) return false;
+    const auto device = a.device().index();
+    if (!dense(a, device) || !dense(b, device) || !dense(gs, device)) return false;
+    dtype = dtype_code(a.scalar_type());
+    if (dtype < 0 || b.scalar_type() != a.scalar_type() || gs.scalar_type() != at::kInt) return false;
+    if (a.dim() != 2 || b.dim() != (tgmm ? 2 : 3) || gs.dim() != 1) return false;
+    m = a.size(0);
+    k = a.size(1);
+    g = gs.size(0);
+    if (tgmm) {
+      if (b.size(0) != m) return false;
+      n = b.size(1);
+    } else {
+      if (b.size(0) != g || b.size(trans_rhs ? 2 : 1) != k) return false;
+      n = b.size(trans_rhs ? 1 : 2);
+    }
+    if (!fits_int(m) || !fits_int(k) || !fits_int(n) || !fits_int(g)) return false;
+    const int mask = dtype == RD_DTYPE_F32 ? 3 : 7;
+    odd = (k & mask) || (n & mask);
+    if (!odd) return aligned16(a) && aligned16(b);
+    return !(dtype == RD_DTYPE_F32 || cfg.set || g > 256 || m > (1 << 20) || m * k + g * k * n + m * n > max_unaligned);
+  }
+
+  // Allocates the result and launches; the caller holds the device guard, and no GIL.
+  int run(void* stream) {
+    out = tgmm ? at::empty({g, k, n}, a.options()) : at::empty({m, n}, a.options());
+    Tensor ws = workspace(m, g, a);
+    if (odd) {
+      const int64_t b_cols = tgmm || !trans_rhs ? n : k, b_rows = tgmm ? m : g * (trans_rhs ? n : k);
+      Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, b_rows, b_cols), a);
+      return tgmm ? rd_tgmm_unaligned(a.data_ptr(), b.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(),
+                                      ws.numel(), scratch.data_ptr(), scratch.numel(), m, k, n, g, dtype, stream)
+                  : rd_gmm_unaligned(a.data_ptr(), b.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(),
+                                     ws.numel(), scratch.data_ptr(), scratch.numel(), m, k, n, g, trans_rhs, dtype,
+                                     stream);
+    }
+    return tgmm ? rd_tgmm(a.data_ptr(), b.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(), m, k,
+                          n, g, dtype, cfg.ptr(), stream)
+                : rd_gmm(a.data_ptr(), b.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(), m, k,
+                         n, g, trans_rhs, dtype, cfg.ptr(), stream);
+  }
+};
+
+py::object run_one(Product p, int64_t max_unaligned) {
+  if (!p.plain(max_unaligned)) return py::none();
+  const c10::cuda::OptionalCUDAGuard guard(p.a.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(p.a.device().index()).stream();
   int rc;
   {
     const py::gil_scoped_release no_gil;
-    y = at::empty({m, n}, x.options());
-    Tensor ws = workspace(m, g, x);
-    if (odd) {
-      const int64_t a_cols = trans_rhs ? k : n, a_rows = g * (trans_rhs ? n : k);
-      Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, a_rows, a_cols), x);
-      rc = rd_gmm_unaligned(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(),
-                            scratch.data_ptr(), scratch.numel(), m, k, n, g, trans_rhs, dtype, stream);
-    } else {
-      rc = rd_gmm(x.data_ptr(), A.data_ptr(), gs.data_ptr<int>(), y.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
-                  trans_rhs, dtype, cfg.ptr(), stream);
-    }
+    rc = p.run(stream);
   }
-  return result(rc, y);
+  return result(rc, p.out);
+}
+
+py::object gmm(const Tensor& x, const Tensor& A, const Tensor& gs, bool trans_rhs, int tile_n, int cta_group,
+               int tile_m, int max_ctas, int flags, int64_t max_unaligned) {
+  return run_one(Product(false, x, A, gs, trans_rhs, Cfg(tile_n, cta_group, tile_m, max_ctas, flags)), max_unaligned);
 }
 
 py::object tgmm(const Tensor& x, const Tensor& y, const Tensor& gs, int tile_n, int cta_group, int tile_m,
                 int max_ctas, int flags, int64_t max_unaligned) {
-  if (!x.is_cuda()) return py::none();
-  const auto device = x.device().index();
-  if (!dense(x, device) || !dense(y, device) || !dense(gs, device)) return py::none();
-  const int dtype = dtype_code(x.scalar_type());
-  if (dtype < 0 || y.scalar_type() != x.scalar_type() || gs.scalar_type() != at::kInt) return py::none();
-  if (x.dim() != 2 || y.dim() != 2 || gs.dim() != 1 || x.size(0) != y.size(0)) return py::none();
-  const int64_t m = x.size(0), k = x.size(1), n = y.size(1), g = gs.size(0);
-  if (!fits_int(m) || !fits_int(k) || !fits_int(n) || !fits_int(g)) return py::none();
-  const int mask = dtype == RD_DTYPE_F32 ? 3 : 7;
-  const bool odd = (k & mask) || (n & mask);
-  if (!odd && (!aligned16(x) || !aligned16(y))) return py::none();
-  const Cfg cfg(tile_n, cta_group, tile_m, max_ctas, flags);
-  if (odd && (dtype == RD_DTYPE_F32 || cfg.set || g > 256 || m > (1 << 20) ||
-              m * k + m * n + g * k * n > max_unaligned))
-    return py::none();
-  const c10::cuda::OptionalCUDAGuard guard(x.device());
-  void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-  Tensor out;
+  return run_one(Product(true, x, y, gs, false, Cfg(tile_n, cta_group, tile_m, max_ctas, flags)), max_unaligned);
+}
+
+// Both products of gmm's backward pass in one call: (dx, dA), None or an error code.  Nothing is launched unless both are of
+// the plain form.  The two calls from Python, on autograd's thread, took 31 us of the host's time.
+py::object gmm_backward(const Tensor& dout, const Tensor& x, const Tensor& A, const Tensor& gs, bool trans_rhs,
+                        int64_t max_unaligned) {
+  const Cfg none(0, 0, 0, 0, 0);
+  Product dx(false, dout, A, gs, !trans_rhs, none);
+  Product dA(true, trans_rhs ? dout : x, trans_rhs ? x : dout, gs, false, none);
+  if (!dx.plain(max_unaligned) || !dA.plain(max_unaligned) || dA.a.device() != dx.a.device()) return py::none();
+  const c10::cuda::OptionalCUDAGuard guard(dout.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(dout.device().index()).stream();
   int rc;
   {
     const py::gil_scoped_release no_gil;
-    out = at::empty({g, k, n}, x.options());
-    Tensor ws = workspace(m, g, x);
-    if (odd) {
-      Tensor scratch = bytes(rd_unaligned_scratch_bytes(m, k, m, n), x);
-      rc = rd_tgmm_unaligned(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(),
-                             scratch.data_ptr(), scratch.numel(), m, k, n, g, dtype, stream);
-    } else {
-      rc = rd_tgmm(x.data_ptr(), y.data_ptr(), gs.data_ptr<int>(), out.data_ptr(), ws.data_ptr(), ws.numel(), m, k, n, g,
-                   dtype, cfg.ptr(), stream);
-    }
+    rc = dx.run(stream);
+    if (rc == RD_OK) rc = dA.run(stream);
   }
-  return result(rc, out);
+  if (rc != RD_OK) return py::int_(rc);
+  return py::make_tuple(dx.out, dA.out);
 }
 
 py::object gmm_fp8(const Tensor& x, const Tensor& A, const Tensor& gs, const c10::optional<Tensor>& scale) {
@@ -172,5 +192,6 @@ py::object gmm_fp8(const Tensor& x, const Tensor& A, const Tensor& gs, const c10
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod) {
   mod.def("gmm", &gmm);
   mod.def("tgmm", &tgmm);
+  mod.def("gmm_backward", &gmm_backward);
   mod.def("gmm_fp8", &gmm_fp8);
 }

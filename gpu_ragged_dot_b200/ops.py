@@ -197,6 +197,22 @@ def _native(where: str, fn, op: str, x, w, group_sizes, m_k_n, cfg, *args):
     return res
 
 
+def _native_backward(do, x, A, group_sizes, trans_rhs: bool):
+    """(dx, dA) of the plain form through one native call, or None: a tile table entry for either product,
+    status checks, or operands the native path does not take."""
+    if _check_status_enabled() or not (_tensors(do, 2, A, 3, group_sizes) and _tensors(x, 2, A, 3, group_sizes)):
+        return None
+    if x.dtype != torch.float32:
+        (m, n), k, g = do.shape, x.shape[1], group_sizes.shape[0]
+        if (tile_table.lookup("gmm" if trans_rhs else "gmm_t", m, n, k, g) is not None
+                or tile_table.lookup("tgmm", m, *((n, k) if trans_rhs else (k, n)), g) is not None):
+            return None
+    res = _lib.host().gmm_backward(do, x, A, group_sizes, trans_rhs, _UNALIGNED_MAX_ELEMENTS)
+    if isinstance(res, int):
+        _lib.check(res, "rd_gmm / rd_tgmm")
+    return res
+
+
 def _use_unaligned(elements: int, m: int, g: int, dtype: torch.dtype, *row_lengths: int) -> bool:
     """Small 16-bit products with rows that are not multiples of 16 bytes: ``rd_gmm_unaligned`` /
     ``rd_tgmm_unaligned`` (two launches) instead of padding with torch, the plain kernel and a copy
@@ -1000,6 +1016,10 @@ class _GmmFn(torch.autograd.Function):
         x, A, group_sizes = ctx.saved_tensors
         cd, pr = ctx.compute_dtype, ctx.precision
         do = do.contiguous()
+        if cd is None and pr != "highest" and ctx.needs_input_grad[0] and ctx.needs_input_grad[1]:
+            both = _native_backward(do, x, A, group_sizes, ctx.trans_rhs)
+            if both is not None:
+                return *both, None, None, None, None
         dx = dA = None
         if ctx.needs_input_grad[0]:
             dx = _gmm_cast(do, A, group_sizes, not ctx.trans_rhs, cd, pr).to(x.dtype)
