@@ -116,7 +116,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t stage_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
 
@@ -183,163 +183,165 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      const uint64_t keep = l2_policy_evict_last();
-      int ready_slot = -1;  // last ready flag this producer has seen set
-      uint64_t waited_ns = 0;
-      const uint64_t t_start = kEp ? global_timer_ns() : 0;
-      for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = decode(tile);
-        const int halves = halves_of(t);
-        const int kb_count = kTgmm ? tgmm_block_count<kSeg>(p, t) : k_blocks_gmm;
-        RowBlocks blocks = first_block(t);
-        if (kEp && p.ready_flags != nullptr) {
-          const int slot = t.group / p.groups_per_flag;
-          if (slot != ready_slot) {
-            const uint64_t w0 = global_timer_ns();
-            if (!wait_flag_ge(p.ready_flags + slot, p.ready_epoch, abort_ptr)) {
-              ok = false;
-              break;
-            }
-            waited_ns += global_timer_ns() - w0;
-            ready_slot = slot;
-          }
-        }
-        for (int kb = 0; kb < kb_count; ++kb, ++it) {
-          const uint32_t s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+    uint32_t it = 0;
+    bool ok = true;
+    const uint64_t keep = l2_policy_evict_last();
+    int ready_slot = -1;  // last ready flag this producer has seen set
+    uint64_t waited_ns = 0;
+    const uint64_t t_start = kEp ? global_timer_ns() : 0;
+    for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
+      const TileCoord t = uniform_coord(decode(tile));
+      const int halves = halves_of(t);
+      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+      RowBlocks blocks = first_block(t);
+      if (kEp && p.ready_flags != nullptr) {
+        const int slot = t.group / p.groups_per_flag;
+        if (slot != ready_slot) {
+          const uint64_t w0 = global_timer_ns();
+          if (!__all_sync(0xffffffffu, wait_flag_ge(p.ready_flags + slot, p.ready_epoch, abort_ptr))) {
             ok = false;
             break;
           }
-          uint32_t full = smem_u32(&bar_full[s]);
-          const uint32_t sa = stage_base + s * kStageBytes;
-          const uint32_t sb = sa + kG2ABytes;
-          const uint32_t own_bytes = halves * kHalfABytes + kBBytes;
-          if (kTgmm) {
-            int r, live;
-            tgmm_block<kSeg>(p, t, blocks, kb, r, live);
-            if (p.blocked_maps) {  // one box per operand; the A box always has both halves
-              mbar_arrive_expect_tx(full, kStageBytes);
-              tma_load_3d_hint(sa, &tmap_a, full, 0, r, t.k0 >> 6, keep);
-              tma_load_3d_hint(sb, &tmap_b, full, 0, r, t.n0 >> 6, keep);
-              continue;
-            }
-            mbar_arrive_expect_tx(full, own_bytes);
-            for (int h = 0; h < halves; ++h) {
-              tma_load_2d_hint(sa + h * kHalfABytes, &tmap_a, full, t.k0 + h * kTileM, r, keep);
-              tma_load_2d_hint(sa + h * kHalfABytes + kBoxBytes, &tmap_a, full, t.k0 + h * kTileM + 64, r, keep);
-            }
+          waited_ns += global_timer_ns() - w0;
+          ready_slot = slot;
+        }
+      }
+      for (int kb = 0; kb < kb_count; ++kb, ++it) {
+        const uint32_t s = it % kStages;
+        const uint32_t ph = (it / kStages) & 1u;
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        int r = 0, live;
+        if (kTgmm) {
+          tgmm_block<kSeg>(p, t, blocks, kb, r, live);
+          if (kSeg) r = __shfl_sync(0xffffffffu, r, 0);
+        }
+        if (!elect_one()) continue;
+        const uint32_t full = smem_u32(&bar_full[s]);
+        const uint32_t sa = stage_base + s * kStageBytes;
+        const uint32_t sb = sa + kG2ABytes;
+        const uint32_t own_bytes = halves * kHalfABytes + kBBytes;
+        if (kTgmm) {
+          if (p.blocked_maps) {  // one box per operand; the A box always has both halves
+            mbar_arrive_expect_tx(full, kStageBytes);
+            tma_load_3d_hint(sa, &tmap_a, full, 0, r, t.k0 >> 6, keep);
+            tma_load_3d_hint(sb, &tmap_b, full, 0, r, t.n0 >> 6, keep);
+            continue;
+          }
+          mbar_arrive_expect_tx(full, own_bytes);
+          for (int h = 0; h < halves; ++h) {
+            tma_load_2d_hint(sa + h * kHalfABytes, &tmap_a, full, t.k0 + h * kTileM, r, keep);
+            tma_load_2d_hint(sa + h * kHalfABytes + kBoxBytes, &tmap_a, full, t.k0 + h * kTileM + 64, r, keep);
+          }
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j)
+            tma_load_2d_hint(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, r, keep);
+        } else {
+          mbar_arrive_expect_tx(full, own_bytes);
+          for (int h = 0; h < halves; ++h)
+            tma_load_2d(sa + h * kHalfABytes, &tmap_a, full, kb * kTileK, t.row0 + h * kTileM);
+          if (kBKMajor) {
+            tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
+          } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d_hint(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, r, keep);
-          } else {
-            mbar_arrive_expect_tx(full, own_bytes);
-            for (int h = 0; h < halves; ++h)
-              tma_load_2d(sa + h * kHalfABytes, &tmap_a, full, kb * kTileK, t.row0 + h * kTileM);
-            if (kBKMajor) {
-              tma_load_3d(sb, &tmap_b, full, kb * kTileK, t.n0, t.weight);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
-            }
+              tma_load_3d(sb + j * kBoxBytes, &tmap_b, full, t.n0 + j * 64, kb * kTileK, t.weight);
           }
         }
       }
-      if (kEp) {
-        // status[2]: longest total wait of a loader for remote rows; status[3]: longest loader
-        // lifetime (microseconds).  Read back by the expert-parallel harness.
-        atomicMax(p.status + 2, static_cast<int32_t>(waited_ns / 1000ull));
-        atomicMax(p.status + 3, static_cast<int32_t>((global_timer_ns() - t_start) / 1000ull));
-      }
+    }
+    if (kEp && lane == 0) {
+      // status[2]: longest total wait of a loader for remote rows; status[3]: longest loader
+      // lifetime (microseconds).  Read back by the expert-parallel harness.
+      atomicMax(p.status + 2, static_cast<int32_t>(waited_ns / 1000ull));
+      atomicMax(p.status + 3, static_cast<int32_t>((global_timer_ns() - t_start) / 1000ull));
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // ONE thread runs the whole loop.  The loop sits on the ring's
-    // critical path -- a stage can be refilled only after its MMAs, and they only start after
-    // this thread has seen the stage land -- and warp-wide steps are expensive there (a
-    // __syncwarp costs about 160 clocks on B200, a stage's MMAs take 1024).  The one warp-wide
-    // job, clearing the rows past a group's end in a tgmm stage, belongs to the fixer warp.
-    if (lane == 0) {
-      const uint32_t idesc =
-          make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM, BN);
-      constexpr uint32_t kAStep = (kTgmm ? 2048u : 32u) >> 4;
-      constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
-      const uint64_t adesc0 = kTgmm ? make_smem_desc(stage_base, kBoxBytes, 1024)
-                                    : make_smem_desc(stage_base, 16, 1024);
-      const uint64_t bdesc0 = kBKMajor ? make_smem_desc(stage_base + kG2ABytes, 16, 1024)
-                                       : make_smem_desc(stage_base + kG2ABytes, kBoxBytes, 1024);
-      const uint32_t adesc0_lo = static_cast<uint32_t>(adesc0);
-      const uint32_t bdesc0_lo = static_cast<uint32_t>(bdesc0);
-      const uint32_t desc_hi = static_cast<uint32_t>(adesc0 >> 32);
-      uint32_t it = 0;
-      uint32_t uses[2] = {0u, 0u};  // how often each half's accumulator has been used
-      uint32_t tail_events = 0;     // stages handed to the fixer warp so far
-      bool ok = true;
-      for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
-        const TileCoord t = decode(tile);
-        const int halves = halves_of(t);
-        const int kb_count = kTgmm ? tgmm_block_count<kSeg>(p, t) : k_blocks_gmm;
-        RowBlocks blocks = first_block(t);
-        const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
+    // The loop sits on the ring's critical path -- a stage can be refilled only after its MMAs, and they only start
+    // after this warp has seen the stage land.  Run by a whole warp that elects a lane per stage (rd_tgmm.cuh), with the
+    // producer, against one thread: m 16384, k 2048, n 7176, 8 groups 427 -> 414 us, 4928, 264, 7232, 4 36.5 -> 34.8.  Clearing the rows past a group's end in a tgmm stage belongs to the
+    // fixer warp.
+    const uint32_t idesc =
+        make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM, BN);
+    constexpr uint32_t kAStep = (kTgmm ? 2048u : 32u) >> 4;
+    constexpr uint32_t kBStep = (kBKMajor ? 32u : 2048u) >> 4;
+    const uint64_t adesc0 = kTgmm ? make_smem_desc(stage_base, kBoxBytes, 1024)
+                                  : make_smem_desc(stage_base, 16, 1024);
+    const uint64_t bdesc0 = kBKMajor ? make_smem_desc(stage_base + kG2ABytes, 16, 1024)
+                                     : make_smem_desc(stage_base + kG2ABytes, kBoxBytes, 1024);
+    const uint32_t adesc0_lo = static_cast<uint32_t>(adesc0);
+    const uint32_t bdesc0_lo = static_cast<uint32_t>(bdesc0);
+    const uint32_t desc_hi = static_cast<uint32_t>(adesc0 >> 32);
+    uint32_t it = 0;
+    uint32_t uses[2] = {0u, 0u};  // how often each half's accumulator has been used
+    uint32_t tail_events = 0;     // stages handed to the fixer warp so far
+    bool ok = true;
+    for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
+      const TileCoord t = uniform_coord(decode(tile));
+      const int halves = halves_of(t);
+      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+      RowBlocks blocks = first_block(t);
+      const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
 
-        if (kb_count == 0) {  // tgmm, empty group: the epilogue writes zeros, nothing to compute
+      if (kb_count == 0) {  // tgmm, empty group: the epilogue writes zeros, nothing to compute
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (h < halves) {
-              if (!mbar_wait(smem_u32(&bar_acc_empty[h]), (uses[h] & 1u) ^ 1u, abort_ptr)) {
+        for (int h = 0; h < 2; ++h) {
+          if (h < halves) {
+            if (!mbar_wait_warp(smem_u32(&bar_acc_empty[h]), (uses[h] & 1u) ^ 1u, abort_ptr)) {
+              ok = false;
+              break;
+            }
+            ++uses[h];
+            if (elect_one()) mbar_arrive(smem_u32(&bar_acc_full[h]));
+          }
+        }
+        continue;
+      }
+
+      uint32_t s = it % kStages;
+      uint32_t ph = (it / kStages) & 1u;
+      for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
+        if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+          ok = false;
+          break;
+        }
+        int live = kTileK;
+        if (kTgmm) {
+          int r;
+          tgmm_block<kSeg>(p, t, blocks, kb, r, live);
+          if (kSeg) live = __shfl_sync(0xffffffffu, live, 0);
+        }
+        const int n_mma = live >= kTileK ? kTileK / kUmmaK : (live + kUmmaK - 1) / kUmmaK;
+        if (kTgmm && (kSeg ? block_needs_clearing(live) : (tail_stage && kb == kb_count - 1))) {
+          // Rows past the end of the group belong to the next group (or to nobody): the fixer
+          // warp clears them before the MMAs read the stage.
+          if (elect_one()) mbar_arrive(smem_u32(&bar_tail_go));
+          if (!mbar_wait_warp(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
+            ok = false;
+            break;
+          }
+          ++tail_events;
+        }
+        const bool last = kb == kb_count - 1;
+        const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
+        tc_fence_after_sync();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h < halves) {
+            if (kb == 0) {  // the half's accumulator must have been drained by the epilogue
+              if (!mbar_wait_warp(smem_u32(&bar_acc_empty[h]), (uses[h] & 1u) ^ 1u, abort_ptr)) {
                 ok = false;
                 break;
               }
               ++uses[h];
-              mbar_arrive(smem_u32(&bar_acc_full[h]));
+              tc_fence_after_sync();
             }
-          }
-          continue;
-        }
-
-        uint32_t s = it % kStages;
-        uint32_t ph = (it / kStages) & 1u;
-        for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
-          if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
-            ok = false;
-            break;
-          }
-          int live = kTileK;
-          if (kTgmm) {
-            int r;
-            tgmm_block<kSeg>(p, t, blocks, kb, r, live);
-          }
-          const int n_mma = live >= kTileK ? kTileK / kUmmaK : (live + kUmmaK - 1) / kUmmaK;
-          if (kTgmm && (kSeg ? block_needs_clearing(live) : (tail_stage && kb == kb_count - 1))) {
-            // Rows past the end of the group belong to the next group (or to nobody): the fixer
-            // warp clears them before the MMAs read the stage.
-            mbar_arrive(smem_u32(&bar_tail_go));
-            if (!mbar_wait(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
-              ok = false;
-              break;
-            }
-            ++tail_events;
-          }
-          const bool last = kb == kb_count - 1;
-          const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
-          tc_fence_after_sync();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (h < halves) {
-              if (kb == 0) {  // the half's accumulator must have been drained by the epilogue
-                if (!mbar_wait(smem_u32(&bar_acc_empty[h]), (uses[h] & 1u) ^ 1u, abort_ptr)) {
-                  ok = false;
-                  break;
-                }
-                ++uses[h];
-                tc_fence_after_sync();
-              }
-              const uint32_t tmem_d = tmem_base + h * BN;
-              const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * (kHalfABytes >> 4);
+            const uint32_t tmem_d = tmem_base + h * BN;
+            const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4) + h * (kHalfABytes >> 4);
+            if (elect_one()) {
               if (kTgmm && n_mma < kTileK / kUmmaK) {
                 for (int kk = 0; kk < n_mma; ++kk) {
                   umma_ab<1, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
@@ -355,14 +357,12 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                   make_desc64(b_lo + kk * kBStep, desc_hi), idesc, 1u);
                 }
               }
-              if (last) {  // this half is complete
-                umma_commit(smem_u32(&bar_acc_full[h]));
-              }
+              if (last) umma_commit(smem_u32(&bar_acc_full[h]));  // this half is complete
             }
           }
-          if (!ok) break;
-          umma_commit(smem_u32(&bar_empty[s]));  // both halves have read the stage
         }
+        if (!ok) break;
+        if (elect_one()) umma_commit(smem_u32(&bar_empty[s]));  // both halves have read the stage
       }
     }
   } else if (warp == kG2FixerWarp) {
