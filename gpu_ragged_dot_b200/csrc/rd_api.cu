@@ -651,16 +651,21 @@ bool choose_two_half(bool tgmm, long long m, int k, int n, int g, int bn, bool f
 }
 
 // float32 tiles on CTA pairs (rd_gemm_f32_pair.cuh).  A caller who asks for three TF32 passes always
-// gets them: only that kernel splits its operands.  One pass: tgmm on groups of 256 rows and more with
-// rows that are multiples of 32.  One CTA against a pair, microseconds: k 1024, n 4096, 32 groups of 256
-// 181 -> 167; n 13056, 17 groups of 399 450 -> 421; k 4096, n 1536, 64 groups of 512 973 -> 939; m/g 1024 equal
-// within 3 %; k 2048, n 4096, 64 groups of 128 413 -> 491; without the column-blocked boxes (n 12976) 457 ->
-// 650.  gmm stays on one CTA: 8192, 4096, 14336, 8 1588 -> 1832, 16384, 1024, 4096, 32 267 -> 302, with
-// trans_rhs 3 % either way.
+// gets them: only that kernel splits its operands.  One pass: tgmm with rows that are multiples of 32, where pairs take no
+// more than a tenth more rounds of tiles; groups of 256 rows from two rounds on one CTA per tile on, of 100 from seven.
+// Of 350 sizes timed on both sides that takes 109, one of them 7 % slower than on one CTA, the others 2 % at most.  One CTA
+// against a pair, microseconds: m 4096, k 1536, n 4096, 32 unequal groups 201 -> 188; 16384, 2048, 2048, 128 506 -> 471; one
+// round: 888, 1184, 2656, 1 15.5 -> 16.4; groups of 245 in five rounds: 14210, 1376, 160, 58 49 -> 57; without the
+// column-blocked boxes (n 12976, 17 groups of 399) 457 -> 650.
+// gmm on long groups takes the swapped kernel instead (choose_swap_f32).
 bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const rd_tile_cfg* cfg) {
   if (cfg && (cfg->flags & RD_CFG_F32_THREE_PASS)) return true;
   if (!tgmm || bn != 256 || g <= 0 || (cfg && (cfg->cta_group == 1 || cfg->tile_m == 128))) return false;
-  return k >= 256 && m / g >= 256 && k % 32 == 0 && n % 32 == 0;
+  if (k % 32 != 0 || n % 32 != 0) return false;
+  const long long sms = sm_count(), cols = (static_cast<long long>(n) + 255) / 256 * g;
+  const long long r1 = ((k + 127) / 128 * cols + sms - 1) / sms;
+  const long long r2 = ((k + 255) / 256 * cols + sms / 2 - 1) / (sms / 2);
+  return 10 * r2 <= 11 * r1 && r1 > 1 && (m / g >= 256 || (m / g >= 100 && r1 > 6));
 }
 
 // tgmm with 256-column tiles (rd_tgmm.cuh): 256 x 256 on CTA pairs, or 128 x 256 on one CTA each?  A pair moves a third
