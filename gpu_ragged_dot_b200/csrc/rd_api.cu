@@ -259,14 +259,15 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 // Groups of 64 rows and less read (or write) weights that no neighbour shares, so there it gains its 2 us too, up to some
 // 512 MB of weights, 80 us: 256 rows, k 4096, n 1536, 64 groups of e4m3 67.7 -> 65.4; 4000, 1024, 1024, 64 30.9 -> 29.5, tgmm
 // 37.0 -> 34.9; 300, 1000, 2000, 100 tgmm 72.5 -> 69.1.  Above, nothing or less: the first in bf16 119.0 -> 119.3; 512, 7168,
-// 2048, 256 755 -> 770.
-bool launch_early(const GemmArgs& args, int ctas_per_tile = 1) {
+// 2048, 256 755 -> 770.  16-bit and float32 weights with rows along the contraction lose sooner: 3383, 8936, 384, 64 109 -> 115;
+// 2000, 3000, 1024, 64 (393 MB) 82 -> 86.
+bool launch_early(const GemmArgs& args, int ctas_per_tile = 1, bool wide_k_major = false) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
                                                : static_cast<long long>(args.m < args.g ? args.m : args.g) + args.m / rd::kTileM;
   if (row_tiles * args.n_tiles * ctas_per_tile <= sm_count()) return true;
   const double weight_bytes = 2.0 * (args.m < args.g ? args.m : args.g) * args.k * args.n;
-  return args.m <= 64LL * args.g && weight_bytes <= 512e6;
+  return args.m <= 64LL * args.g && weight_bytes <= (wide_k_major ? 150e6 : 512e6);
 }
 
 // How many clusters of two CTAs can be resident at once (0: the query failed).
@@ -333,7 +334,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
       cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1, launch_early(args), stream, ta, tb, tout,
+  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1, launch_early(args, 1, kBKMajor && !kFp8), stream, ta, tb, tout,
                        args);
 }
 
@@ -347,7 +348,7 @@ int launch_gemm_unaligned(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
   auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, 1, false, false, true>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1, launch_early(args), stream, ta, tb, ta, args);
+  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1, launch_early(args, 1, kBKMajor), stream, ta, tb, ta, args);
 }
 
 template <int BN, bool kBKMajor, bool kTgmm>
@@ -360,7 +361,7 @@ int launch_gemm_f32(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensor
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
       cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kGemmThreads, kSmem, 1, launch_early(args), stream, ta, tb, tout, args);
+  return launch_kernel(kernel, ctas, rd::kGemmThreads, kSmem, 1, launch_early(args, 1, kBKMajor), stream, ta, tb, tout, args);
 }
 
 template <int BN, bool kBKMajor, bool kTgmm>
@@ -398,7 +399,7 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rd::kG2SmemBytes) !=
       cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kG2Threads, rd::kG2SmemBytes, 1, launch_early(args), stream, ta, tb, tout,
+  return launch_kernel(kernel, ctas, rd::kG2Threads, rd::kG2SmemBytes, 1, launch_early(args, 1, kBKMajor), stream, ta, tb, tout,
                        args);
 }
 
