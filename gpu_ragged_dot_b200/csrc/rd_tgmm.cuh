@@ -3,7 +3,7 @@
 // A tile contracts over the rows of one group only, often a few 64-row stages, so what bounds it is as
 // much the way from one tile to the next as the MMAs.  A CTA owns 128 x 256 tiles (kCtas 2: a pair
 // 256 x 256, each CTA its own 128 rows of x^T and half of dout's columns) and has two of them in tensor
-// memory: while the MMAs fill one, four of eight epilogue warps drain the other.  The 256 x 256 tiles per CTA
+// memory: while the MMAs fill one, four of eight epilogue warps (all eight on one CTA) drain the other.  The 256 x 256 tiles per CTA
 // that stood here before moved less per flop but left the drain exposed, 5000 clocks per tile.
 //
 // What made the smaller tiles fast enough is the issue path.  A 64-row stage takes 512 clocks of MMAs here.
