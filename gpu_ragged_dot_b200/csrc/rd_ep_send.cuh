@@ -78,7 +78,7 @@ __device__ __noinline__ void ep_sender_role(const EpSendArgs a, int epoch, int s
   if (warp == 0) {
     // ---- signaller
     for (int p = 1; p < a.world && ok; ++p) {
-      if (!mbar_wait(phase_bars + 8 * p, 0u, abort_flag)) {
+      if (!mbar_wait_warp(phase_bars + 8 * p, 0u, abort_flag)) {
         ok = false;
         break;
       }
@@ -151,7 +151,7 @@ __device__ __noinline__ void ep_sender_role(const EpSendArgs a, int epoch, int s
       const int by = __shfl_sync(0xffffffffu, bytes_c, t & 31);
       if (by > 0) {
         const int slot = t % kEpSlots;
-        if (!mbar_wait(bars + 8 * slot, (parity >> slot) & 1u, abort_flag)) {
+        if (!mbar_wait_warp(bars + 8 * slot, (parity >> slot) & 1u, abort_flag)) {
           ok = false;
           break;
         }

@@ -32,7 +32,7 @@
 //   MN-major operand tile [64 k][64 mn] : boxes of 8 KB; K-groups of 8 rows 1024 B apart,
 //                                         next 64 M/N elements in the next box (8192 B)
 //
-// Every mbarrier wait is bounded (rd_ptx.cuh: mbar_wait); on expiry the CTA records a status
+// Every mbarrier wait is bounded (rd_ptx.cuh: mbar_wait_warp); on expiry the CTA records a status
 // word, drains and frees its TMEM instead of spinning.
 #pragma once
 
@@ -725,7 +725,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (!(kSeg ? block_needs_clearing(live) : tail_stage)) continue;
           const uint32_t s = (it + kb) % kStages;
-          if (!mbar_wait<kPair>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
+          if (!mbar_wait_warp<kPair>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
             ok = false;
             break;
           }
@@ -735,7 +735,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (!leader) {
               const uint32_t par = (own_parity >> s) & 1u;
               own_parity ^= 1u << s;
-              if (!mbar_wait(smem_u32(&bar_full[s]), par, abort_ptr)) {
+              if (!mbar_wait_warp(smem_u32(&bar_full[s]), par, abort_ptr)) {
                 ok = false;
                 break;
               }
@@ -770,7 +770,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int n0 = t.n0;
       const uint32_t acc = local_tile & 1u;
       const uint32_t acc_ph = (local_tile >> 1) & 1u;
-      if (!mbar_wait<kPair>(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
+      if (!mbar_wait_warp<kPair>(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
         ok = false;
         break;
       }

@@ -384,7 +384,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (!(kSeg ? block_needs_clearing(live) : tail_stage)) continue;
           const uint32_t s = (it + kb) % kStages;
-          if (!mbar_wait(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
+          if (!mbar_wait_warp(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
             ok = false;
             break;
           }
@@ -412,7 +412,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const TileCoord t = decode(tile);
       if (half >= halves_of(t)) continue;  // this half does not exist in this tile
       const int n0 = t.n0;
-      if (!mbar_wait(smem_u32(&bar_acc_full[half]), uses & 1u, abort_ptr)) {
+      if (!mbar_wait_warp(smem_u32(&bar_acc_full[half]), uses & 1u, abort_ptr)) {
         ok = false;
         break;
       }

@@ -319,7 +319,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+          if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
             ok = false;
             break;
           }
@@ -378,14 +378,14 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         it += kb_count;
         if (kb_count == 0 || !tail_needs_clearing_f32(t.rows)) continue;
         const uint32_t s = (it - 1) % kStages;
-        if (!mbar_wait<true>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
+        if (!mbar_wait_warp<true>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
           ok = false;
           break;
         }
         if (!leader) {  // the peer's bytes of such a stage are counted on its own barrier
           const uint32_t par = (own_parity >> s) & 1u;
           own_parity ^= 1u << s;
-          if (!mbar_wait(smem_u32(&bar_full[s]), par, abort_ptr)) {
+          if (!mbar_wait_warp(smem_u32(&bar_full[s]), par, abort_ptr)) {
             ok = false;
             break;
           }
@@ -411,7 +411,7 @@ ragged_gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int n0 = t.n0;
       const uint32_t acc = kSplit ? 0u : (local_tile & 1u);
       const uint32_t acc_ph = kSplit ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
-      if (!mbar_wait<true>(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
+      if (!mbar_wait_warp<true>(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
         ok = false;
         break;
       }

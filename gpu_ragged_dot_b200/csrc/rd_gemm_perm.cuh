@@ -219,7 +219,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
             di_next[i] = gather_b ? q.b_rows[r] : 0;
           }
         }
-        if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
           ok = false;
           break;
         }
@@ -405,7 +405,7 @@ ragged_gemm_perm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         scatter_row = row_ok ? dst_row : -1;
       }
 
-      if (!mbar_wait(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
+      if (!mbar_wait_warp(smem_u32(&bar_acc_full[acc]), acc_ph, abort_ptr)) {
         ok = false;
         break;
       }

@@ -159,7 +159,7 @@ ragged_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     } else {
       // The accumulator is complete when all MMAs have retired, so the ring is idle and its memory
       // free: the loader does not start on the next tile before the barriers below.
-      if (ok && !mbar_wait(smem_u32(&bar_acc_full), local_tile & 1u, abort_ptr)) ok = false;
+      if (ok && !mbar_wait_warp(smem_u32(&bar_acc_full), local_tile & 1u, abort_ptr)) ok = false;
       __syncwarp();
       tc_fence_after_sync();
       const int quarter = warp & 3;

@@ -369,7 +369,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       const SwapTile t = decode_swap_tile<kStep>(p, &group_table, work, tile);
       if (half >= t.halves) continue;
       const int col0 = t.n0 + (cta_rank * t.halves + half) * kTileM + quarter * 32;  // this warp's first output column; lane = column
-      if (!mbar_wait<true>(smem_u32(&bar_acc_full[half]), uses & 1u, abort_ptr)) {
+      if (!mbar_wait_warp<true>(smem_u32(&bar_acc_full[half]), uses & 1u, abort_ptr)) {
         ok = false;
         break;
       }

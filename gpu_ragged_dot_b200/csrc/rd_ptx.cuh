@@ -159,7 +159,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
-// The same wait by a whole warp, whose result every lane (and the compiler) knows to be the same.
+// The same wait by a whole warp, whose result every lane (and the compiler) knows to be the same.  Roles that run as
+// whole warps wait in this form only: were some lanes to give up while others still saw the phase end, the latter would
+// go on to a __syncwarp, a tcgen05.ld or a vote that the former never reach.
 template <bool kClusterScope = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile WaitCtl* ctl) {
   return __all_sync(0xffffffffu, mbar_wait<kClusterScope>(bar, parity, ctl));

@@ -330,7 +330,7 @@ ragged_tgmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       it += kb_count;
       if (kb_count == 0 || !tail_needs_clearing(t.rows)) continue;
       const uint32_t s = (it - 1) % kStages;
-      if (!mbar_wait(smem_u32(&bar_land[s]), (parity >> s) & 1u, abort_ptr)) break;
+      if (!mbar_wait_warp(smem_u32(&bar_land[s]), (parity >> s) & 1u, abort_ptr)) break;
       parity ^= 1u << s;
       clear_tail_rows<kStageBytes / kBoxBytes>(stage_base + s * kStageBytes, t.rows - (kb_count - 1) * kTileK, lane);
       __syncwarp();
@@ -360,7 +360,7 @@ ragged_tgmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       const int first = kPair ? 0 : 2 * side;  // 64-column blocks [first, chunks) are this warp's
       const int chunks = out_row0 < p.k ? imin(t.blocks, kPair ? 4 : first + 2) : 0;
       const bool zero_only = t.rows <= 0;
-      if (!mbar_wait<kPair>(smem_u32(&bar_acc_full[acc]), phase, abort_ptr)) break;
+      if (!mbar_wait_warp<kPair>(smem_u32(&bar_acc_full[acc]), phase, abort_ptr)) break;
       tc_fence_after_sync();
       auto hand_back = [&]() {  // everything this warp needs of the accumulator is in registers
         tc_fence_before_sync();
