@@ -22,10 +22,7 @@
 //             what bounds the 1-CTA kernel.  Every CTA loads only its own tiles (nothing is
 //             broadcast); the peer's loads count their bytes on the LEADER's "full" barrier
 //             (cta_group::2 TMA form), so the leader sees one barrier per stage, and
-//             tcgen05.commit frees the stage in both CTAs.  The one stage per tgmm tile whose
-//             tail rows must be cleared goes through a slower hand-shake (the peer's bytes
-//             land on its own barrier, either CTA's fixer warp clears its rows and arrives on
-//             the leader's tail_done barrier).
+//             tcgen05.commit frees the stage in both CTAs.  gmm only: rd_tgmm.cuh has tgmm's pairs.
 //
 // Operand layouts (all 128-byte-swizzled, written by TMA, read through UMMA descriptors):
 //   K-major  operand tile [rows][64 k]  : one box, 8-row groups 1024 B apart
@@ -428,7 +425,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   static_assert(BN == 64 || BN == 128 || BN == 256, "BN must be 64, 128 or 256");
   static_assert(!(kTgmm && kBKMajor), "tgmm reads both operands MN-major");
   static_assert(kCtas == 1 || (kCtas == 2 && BN >= 128), "a CTA pair needs BN >= 128");
-  static_assert(!kSeg || (kTgmm && kCtas == 1), "strided segments: tgmm on one CTA per tile");
+  static_assert(!kTgmm || kCtas == 1, "tgmm on CTA pairs: rd_tgmm.cuh");
+  static_assert(!kSeg || kTgmm, "strided segments: tgmm");
   // 8-bit inputs (e4m3): both operands K-major (x[m,k], W[g,n,k]), so the tiles are byte for byte
   // those of a 16-bit problem with k/2 elements per row (which is what the tensor maps and
   // GemmArgs::k describe); only the MMA kind differs, 32 elements = 32 bytes per instruction, and
@@ -445,8 +443,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t bar_full[kStages];        // TMA data of this CTA landed
   __shared__ __align__(8) uint64_t bar_empty[kStages];       // MMAs reading the stage retired
-  __shared__ __align__(8) uint64_t bar_tail_go;    // MMA thread -> fixer warp(s): a stage with tail rows has landed
-  __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp(s) -> MMA thread (pair: the leader's is used)
+  __shared__ __align__(8) uint64_t bar_tail_go;    // MMA warp -> fixer warp: a stage with tail rows has landed
+  __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp -> MMA warp
   __shared__ __align__(8) uint64_t bar_acc_full[2];
   __shared__ __align__(8) uint64_t bar_acc_empty[2];  // leader only when paired
   __shared__ uint32_t tmem_slot;
@@ -482,7 +480,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     mbar_init(smem_u32(&bar_tail_go), 1);
-    mbar_init(smem_u32(&bar_tail_done), kCtas);  // one arrival per CTA's fixer warp
+    mbar_init(smem_u32(&bar_tail_done), 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bar_acc_full[a]), 1);
       mbar_init(smem_u32(&bar_acc_empty[a]), 4 * kCtas);  // one arrival per epilogue warp
@@ -554,19 +552,13 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (kSeg) r = __shfl_sync(0xffffffffu, r, 0);
         }
-        // In a pair the peer's bytes are counted on the leader's barrier, except for a stage
-        // whose tail rows the peer has to clear first (it then needs to see its own data land).
-        const bool local_stage = !kPair || (kTgmm && kb == kb_count - 1 && tail_needs_clearing(t.rows));
         if (elect_one()) {
           uint32_t full = smem_u32(&bar_full[s]);
-          bool remote_bar = false;
-          if (leader) {
-            mbar_arrive_expect_tx(full, local_stage ? kStageBytes : 2 * kStageBytes);
-          } else if (local_stage) {
-            mbar_arrive_expect_tx(full, kStageBytes);
-          } else {
+          const bool remote_bar = kPair && !leader;  // the peer's bytes are counted on the leader's barrier
+          if (remote_bar) {
             full = map_to_cta(full, 0);
-            remote_bar = true;
+          } else {
+            mbar_arrive_expect_tx(full, kCtas * kStageBytes);
           }
           if (kTgmm) {
             load_2d(remote_bar, sa, &tmap_a, full, t.k0, r);
@@ -647,14 +639,11 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           const int n_mma = live >= kTileK ? kTileK / kUmmaK : (live + kUmmaK - 1) / kUmmaK;
           if (kTgmm && (kSeg ? block_needs_clearing(live) : (tail_stage && kb == kb_count - 1))) {
             // Rows past the end of the group belong to the next group (or to nobody): the fixer
-            // warp (of either CTA in a pair) clears them, up to the end of the last MMA that is
-            // issued, in every box of this stage, so they add nothing to the reduction.  (In gmm
-            // the columns past k are zero-filled by TMA.)
-            if (elect_one()) {
-              mbar_arrive(smem_u32(&bar_tail_go));
-              if constexpr (kPair) mbar_arrive_cluster(smem_u32(&bar_tail_go), 1);
-            }
-            if (!mbar_wait_warp<kPair>(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
+            // warp clears them, up to the end of the last MMA that is issued, in every box of this
+            // stage, so they add nothing to the reduction.  (In gmm the columns past k are
+            // zero-filled by TMA.)
+            if (elect_one()) mbar_arrive(smem_u32(&bar_tail_go));
+            if (!mbar_wait_warp(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
               ok = false;
               break;
             }
@@ -700,20 +689,18 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
           } else {  // empty group: nothing to wait for
             mbar_arrive(bar);
-            if (kPair) mbar_arrive_cluster(bar, 1);
           }
         }
       }
     }
   } else if (warp == kGemmFixerWarp) {
     // ------------------------------------------------------------ tail fixer (tgmm)
-    // Walks the tiles like the MMA thread and, for every stage whose last 16-deep MMA reaches past
-    // the end of its group, waits for the MMA thread's go (the stage has landed), clears those
-    // rows in every box of the stage in THIS CTA's shared memory and reports back.
+    // Walks the tiles like the MMA warp and, for every stage whose last 16-deep MMA reaches past
+    // the end of its group, waits for the MMA warp's go (the stage has landed), clears those
+    // rows in every box of the stage and reports back.
     if constexpr (kTgmm) {
       uint32_t it = 0;
       uint32_t events = 0;
-      uint32_t own_parity = 0;  // peer of a pair, bit s: parity of the next landing on its own barrier of slot s
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
         const TileCoord t = decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
@@ -725,32 +712,14 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (!(kSeg ? block_needs_clearing(live) : tail_stage)) continue;
           const uint32_t s = (it + kb) % kStages;
-          if (!mbar_wait_warp<kPair>(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
+          if (!mbar_wait_warp(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
             ok = false;
             break;
-          }
-          if constexpr (kPair) {
-            // The peer's bytes of such a stage are counted on its own barrier of that slot (see
-            // the producer), which is used for nothing else.
-            if (!leader) {
-              const uint32_t par = (own_parity >> s) & 1u;
-              own_parity ^= 1u << s;
-              if (!mbar_wait_warp(smem_u32(&bar_full[s]), par, abort_ptr)) {
-                ok = false;
-                break;
-              }
-            }
           }
           ++events;
           clear_tail_rows<(kABytes + kBBytes) / kBoxBytes>(stage_base + s * kStageBytes, live, lane);
           __syncwarp();
-          if (lane == 0) {
-            if constexpr (kPair) {
-              mbar_arrive_cluster(smem_u32(&bar_tail_done), 0);
-            } else {
-              mbar_arrive(smem_u32(&bar_tail_done));
-            }
-          }
+          if (lane == 0) mbar_arrive(smem_u32(&bar_tail_done));
         }
         it += kb_count;
       }

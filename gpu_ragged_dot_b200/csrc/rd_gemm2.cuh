@@ -21,8 +21,9 @@
 // Blocked operand maps (GemmArgs::blocked_maps, tgmm): x and dout are described to TMA as
 // (64 columns, rows, blocks of 64 columns), so ONE box of (64, 64 rows, 4 blocks) = 32 KB lands as
 // the same four [64 rows][128 B] slabs that four 2-D boxes would write: two TMA instructions per
-// stage instead of eight (about 1 % on the Mixtral-shaped weight gradient).  Needs k and n to be
+// stage instead of eight (1 % of a compute-bound product).  Needs k and n to be
 // multiples of 64; otherwise one 2-D box per 64 columns, as in rd_gemm.cuh.
+// tgmm here is the strided form, a block of the output summed over several row ranges; plain tgmm: rd_tgmm.cuh.
 #pragma once
 
 #include "rd_gemm.cuh"
@@ -58,7 +59,6 @@ __device__ __forceinline__ TileCoord decode_gmm_tile256(const GemmArgs& p, const
   return t;
 }
 
-template <int kRows = kG2TileRows>
 __device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, const GroupTable* tab, int tile) {
   const int per_group = p.k_tiles * p.n_tiles;
   const int gi = tile / per_group;
@@ -77,7 +77,7 @@ __device__ __forceinline__ TileCoord decode_tgmm_tile256(const GemmArgs& p, cons
   t.weight = gi;
   group_rows(p, tab, gi, t.row0, t.rows);
   t.n0 = nt * kG2TileN;
-  t.k0 = kt * kRows;
+  t.k0 = kt * kG2TileRows;
   return t;
 }
 
@@ -97,7 +97,6 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   static_assert(!kFp8 || (kBKMajor && !kTgmm && !kVariant), "8-bit inputs: plain gmm, K-major weights");
   static_assert(!kTgmm || kVariant, "plain tgmm: rd_tgmm.cuh");
   constexpr bool kEp = !kTgmm && kVariant;
-  constexpr bool kSeg = kTgmm && kVariant;
   constexpr int BN = kG2TileN;
   constexpr int kStages = kG2Stages;
   constexpr uint32_t kHalfABytes = kTileM * kTileK * 2;  // 16 KB
@@ -110,8 +109,8 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ __align__(8) uint64_t bar_empty[kStages];
   __shared__ __align__(8) uint64_t bar_acc_full[2];   // per half
   __shared__ __align__(8) uint64_t bar_acc_empty[2];  // per half
-  __shared__ __align__(8) uint64_t bar_tail_go;    // MMA thread -> fixer warp(s): a stage with tail rows has landed
-  __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp(s) -> MMA thread: its tail rows are cleared
+  __shared__ __align__(8) uint64_t bar_tail_go;    // MMA warp -> fixer warp: a stage with tail rows has landed
+  __shared__ __align__(8) uint64_t bar_tail_done;  // fixer warp -> MMA warp: its tail rows are cleared
   __shared__ uint32_t tmem_slot;
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
@@ -192,7 +191,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
       const TileCoord t = uniform_coord(decode(tile));
       const int halves = halves_of(t);
-      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<true>(p, t), 0) : k_blocks_gmm;
       RowBlocks blocks = first_block(t);
       if (kEp && p.ready_flags != nullptr) {
         const int slot = t.group / p.groups_per_flag;
@@ -215,8 +214,8 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         int r = 0, live;
         if (kTgmm) {
-          tgmm_block<kSeg>(p, t, blocks, kb, r, live);
-          if (kSeg) r = __shfl_sync(0xffffffffu, r, 0);
+          tgmm_block<true>(p, t, blocks, kb, r, live);
+          r = __shfl_sync(0xffffffffu, r, 0);
         }
         if (!elect_one()) continue;
         const uint32_t full = smem_u32(&bar_full[s]);
@@ -262,8 +261,8 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // ------------------------------------------------------------ MMA issuer
     // The loop sits on the ring's critical path -- a stage can be refilled only after its MMAs, and they only start
     // after this warp has seen the stage land.  Run by a whole warp that elects a lane per stage (rd_tgmm.cuh), with the
-    // producer, against one thread: m 16384, k 2048, n 7176, 8 groups 427 -> 414 us, 4928, 264, 7232, 4 36.5 -> 34.8.  Clearing the rows past a group's end in a tgmm stage belongs to the
-    // fixer warp.
+    // producer, against one thread: m 16384, k 2048, n 7176, 8 groups 427 -> 414 us, 4928, 264, 7232, 4 36.5 -> 34.8.
+    // Clearing the rows past a segment's end in a tgmm stage belongs to the fixer warp.
     const uint32_t idesc =
         make_idesc_f16(kFp8 ? 0 : p.ab_format, kTgmm ? 1 : 0, kBKMajor ? 0 : 1, kTileM, BN);
     constexpr uint32_t kAStep = (kTgmm ? 2048u : 32u) >> 4;
@@ -282,9 +281,8 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
       const TileCoord t = uniform_coord(decode(tile));
       const int halves = halves_of(t);
-      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<true>(p, t), 0) : k_blocks_gmm;
       RowBlocks blocks = first_block(t);
-      const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
 
       if (kb_count == 0) {  // tgmm, empty group: the epilogue writes zeros, nothing to compute
 #pragma unroll
@@ -311,11 +309,11 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         int live = kTileK;
         if (kTgmm) {
           int r;
-          tgmm_block<kSeg>(p, t, blocks, kb, r, live);
-          if (kSeg) live = __shfl_sync(0xffffffffu, live, 0);
+          tgmm_block<true>(p, t, blocks, kb, r, live);
+          live = __shfl_sync(0xffffffffu, live, 0);
         }
         const int n_mma = live >= kTileK ? kTileK / kUmmaK : (live + kUmmaK - 1) / kUmmaK;
-        if (kTgmm && (kSeg ? block_needs_clearing(live) : (tail_stage && kb == kb_count - 1))) {
+        if (kTgmm && block_needs_clearing(live)) {
           // Rows past the end of the group belong to the next group (or to nobody): the fixer
           // warp clears them before the MMAs read the stage.
           if (elect_one()) mbar_arrive(smem_u32(&bar_tail_go));
@@ -367,22 +365,21 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == kG2FixerWarp) {
     // ------------------------------------------------------------ tail fixer (tgmm)
-    // Walks the tiles like the MMA thread and, for every stage whose last 16-deep MMA reaches past
-    // the end of its group, waits for the MMA thread's go (the stage has landed), clears those
-    // rows in every box of the stage in THIS CTA's shared memory and reports back.
+    // Walks the tiles like the MMA warp and, for every stage whose last 16-deep MMA reaches past
+    // the end of its segment, waits for the MMA warp's go (the stage has landed), clears those
+    // rows in every box of the stage and reports back.
     if constexpr (kTgmm) {
       uint32_t it = 0;
       uint32_t events = 0;
       bool ok = true;
       for (int tile = first_tile(); tile < num_tiles && ok; tile += tile_step) {
         const TileCoord t = decode(tile);
-        const int kb_count = tgmm_block_count<kSeg>(p, t);
+        const int kb_count = tgmm_block_count<true>(p, t);
         RowBlocks blocks = first_block(t);
-        const bool tail_stage = kb_count > 0 && tail_needs_clearing(t.rows);
-        for (int kb = kSeg ? 0 : imax(kb_count - 1, 0); kb < kb_count; ++kb) {
+        for (int kb = 0; kb < kb_count; ++kb) {
           int r, live;
-          tgmm_block<kSeg>(p, t, blocks, kb, r, live);
-          if (!(kSeg ? block_needs_clearing(live) : tail_stage)) continue;
+          tgmm_block<true>(p, t, blocks, kb, r, live);
+          if (!block_needs_clearing(live)) continue;
           const uint32_t s = (it + kb) % kStages;
           if (!mbar_wait_warp(smem_u32(&bar_tail_go), events & 1u, abort_ptr)) {
             ok = false;
@@ -430,7 +427,7 @@ ragged_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         warp_has_rows = out_row0 < p.k;
         slab_by_tma = true;
         row_off = (static_cast<size_t>(t.group) * p.k + kr) * static_cast<size_t>(p.n);
-        zero_only = kSeg ? tgmm_block_count<kSeg>(p, t) == 0 : t.rows <= 0;
+        zero_only = tgmm_block_count<true>(p, t) == 0;
       } else {
         out_row0 = t.row0 + slab0;
         row_ok = r_in_tile < t.rows;
