@@ -204,21 +204,21 @@ def test_256_row_tiles_ragged_boundaries(cta_group, tile_m, trans_rhs):
 @pytest.mark.parametrize("cta_group", [1, 2])
 @pytest.mark.parametrize("k,n", [(136, 392), (264, 392), (392, 392), (520, 392), (1032, 392),
                                  (64, 64), (128, 192), (320, 448), (576, 256), (1024, 512)])
-def test_tgmm_256_row_tiles_all_load_paths(k, n, cta_group):
-    """tgmm with 256-row tiles on one CTA and with 512 x 256 tiles on CTA pairs (tile_m 256,
-    cta_group 1 / 2).  k values that end inside the first CTA's rows, the second CTA's rows, the
-    second half and the second tile; k and n that are multiples of 64 (one column-blocked TMA box
-    per operand and stage, also where the box is wider than the tensor) and that are not (one box
-    per 64 columns); group sizes around the 64-row reduction step and the 16-row MMA depth (the
-    fixer warp of either CTA clears the tail rows); empty groups; rows past the last group hold
-    NaN and must not reach any output."""
+def test_tgmm_256_columns_all_load_paths(k, n, cta_group):
+    """tgmm with 256-column tiles on one CTA and on pairs (tile_m 256 is taken, and means the same as 128).
+    k values that end inside the first CTA's rows, the second CTA's rows and later tiles; k and n
+    that are multiples of 64 (one column-blocked TMA box per operand and stage, also where the box
+    is wider than the tensor) and that are not (one box per 64 columns at the edge); narrow column
+    tiles; group sizes around the 64-row reduction step and the 16-row MMA depth (the fixer warp of
+    either CTA clears the tail rows); empty groups; rows past the last group hold NaN and must not
+    reach any output."""
     sizes = [1, 63, 64, 65, 0, 130, 15, 16, 17, 0, 300, 77]
     m = sum(sizes) + 40
     x, _, dout = _inputs(8, m, k, n, len(sizes))
     x[sum(sizes):] = float("nan")
     dout[sum(sizes):] = float("nan")
     got = _check_tgmm(x, dout, sizes, cfg=_lib.TileCfg(256, 0, cta_group, 256),
-                      what=f"256-row tgmm k={k} n={n} ctas={cta_group}")
+                      what=f"tgmm k={k} n={n} ctas={cta_group}")
     assert torch.isfinite(got.float()).all()
 
 
@@ -853,6 +853,35 @@ def test_tgmm_strided_matches_oracle(n, tile_m):
     assert torch.equal(plain.view(torch.int16), one.view(torch.int16))
 
 
+@pytest.mark.parametrize("tile_m", [128, 256])
+@pytest.mark.parametrize("k,n", [(264, 392), (392, 392), (520, 392), (320, 448), (576, 256), (1024, 512)])
+def test_tgmm_strided_all_load_paths(k, n, tile_m):
+    """tgmm over strided segments on 128-row and 256-row tiles: k that ends in the first or the second half of a
+    tile, several row tiles; k and n that are multiples of 64 (256 rows: one column-blocked box per operand and
+    stage, also where the box is wider than the tensor) and that are not (one box per 64 columns); segments around
+    the 64-row stage and the 16-row MMA depth, empty ones; rows past the last group hold NaN."""
+    g, seg = 4, 3
+    sizes = [1, 63, 64, 0,   65, 0, 130, 15,   16, 17, 300, 0]  # segment-major: [q][i]
+    total = sum(sizes)
+    m = total + 40
+    x, _, dout = _inputs(8, m, k, n, 1)
+    x[total:], dout[total:] = float("nan"), float("nan")
+    offs = np.concatenate([[0], np.cumsum(sizes)])
+    want = torch.zeros((g, k, n), dtype=torch.float32)
+    for j, (lo, hi) in enumerate(zip(offs[:-1], offs[1:])):
+        want[j % g] += x[lo:hi].float().T @ dout[lo:hi].float()
+    ws = ops._workspace(m, len(sizes), DEV)
+    xd, dd, gd = _to_dev(x, dout, torch.tensor(sizes, dtype=torch.int32))
+    got, names = launched.kernels(lambda: ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, 1, tile_m, 0),
+                                                           workspace=ws, seg_count=seg))
+    kernel = "ragged_gemm2_kernel<" if tile_m == 256 else "ragged_gemm_kernel<256"
+    assert any(kernel in name for name in names), names
+    assert ops.device_status(ws) == 0
+    assert torch.isfinite(got.float()).all()
+    _assert_close(got.cpu(), want.to(torch.bfloat16), "tgmm strided")
+    assert float(oracle.rel_l2_err(got.cpu(), want, axis=(-1, -2)).max()) < EPS_GROUPS_BF16
+
+
 @pytest.mark.parametrize("sizes,m,n", [([1000], 256, 1024), ([100, 300, 50], 256, 520), ([0, 5000, 7], 700, 264)])
 @pytest.mark.parametrize("tile_m", [128, 256])
 def test_group_sizes_overshooting_m(sizes, m, n, tile_m):
@@ -1446,6 +1475,7 @@ def test_launched_before_the_predecessor_ends():
     (1540, 576, 19456, [256, 257, 1027]),                # exactly one tile; one row more
     (2600, 1040, 11776, [31, 33, 2500]),                 # around one 32-row step; unowned rows
     (1030, 576, 32744, [5, 1020]),                       # trans_rhs: n ends inside a 32-column block
+    (1030, 584, 32960, [5, 1025]),                       # the last tile of a row has 192 columns; a last round in half tiles
 ])
 def test_rows_on_the_n_side(dtype, m, k, n, sizes):
     """The swapped kernel at the edges of its row shares, against the oracle and the 128-row kernel (the
@@ -1523,8 +1553,9 @@ def test_tiles_of_long_groups(dtype, m, k, n, g, kernel):
 @pytest.mark.parametrize("n", [8, 248, 264, 520, 1432])
 @pytest.mark.parametrize("tile", [(256, 1, 256), (256, 2, 256), None])
 def test_tgmm_rows_that_split_sectors(n, tile):
-    """n % 16 == 8: output rows begin inside a 32-byte sector.  Every tile and the library's choice, bit-equal
-    to the 128-row kernel, k around the tile heights, an empty group's zeros included."""
+    """n % 16 == 8: output rows begin inside a 32-byte sector.  256-column tiles on one CTA and on pairs and the
+    library's choice, bit-equal to the kernel with 128-column tiles, k around the tile heights, an empty group's
+    zeros included."""
     g = 3
     for k in (256, 520, 776):
         gs = torch.tensor([70, 0, 133], dtype=torch.int32)
@@ -1533,20 +1564,28 @@ def test_tgmm_rows_that_split_sectors(n, tile):
         cfg = _lib.TileCfg(tile[0], 0, tile[1], tile[2], 0) if tile else None
         out = torch.full((g, k, n), float("nan"), dtype=x.dtype, device=DEV)
         ops.tgmm_forward(xd, dd, gd, cfg=cfg, out=out)
-        ref = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
+        ref = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(128, 0, 1, 128, 0))
         assert torch.equal(out, ref), (k, n)
         assert float(out[1].abs().max()) == 0.0
 
 
-@pytest.mark.parametrize("m,k,n,g", [(300, 256, 264, 2), (900, 1032, 1024, 4), (2000, 776, 3072, 8), (700, 4104, 4096, 1)])
-def test_tgmm_tile_by_rounds(m, k, n, g):
-    """Sizes on either side of the rule that picks the tile height from rounds of tiles: the library's choice
-    has the bits of every tile height."""
+@pytest.mark.parametrize("m,k,n,g,kernel", [
+    (300, 256, 264, 2, "ragged_tgmm_kernel<1>"),      # fewer tiles than CTAs
+    (900, 1032, 1024, 4, "ragged_tgmm_kernel<1>"),    # one round on one CTA, two on pairs
+    (2000, 776, 3072, 8, "ragged_tgmm_kernel<1>"),    # groups of 250, five rounds against six
+    (2048, 776, 3072, 8, "ragged_tgmm_kernel<2>"),    # of 256: up to a quarter more rounds
+    (1600, 512, 3072, 8, "ragged_tgmm_kernel<2>"),    # of 200, three against three
+    (700, 4104, 4096, 1, "ragged_tgmm_kernel<2>"),    # one group, four against four
+])
+def test_tgmm_one_cta_or_pair(m, k, n, g, kernel):
+    """Sizes on either side of the rule that picks pairs from rounds of tiles and rows per group: the kernel it
+    takes, and the bits of the kernel with 128-column tiles, whatever the choice."""
     x, _, dout = _inputs(17, m, k, n, g)
     gs = torch.from_numpy(oracle.reference_group_sizes(5, g, m - 3))
     xd, dd, gd = _to_dev(x, dout, gs)
-    out = ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(0, 0, 0, 0, 0))
-    for cfg in (_lib.TileCfg(256, 0, 1, 128, 0), _lib.TileCfg(256, 0, 1, 256, 0), _lib.TileCfg(256, 0, 2, 256, 0)):
+    out, names = launched.kernels(lambda: ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(0, 0, 0, 0, 0)))
+    assert any(kernel in name for name in names), names
+    for cfg in (_lib.TileCfg(128, 0, 1, 128, 0), _lib.TileCfg(256, 0, 1, 128, 0), _lib.TileCfg(256, 0, 2, 128, 0)):
         assert torch.equal(out, ops.tgmm_forward(xd, dd, gd, cfg=cfg))
 
 

@@ -52,3 +52,26 @@ def test_tgmm_two_accumulators(m, k, n, g, kernel, dtype, rel):
     assert torch.isfinite(got).all()
     # float32 sums in another order, and one rounding to 16 bits (2^-9 or 2^-12 at most)
     assert float((got - want).norm() / want.norm()) < rel
+
+
+@pytest.mark.parametrize("m,k,n,g,kernel", [
+    (2570, 160, 4096, 10, "ragged_gemm_f32_pair_kernel"),  # three rounds of either; the peer's rows begin inside k
+    (2570, 128, 4096, 10, "ragged_gemm_f32_kernel"),       # two rounds against three
+    (2000, 160, 4096, 10, "ragged_gemm_f32_kernel"),       # groups of 200 and few rounds
+    (1500, 1024, 4096, 10, "ragged_gemm_f32_pair_kernel"),  # of 150 in nine rounds
+    (2570, 164, 4096, 10, "ragged_gemm_f32_kernel"),       # rows that are not multiples of 32
+])
+def test_float32_one_cta_or_pair(m, k, n, g, kernel):
+    """Either side of the rule that puts one-pass float32 tgmm on pairs: the same TF32 products, added in the same
+    order, so the bits of one CTA per tile; NaN in the rows of no group."""
+    rng = np.random.default_rng(m + k)
+    live = m - 70
+    gs = torch.from_numpy(rng.multinomial(live, rng.dirichlet(np.full(g, 0.7))).astype(np.int32)).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), device="cuda", generator=gen)
+    dout = torch.randn((m, n), device="cuda", generator=gen)
+    x[live:], dout[live:] = float("nan"), float("nan")
+    got, names = launched.kernels(lambda: ops.tgmm_forward(x, dout, gs))
+    assert any(kernel in name for name in names), names
+    one = ops.tgmm_forward(x, dout, gs, cfg=_lib.TileCfg(256, 0, 1, 128))
+    assert torch.isfinite(got).all() and torch.equal(got, one)
