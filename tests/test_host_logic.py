@@ -79,6 +79,18 @@ def test_tuner_writes_no_entry_where_the_rules_win(tmp_path, monkeypatch):
     assert [e["op"] for e in json.loads(path.read_text())["entries"]] == ["tgmm"]
 
 
+def test_tuner_writes_no_ties():
+    """Choices that are one kernel are timed once, and a choice as fast as the rules, within noise, is no entry."""
+    from gpu_ragged_dot_b200 import tune
+
+    assert {c[:2] for c in tune.candidates("tgmm")} == {c[:2] for c in tune.candidates("gmm")}
+    assert len({c[:2] for c in tune.candidates("tgmm")}) == len(tune.candidates("tgmm"))  # the height means nothing there
+    assert tune.winner([(1.00, (256, 1, 128)), (1.01, tune.RULES)]) is None
+    assert tune.winner([(1.00, tune.RULES), (1.20, (256, 1, 128))]) is None
+    assert tune.winner([(1.00, (256, 2, 128)), (1.10, tune.RULES)]) == (1.00, (256, 2, 128))
+    assert tune.winner([(1.00, (64, 1, 128))]) == (1.00, (64, 1, 128))
+
+
 def test_reference_signature_is_kept():
     import inspect
 
