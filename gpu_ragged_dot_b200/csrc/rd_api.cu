@@ -256,18 +256,22 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 // then land on SMs in the order in which the kernel before leaves them, and neighbours in the tile
 // order, which share operand panels, no longer lie side by side (Mixtral-shaped training step 2.57 ->
 // 2.70 ms, 64 groups 1.41 -> 1.54 ms, 256 groups 5.1 -> 5.5 ms).
-// Groups of 64 rows and less read (or write) weights that no neighbour shares, so there it gains its 2 us too, up to some
-// 512 MB of weights, 80 us: 256 rows, k 4096, n 1536, 64 groups of e4m3 67.7 -> 65.4; 4000, 1024, 1024, 64 30.9 -> 29.5, tgmm
-// 37.0 -> 34.9; 300, 1000, 2000, 100 tgmm 72.5 -> 69.1.  Above, nothing or less: the first in bf16 119.0 -> 119.3; 512, 7168,
-// 2048, 256 755 -> 770.  16-bit and float32 weights with rows along the contraction lose sooner: 3383, 8936, 384, 64 109 -> 115;
-// 2000, 3000, 1024, 64 (393 MB) 82 -> 86.
+// Groups of 64 rows and less read (or write) weights that no neighbour shares, so there it gains its 2 us too, up to 256
+// million weights, 80 us and more (counted for the groups that can have rows, in elements of any type, e4m3 in pairs): 256
+// rows, k 4096, n 1536, 64 groups of e4m3 67.7 -> 65.4; 4000, 1024, 1024, 64 30.9 -> 29.5, tgmm 37.0 -> 34.9; 300, 1000,
+// 2000, 100 tgmm 72.5 -> 69.1; float32 2000, 1024, 2048, 64 (537 MB) 99 -> 98, tgmm 114 -> 107; tgmm of 64 rows in 256 groups,
+// k 1536, n 1536, float32 (2.4 GB) 422 -> 410.  Above, nothing or less: the first in bf16 119.0 -> 119.3; 512, 7168, 2048, 256
+// 755 -> 770.  Weights with rows along the contraction lose sooner, where it is long, so of these 75 million: bf16 3383, 8936,
+// 384, 64 109 -> 115; 2000, 3000, 1024, 64 (393 MB) 82 -> 86.  (Short contractions would gain: float32 2000, 1024, 1024, 64 54 ->
+// 52.)  On pairs, which take such weights for three float32 products only, it does no harm: 2000, 768, 1024, 64 121 -> 119,
+// 1536, 2048 429 -> 427.
 bool launch_early(const GemmArgs& args, int ctas_per_tile = 1, bool wide_k_major = false) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
                                                : static_cast<long long>(args.m < args.g ? args.m : args.g) + args.m / rd::kTileM;
   if (row_tiles * args.n_tiles * ctas_per_tile <= sm_count()) return true;
-  const double weight_bytes = 2.0 * (args.m < args.g ? args.m : args.g) * args.k * args.n;
-  return args.m <= 64LL * args.g && weight_bytes <= (wide_k_major ? 150e6 : 512e6);
+  const double weights = 1.0 * (args.m < args.g ? args.m : args.g) * args.k * args.n;
+  return args.m <= 64LL * args.g && weights <= (wide_k_major ? 75e6 : 256e6);
 }
 
 // How many clusters of two CTAs can be resident at once (0: the query failed).
