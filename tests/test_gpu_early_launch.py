@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from gpu_ragged_dot_b200 import ops
+from tests import launched
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda", 0)
@@ -14,19 +15,11 @@ DEV = torch.device("cuda", 0)
 
 def _capture(fn):
     """fn captured: the graph, what fn returned, and for every edge whether it lets its end start early."""
-    side = torch.cuda.Stream()
-    with torch.cuda.stream(side):
-        fn()
-    torch.cuda.synchronize()
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        res = fn()
+    graph, res = launched.graph_of(fn)
     get = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2
     handle, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
     assert get(handle, None, None, None, ctypes.byref(n)) == 0
-    ends, data = (ctypes.c_void_p * (2 * n.value))(), (ctypes.c_uint8 * (8 * n.value))()
-    starts = (ctypes.c_void_p * n.value).from_buffer(ends)
-    stops = (ctypes.c_void_p * n.value).from_buffer(ends, 8 * n.value)
+    starts, stops, data = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (ctypes.c_uint8 * (8 * n.value))()
     assert get(handle, starts, stops, data, ctypes.byref(n)) == 0
     return graph, res, [data[8 * i + 2] == 1 for i in range(n.value)]  # byte 2: the type, 1 = programmatic
 

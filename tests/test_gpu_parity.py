@@ -1306,9 +1306,10 @@ def test_gmm_fp8_on_256_row_tiles():
     rng = np.random.default_rng(5)
     x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
     A = torch.from_numpy(rng.standard_normal((8, n, k)).astype(np.float32)).to(torch.float8_e4m3fn).to(DEV)
+    gd = gs.to(DEV)
     for scale in (None, torch.rand(8, device=DEV) + 0.5):
-        want = ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale, cfg=_lib.TileCfg(256, 0, 0, 128, 0))
-        got, names = launched.kernels(lambda: ops.gmm_fp8_forward(x, A, gs.to(DEV), weight_scale=scale))
+        want = ops.gmm_fp8_forward(x, A, gd, weight_scale=scale, cfg=_lib.TileCfg(256, 0, 0, 128, 0))
+        got, names = launched.kernels(lambda: ops.gmm_fp8_forward(x, A, gd, weight_scale=scale))
         assert any("ragged_gemm2_kernel" in name for name in names), names
         assert torch.equal(got, want) and float(got[int(gs.sum()):].abs().max()) == 0.0
 
