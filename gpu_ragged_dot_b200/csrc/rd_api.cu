@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <numeric>
 
 #include "../../include/ragged_dot_b200.h"
 #include "rd_gemm.cuh"
@@ -265,11 +266,14 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 // 384, 64 109 -> 115; 2000, 3000, 1024, 64 (393 MB) 82 -> 86.  (Short contractions would gain: float32 2000, 1024, 1024, 64 54 ->
 // 52.)  On pairs, which take such weights for three float32 products only, it does no harm: 2000, 768, 1024, 64 121 -> 119,
 // 1536, 2048 429 -> 427.
-bool launch_early(const GemmArgs& args, int ctas_per_tile = 1, bool wide_k_major = false) {
+// tgmm on 256 columns: two tiles per CTA (`rounds`); there the launch is a good part of the time as well, 20 sizes of two
+// rounds 1.25 times as fast below 256 rows per group, 1.15 below 768, 1.05 above (128 CTAs' worth of such tiles is one
+// round of tiles twice as tall).
+bool launch_early(const GemmArgs& args, int ctas_per_tile = 1, bool wide_k_major = false, int rounds = 1) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
                                                : static_cast<long long>(args.m < args.g ? args.m : args.g) + args.m / rd::kTileM;
-  if (row_tiles * args.n_tiles * ctas_per_tile <= sm_count()) return true;
+  if (row_tiles * args.n_tiles * ctas_per_tile <= static_cast<long long>(rounds) * sm_count()) return true;
   const double weights = 1.0 * (args.m < args.g ? args.m : args.g) * args.k * args.n;
   return args.m <= 64LL * args.g && weights <= (wide_k_major ? 75e6 : 256e6);
 }
@@ -312,7 +316,7 @@ int resident_pairs_once(int threads, size_t smem_bytes) {
 }
 
 // A persistent grid of pairs must be fully co-resident.
-template <auto kKernel, typename... Maps>
+template <auto kKernel, int kEarlyRounds = 1, typename... Maps>
 int launch_pairs(int threads, int smem_bytes, const GemmArgs& args, int ctas, cudaStream_t stream,
                  const Maps&... maps) {
   if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
@@ -322,24 +326,25 @@ int launch_pairs(int threads, int smem_bytes, const GemmArgs& args, int ctas, cu
   int pairs = ctas / 2;
   if (pairs > clusters) pairs = clusters;
   if (pairs < 1) pairs = 1;
-  return launch_kernel(kKernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args, 2), stream, maps..., args);
+  return launch_kernel(kKernel, 2 * pairs, threads, smem_bytes, 2, launch_early(args, 2, false, kEarlyRounds), stream,
+                       maps..., args);
 }
 
-template <int BN, bool kBKMajor, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false>
+template <int BN, bool kBKMajor, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false, bool kOneThread = false>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tout,
                 const GemmArgs& args, int ctas, cudaStream_t stream) {
   constexpr int kStageBytes = rd::stage_bytes<BN, kCtas>();
   constexpr int kStages = (196608 / kStageBytes) > 8 ? 8 : (196608 / kStageBytes);
   constexpr int kSmem = kStages * kStageBytes + rd::kOutStagingBytes + 1024;
-  constexpr auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, kCtas, kSeg, kFp8>;
+  constexpr auto kernel = rd::ragged_gemm_kernel<BN, kBKMajor, kStages, kTgmm, kCtas, kSeg, kFp8, false, kOneThread>;
   if constexpr (kCtas == 2) return launch_pairs<kernel>(rd::kGemmFixerThreads, kSmem, args, ctas, stream, ta, tb, tout);
   // The attribute is per device; setting it again is cheap, so do it on every call rather
   // than track which devices have seen it.
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
       cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1, launch_early(args, 1, kBKMajor && !kFp8), stream, ta, tb, tout,
-                       args);
+  return launch_kernel(kernel, ctas, rd::kGemmFixerThreads, kSmem, 1,
+                       launch_early(args, 1, kBKMajor && !kFp8, kTgmm && BN == 256 ? 2 : 1), stream, ta, tb, tout, args);
 }
 
 // Rows that are not multiples of 16 bytes (see kUnaligned in rd_gemm.cuh).
@@ -598,10 +603,11 @@ int launch_tgmm(const void* x, const void* dout, const CUtensorMap& tout, int dt
   constexpr auto kernel = rd::ragged_tgmm_kernel<kCtas>;
   constexpr int kSmem = rd::tg_smem_bytes<kCtas>();
   if constexpr (kCtas == 2)
-    return launch_pairs<kernel>(rd::kTgThreads, kSmem, args, ctas, stream, ta, ta2, tb, tb2, tout);
+    return launch_pairs<kernel, 2>(rd::kTgThreads, kSmem, args, ctas, stream, ta, ta2, tb, tb2, tout);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
     return RD_ERR_LAUNCH;
-  return launch_kernel(kernel, ctas, rd::kTgThreads, kSmem, 1, launch_early(args), stream, ta, ta2, tb, tb2, tout, args);
+  return launch_kernel(kernel, ctas, rd::kTgThreads, kSmem, 1, launch_early(args, 1, false, 2), stream, ta, ta2, tb, tb2, tout,
+                       args);
 }
 
 // Upper bound on the live 128 x 256 tiles of a gmm: a group has at least one row, and only whole
@@ -673,50 +679,44 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
   return 10 * r2 <= 11 * r1 && r1 > 1 && (m / g >= 256 || (m / g >= 100 && r1 > 6));
 }
 
-// tgmm with 256-column tiles (rd_tgmm.cuh): 256 x 256 on CTA pairs, or 128 x 256 on one CTA each?  A pair moves a third
-// less data into shared memory.  Microseconds in a row, one CTA against a pair:
-// - Groups of 256 rows and more: pairs, up to a quarter more rounds of tiles (m 8192, k 4096, n 14336, 8 groups 908 ->
-//   722; 21272, 600, 5440, 49, 37 rounds against 44, 207 -> 190; 20312, 288, 280, 38, 2 against 3, equal).
-// - Groups of less than 64 rows: one CTA (5331, 4096, 1536, 128 299 against 325; 2816 548 against 586; at 64 rows equal).
-// - Groups between: pairs where they take no more rounds and more than two (16384, 7168, 2048, 128 972 -> 851; 3000,
-//   2048, 2048, 30 72 -> 69; 5024, 272, 1352, 124, 16 against 21 rounds, 35 -> 37).  With one or two rounds the start of a
-//   cluster is a good part of the time (512, 256, 384, 8, one round, alone 11 -> 13).
-// - Output rows that are not multiples of 32 bytes, groups of 100 rows and less: boxes begin and end inside sectors,
-//   which costs L2 reads of what it has not got; the one-CTA tiles, whose boxes of a row follow one another more
-//   closely, suffer less (4365, 11600, 3240, 45 1134 -> 1299; 6192, 3480, 840, 74 147 -> 173; 103 rows per group, 3512,
-//   8168, 648, 34 119 -> 112).  Rows that are not whole 256 bytes likewise, below 100 rows (5331, 4096, 1216, 128 242 -> 276;
-//   n 1600 293 -> 358).
-bool choose_tgmm_pair(long long m, int k, int n, int g) {
-  const long long sms = sm_count(), cols = (static_cast<long long>(n) + 255) / 256 * g;
-  const long long r1 = ((k + 127) / 128 * cols + sms - 1) / sms;
-  const long long r2 = ((k + 255) / 256 * cols + sms / 2 - 1) / (sms / 2);
-  if (m / g >= 256) return 4 * r2 <= 5 * r1;
-  if (n % 16 != 0 && m / g <= 100) return false;
-  if (m / g < (n % 128 != 0 ? 100 : 64)) return false;
-  return r2 <= r1 && r1 > 2;
-}
-
-// 128 x 256 tiles on one CTA each, groups that are not long and output rows that are not whole 256 bytes: a column tile's
-// edge falls inside 256 bytes (or a sector) of every other row, and what counts is that the CTAs that write either side
-// of it stay side by side.  A CTA steps over `ctas` tiles; `d` is what that shares with the tiles of a row.
-// - d > 1 and CTAs that would meet more wide columns than others: the order is turned.  128 groups of 42, k 4096, plain kernel
-//   (rd_gemm.cuh), two accumulators, those turned, microseconds: n 776 301, 327, 196; 1288 546, 509, 370; 1800 714, 716, 542.
-// - d > 1, narrow columns spread over all of them: as it is; n 1392 360, 261, 263; 1400 560, 428, 422.
-// - otherwise the plain kernel, whose CTAs write one tile at a time: n 1160 275, 319, 381; 1560 388, 443, 463; 1600 293, 331, 302;
-//   1000 231, 281, 277; 2112 391, 484, 440; groups of 8, k 2048, n 1216 109, 104, 107.
-enum class TgmmOneCta { kAsIs, kTurned, kPlain };
-TgmmOneCta tgmm_one_cta(long long m, int n, int g, int ctas) {
-  const int tiles = (n + 255) / 256;
-  if (n % 128 == 0 || tiles == 1 || m / g >= 256) return TgmmOneCta::kAsIs;
-  int d = tiles;
-  for (int r = ctas; r != 0;) {
-    const int t = d % r;
-    d = r;
-    r = t;
+// tgmm with 256-column tiles: which kernel?  By rounds of tiles (128 x 256 on one CTA, 256 x 256 on a pair) and the mean rows of
+// a group.  Timed all five ways on 640 sizes (16 to 32768 rows per call, 1 to 256 groups, equal to heavy-tailed) the choice takes
+// 1.5 % longer than the best of them on average.  Microseconds in a row, sizes m, k, n, groups:
+// - One round: the plain 128-row kernel (rd_gemm.cuh), which starts sooner and has a stage more (171, 1880, 768, 3 6.3 against 7.5 on two
+//   accumulators; 260, 1056, 3432, 1 7.7 against 9.2); from 768 rows per group on the MMAs count, and a pair moves a third less
+//   data (2077, 344, 880, 1 19.8 -> 17.6; 9424, 640, 360, 2 37 -> 27; just above equal: 884, 4408, 536, 1 13.4 -> 12.8).
+// - Groups of 512 rows and more: pairs, up to a quarter more rounds (m 8192, k 4096, n 14336, 8 groups 908 -> 722); of 256 rows up to
+//   three rounds only with no more of them (2683, 472, 2600, 6 26.6 -> 23.1; three against two, 4150, 544, 1152, 10 16.4 -> 18.4).
+// - Groups of 64 to 255 rows: pairs likewise, but from seven rounds on (9101, 4496, 1944, 37 307 -> 248; 672, 7288, 11816, 4 257 ->
+//   232); up to six the plain kernel (7474, 376, 1280, 44 27.1 against 28.6; 579, 320, 8192, 3 10.7 against 14.3).
+// - Groups of less than 64 rows: up to three rounds the plain kernel, then by the output's rows.  Whole 256 bytes: two accumulators
+//   (1085, 520, 2048, 67 33.2 plain, 29.2).  Other rows: a column tile's edge falls inside 256 bytes (or a sector) of every other
+//   row, and what counts is that the CTAs that write either side of it stay side by side.  Whole sectors: two accumulators with the
+//   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
+//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where the columns of up to twelve tiles are unequal and a
+//   CTA's step, `ctas` tiles, shares a factor with them (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1800
+//   724, 696, 528); otherwise the plain kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37
+//   rounds on (kOneThread, rd_gemm.cuh).
+enum class TgmmWay { kPair, kPlain, kOneThread, kTwoAcc, kTurned };
+TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
+  const long long rows = m / g, tiles = (static_cast<long long>(n) + 255) / 256, blocks = (static_cast<long long>(n) + 63) / 64;
+  const long long r1 = ((k + 127) / 128 * tiles * g + ctas - 1) / ctas;
+  if (cta_group == 2) return TgmmWay::kPair;
+  if (cta_group == 0) {
+    const long long pairs = sm_count() / 2, r2 = ((k + 255) / 256 * tiles * g + pairs - 1) / pairs;
+    if (r1 <= 1) {
+      if (rows >= 768 && r2 <= 1) return TgmmWay::kPair;
+    } else if (rows >= 512 || (rows >= 256 && r1 > 3) || (rows >= 64 && r1 > 6)) {
+      if (4 * r2 <= 5 * r1) return TgmmWay::kPair;
+    } else if (rows >= 256) {
+      if (r2 <= r1) return TgmmWay::kPair;
+    }
   }
-  const int wide = (n + 63) / 64 % tiles;  // tiles with a block of 64 columns more than the others
-  if (d > 1 && (wide % d != 0 || (n % 64 != 0 && n % 64 < 40))) return TgmmOneCta::kTurned;
-  return d > 1 && wide != 0 ? TgmmOneCta::kAsIs : TgmmOneCta::kPlain;
+  if (r1 <= 3 || rows >= 64) return TgmmWay::kPlain;
+  if (n % 128 == 0 || tiles == 1) return TgmmWay::kTwoAcc;
+  if (n % 16 == 0) return TgmmWay::kTurned;
+  if (tiles <= 12 && blocks != 4 * tiles && std::gcd(tiles, static_cast<long long>(ctas)) > 1) return TgmmWay::kTurned;
+  return r1 > 36 ? TgmmWay::kOneThread : TgmmWay::kPlain;
 }
 
 // Limit of every bounded wait inside a kernel, in microseconds: rd_tile_cfg.wait_limit_ms if
@@ -1317,11 +1317,14 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (cta_group == 2) return RD_ERR_BAD_CONFIG;
     cta_group = 1;
   }
-  // 256 columns, plain: the kernel with two accumulators, whatever tile height the caller names.
+  // 256 columns, plain: 128 rows per CTA, whatever tile height the caller names.
   const bool two_acc = !f32 && bn == 256 && seg_count == 1;
+  const int ctas = pick_ctas(cfg);
+  TgmmWay way = TgmmWay::kPlain;
   if (two_acc) {
     tile_m = 128;
-    if (cta_group == 0) cta_group = choose_tgmm_pair(m, k, n, g) ? 2 : 1;
+    way = tgmm_way(m, k, n, g, ctas, cta_group);
+    cta_group = way == TgmmWay::kPair ? 2 : 1;
   }
   if (cta_group == 0) cta_group = 1;
   if (tile_m == 0) tile_m = choose_two_half(true, m, k, n, g, bn) ? 256 : 128;
@@ -1399,7 +1402,6 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
   args.status = w.status();
   args.out = out;
 
-  const int ctas = pick_ctas(cfg);
   if (f32_pair)
     return three_pass ? launch_gemm_f32_pair<false, true, true>(ta, tb, tout, args, ctas, stream)
                       : launch_gemm_f32_pair<false, true, false>(ta, tb, tout, args, ctas, stream);
@@ -1414,14 +1416,15 @@ static int tgmm_impl(const void* x, const void* dout, const int32_t* group_sizes
     if (bn == 128) return launch_gemm<128, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
     return launch_gemm<64, false, true, 1, true>(ta, tb, tout, args, ctas, stream);
   }
-  if (two_acc && cta_group == 1) {
-    const TgmmOneCta way = tgmm_one_cta(m, n, g, ctas);
-    if (way == TgmmOneCta::kPlain) return launch_gemm<256, false, true, 1>(ta, tb, tout, args, ctas, stream);
-    args.turn_columns = way == TgmmOneCta::kTurned ? 1 : 0;
+  if (two_acc) {
+    args.turn_columns = way == TgmmWay::kTurned ? 1 : 0;
+    switch (way) {
+      case TgmmWay::kPair: return launch_tgmm<2>(x, dout, tout, dtype, args, ctas, stream);
+      case TgmmWay::kPlain: return launch_gemm<256, false, true, 1>(ta, tb, tout, args, ctas, stream);
+      case TgmmWay::kOneThread: return launch_gemm<256, false, true, 1, false, false, true>(ta, tb, tout, args, ctas, stream);
+      default: return launch_tgmm<1>(x, dout, tout, dtype, args, ctas, stream);
+    }
   }
-  if (two_acc)
-    return cta_group == 2 ? launch_tgmm<2>(x, dout, tout, dtype, args, ctas, stream)
-                          : launch_tgmm<1>(x, dout, tout, dtype, args, ctas, stream);
   if (bn == 128) return launch_gemm<128, false, true, 1>(ta, tb, tout, args, ctas, stream);
   return launch_gemm<64, false, true, 1>(ta, tb, tout, args, ctas, stream);
 }

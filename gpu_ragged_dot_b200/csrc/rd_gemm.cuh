@@ -416,8 +416,14 @@ constexpr int stage_bytes() {
 // kUnaligned: rows of the output are not multiples of 16 bytes (n odd, say).  Operands come through
 // maps whose rows have a pitch of their own; the output is staged as usual and stored element
 // by element, a warp covering 32 consecutive columns of a row at a time.
+// kOneThread (tgmm): producer and MMA loops run by one thread each, and nothing in the kernel knows its warp to be
+// uniform, instead of a whole warp that elects a lane.  Slower to issue, and where an output of more than some 36 rounds of tiles
+// has rows that begin inside a sector (n % 16 == 8) that is what keeps the CTAs that write either side of a column tile's edge
+// abreast.  128 heavy-tailed groups of 42 rows, k 4096, microseconds in a row, whole warps against one thread: n 1224 344 -> 318,
+// 1592 464 -> 416, 1720 514 -> 422, 2040 609 -> 514; 494, 6600, 1176, 136 597 -> 448; 108, 2624, 4584, 68 444 -> 323.  Fewer rounds
+// the other way: 171, 1880, 768, 3 (one) 6.7 -> 6.1.  Choice: tgmm_way in rd_api.cu.
 template <int BN, bool kBKMajor, int kStages, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false,
-          bool kUnaligned = false>
+          bool kUnaligned = false, bool kOneThread = false>
 __global__ void __launch_bounds__(kGemmFixerThreads, 1)
 ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                    const __grid_constant__ CUtensorMap tmap_b,
@@ -427,6 +433,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   static_assert(kCtas == 1 || (kCtas == 2 && BN >= 128), "a CTA pair needs BN >= 128");
   static_assert(!kTgmm || kCtas == 1, "tgmm on CTA pairs: rd_tgmm.cuh");
   static_assert(!kSeg || kTgmm, "strided segments: tgmm");
+  static_assert(!kOneThread || (kTgmm && !kSeg), "loops of one thread: plain tgmm");
   // 8-bit inputs (e4m3): both operands K-major (x[m,k], W[g,n,k]), so the tiles are byte for byte
   // those of a 16-bit problem with k/2 elements per row (which is what the tensor maps and
   // GemmArgs::k describe); only the MMA kind differs, 32 elements = 32 bytes per instruction, and
@@ -451,7 +458,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __shared__ WaitCtl wait_ctl;
   __shared__ GroupTable group_table;
 
-  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int warp = kOneThread ? static_cast<int>(threadIdx.x >> 5)
+                              : __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int cta_rank = kPair ? static_cast<int>(cluster_cta_rank()) : 0;
   const bool leader = cta_rank == 0;
@@ -513,20 +521,39 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     return kTgmm ? decode_tgmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank)
                  : decode_gmm_tile<BN, kCtas>(p, &group_table, tile, cta_rank);
   };
+  // How producer and MMA loop run: as whole warps on uniform values, or by one thread.
+  auto coord = [&](int tile) -> TileCoord {
+    if constexpr (kOneThread) return decode(tile);
+    return uniform_coord(decode(tile));
+  };
+  auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+    if constexpr (kOneThread) return mbar_wait(bar, parity, abort_ptr);
+    return mbar_wait_warp(bar, parity, abort_ptr);
+  };
+  auto elected = [&]() -> bool {
+    if constexpr (kOneThread) return true;
+    return elect_one();
+  };
+  auto uniform = [&](int v) -> int {
+    if constexpr (kOneThread) return v;
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
 
   // The producer and the MMA warp run their loops as whole warps on uniform values and elect a lane for each
   // stage's instructions.  Against loops of one thread, microseconds in a row: m 32768, k 7168, n 2048, 256
   // heavy-tailed groups 1467 -> 1370, trans_rhs 1513 -> 1459; decode, 256 rows 121.8 -> 120.4, e4m3 67.7 -> 66.9;
   // 1024 rows, k 1024, n 1024, 8 groups 11.0 -> 10.4.
-  if (warp == 0) {
+  if (kOneThread && warp < 2 && lane != 0) {
+    // one thread runs either loop
+  } else if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     uint32_t it = 0;
     bool ok = true;
     int ready_slot = -1;  // last ready flag this producer has seen set
     for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step) {
-      const TileCoord t = uniform_coord(decode(tile));
+      const TileCoord t = coord(tile);
       const int nb = t.n0 + cta_rank * kBCols;  // first B column this CTA loads
-      const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+      const int kb_count = kTgmm ? uniform(tgmm_block_count<kSeg>(p, t)) : k_blocks_gmm;
       RowBlocks blocks = first_block(t);
       if (!kTgmm && p.ready_flags != nullptr) {
         const int slot = t.group / p.groups_per_flag;
@@ -541,7 +568,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       for (int kb = 0; kb < kb_count; ++kb, ++it) {
         const uint32_t s = it % kStages;
         const uint32_t ph = (it / kStages) & 1u;
-        if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1u, abort_ptr)) {
+        if (!wait(smem_u32(&bar_empty[s]), ph ^ 1u)) {
           ok = false;
           break;
         }
@@ -552,7 +579,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tgmm_block<kSeg>(p, t, blocks, kb, r, live);
           if (kSeg) r = __shfl_sync(0xffffffffu, r, 0);
         }
-        if (elect_one()) {
+        if (elected()) {
           uint32_t full = smem_u32(&bar_full[s]);
           const bool remote_bar = kPair && !leader;  // the peer's bytes are counted on the leader's barrier
           if (remote_bar) {
@@ -606,15 +633,15 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint32_t tail_events = 0;  // stages handed to the fixer warp so far
       bool ok = true;
       for (int tile = tile_start; tile < num_tiles && ok; tile += tile_step, ++local_tile) {
-        const TileCoord t = uniform_coord(decode(tile));
-        const int kb_count = kTgmm ? __shfl_sync(0xffffffffu, tgmm_block_count<kSeg>(p, t), 0) : k_blocks_gmm;
+        const TileCoord t = coord(tile);
+        const int kb_count = kTgmm ? uniform(tgmm_block_count<kSeg>(p, t)) : k_blocks_gmm;
         const bool tail_stage = kTgmm && kb_count > 0 && tail_needs_clearing(t.rows);
         RowBlocks blocks = first_block(t);
         const uint32_t idesc = (!kTgmm && !kPair && t.rows <= 64) ? idesc_half : idesc_full;
 
         const uint32_t acc = local_tile & 1u;
         const uint32_t acc_ph = (local_tile >> 1) & 1u;
-        if (!mbar_wait_warp(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u, abort_ptr)) {
+        if (!wait(smem_u32(&bar_acc_empty[acc]), acc_ph ^ 1u)) {
           ok = false;
           break;
         }
@@ -623,7 +650,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         uint32_t s = it % kStages;
         uint32_t ph = (it / kStages) & 1u;
         for (int kb = 0; kb < kb_count; ++kb, ++it, s = (s + 1 == kStages ? 0 : s + 1), ph ^= (s == 0)) {
-          if (!mbar_wait_warp(smem_u32(&bar_full[s]), ph, abort_ptr)) {
+          if (!wait(smem_u32(&bar_full[s]), ph)) {
             ok = false;
             break;
           }
@@ -642,8 +669,8 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
             // warp clears them, up to the end of the last MMA that is issued, in every box of this
             // stage, so they add nothing to the reduction.  (In gmm the columns past k are
             // zero-filled by TMA.)
-            if (elect_one()) mbar_arrive(smem_u32(&bar_tail_go));
-            if (!mbar_wait_warp(smem_u32(&bar_tail_done), tail_events & 1u, abort_ptr)) {
+            if (elected()) mbar_arrive(smem_u32(&bar_tail_go));
+            if (!wait(smem_u32(&bar_tail_done), tail_events & 1u)) {
               ok = false;
               break;
             }
@@ -654,7 +681,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // address field, and only a tgmm tile's last stage looks at n_mma.
           const uint32_t a_lo = adesc0_lo + s * (kStageBytes >> 4);
           const uint32_t b_lo = bdesc0_lo + s * (kStageBytes >> 4);
-          if (elect_one()) {
+          if (elected()) {
             if (kTgmm && n_mma < kTileK / kUmmaK) {
               for (int kk = 0; kk < n_mma; ++kk) {
                 umma_ab<kCtas, kFp8>(tmem_d, make_desc64(a_lo + kk * kAStep, desc_hi),
@@ -680,7 +707,7 @@ ragged_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         if (!ok) break;
         const uint32_t bar = smem_u32(&bar_acc_full[acc]);
-        if (elect_one()) {
+        if (elected()) {
           if (kb_count > 0) {
             if (kPair) {
               umma_commit_pair(bar, 0x3);

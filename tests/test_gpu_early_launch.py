@@ -39,6 +39,10 @@ def _capture(fn):
     ("tgmm", 640, 2000, 2000, 64, torch.bfloat16, True),
     ("tgmm", 640, 2000, 2008, 64, torch.bfloat16, False),
     ("tgmm", 16, 2000, 2008, 64, torch.float32, True),      # 16 groups at most have rows
+    ("tgmm", 1000, 520, 1024, 14, torch.bfloat16, True),    # two tiles per CTA at most (280 tiles)
+    ("tgmm", 1000, 520, 1024, 15, torch.bfloat16, False),   # 300
+    ("tgmm", 2000, 520, 1024, 2, torch.bfloat16, True),     # 24 on pairs
+    ("tgmm", 1000, 520, 1024, 14, torch.float32, False),    # float32: one tile per CTA
 ])
 def test_which_calls_start_early(op, m, k, n, g, dtype, early):
     gs = torch.full((g,), m // g, dtype=torch.int32, device=DEV)

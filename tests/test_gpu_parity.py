@@ -1571,16 +1571,26 @@ def test_tgmm_rows_that_split_sectors(n, tile):
 
 
 @pytest.mark.parametrize("m,k,n,g,kernel", [
-    (300, 256, 264, 2, "ragged_tgmm_kernel<1>"),      # fewer tiles than CTAs
-    (900, 1032, 1024, 4, "ragged_tgmm_kernel<1>"),    # one round on one CTA, two on pairs
-    (2000, 776, 3072, 8, "ragged_tgmm_kernel<1>"),    # groups of 250, five rounds against six
+    (300, 256, 264, 2, "ragged_gemm_kernel<256"),     # one round
+    (1534, 776, 264, 2, "ragged_gemm_kernel<256"),    # one round of 767 rows per group
+    (1536, 776, 264, 2, "ragged_tgmm_kernel<2>"),     # of 768
+    (900, 1032, 1024, 4, "ragged_gemm_kernel<256"),   # one round on one CTA, two on pairs
+    (2000, 776, 3072, 8, "ragged_gemm_kernel<256"),   # groups of 250, five rounds
     (2048, 776, 3072, 8, "ragged_tgmm_kernel<2>"),    # of 256: up to a quarter more rounds
-    (1600, 512, 3072, 8, "ragged_tgmm_kernel<2>"),    # of 200, three against three
+    (1600, 512, 3072, 8, "ragged_gemm_kernel<256"),   # of 200, three against three
+    (2000, 512, 3072, 20, "ragged_tgmm_kernel<2>"),   # of 100, seven against seven
+    (2000, 264, 3072, 31, "ragged_gemm_kernel<256"),  # of 64, eight against eleven
+    (620, 520, 3072, 10, "ragged_tgmm_kernel<1>"),    # of 62, five rounds
+    (640, 520, 3072, 10, "ragged_gemm_kernel<256"),   # of 64
     (700, 4104, 4096, 1, "ragged_tgmm_kernel<2>"),    # one group, four against four
+    (300, 2048, 1160, 66, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, false>"),  # 36 rounds
+    (300, 2048, 1160, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # a round more
+    (300, 2048, 1176, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # five tiles still
+    (300, 2048, 1168, 67, "ragged_tgmm_kernel<1>"),   # rows of whole sectors
 ])
 def test_tgmm_one_cta_or_pair(m, k, n, g, kernel):
-    """Sizes on either side of the rule that picks pairs from rounds of tiles and rows per group: the kernel it
-    takes, and the bits of the kernel with 128-column tiles, whatever the choice."""
+    """Sizes on either side of the rule that picks a kernel from rounds of tiles, rows per group and the output's rows: what
+    it takes, and the bits of the kernel with 128-column tiles, whatever the choice."""
     x, _, dout = _inputs(17, m, k, n, g)
     gs = torch.from_numpy(oracle.reference_group_sizes(5, g, m - 3))
     xd, dd, gd = _to_dev(x, dout, gs)

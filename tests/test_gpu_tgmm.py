@@ -11,24 +11,27 @@ from tests import launched
 
 pytestmark = pytest.mark.gpu
 ONE, PAIR = "ragged_tgmm_kernel<1>", "ragged_tgmm_kernel<2>"
-PLAIN = "ragged_gemm_kernel<256"  # one accumulator drained at a time
+PLAIN = "ragged_gemm_kernel<256"  # tiles written one at a time
 
 
 @pytest.mark.parametrize("dtype,rel", [(torch.bfloat16, 2e-3), (torch.float16, 3e-4)])
 @pytest.mark.parametrize("m,k,n,g,kernel", [
-    (40, 136, 264, 3, ONE),        # fewer tiles than CTAs
-    (900, 520, 2384, 9, PAIR),     # two bands of column tiles, the last tile 80 wide, rows not of whole blocks
-    (700, 1032, 2176, 4, PAIR),    # the same with a last tile of 128 and whole blocks in n only
+    (40, 136, 264, 3, PLAIN),      # fewer tiles than CTAs
+    (1300, 1000, 2384, 13, PAIR),  # two bands of column tiles, the last tile 80 wide, rows not of whole blocks
+    (2275, 1016, 2176, 13, PAIR),  # the same with a last tile of 128 and whole blocks in n only
     (64, 504, 2176, 40, ONE),      # two rows per group
     (3200, 504, 2176, 40, PAIR),   # eighty
     (300, 392, 840, 60, ONE),      # output rows that split sectors, short groups
-    (3000, 320, 2048, 3, PAIR),    # long groups: several stages per tile
+    (3000, 320, 2048, 3, PAIR),    # long groups: several stages per tile, one round
     (700, 1288, 776, 31, ONE),     # four tiles per row of 4, 3, 3 and 3 blocks, the order turned
-    (500, 392, 1288, 13, ONE),     # six tiles, as many wide as narrow, turned
-    (500, 392, 1392, 13, ONE),     # six tiles, narrow ones spread over all CTAs
-    (500, 392, 2312, 9, ONE),      # ten tiles in two bands, turned
-    (700, 392, 1160, 17, PLAIN),   # five tiles
+    (500, 392, 1288, 30, ONE),     # six tiles, as many wide as narrow, turned
+    (500, 392, 1392, 30, ONE),     # six tiles, rows of whole sectors, turned
+    (500, 392, 2312, 20, ONE),     # ten tiles in two bands, turned
+    (500, 392, 2320, 20, ONE),     # the same in whole sectors
+    (500, 520, 1408, 30, ONE),     # rows of whole 256 bytes
+    (700, 392, 1160, 17, PLAIN),   # five tiles, three rounds
     (700, 264, 1000, 40, PLAIN),   # four tiles, equally wide
+    (300, 2048, 1160, 68, PLAIN),  # 37 rounds of tiles: loops run by one thread
     (500, 264, 136, 300, ONE),     # more groups than the table in shared memory holds; most rounds on one CTA
 ])
 def test_tgmm_two_accumulators(m, k, n, g, kernel, dtype, rel):
