@@ -489,25 +489,39 @@ int launch_gemm_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
 
 // Fewer rounds than choose_swap asks for: the clocks of both kernels, from their rounds of tiles.  A pair takes 4 clocks per
 // row and block of the contraction and 5000 to drain a tile, a last half round costs 0.55 of one (SwapWork), one CTA 560
-// per block of a 128 x 256 tile; a group's last tile is half full on average.  Timed on both sides on 400 float32, 600
-// 16-bit and 350 e4m3 sizes (1 to 64 groups, equal and unequal, 256 to 14336 deep and wide), this and the rules
-// below against the rules below alone: float32 1.019 times as fast on average over all sizes instead of 1.012, 16 bits
-// 1.010 instead of 1.004, e4m3 1.005 instead of 1.001; slower by more than 2 % in 0, 2 and 0 of them, 4 % at most.  A
-// last tile of a row that is a half tile counts whole: pairs do not share such tiles evenly (counted half, 704 columns
-// were up to 29 % slower).  Under half a round, and for groups shorter than `least`, it is wrong too often.
+// per block of a 128 x 256 tile; a group's last tile is half full on average.  A last tile of a row that is a half tile counts
+// whole: pairs do not share such tiles evenly (counted half, 704 columns were up to 29 % slower).  The tiles of a single
+// group are counted: 590 rows, k 10912, n 12640, float32, are 75 tiles for 74 pairs (293 -> 372 us where an average of 70
+// had said one round).  Under half a round, and for groups shorter than `least`, it is wrong too often.
+// Timed on both sides on 477 sizes that this takes and the rules below do not (1 to 256 groups, equal to heavy-tailed): 16 bits
+// 1.17 times as fast on average, slower by more than 5 % in 7 of 191; e4m3 1.17, 22 of 189; float32 1.14, 2 of 97.  Most of the slower
+// ones are heavy-tailed, which the host cannot know: worst, e4m3 4842, 3840, 584, 28 groups 28 -> 43, 16 bits 4567, 3216, 3192, 7
+// 95 -> 114.  e4m3 within a twentieth of one whole round is as often slower as faster (11257, 5632, 432, 62 55 -> 74; 2595, 5200,
+// 2296, 9 67 -> 46).
 bool swap_takes_less(long long m, int k_blocks, int n, int g, int least, double margin) {
   if (m / g < least) return false;
-  const double sms = sm_count(), rows = static_cast<double>(m) / g;
-  const double per = rows > 128.0 ? rows / rd::kSwapRows + 0.5 : 1.0;
-  const double exact = g * per * ((n + rd::kSwapCols - 1) / rd::kSwapCols) / (sms / 2);
-  if (exact < 0.5) return false;
-  if (exact < 1.0) margin = 1.25;
-  const double whole = static_cast<double>(static_cast<long long>(exact)), left = exact - whole;
-  const double rounds = whole + (left < 0.03 ? 0.0 : left <= 0.5 ? 0.55 : 1.0);
-  double height = rows / per + 8.0;
+  const long long sms = sm_count(), pairs = sms / 2;
+  const long long cols = (n + rd::kSwapCols - 1) / rd::kSwapCols, cols128 = (n + 255) / 256;
+  double rounds, height, rounds128;
+  if (g == 1) {
+    const long long per = (m + rd::kSwapRows - 1) / rd::kSwapRows, tiles = per * cols, left = tiles % pairs;
+    if (2 * tiles < pairs) return false;
+    rounds = static_cast<double>(tiles / pairs) + (left == 0 ? 0.0 : 2 * left <= pairs ? 0.55 : 1.0);
+    height = static_cast<double>((m + 16 * per - 1) / (16 * per) * 16);
+    rounds128 = static_cast<double>(((m + rd::kTileM - 1) / rd::kTileM * cols128 + sms - 1) / sms);
+    margin = 1.0;
+  } else {
+    const double rows = static_cast<double>(m) / g, per = rows > 128.0 ? rows / rd::kSwapRows + 0.5 : 1.0;
+    const double exact = g * per * cols / pairs;
+    if (exact < 0.5) return false;
+    if (exact < 1.0) margin = 1.25;
+    const double whole = static_cast<double>(static_cast<long long>(exact)), left = exact - whole;
+    rounds = whole + (left < 0.03 ? 0.0 : left <= 0.5 ? 0.55 : 1.0);
+    height = rows / per + 8.0;
+    const double per128 = rows > 64.0 ? rows / rd::kTileM + 0.5 : 1.0;
+    rounds128 = static_cast<double>(static_cast<long long>(g * per128 * cols128 / sms + 0.97));
+  }
   if (height > rd::kSwapRows) height = rd::kSwapRows;
-  const double per128 = rows > 64.0 ? rows / rd::kTileM + 0.5 : 1.0;
-  const double rounds128 = static_cast<double>(static_cast<long long>(g * per128 * ((n + 255) / 256) / sms + 0.97));
   return rounds * (4.0 * height * k_blocks + 5000.0) * margin < (rounds128 > 1.0 ? rounds128 : 1.0) * 560.0 * k_blocks;
 }
 
@@ -538,9 +552,10 @@ bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool f
          static_cast<double>((tiles128 + 2 * pairs - 1) / (2 * pairs));
 }
 
-// The same for float32 in one pass (128-row tiles on one CTA otherwise), k_blocks of 32.  Of 260 sizes timed on both
-// sides it takes 15, 1.11 times as fast on average and 6 % slower in one: m 32768, k 2624, n 928, 26 groups 282 -> 237
-// us, 32768, 368, 7584, 28 384 -> 349.  Below three rounds either side wins by up to 1.6, by how rounds fall.
+// The same for float32 in one pass (128-row tiles on one CTA otherwise), k_blocks of 32.  70 sizes that it takes and
+// swap_takes_less does not, timed on both sides: 1.10 times as fast on average (m 32768, k 2624, n 928, 26 groups 282 -> 237 us; 15103,
+// 584, 8480, 16 402 -> 316), slower by more than 5 % in four (worst 8835, 384, 4192, 2, 12 blocks and a narrow last tile, 67 -> 75).
+// Below three rounds either side wins by up to 1.6, by how rounds fall.
 bool choose_swap_f32(long long m, int k_blocks, int n, int g, bool trans_rhs) {
   if (g <= 0 || (!trans_rhs && n % 32 != 0)) return false;
   if (swap_takes_less(m, k_blocks, n, g, 384, 1.0)) return true;

@@ -69,3 +69,23 @@ def test_float32_rows_in_steps_of_16(m, k, n, g, trans):
     ref = ops.gmm_forward(x, w, gs, trans_rhs=trans, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
     assert torch.equal(got[:m - 5], ref[:m - 5])  # the same TF32 products, added in the same order
     assert float(got[m - 5:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype,m,k,n,swapped", [
+    (torch.float32, 590, 8192, 12640, False),        # 75 tiles for 74 pairs
+    (torch.float32, 512, 8192, 12640, True),         # 50, in one round against two
+    (torch.float8_e4m3fn, 338, 8416, 12520, False),  # one round of either kernel
+    (torch.bfloat16, 1785, 4096, 4672, True),        # 70 tiles
+])
+def test_one_group_is_counted(dtype, m, k, n, swapped):
+    """The rule for few rounds on one group, whose tiles the host can count."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), device="cuda", generator=gen).to(dtype)
+    w = torch.randn((1, n, k), device="cuda", generator=gen, dtype=torch.bfloat16).to(dtype)
+    gs = torch.tensor([m - 3], dtype=torch.int32, device="cuda")
+    fn = ops.gmm_fp8_forward if dtype == torch.float8_e4m3fn else lambda *a, **kw: ops.gmm_forward(*a, trans_rhs=True, **kw)
+    got, names = launched.kernels(lambda: fn(x, w, gs))
+    assert any("ragged_gemm_swap_kernel" in name for name in names) == swapped, names
+    ref = fn(x, w, gs, cfg=_lib.TileCfg(256, 0, 1, 128, 0))
+    assert float((got.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
+    assert float(got[m - 3:].float().abs().max()) == 0.0
