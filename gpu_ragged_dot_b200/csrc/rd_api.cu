@@ -525,18 +525,18 @@ bool swap_takes_less(long long m, int k_blocks, int n, int g, int least, double 
   return rounds * (4.0 * height * k_blocks + 5000.0) * margin < (rounds128 > 1.0 ? rounds128 : 1.0) * 560.0 * k_blocks;
 }
 
-// Should a gmm put its rows on the N side of the MMAs (rd_gemm_swap.cuh)?  When groups are long, there
-// are at least three rounds of tiles for the pairs and the last 512-column tile is nearly full.
-// Microseconds, one-CTA tiles (better of the two heights) against swapped: m 8192, k 4096, n 14336, 8
-// groups 694 -> 687, trans_rhs with k 14336, n 4096 687 -> 669 (alone; in a row with the backward pass
-// 2.58 -> 2.48 ms a step); 13304, 2824, 11264, 16 804 -> 683; 28320, 5656, 1536, 32 605 -> 523; 64 groups of 512, k
-// 4096, n 1536 402 -> 384.  Below: 4096, 4096, 4096, 8 (1.7 rounds) 177 -> 212; n 2304 (last tile half full)
-// 160 -> 171; 256 rows per group 288 -> 273 at best, 1058 -> 1160 at worst; 128 rows 222 -> 233.
+// Should a gmm put its rows on the N side of the MMAs (rd_gemm_swap.cuh)?  Where swap_takes_less says so; and when groups are
+// long, there are at least three rounds of tiles for the pairs and the last 512-column tile is nearly full.
+// Microseconds in a row, one-CTA tiles (better of the two heights) against swapped: m 8192, k 4096, n 14336, 8
+// groups 726 -> 659, trans_rhs with k 14336, n 4096 723 -> 703; 13304, 2824, 11264, 16 685 -> 627; 28320, 5656, 1536, 32
+// 430 -> 410; 64 groups of 512, k 4096, n 1536, fp16 339 -> 333; e4m3 8192, 4096, 14336, 8 397 -> 370.  Not there: 4096, 4096, 4096, 8 (1.7
+// rounds) 107 -> 109 with equal groups, 120 -> 126 with unequal ones; 8192, 4096, 2304, 8 (last tile half full, equal groups) 107 -> 134.
 // A short contraction (fewer than nine 64-deep blocks) leaves the drain of both accumulators exposed once per
-// tile: 4928, 264, 7232, 4 40 -> 50, 22000, 512, 4032, 12 112 -> 120; 16 bits win again from twenty rounds on (17184, 456,
-// 13568, 32 288 -> 255), e4m3 does not (25960, 448, 4928, 24 112 -> 124).
+// tile: 4928, 264, 7232, 4 29 -> 33, 22000, 512, 4032, 12 90 -> 86 with equal groups, 95 -> 97 with unequal ones; 16 bits win again
+// from twenty rounds on (17184, 456, 13568, 32 272 -> 247), e4m3 does not (25960, 448, 4928, 24 96 -> 97, unequal 105 -> 111).
 // e4m3 (128-row tiles otherwise) with few rounds: they are compared, a swapped tile taking 1.7 times as long
-// as a 128-row one; 8192, 14336, 4096, 16 (5 against 8) 422 -> 433, in a row 425 -> 453.
+// as a 128-row one.  (That was fitted to a slower swapped kernel: 8192, 14336, 4096, 16, five rounds against eight, is refused and would
+// take 357 instead of 392, with unequal groups 422 instead of 437.)
 bool choose_swap(long long m, int k_blocks, int n, int g, bool trans_rhs, bool fp8) {
   if (g <= 0 || (!trans_rhs && n % 64 != 0)) return false;
   if (swap_takes_less(m, k_blocks, n, g, fp8 ? 128 : 384, fp8 ? 1.2 : 1.0)) return true;
@@ -647,14 +647,14 @@ bool split_allowed(const rd_tile_cfg* cfg) {
 // They pay off when a tile's second half usually exists: tgmm with k >= 256, and gmm when the
 // groups are long (a half without rows is skipped, so the cost of a wrong guess is only a
 // shallower smem ring) -- unless the larger tiles fill the SMs badly.
-// 512 rows per group and more: always from three rounds of 256-row tiles on (128 rows against 256, microseconds, m,
-// k, n, groups: 6120, 6528, 3304, 8 390 -> 319; 8304, 1768, 5112, 16 198 -> 173; 28448, 952, 576, 16 75 -> 69; 24104, 304, 2560, 6
-// 75 -> 68).  Below, the rounds are compared, a 256-row tile taking 1.5 times as long as a 128-row one: 4096, 4096,
-// 4096, 8 (4 rounds against 3) 177 -> 210; 512, 4096, 4096, 1 (1 against 1) 36 -> 52; but 6000, 4096, 1024, 8 (2 against 1)
-// 77 -> 70; 4352, 2928, 2232, 2 (3 against 2) 103 -> 93; 7184, 448, 2296, 8 (4 against 2) 38 -> 32.
+// 512 rows per group and more: always from three rounds of 256-row tiles on (128 rows against 256, microseconds in a row, m,
+// k, n, groups: 6120, 6528, 3304, 8 279 -> 237; 8304, 1768, 5112, 16 229 -> 182; equal on narrow outputs, 28448, 952, 576, 16 43 -> 45;
+// 24104, 304, 2560, 6 50 -> 51).  Below, the rounds are compared, a 256-row tile taking 1.5 times as long as a 128-row one: 4096,
+// 4096, 4096, 8 (4 rounds against 3, unequal groups) 120 -> 152; 512, 4096, 4096, 1 (1 against 1) 24 -> 42; but 6000, 4096, 1024, 8
+// (2 against 1) 57 -> 50; 4352, 2928, 2232, 2 (3 against 2) 78 -> 70; 7184, 448, 2296, 8 (4 against 2) 24.7 -> 20.5.
 // 256 to 511 rows: only where 256-row tiles need fewer rounds even with a tile more per group than m asks for and
-// no tile more for 128 rows; 2048, 7168, 2048, 8 would take 2 rounds against 1 with unequal groups (116 -> 101) but
-// 1 against 1 with equal ones (74 -> 91), and 6352, 968, 896, 24 loses (30 -> 40).
+// no tile more for 128 rows; 2048, 7168, 2048, 8 would take 2 rounds against 1 with unequal groups (90 -> 80) but
+// 1 against 1 with equal ones (59 -> 92), and 6352, 968, 896, 24 loses (20 -> 30).
 // e4m3, whose MMAs take half as long: 1.7 times, always from six rounds on, never with fewer than nine blocks of
 // the contraction (m 8192, k 4096, n 14336, 8 groups 390 -> 378; but 8192, 14336, 4096, 16, five rounds against
 // eight, 422 -> 472; 31480, 640, 1088, 32, five blocks, 46 -> 48).

@@ -374,7 +374,7 @@ __device__ __forceinline__ void clear_tail_rows(uint32_t stage_addr, int live, i
 }
 
 // The fields of a tile that the producer and the MMA warp use, as values every lane (and the compiler) knows to be
-// the same: loops on them run in uniform registers, which TMA and tcgen05 instructions read (rd_tgmm.cuh).
+// the same: stages of loops on them are issued faster (rd_tgmm.cuh).
 __device__ __forceinline__ TileCoord uniform_coord(TileCoord t) {
   t.group = __shfl_sync(0xffffffffu, t.group, 0);
   t.weight = __shfl_sync(0xffffffffu, t.weight, 0);

@@ -232,7 +232,7 @@ ragged_gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const int k_blocks = (p.k + kDeep - 1) / kDeep;
 
   // The producer and the MMA warp run their loops as whole warps on values that the compiler knows to be uniform
-  // and elect a lane for the TMA and tcgen05 instructions alone, which take uniform registers (rd_tgmm.cuh).
+  // and elect a lane for the TMA and tcgen05 instructions alone (rd_tgmm.cuh).
   auto uniform_tile = [&](int tile) {
     SwapTile t = decode_swap_tile<kStep>(p, &group_table, work, tile);
     t.weight = __shfl_sync(0xffffffffu, t.weight, 0);

@@ -7,11 +7,10 @@
 // that stood here before moved less per flop but left the drain exposed, 5000 clocks per tile.
 //
 // What made the smaller tiles fast enough is the issue path.  A 64-row stage takes 512 clocks of MMAs here.
-// With producer and MMA loops run by one thread (lane == 0) the compiler keeps their values in ordinary
-// registers and moves every descriptor, coordinate and barrier address to the uniform registers that
-// TMA and tcgen05 instructions read: 420 clocks to issue a stage's four MMAs and commit, and 395 for two boxes
-// of loads, beside the waits.  Run by a whole warp on values known to be uniform, with a lane elected for the
-// instructions alone, they take 240 and 290 (the same kernel: m 8192, k 4096, n 14336, 8 groups 938 -> 722 us).
+// With producer and MMA loops run by one thread (lane == 0) a stage's four MMAs and commit take 420 clocks to issue, and
+// its two boxes of loads 395, beside the waits (clock64 around them).  Run by a whole warp on values that the compiler knows to
+// be the same in every lane, with a lane elected for the instructions alone, they take 240 and 290 (the same kernel: m 8192,
+// k 4096, n 14336, 8 groups 938 -> 722 us).
 // The order of tiles is walked without divisions (TgmmWalk), which had taken 650 clocks a tile.
 //
 // Rows past a group's end in its last stage are cleared by a fixer warp as soon as the stage has landed,
@@ -176,7 +175,7 @@ ragged_tgmm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const int tile_step = static_cast<int>(gridDim.x) / kCtas;
   using Walk = TgmmWalk<kTileM * kCtas>;
   // The producer and the MMA warp run their loops as whole warps whose values the compiler knows to be
-  // uniform, and elect a lane for each stage's instructions: these take uniform registers.
+  // uniform, and elect a lane for each stage's instructions alone (see above).
   auto uniform_coord = [&](const Walk& w) {
     TgmmTile t = w.coord(p, &group_table);
     t.row0 = __shfl_sync(0xffffffffu, t.row0, 0);
