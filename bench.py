@@ -36,15 +36,15 @@ if ROOT not in sys.path:
 
 
 
-def dram_traffic_per_launch():
-    """dram__bytes_read.sum + dram__bytes_write.sum of one launch of each kernel on the Mixtral
-    workload, from the profiler capture whose figures are kept in a small JSON file beside its
-    summary; None for a kernel that file does not list."""
+def captured_launches():
+    """Per product of the bf16 Mixtral workload, from the profiler captures whose figures are kept in a small JSON file
+    beside their summaries: the kernel's name and dram__bytes_read.sum + dram__bytes_write.sum of one launch."""
     path = os.path.join(ROOT, "profiles", "ragged_gemm_mixtral_dram_traffic.json")
     try:
         with open(path) as f:
             d = json.load(f)
-        return {k: float(v["dram_read_bytes"]) + float(v["dram_write_bytes"]) for k, v in d["kernels"].items()}
+        return {k: (v["kernel"], float(v["dram_read_bytes"]) + float(v["dram_write_bytes"]))
+                for k, v in d["kernels"].items()}
     except Exception:
         return {}
 
@@ -443,7 +443,9 @@ def run_single(args):
         tf = gemm_flops / (ms * 1e-3) / 1e12
         per_kernel[name] = {"ms": ms, "tflops": tf, "frac_of_measured_burst": tf / peaks["bf16_tflops"],
                             "frac_of_measured_sustained": tf / peaks["bf16_tflops_sustained"]}
-    traffic = dram_traffic_per_launch() if args.workload == "mixtral" else {}
+    captured = captured_launches() if args.workload == "mixtral" and args.dtype == "bf16" else {}
+    kernel, traffic = captured.get(dom, ({"fwd": "gmm", "dlhs": "gmm, trans_rhs", "drhs": "tgmm"}[dom]
+                                         + ": the kernel that the rules of rd_api.cu pick", None))
     gplus_f, gplus_b = int((gs_fwd_np > 0).sum()), int((gs_bwd_np > 0).sum())
     alg_bytes = {
         "fwd": (1.0 * (shape.m * shape.k + gplus_f * shape.k * shape.n) + 2.0 * shape.m * shape.n) if fp8 else
@@ -459,8 +461,7 @@ def run_single(args):
     if hbm_bound:
         roofline = {
             "bound": "hbm",
-            "kernel": {"fwd": "ragged_gemm(2)_kernel<gmm>", "dlhs": "ragged_gemm(2)_kernel<gmm, trans_rhs>",
-                       "drhs": "ragged_gemm2_kernel<tgmm>"}[dom],
+            "kernel": kernel,
             "achieved": per_kernel[dom]["algorithmic_GBps"], "peak": peaks["hbm_gbs"],
             "peak_source": f"{peaks['source']} (copy bandwidth)", "unit": "GB/s",
             "frac": per_kernel[dom]["frac_of_measured_hbm"], "traffic": None,
@@ -470,15 +471,14 @@ def run_single(args):
     else:
         roofline = {
             "bound": "tensor",
-            "kernel": {"fwd": "ragged_gemm2_kernel<gmm>", "dlhs": "ragged_gemm2_kernel<gmm, trans_rhs>",
-                       "drhs": "ragged_gemm2_kernel<tgmm>"}[dom],
+            "kernel": kernel,
             "achieved": per_kernel[dom]["tflops"],
             "peak": peaks["bf16_tflops"],
             "peak_source": f"{peaks['source']} (burst cuBLAS bf16); sustained {peaks['bf16_tflops_sustained']}",
             "unit": "TFLOP/s",
             "frac": per_kernel[dom]["tflops"] / peaks["bf16_tflops"],
             "frac_of_sustained": per_kernel[dom]["tflops"] / peaks["bf16_tflops_sustained"],
-            "traffic": traffic.get(dom),
+            "traffic": traffic,
             "algorithmic_flops_per_launch": gemm_flops,
             "algorithmic_bytes_per_launch": alg_bytes[dom],
             "per_kernel": per_kernel,
