@@ -419,9 +419,9 @@ constexpr int stage_bytes() {
 // kOneThread (tgmm): producer and MMA loops run by one thread each, and nothing in the kernel knows its warp to be
 // uniform, instead of a whole warp that elects a lane.  Slower to issue, and where an output of more than some 36 rounds of tiles
 // has rows that begin inside a sector (n % 16 == 8) that is what keeps the CTAs that write either side of a column tile's edge
-// abreast.  128 heavy-tailed groups of 42 rows, k 4096, microseconds in a row, whole warps against one thread: n 1224 344 -> 318,
-// 1592 464 -> 416, 1720 514 -> 422, 2040 609 -> 514; 494, 6600, 1176, 136 597 -> 448; 108, 2624, 4584, 68 444 -> 323.  Fewer rounds
-// the other way: 171, 1880, 768, 3 (one) 6.7 -> 6.1.  Choice: tgmm_way in rd_api.cu.
+// abreast.  128 heavy-tailed groups of 42 rows, k 4096, microseconds in a row, whole warps against one thread: n 1224 350 -> 313,
+// 1592 457 -> 411, 1720 528 -> 453, 2040 614 -> 518; 494, 6600, 1176, 136 592 -> 450; 108, 2624, 4584, 68 444 -> 362.  Fewer rounds
+// the other way: 171, 1880, 768, 3 (one) 6.3 against 6.9.  Choice: tgmm_way in rd_api.cu.
 template <int BN, bool kBKMajor, int kStages, bool kTgmm, int kCtas, bool kSeg = false, bool kFp8 = false,
           bool kUnaligned = false, bool kOneThread = false>
 __global__ void __launch_bounds__(kGemmFixerThreads, 1)
