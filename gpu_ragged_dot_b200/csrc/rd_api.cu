@@ -703,34 +703,43 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 // - Groups of 512 rows and more: pairs, up to a quarter more rounds (m 8192, k 4096, n 14336, 8 groups 908 -> 722); of 256 rows up to
 //   three rounds only with no more of them (2683, 472, 2600, 6 26.6 -> 23.1; three against two, 4150, 544, 1152, 10 16.4 -> 18.4).
 // - Groups of 64 to 255 rows: pairs likewise, but from seven rounds on (9101, 4496, 1944, 37 307 -> 248; 672, 7288, 11816, 4 257 ->
-//   232); up to six the plain kernel (7474, 376, 1280, 44 27.1 against 28.6; 579, 320, 8192, 3 10.7 against 14.3).
+//   232); up to six the plain kernel (7474, 376, 1280, 44 27.1 against 28.6; 579, 320, 8192, 3 10.7 against 14.3).  Up to 100 rows, more
+//   than 36 rounds and rows that begin inside a sector: as below 64 rows (16612, 4216, 1576, 174 715 plain, pair 897; 4108, 11704, 424,
+//   52 turned 160, 211).
 // - Groups of less than 64 rows: up to three rounds the plain kernel, then by the output's rows.  Whole 256 bytes: two accumulators
 //   (1085, 520, 2048, 67 33.2 plain, 29.2).  Other rows: a column tile's edge falls inside 256 bytes (or a sector) of every other
 //   row, and what counts is that the CTAs that write either side of it stay side by side.  Whole sectors: two accumulators with the
 //   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
-//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where the columns of up to twelve tiles are unequal and a
-//   CTA's step, `ctas` tiles, shares a factor with them (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1800
-//   724, 696, 528); otherwise the plain kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37
-//   rounds on (kOneThread, rd_gemm.cuh).
+//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where columns are unequal and a CTA's step, `ctas` tiles,
+//   shares a factor with the tiles of a row (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1800 724, 696,
+//   528), up to twelve of them or up to sixteen tiles of rows (320 deep, 40 tiles 78 plain, 74; but 13272 deep, 22 tiles 101, 118);
+//   otherwise the plain kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on
+//   (kOneThread, rd_gemm.cuh).
+// - Few columns (n 296: 512 are multiplied by the plain kernel, 320 here, dealt evenly): two accumulators or pairs from four rounds on,
+//   whatever the rows up to 36 (1796, 5480, 304, 10 24.6 plain, 20.6; groups below 64 rows 1.07 to 1.4 times as fast; but with 140
+//   rounds 67, 11464, 520, 77 one thread 205, turned 241).
 enum class TgmmWay { kPair, kPlain, kOneThread, kTwoAcc, kTurned };
 TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
   const long long rows = m / g, tiles = (static_cast<long long>(n) + 255) / 256, blocks = (static_cast<long long>(n) + 63) / 64;
   const long long r1 = ((k + 127) / 128 * tiles * g + ctas - 1) / ctas;
+  const bool narrow = 40 * tiles >= 13 * blocks;  // tiles of 256 columns are 1.3 times the columns there are
+  const bool split = n % 16 != 0 && rows <= 100 && r1 > 36;  // sectors in two parts, more output than L2 holds
   if (cta_group == 2) return TgmmWay::kPair;
   if (cta_group == 0) {
     const long long pairs = sm_count() / 2, r2 = ((k + 255) / 256 * tiles * g + pairs - 1) / pairs;
     if (r1 <= 1) {
       if (rows >= 768 && r2 <= 1) return TgmmWay::kPair;
-    } else if (rows >= 512 || (rows >= 256 && r1 > 3) || (rows >= 64 && r1 > 6)) {
+    } else if (rows >= 512 || (rows >= 256 && r1 > 3) || (rows >= 64 && r1 > (narrow ? 3 : 6) && !split)) {
       if (4 * r2 <= 5 * r1) return TgmmWay::kPair;
     } else if (rows >= 256) {
       if (r2 <= r1) return TgmmWay::kPair;
     }
   }
-  if (r1 <= 3 || rows >= 64) return TgmmWay::kPlain;
+  if (r1 <= 3 || (rows >= 64 && !narrow && !split)) return TgmmWay::kPlain;
   if (n % 128 == 0 || tiles == 1) return TgmmWay::kTwoAcc;
-  if (n % 16 == 0) return TgmmWay::kTurned;
-  if (tiles <= 12 && blocks != 4 * tiles && std::gcd(tiles, static_cast<long long>(ctas)) > 1) return TgmmWay::kTurned;
+  if (n % 16 == 0 || (narrow && r1 <= 36)) return TgmmWay::kTurned;
+  if ((tiles <= 12 || k <= 2048) && blocks != 4 * tiles && std::gcd(tiles, static_cast<long long>(ctas)) > 1)
+    return TgmmWay::kTurned;
   return r1 > 36 ? TgmmWay::kOneThread : TgmmWay::kPlain;
 }
 

@@ -1583,6 +1583,17 @@ def test_tgmm_rows_that_split_sectors(n, tile):
     (620, 520, 3072, 10, "ragged_tgmm_kernel<1>"),    # of 62, five rounds
     (640, 520, 3072, 10, "ragged_gemm_kernel<256"),   # of 64
     (700, 4104, 4096, 1, "ragged_tgmm_kernel<2>"),    # one group, four against four
+    (6800, 2048, 1160, 68, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # of 100, 37 rounds
+    (6868, 2048, 1160, 68, "ragged_tgmm_kernel<2>"),  # of 101
+    (6800, 2048, 1168, 68, "ragged_tgmm_kernel<2>"),  # rows of whole sectors
+    (1600, 1032, 296, 30, "ragged_tgmm_kernel<1>"),   # few columns, four rounds, groups of 53
+    (2400, 1032, 296, 30, "ragged_tgmm_kernel<2>"),   # of 80
+    (100, 1032, 520, 30, "ragged_tgmm_kernel<1>"),    # three tiles, no factor shared, six rounds
+    (100, 2048, 520, 112, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 37
+    (2400, 1032, 424, 30, "ragged_gemm_kernel<256"),  # more columns
+    (300, 2048, 3592, 24, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 15 tiles: no factor shared
+    (300, 2048, 3464, 26, "ragged_tgmm_kernel<1>"),   # 14 tiles, unequal
+    (300, 2056, 3464, 26, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # one row tile more
     (300, 2048, 1160, 66, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, false>"),  # 36 rounds
     (300, 2048, 1160, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # a round more
     (300, 2048, 1176, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # five tiles still
