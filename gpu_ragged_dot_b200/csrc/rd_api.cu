@@ -266,9 +266,8 @@ int launch_kernel(void (*kernel)(Params...), int ctas, int threads, size_t smem_
 // 384, 64 109 -> 115; 2000, 3000, 1024, 64 (393 MB) 82 -> 86.  (Short contractions would gain: float32 2000, 1024, 1024, 64 54 ->
 // 52.)  On pairs, which take such weights for three float32 products only, it does no harm: 2000, 768, 1024, 64 121 -> 119,
 // 1536, 2048 429 -> 427.
-// tgmm on 256 columns: two tiles per CTA (`rounds`); there the launch is a good part of the time as well, 20 sizes of two
-// rounds 1.25 times as fast below 256 rows per group, 1.15 below 768, 1.05 above (128 CTAs' worth of such tiles is one
-// round of tiles twice as tall).
+// tgmm on 256 columns, whose tiles are a few stages each: up to two tiles per CTA (`rounds`).  82 sizes of one to two rounds: 1.25
+// times as fast below 256 rows per group, 1.15 below 768, 1.05 above.
 bool launch_early(const GemmArgs& args, int ctas_per_tile = 1, bool wide_k_major = false, int rounds = 1) {
   if (!args.inline_groups) return false;
   const long long row_tiles = args.k_tiles > 0 ? static_cast<long long>(args.g) * args.k_tiles
@@ -696,7 +695,7 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 
 // tgmm with 256-column tiles: which kernel?  By rounds of tiles (128 x 256 on one CTA, 256 x 256 on a pair) and the mean rows of
 // a group.  Timed all five ways on 640 sizes (16 to 32768 rows per call, 1 to 256 groups, equal to heavy-tailed) the choice takes
-// 1.5 % longer than the best of them on average.  Microseconds in a row, sizes m, k, n, groups:
+// 1.1 % longer than the best of them on average.  Microseconds in a row, sizes m, k, n, groups:
 // - One round: the plain 128-row kernel (rd_gemm.cuh), which starts sooner and has a stage more (171, 1880, 768, 3 6.3 against 7.5 on two
 //   accumulators; 260, 1056, 3432, 1 7.7 against 9.2); from 768 rows per group on the MMAs count, and a pair moves a third less
 //   data (2077, 344, 880, 1 19.8 -> 17.6; 9424, 640, 360, 2 37 -> 27; just above equal: 884, 4408, 536, 1 13.4 -> 12.8).
@@ -712,7 +711,7 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 //   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
 //   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where columns are unequal and a CTA's step, `ctas` tiles,
 //   shares a factor with the tiles of a row (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1800 724, 696,
-//   528), up to twelve of them or up to sixteen tiles of rows (320 deep, 40 tiles 78 plain, 74; but 13272 deep, 22 tiles 101, 118);
+//   528), up to twelve of them or up to sixteen tiles of rows (320 deep, 40 tiles 73 plain, 69; but 13272 deep, 22 tiles 101, 118);
 //   otherwise the plain kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on
 //   (kOneThread, rd_gemm.cuh).
 // - Few columns (n 296: 512 are multiplied by the plain kernel, 320 here, dealt evenly): two accumulators or pairs from four rounds on,
