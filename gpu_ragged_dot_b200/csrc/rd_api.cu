@@ -709,11 +709,12 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 //   (1085, 520, 2048, 67 33.2 plain, 29.2).  Other rows: a column tile's edge falls inside 256 bytes (or a sector) of every other
 //   row, and what counts is that the CTAs that write either side of it stay side by side.  Whole sectors: two accumulators with the
 //   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
-//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where columns are unequal and a CTA's step, `ctas` tiles,
-//   shares a factor with the tiles of a row (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1800 724, 696,
-//   528), up to twelve of them or up to sixteen tiles of rows (320 deep, 40 tiles 73 plain, 69; but 13272 deep, 22 tiles 101, 118);
-//   otherwise the plain kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on
-//   (kOneThread, rd_gemm.cuh).
+//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where a CTA's step, `ctas` tiles, shares a factor with
+//   the tiles of a row and the plain kernel's last tile pads every row: by a thirty-second or more (128 groups of 42, k 4096, n 776
+//   290 plain, 323, 195; 1288 551, 485, 362), or up to five tiles of rows (527, 280, 8984, 31 47 plain, 42), or from 160 rounds on
+//   (682, 9936, 3896, 48 1353 plain, 1159; but in fewer rounds 754, 4160, 10520, 13 one thread 270, 333).  Otherwise the plain kernel,
+//   whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on (kOneThread, rd_gemm.cuh; no padding: 396,
+//   4928, 2504, 66 turned 467, 324).  On 628 sizes the better of the two within 1 % on average.
 // - Few columns (n 296: 512 are multiplied by the plain kernel, 320 here, dealt evenly): two accumulators or pairs from four rounds on,
 //   whatever the rows up to 36 (1796, 5480, 304, 10 24.6 plain, 20.6; groups below 64 rows 1.07 to 1.4 times as fast; but with 140
 //   rounds 67, 11464, 520, 77 one thread 205, turned 241).
@@ -737,7 +738,8 @@ TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
   if (r1 <= 3 || (rows >= 64 && !narrow && !split)) return TgmmWay::kPlain;
   if (n % 128 == 0 || tiles == 1) return TgmmWay::kTwoAcc;
   if (n % 16 == 0 || (narrow && r1 <= 36)) return TgmmWay::kTurned;
-  if ((tiles <= 12 || k <= 2048) && blocks != 4 * tiles && std::gcd(tiles, static_cast<long long>(ctas)) > 1)
+  const long long padding = 4 * tiles - blocks;  // of 4 * tiles
+  if (padding > 0 && (8 * padding >= tiles || r1 >= 160 || k <= 640) && std::gcd(tiles, static_cast<long long>(ctas)) > 1)
     return TgmmWay::kTurned;
   return r1 > 36 ? TgmmWay::kOneThread : TgmmWay::kPlain;
 }

@@ -1592,8 +1592,12 @@ def test_tgmm_rows_that_split_sectors(n, tile):
     (100, 2048, 520, 112, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 37
     (2400, 1032, 424, 30, "ragged_gemm_kernel<256"),  # more columns
     (300, 2048, 3592, 24, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 15 tiles: no factor shared
-    (300, 2048, 3464, 26, "ragged_tgmm_kernel<1>"),   # 14 tiles, unequal
-    (300, 2056, 3464, 26, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # one row tile more
+    (300, 2048, 3400, 26, "ragged_tgmm_kernel<1>"),   # 14 tiles, two of 56 blocks padding
+    (300, 2048, 3464, 26, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # one
+    (300, 648, 2440, 393, "ragged_tgmm_kernel<1>"),   # one of 40, 160 rounds
+    (300, 648, 2440, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 159
+    (300, 640, 2440, 392, "ragged_tgmm_kernel<1>"),   # five row tiles
+    (300, 640, 2504, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # no padding
     (300, 2048, 1160, 66, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, false>"),  # 36 rounds
     (300, 2048, 1160, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # a round more
     (300, 2048, 1176, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # five tiles still
@@ -1602,7 +1606,7 @@ def test_tgmm_rows_that_split_sectors(n, tile):
 def test_tgmm_one_cta_or_pair(m, k, n, g, kernel):
     """Sizes on either side of the rule that picks a kernel from rounds of tiles, rows per group and the output's rows: what
     it takes, and the bits of the kernel with 128-column tiles, whatever the choice."""
-    x, _, dout = _inputs(17, m, k, n, g)
+    x, _, dout = _inputs(17, m, k, n, 1)
     gs = torch.from_numpy(oracle.reference_group_sizes(5, g, m - 3))
     xd, dd, gd = _to_dev(x, dout, gs)
     out, names = launched.kernels(lambda: ops.tgmm_forward(xd, dd, gd, cfg=_lib.TileCfg(0, 0, 0, 0, 0)))
