@@ -716,8 +716,9 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 //   whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on (kOneThread, rd_gemm.cuh; no padding: 396,
 //   4928, 2504, 66 turned 467, 324).  On 628 sizes the better of the two within 1 % on average.
 // - Few columns (n 296: 512 are multiplied by the plain kernel, 320 here, dealt evenly): two accumulators or pairs from four rounds on,
-//   whatever the rows up to 36 (1796, 5480, 304, 10 24.6 plain, 20.6; groups below 64 rows 1.07 to 1.4 times as fast; but with 140
-//   rounds 67, 11464, 520, 77 one thread 205, turned 241).
+//   with less than 64 rows from three (90, 11464, 312, 2 9.9 plain, 8.5; two rounds equal), whatever the output's rows up to 36 rounds
+//   (1796, 5480, 304, 10 24.6 plain, 20.6; groups below 64 rows 1.07 to 1.4 times as fast; but with 140 rounds 67, 11464, 520, 77 one
+//   thread 205, turned 241).
 enum class TgmmWay { kPair, kPlain, kOneThread, kTwoAcc, kTurned };
 TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
   const long long rows = m / g, tiles = (static_cast<long long>(n) + 255) / 256, blocks = (static_cast<long long>(n) + 63) / 64;
@@ -735,7 +736,7 @@ TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
       if (r2 <= r1) return TgmmWay::kPair;
     }
   }
-  if (r1 <= 3 || (rows >= 64 && !narrow && !split)) return TgmmWay::kPlain;
+  if (r1 <= (narrow && rows < 64 ? 2 : 3) || (rows >= 64 && !narrow && !split)) return TgmmWay::kPlain;
   if (n % 128 == 0 || tiles == 1) return TgmmWay::kTwoAcc;
   if (n % 16 == 0 || (narrow && r1 <= 36)) return TgmmWay::kTurned;
   const long long padding = 4 * tiles - blocks;  // of 4 * tiles

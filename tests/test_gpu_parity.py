@@ -1587,6 +1587,10 @@ def test_tgmm_rows_that_split_sectors(n, tile):
     (6868, 2048, 1160, 68, "ragged_tgmm_kernel<2>"),  # of 101
     (6800, 2048, 1168, 68, "ragged_tgmm_kernel<2>"),  # rows of whole sectors
     (1600, 1032, 296, 30, "ragged_tgmm_kernel<1>"),   # few columns, four rounds, groups of 53
+    (1000, 1016, 296, 20, "ragged_tgmm_kernel<1>"),   # three rounds, of 50
+    (1280, 1016, 296, 20, "ragged_gemm_kernel<256"),  # of 64
+    (1000, 896, 296, 20, "ragged_gemm_kernel<256"),   # two rounds
+    (1000, 1016, 424, 20, "ragged_gemm_kernel<256"),  # more columns
     (2400, 1032, 296, 30, "ragged_tgmm_kernel<2>"),   # of 80
     (100, 1032, 520, 30, "ragged_tgmm_kernel<1>"),    # three tiles, no factor shared, six rounds
     (100, 2048, 520, 112, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 37
