@@ -709,7 +709,9 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 //   (1085, 520, 2048, 67 33.2 plain, 29.2).  Other rows: a column tile's edge falls inside 256 bytes (or a sector) of every other
 //   row, and what counts is that the CTAs that write either side of it stay side by side.  Whole sectors: two accumulators with the
 //   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
-//   68, turned 61).  Rows that begin inside a sector (n % 16 == 8): the same where a CTA's step, `ctas` tiles, shares a factor with
+//   68, turned 61); but the plain kernel with fewer rows than groups, tiles of which no CTA meets the same columns anyway and more than
+//   63 rounds, nearly all of them zeros (18, 5912, 3680, 42 288 plain, turned 349; 25 such sizes 0.90, up to 63 rounds 1.08 times as
+//   fast turned).  Rows that begin inside a sector (n % 16 == 8): the same where a CTA's step, `ctas` tiles, shares a factor with
 //   the tiles of a row and the plain kernel's last tile pads every row: by a thirty-second or more (128 groups of 42, k 4096, n 776
 //   290 plain, 323, 195; 1288 551, 485, 362), or up to five tiles of rows (527, 280, 8984, 31 47 plain, 42), or from 160 rounds on
 //   (682, 9936, 3896, 48 1353 plain, 1159; but in fewer rounds 754, 4160, 10520, 13 one thread 270, 333).  Otherwise the plain kernel,
@@ -738,10 +740,11 @@ TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
   }
   if (r1 <= (narrow && rows < 64 ? 2 : 3) || (rows >= 64 && !narrow && !split)) return TgmmWay::kPlain;
   if (n % 128 == 0 || tiles == 1) return TgmmWay::kTwoAcc;
+  const bool shared = std::gcd(tiles, static_cast<long long>(ctas)) > 1;
+  if (n % 16 == 0 && rows == 0 && r1 > 63 && !shared && !narrow) return TgmmWay::kPlain;
   if (n % 16 == 0 || (narrow && r1 <= 36)) return TgmmWay::kTurned;
   const long long padding = 4 * tiles - blocks;  // of 4 * tiles
-  if (padding > 0 && (8 * padding >= tiles || r1 >= 160 || k <= 640) && std::gcd(tiles, static_cast<long long>(ctas)) > 1)
-    return TgmmWay::kTurned;
+  if (padding > 0 && (8 * padding >= tiles || r1 >= 160 || k <= 640) && shared) return TgmmWay::kTurned;
   return r1 > 36 ? TgmmWay::kOneThread : TgmmWay::kPlain;
 }
 
