@@ -711,12 +711,13 @@ bool choose_f32_pair(bool tgmm, long long m, int k, int n, int g, int bn, const 
 //   order of columns turned by a place per row, so that no CTA meets the same columns again and again (115, 2248, 912, 93 73 plain,
 //   68, turned 61); but the plain kernel with fewer rows than groups, tiles of which no CTA meets the same columns anyway and more than
 //   63 rounds, nearly all of them zeros (18, 5912, 3680, 42 288 plain, turned 349; 25 such sizes 0.90, up to 63 rounds 1.08 times as
-//   fast turned).  Rows that begin inside a sector (n % 16 == 8): the same where a CTA's step, `ctas` tiles, shares a factor with
-//   the tiles of a row and the plain kernel's last tile pads every row: by a thirty-second or more (128 groups of 42, k 4096, n 776
-//   290 plain, 323, 195; 1288 551, 485, 362), or up to five tiles of rows (527, 280, 8984, 31 47 plain, 42), or from 160 rounds on
-//   (682, 9936, 3896, 48 1353 plain, 1159; but in fewer rounds 754, 4160, 10520, 13 one thread 270, 333).  Otherwise the plain kernel,
-//   whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on (kOneThread, rd_gemm.cuh; no padding: 396,
-//   4928, 2504, 66 turned 467, 324).  On 628 sizes the better of the two within 1 % on average.
+//   fast turned).  Rows that begin inside a sector (n % 16 == 8): the same where a CTA's step, `ctas`
+//   tiles, shares a factor with the tiles of a row and the plain kernel's last tile, less to write than the others, always falls to the
+//   same CTAs: where it pads a thirty-second of the row (128 groups of 42, k 4096, n 776 290 plain, 323, 195; 1288 551, 485, 362; 1104,
+//   14168, 984, 92 one thread 831, 692), or a block of 64 with up to five tiles of rows (527, 280, 8984, 31 47 plain, 42) or from 160
+//   rounds on (585, 3416, 9048, 65 one thread 1315, 1238; but in fewer rounds 280, 2688, 9320, 20 223, 268).  Otherwise the plain
+//   kernel, whose CTAs write one tile at a time, its loops issued by one thread from 37 rounds on (kOneThread, rd_gemm.cuh; no padding:
+//   396, 4928, 2504, 66 turned 467, 324).  On 775 sizes the better of the two within 1 % on average.
 // - Few columns (n 296: 512 are multiplied by the plain kernel, 320 here, dealt evenly): two accumulators or pairs from four rounds on,
 //   with less than 64 rows from three (90, 11464, 312, 2 9.9 plain, 8.5; two rounds equal), whatever the output's rows up to 36 rounds
 //   (1796, 5480, 304, 10 24.6 plain, 20.6; groups below 64 rows 1.07 to 1.4 times as fast; but with 140 rounds 67, 11464, 520, 77 one
@@ -743,8 +744,8 @@ TgmmWay tgmm_way(long long m, int k, int n, int g, int ctas, int cta_group) {
   const bool shared = std::gcd(tiles, static_cast<long long>(ctas)) > 1;
   if (n % 16 == 0 && rows == 0 && r1 > 63 && !shared && !narrow) return TgmmWay::kPlain;
   if (n % 16 == 0 || (narrow && r1 <= 36)) return TgmmWay::kTurned;
-  const long long padding = 4 * tiles - blocks;  // of 4 * tiles
-  if (padding > 0 && (8 * padding >= tiles || r1 >= 160 || k <= 640) && shared) return TgmmWay::kTurned;
+  const long long padding = 256 * tiles - n;
+  if (shared && (padding >= 8 * tiles || (padding >= 64 && (r1 >= 160 || k <= 640)))) return TgmmWay::kTurned;
   return r1 > 36 ? TgmmWay::kOneThread : TgmmWay::kPlain;
 }
 

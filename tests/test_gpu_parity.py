@@ -1596,16 +1596,16 @@ def test_tgmm_rows_that_split_sectors(n, tile):
     (100, 2048, 520, 112, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 37
     (2400, 1032, 424, 30, "ragged_gemm_kernel<256"),  # more columns
     (300, 2048, 3592, 24, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 15 tiles: no factor shared
-    (300, 2048, 3400, 26, "ragged_tgmm_kernel<1>"),   # 14 tiles, two of 56 blocks padding
-    (300, 2048, 3464, 26, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # one
+    (300, 2048, 3464, 26, "ragged_tgmm_kernel<1>"),   # 14 tiles, a thirty-second of 3584 columns padding
+    (300, 2048, 3480, 26, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # less
     (100, 1016, 1168, 234, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, false>"),  # no rows to speak of, 64 rounds
     (100, 1016, 1168, 233, "ragged_tgmm_kernel<1>"),  # 63
     (234, 1016, 1168, 234, "ragged_tgmm_kernel<1>"),  # a row per group
     (100, 1016, 1424, 234, "ragged_tgmm_kernel<1>"),  # six tiles: a factor shared
-    (300, 648, 2440, 393, "ragged_tgmm_kernel<1>"),   # one of 40, 160 rounds
-    (300, 648, 2440, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 159
-    (300, 640, 2440, 392, "ragged_tgmm_kernel<1>"),   # five row tiles
-    (300, 640, 2504, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # no padding
+    (300, 648, 2488, 393, "ragged_tgmm_kernel<1>"),   # ten tiles, a block padding, 160 rounds
+    (300, 648, 2488, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # 159
+    (300, 640, 2488, 392, "ragged_tgmm_kernel<1>"),   # five row tiles
+    (300, 640, 2504, 392, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),  # less than a block
     (300, 2048, 1160, 66, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, false>"),  # 36 rounds
     (300, 2048, 1160, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # a round more
     (300, 2048, 1176, 67, "ragged_gemm_kernel<256, false, 4, true, 1, false, false, false, true>"),   # five tiles still
